@@ -639,7 +639,48 @@ int ensure_split(imsrg_space* sp)
   return IMSRG_OK;
 }
 
-// overwrite: Z2 is known to be zero (fresh commutator), so the split product
+bool capturing(cudaStream_t st)
+{
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
+
+// the plan in *slot, made on first use outside a capture; null where it
+// cannot be (no room for its planes, or first used inside a capture)
+DgemmPlan* fp64_plan(DgemmPlan** slot, bool* tried, const std::vector<GemmJobDev>& jobs, int family, cudaStream_t st)
+{
+  if (!*slot && !*tried && !capturing(st)) {
+    *tried = true;
+    try {
+      *slot = dgemm_plan_create(jobs, family);
+    } catch (std::exception&) {
+    }
+  }
+  return *slot;
+}
+
+// the FP64 ladder as a term of its own, on planes of its own: launches from
+// several threads and streams follow each other; a capture takes the
+// FP64-pipe kernel, which keeps nothing
+int ladder_term_fp64(imsrg_space* sp, const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
+{
+  Space& s = *sp->s;
+  std::lock_guard<std::mutex> g(sp->fp64_mu);
+  DgemmPlan* p = capturing(st) ? nullptr : fp64_plan(&sp->fp64_term, &sp->fp64_tried[2], sp->ladder_jobs, 0, st);
+  if (p) {
+    if (!sp->fp64_ev) CUDA_TRY(cudaEventCreateWithFlags(&sp->fp64_ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaStreamWaitEvent(st, sp->fp64_ev, 0));
+    CUDA_TRY(launch_dgemm(p, X->d, Y->d, Y->d, Z->d, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm,
+                          (double)Y->herm, -1, true, st));
+    CUDA_TRY(cudaEventRecord(sp->fp64_ev, st));
+    return IMSRG_OK;
+  }
+  CUDA_TRY(launch_symgemm_fp64(sp->d_ladder_jobs, sp->d_ladder_pairs, sp->n_ladder_pairs, X->d, Y->d, Y->d, Z->d,
+                               s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, st));
+  return IMSRG_OK;
+}
+
+// overwrite: Z2 is known to be zero (fresh commutator), so the product
 // writes its blocks instead of read-modify-write
 int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st, bool overwrite = false)
 {
@@ -655,6 +696,12 @@ int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaS
     return IMSRG_OK;
   }
   if (prec != IMSRG_PREC_FP64) return fail(IMSRG_ERR_ARG, "unknown precision");
+  if (!overwrite) return ladder_term_fp64(sp, X, Y, Z, st);
+  if (DgemmPlan* p = fp64_plan(&sp->fp64_ladder, &sp->fp64_tried[0], sp->ladder_jobs, 0, st)) {
+    CUDA_TRY(launch_dgemm(p, X->d, Y->d, Y->d, Z->d, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm,
+                          (double)Y->herm, 0, true, st));
+    return IMSRG_OK;
+  }
   CUDA_TRY(launch_symgemm_fp64(sp->d_ladder_jobs, sp->d_ladder_pairs, sp->n_ladder_pairs, X->d, Y->d, Y->d, Z->d,
                                s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, st));
   return IMSRG_OK;
@@ -694,8 +741,13 @@ int do_ph(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStrea
     CUDA_TRY(launch_symgemm_split(sp->split_zbar, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx,
                                   s.work.kweight, s.work.phase_tab, sp->d_status, Z->herm, 1.0, st));
   } else if (prec == IMSRG_PREC_FP64) {
-    CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
-                                 sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, 1.0, st));
+    if (DgemmPlan* p = fp64_plan(&sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
+      // the descriptor inverse kernel reads only Zbar's upper triangle
+      CUDA_TRY(launch_dgemm(p, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab,
+                            Z->herm, 1.0, 0, sp->inv_fp64 == 0, st));
+    else
+      CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
+                                   sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, 1.0, st));
   } else {
     return fail(IMSRG_ERR_ARG, "unknown precision");
   }
@@ -1483,7 +1535,9 @@ struct GroupedProducts {
   int prec = IMSRG_PREC_SPLIT;
   SplitPlan* ladder = nullptr;  // split form
   SplitPlan* zbar = nullptr;
-  // FP64 form: every pair's jobs and tile pairs in one list per product
+  // FP64 form: tensor-core plans over every pair's jobs; where they do not fit,
+  // the jobs and tile pairs in one list per product
+  DgemmPlan *fp64_ladder = nullptr, *fp64_zbar = nullptr;
   GemmJobDev *d_lj = nullptr, *d_zj = nullptr;
   int *d_lp = nullptr, *d_zp = nullptr;
   int n_lp = 0, n_zp = 0;
@@ -1494,6 +1548,8 @@ struct GroupedProducts {
   {
     if (ladder) split_plan_destroy(ladder);
     if (zbar) split_plan_destroy(zbar);
+    dgemm_plan_destroy(fp64_ladder);
+    dgemm_plan_destroy(fp64_zbar);
     if (d_zoff) cudaFree(d_zoff);
     for (void* p : {(void*)d_lj, (void*)d_zj, (void*)d_lp, (void*)d_zp})
       if (p) cudaFree(p);
@@ -1570,7 +1626,15 @@ GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, 
       g->ladder = split_plan_create(*s0->s, lj, 0, s0->opt_ladder);
       g->zbar = split_plan_create(*s0->s, zj, 1, s0->opt_zbar);
     } else {
-      // the FP64 products' tile pairs over every pair's jobs (offsets from pair 0's arrays)
+      // (offsets from pair 0's arrays)
+      try {
+        g->fp64_ladder = dgemm_plan_create(lj, 0);
+      } catch (std::exception&) {
+      }
+      try {
+        g->fp64_zbar = dgemm_plan_create(zj, 1);
+      } catch (std::exception&) {
+      }
       std::vector<int> lp = tile_pairs(lj, symgemm_fp64_tile()), zp = tile_pairs(zj, symgemm_fp64_tile());
       g->d_lj = dcopy(lj);
       g->d_zj = dcopy(zj);
@@ -1659,6 +1723,11 @@ int grouped_ladder(GroupedProducts* g, cudaStream_t st)
 {
   imsrg_space* s0 = g->X[0]->sp;
   const Space& s = *s0->s;
+  if (g->fp64_ladder) {  // Z was zeroed in the pre phase
+    CUDA_TRY(launch_dgemm(g->fp64_ladder, g->X[0]->d, g->Y[0]->d, g->Y[0]->d, g->Z[0]->d, s.work.kidx, s.work.kweight,
+                          s.work.phase_tab, g->Z[0]->herm, (double)g->Y[0]->herm, 0, true, st));
+    return IMSRG_OK;
+  }
   if (g->prec == IMSRG_PREC_FP64) {
     CUDA_TRY(launch_symgemm_fp64(g->d_lj, g->d_lp, g->n_lp, g->X[0]->d, g->Y[0]->d, g->Y[0]->d, g->Z[0]->d,
                                  s.work.kidx, s.work.kweight, s.work.phase_tab, g->Z[0]->herm,
@@ -1676,6 +1745,11 @@ int grouped_zbar(GroupedProducts* g, cudaStream_t st)
 {
   imsrg_space* s0 = g->X[0]->sp;
   const Space& s = *s0->s;
+  if (g->fp64_zbar) {
+    CUDA_TRY(launch_dgemm(g->fp64_zbar, s0->d_xb, s0->d_yt, s0->d_yf, s0->d_zb, s.work.kidx, s.work.kweight,
+                          s.work.phase_tab, g->Z[0]->herm, 1.0, 0, s0->inv_fp64 == 0, st));
+    return IMSRG_OK;
+  }
   if (g->prec == IMSRG_PREC_FP64) {
     CUDA_TRY(launch_symgemm_fp64(g->d_zj, g->d_zp, g->n_zp, s0->d_xb, s0->d_yt, s0->d_yf, s0->d_zb, s.work.kidx,
                                  s.work.kweight, s.work.phase_tab, g->Z[0]->herm, 1.0, st));

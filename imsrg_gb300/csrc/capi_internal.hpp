@@ -103,6 +103,15 @@ struct imsrg_space {
   // split-precision plans
   SplitPlan* split_ladder = nullptr;
   SplitPlan* split_zbar = nullptr;
+  // FP64 products on the tensor cores (built on first use; null where their
+  // planes do not fit: the FP64-pipe kernel runs then).  The ladder term on
+  // its own, unlike the whole commutator and the ph term, uses no scratch of
+  // the space and may run on several streams, so it has planes of its own,
+  // and fp64_ev orders their uses
+  imsrg::DgemmPlan *fp64_ladder = nullptr, *fp64_zbar = nullptr, *fp64_term = nullptr;
+  bool fp64_tried[3] = {false, false, false};
+  std::mutex fp64_mu;
+  cudaEvent_t fp64_ev = nullptr;
   // BCH work operators (d_prod: BCH_Product result when Z aliases X or Y)
   double *d_nested = nullptr, *d_next = nullptr, *d_prod = nullptr;
   // generator scratch: monopoles V(ab, ab) of H, norb^2
@@ -137,6 +146,10 @@ struct imsrg_space {
   {
     if (split_ladder) split_plan_destroy(split_ladder);
     if (split_zbar) split_plan_destroy(split_zbar);
+    dgemm_plan_destroy(fp64_ladder);
+    dgemm_plan_destroy(fp64_zbar);
+    dgemm_plan_destroy(fp64_term);
+    if (fp64_ev) cudaEventDestroy(fp64_ev);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (side) cudaStreamDestroy(side);

@@ -175,6 +175,19 @@ cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int np
                                 const double* B0, const double* B1, double* O, const int* kidx, const double* kw,
                                 const int* phase, int gsign, double gbscale, cudaStream_t st);
 
+// kernels_dgemm.cu: the same products, and plain ones (nosym), to FP64 accuracy
+// on the tensor cores.  create throws when its planes do not fit in device
+// memory; a launch reuses the plan's planes, so launches of one plan run in
+// order.  family: 0 ladder, 1 Zbar (phase timers)
+struct DgemmPlan;
+DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs, int family);
+void dgemm_plan_destroy(DgemmPlan* p);
+// accum: -1 each job's own flag, 0 overwrite, 1 accumulate; mirror false:
+// symmetrised jobs write only their upper triangle
+cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, const double* B1, double* O, const int* kidx,
+                         const double* kw, const int* phase, int gsign, double gbscale, int accum, bool mirror,
+                         cudaStream_t st);
+
 // kernels_split.cu (Ozaki-style sliced BF16 products on tcgen05)
 struct SplitPlan;
 // Tile shape and schedule of a plan: tn x nacc in {64 x 1, 32 x 2} (tile

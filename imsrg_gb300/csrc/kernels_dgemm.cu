@@ -1,0 +1,1026 @@
+// FP64 channel products on the Blackwell tensor cores.
+//
+// The products of the FP64 form, for every job (a channel block),
+//     Out (+)= P + s phi_i phi_j P^T,   P = A B^T,   A, B: m x K FP64
+// (or Out (+)= A B^T, A: m x K, B: n x K, for a plain job), to FP64 accuracy
+// but not on the FP64 pipe, which runs at 1.2 TFLOP/s on this part: each row
+// of A and of B is taken as 62-bit fixed point below its own exponent, cut
+// into S = 9 balanced base-2^7 digits, exact in BF16, and the digit products
+// of weight s + t < S are summed by tcgen05.mma into one FP32 tensor-memory
+// accumulator per weight.
+//
+//  * Exactness.  The reduction is cut into chunks of at most CH x 32 elements,
+//    so the sums of the six leading weights stay below 2^24 and are exact
+//    integers; what the others round is below 2^-66 of the row maxima's
+//    product.  Each chunk's sums are added as 64-bit integers (two words: the
+//    leading five weights, the trailing four) and converted to FP64 once per
+//    half of the product.
+//  * The two halves, A B^T and s phi B A^T, have their own row exponents (a_i
+//    + b_j and b_i + a_j), so they are separate chunks of one tile: only the
+//    tiles of the upper triangle are computed, each written with its mirror.
+//  * Error.  Fixed point is exact to 2^-63 of each row's largest element, FP64
+//    to 2^-53 of each element, so the two differ where a sum is small against
+//    its rows' maxima.  A tenth plane holds |a| and |b| as BF16 magnitudes
+//    (exponents clamped at 2^-60), and one more MMA a step gives sum |a||b| of
+//    every output and chunk.  The digit error is about sqrt(K) 2^-63 (unit:
+//    the rows' exponents) and that of an FP64 sum about 2^-54 sum |a||b|, so
+//    an element with 0 < sum |a||b| < 2^-9 sqrt(K) is not written but listed,
+//    and k_dgemm_exact evaluates it with FP64 FMAs.  A tile with many such
+//    elements is listed whole, and so are tiles with a row that holds an
+//    infinity, a NaN or magnitudes outside 2^-423 .. 2^477, and tiles that a
+//    timed-out wait left undone.  (Random operators list a few elements of
+//    the channels with K < 8; listing whole tiles for those cost 30 us a
+//    product at emax=10.)
+//
+// What bounds it: for the long products the MMAs, 46 of 128 x 32 x 16 a K16
+// step (merged to 11 instructions), next to the TMA stream of the ten planes
+// (the emax=10 ladder: 2.6 ms, tensor pipe 58%, 13.4 TB/s from L2); for the
+// short ones (Zbar, K <= 132) the epilogue.  With the FP64-pipe kernel the
+// commutator takes 142 us at emax 2, 1.26 ms at emax 6, 87.2 ms at emax 10;
+// with this one 116 us, 0.38 ms and 7.7 ms: it is used at every size, and
+// the FP64-pipe kernel only where the planes do not fit (40 bytes an element
+// pair of the operands) or inside a capture that comes before them.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <stdexcept>
+#include <vector>
+
+#include "kernels.cuh"
+#include "prof.hpp"
+#include "tcgen05.cuh"
+
+namespace imsrg {
+
+namespace {
+
+constexpr int KB = 32;       // K elements per pipeline stage: one 64-byte swizzle row
+constexpr int TM = 128;      // tile rows (UMMA M)
+constexpr int TN = 32;       // tile columns (UMMA N per digit)
+constexpr int S = 9;         // digits per element
+constexpr int BETA = 7;      // bits between digits
+constexpr int P = 62;        // bits of the fixed point: 6 in the top digit, 7 in each other
+constexpr int NP = S + 1;    // planes: digits, then magnitudes
+constexpr int NHI = 5;       // weights summed in the leading integer word
+constexpr int CH = 20;       // K blocks per chunk: 6 x 65^2 x 32 CH < 2^24
+constexpr int NSTAGE = 2;    // 2 x 100 KB of 227 KB
+constexpr int NINFO = 3;     // tiles whose job, exponents and phases wait in shared memory
+constexpr int EPIW = 8;      // epilogue warps: two per TMEM lane quarter, 16 columns each
+constexpr int COLS_W = TN / 2;
+constexpr int NB = 512 / TN;         // tensor-memory blocks
+constexpr int OV = 2 * NP - NB;      // blocks that consecutive chunks share (see k_dgemm)
+constexpr unsigned A_SLICE = TM * KB * 2, B_SLICE = TN * KB * 2;
+constexpr unsigned STAGE = NP * (A_SLICE + B_SLICE);
+constexpr int RAW_MIN = 600, RAW_MAX = 1500;  // biased exponents of rows whose products stay normal
+
+static_assert(OV >= 0 && OV < NP, "a chunk's blocks exceed tensor memory");
+
+struct DJob {
+  long long a_off, b_off, out_off;
+  double bscale;
+  int m, n, K, lda, ldb, ldo;
+  int kidx_off, w_off, phase_off;
+  int bsel, sign, accumulate, nosym;
+  int m_pad, nkb, nchunk;
+  int exp_base;       // first row in the exponent arrays
+  int row_base;       // first row in the planes: K block kb, row i is row_base + kb m_pad + i
+};
+
+struct DTile {
+  int job, I, J;
+};
+
+// at most MAX_LISTED threads of a tile list their elements (each up to
+// COLS_W); with more the tile is listed
+constexpr int MAX_LISTED = 8;
+struct DElem {
+  int tile, ij;  // row and column within the tile: row | column << 16
+};
+
+__host__ __device__ __forceinline__ int chunk_begin(int nkb, int nchunk, int c) { return (int)((long long)nkb * c / nchunk); }
+
+}  // namespace
+
+struct DgemmPlan {
+  int family = 0;
+  int njobs = 0, ntiles = 0, grid = 0;
+  long long rows = 0, exp_rows = 0;
+  DJob* d_jobs = nullptr;
+  DTile* d_tiles = nullptr;
+  int* d_cta = nullptr;
+  __nv_bfloat16* arr[2] = {nullptr, nullptr};  // planes of A and of B
+  int* d_exp = nullptr;   // [2 exp_rows] raw row exponents of A, of B; then the counts of listed tiles and elements
+  int* d_list = nullptr;  // tiles to evaluate exactly
+  DElem* d_elem = nullptr;
+  int4 *d_rblk = nullptr, *d_dblk = nullptr;
+  int n_rblk = 0, n_dblk = 0;
+  CUtensorMap maps[4];  // A rows of A, of B (128-row boxes); B rows of A, of B (32-row boxes)
+  size_t smem = 0;
+};
+
+// ----------------------------------------------------------------- device
+namespace {
+
+// biased exponent; 1 for a subnormal, so that only a zero gives 0
+__device__ __forceinline__ int dexp1(double v)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+  const int E = (int)(b >> 52);
+  return E == 0 && b != 0 ? 1 : E;
+}
+
+// B's column scale (job scale x launch scale x ladder weight): every weight of
+// a closed shell is +-1, a sign flip; any other is an FP64 multiply, rounded
+// as the FP64 kernel rounds it.  (The slicing passes spend one FP64
+// instruction an element otherwise: 250 us instead of 55 for the emax=10
+// ladder's exponents.)
+enum { SC_PLUS = 0, SC_MINUS = 1, SC_OTHER = 2 };
+__device__ __forceinline__ int scale_kind(double sc) { return sc == 1.0 ? SC_PLUS : sc == -1.0 ? SC_MINUS : SC_OTHER; }
+__device__ __forceinline__ double scaled(double v, int kind, double sc)
+{
+  if (kind == SC_OTHER) return v * sc;
+  return __longlong_as_double(__double_as_longlong(v) ^ ((long long)kind << 63));
+}
+
+__device__ __forceinline__ bool row_bad(int raw) { return raw != 0 && (raw < RAW_MIN || raw > RAW_MAX); }
+__device__ __forceinline__ int row_e(int raw) { return raw - 1022; }
+
+// Raw row exponents of A and B (largest biased exponent of the row): a block
+// per listed (job, 32-row group, 256-column chunk), partial maxima combined
+// by atomicMax.  Bound by its operand loads: four columns in flight a thread.
+__global__ void __launch_bounds__(256) k_dgemm_rowexp(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
+                                                      const double* __restrict__ Abase, const double* __restrict__ B0,
+                                                      const double* __restrict__ B1, const int* __restrict__ kidx,
+                                                      const double* __restrict__ kw, double gbscale,
+                                                      int* __restrict__ rexpA, int* __restrict__ rexpB)
+{
+  __shared__ int sa[8][33], sb[8][33];
+  __shared__ int s_col[256], s_kind[256];
+  __shared__ double s_sc[256];
+  const int4 bk = blocks[blockIdx.x];
+  const DJob jb = jobs[bk.x];
+  const int r = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int i = bk.y * 32 + r;
+  const int t0 = bk.z * 256, tend = min(jb.K, t0 + 256);
+  {
+    const int t = t0 + threadIdx.x;
+    if (t < tend) {
+      s_col[threadIdx.x] = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
+      s_sc[threadIdx.x] = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
+      s_kind[threadIdx.x] = scale_kind(s_sc[threadIdx.x]);
+    }
+  }
+  __syncthreads();
+  const double* A = Abase + jb.a_off;
+  const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
+  const bool oka = i < jb.m, okb = i < jb.n;
+  int ea = 0, eb = 0;
+  int t = t0 + ty;
+  for (; t + 24 < tend; t += 32) {
+    double a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long col = s_col[t + 8 * u - t0];
+      a[u] = oka ? A[col * jb.lda + i] : 0.0;
+      b[u] = okb ? B[col * jb.ldb + i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      ea = max(ea, dexp1(a[u]));
+      eb = max(eb, dexp1(scaled(b[u], s_kind[t + 8 * u - t0], s_sc[t + 8 * u - t0])));
+    }
+  }
+  for (; t < tend; t += 8) {
+    const long long col = s_col[t - t0];
+    if (oka) ea = max(ea, dexp1(A[col * jb.lda + i]));
+    if (okb) eb = max(eb, dexp1(scaled(B[col * jb.ldb + i], s_kind[t - t0], s_sc[t - t0])));
+  }
+  sa[ty][r] = ea;
+  sb[ty][r] = eb;
+  __syncthreads();
+  if (ty == 0) {
+    for (int y = 1; y < 8; ++y) {
+      ea = max(ea, sa[y][r]);
+      eb = max(eb, sb[y][r]);
+    }
+    if (ea) atomicMax(rexpA + jb.exp_base + i, ea);
+    if (eb) atomicMax(rexpB + jb.exp_base + i, eb);
+  }
+}
+
+// v 2^(P - e), rounded to an integer, for |v| < 2^e (v of a row in range)
+__device__ __forceinline__ long long fixed_of(double v, int e)
+{
+  const long long bits = __double_as_longlong(v);
+  const int E = (int)((bits >> 52) & 0x7FF);
+  if (E == 0) return 0;
+  const long long M = (bits & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll;
+  const int r = 1075 - E - P + e;  // right shift, >= 53 - P
+  if (r > 54) return 0;
+  const long long q = r <= 0 ? M << min(-r, P - 53) : (M + (1ll << (r - 1))) >> r;
+  return bits < 0 ? -q : q;
+}
+
+// |v| 2^-e as BF16 (truncated), exponents clamped at 2^-60; 0 only for v = 0
+__device__ __forceinline__ unsigned magnitude_of(double v, int e)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+  if (b == 0) return 0;
+  const int x = (int)(b >> 52) - 1023 - e;  // <= -1
+  if (x < -60) return (unsigned)(127 - 60) << 7;
+  return ((unsigned)(127 + min(x, 0)) << 7) | (unsigned)((b >> 45) & 0x7F);
+}
+
+// The ten planes of A and of B: a block per listed (job, 32-row group, KB-column group), through shared
+// memory to 16-byte stores (a plane's 32 x KB values are 2 KB in a row).
+// Bound by HBM: 16 bytes read and 40 written per element pair; every operand
+// load of a thread is issued before its first conversion.
+__global__ void __launch_bounds__(256) k_dgemm_digits(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
+                                                      const double* __restrict__ Abase, const double* __restrict__ B0,
+                                                      const double* __restrict__ B1, const int* __restrict__ kidx,
+                                                      const double* __restrict__ kw, double gbscale,
+                                                      const int* __restrict__ rexpA, const int* __restrict__ rexpB,
+                                                      long long plane_rows, __nv_bfloat16* __restrict__ pA,
+                                                      __nv_bfloat16* __restrict__ pB)
+{
+  constexpr int RW = (KB + 2) / 2;  // 17 words a row: a warp's 32 rows in 32 banks
+  __shared__ unsigned dg[NP][32][RW];
+  __shared__ int s_e[2][32], s_col[KB], s_kind[KB];
+  __shared__ double s_sc[KB];
+  const int4 bk = blocks[blockIdx.x];
+  const DJob jb = jobs[bk.x];
+  const int r0 = bk.y * 32, t0 = bk.z * KB;
+  if (threadIdx.x < 32) {
+    s_e[0][threadIdx.x] = row_e(rexpA[jb.exp_base + r0 + threadIdx.x]);
+    s_e[1][threadIdx.x] = row_e(rexpB[jb.exp_base + r0 + threadIdx.x]);
+  } else if (threadIdx.x < 32 + KB) {
+    const int tt = threadIdx.x - 32, t = t0 + tt;
+    s_col[tt] = t < jb.K ? (jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t) : 0;
+    s_sc[tt] = t < jb.K ? jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0) : 1.0;
+    s_kind[tt] = scale_kind(s_sc[tt]);
+  }
+  __syncthreads();
+  const double* A = Abase + jb.a_off;
+  const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
+  constexpr int NIT = 32 * (KB / 2) / 256;
+  double v[2][NIT][2];
+#pragma unroll
+  for (int u = 0; u < NIT; ++u) {
+    const int e = threadIdx.x + u * 256, r = e & 31, i = r0 + r;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int tt = 2 * (e >> 5) + h;
+      const bool ok = t0 + tt < jb.K;
+      v[0][u][h] = ok && i < jb.m ? A[(long long)s_col[tt] * jb.lda + i] : 0.0;
+      v[1][u][h] = ok && i < jb.n ? B[(long long)s_col[tt] * jb.ldb + i] : 0.0;
+    }
+  }
+  long long bias = 0;  // half a digit in every lower digit: the fields of q + bias minus half are balanced
+#pragma unroll
+  for (int s = 1; s < S; ++s) bias += 1ll << (BETA * (S - 1 - s) + BETA - 1);
+#pragma unroll
+  for (int op = 0; op < 2; ++op) {
+#pragma unroll
+    for (int u = 0; u < NIT; ++u) {
+      const int e = threadIdx.x + u * 256, r = e & 31, tp = e >> 5;
+      long long q[2];
+      unsigned mag[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double x = op ? scaled(v[1][u][h], s_kind[2 * tp + h], s_sc[2 * tp + h]) : v[0][u][h];
+        q[h] = fixed_of(x, s_e[op][r]) + bias;
+        mag[h] = magnitude_of(x, s_e[op][r]);
+      }
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const int sh = BETA * (S - 1 - s);
+        // small integer -> BF16: 1.5 * 2^23 + x minus 1.5 * 2^23, upper half; "- half" rides in the constant
+        const int mg = s == 0 ? 0x4B400000 : 0x4B400000 - (1 << (BETA - 1));
+        float f[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int x = s == 0 ? (int)(q[h] >> sh) : (int)((unsigned)(q[h] >> sh) & ((1u << BETA) - 1));
+          f[h] = __int_as_float(mg + x) - 12582912.0f;
+        }
+        dg[s][r][tp] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
+      }
+      dg[S][r][tp] = mag[0] | (mag[1] << 16);
+    }
+    __syncthreads();
+    __nv_bfloat16* out = op ? pB : pA;
+    const long long row0 = jb.row_base + (long long)bk.z * jb.m_pad + r0;
+    for (int e = threadIdx.x; e < NP * 32 * (KB / 8); e += 256) {
+      const int x = e % (KB / 8), r = (e / (KB / 8)) & 31, s = e / (32 * (KB / 8));
+      const unsigned* d = &dg[s][r][x * 4];
+      *(uint4*)(out + ((long long)s * plane_rows + row0 + r) * KB + x * 8) = make_uint4(d[0], d[1], d[2], d[3]);
+    }
+    __syncthreads();
+  }
+}
+
+struct DArgs {
+  const DJob* jobs;
+  const DTile* tiles;
+  const int* cta_first;
+  const int *rexpA, *rexpB;
+  const int* phase;
+  double* out;
+  int* nlist;  // to evaluate exactly: counts of tiles and elements, then the lists
+  int* list;
+  DElem* elem;
+  int gsign, accum, nomirror;
+};
+
+// what the roles of a CTA need to know of a tile, gathered one or two tiles
+// ahead by a warp of its own: a chain of three dependent loads (tile, job,
+// exponents), and sixteen exponent and phase loads a thread, cost the
+// epilogue 30k of its 45k cycles a tile of the emax=10 Zbar product
+struct TileInfo {
+  double* O;
+  int m, n, K, ldo, nosym, nkb, nchunk, m_pad, row_base, accumulate, I, J;
+  int rrow[2][TM], rcol[2][TN];  // raw exponents of the tile's rows and columns, in each half
+  int prow[TM], pcol[TN];        // phases (rows carry the job's sign too)
+};
+
+// adds 16 columns of block g (a weight, or the magnitudes) to the thread's sums
+template <int G>
+__device__ __forceinline__ void take(unsigned taddr, long long (&hi)[COLS_W], long long (&lo)[COLS_W], float tau, unsigned& bad)
+{
+  unsigned r[2][8];
+  tmem_ld8(taddr, r[0]);
+  tmem_ld8(taddr + 8, r[1]);
+  tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < COLS_W; ++c) {
+    const float x = __uint_as_float(r[c >> 3][c & 7]);
+    if (G == S)
+      bad |= (x != 0.f && x < tau ? 1u : 0u) << c;
+    else if (G < NHI)
+      hi[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (NHI - 1 - (G < NHI ? G : 0))));
+    else
+      lo[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (S - 1 - (G < S ? G : 0))));
+  }
+}
+
+template <int G, int N>
+__device__ __forceinline__ void take_run(unsigned base, long long (&hi)[COLS_W], long long (&lo)[COLS_W], float tau, unsigned& bad)
+{
+  if constexpr (N > 0) {
+    take<G>(base + G * TN, hi, lo, tau, bad);
+    take_run<G + 1, N - 1>(base, hi, lo, tau, bad);
+  }
+}
+
+// (hi + lo 2^-28) 2^X as FP64, rounded once to nearest even (rows in range
+// keep it normal).  Three 32-bit words and no branch: conversions and an FMA
+// would run on the FP64 pipe, and the same steps with 64-bit shifts and
+// branches took the emax=10 commutator from 7.71 to 8.02 ms.
+__device__ __forceinline__ double value_of(long long hi, long long lo, int X)
+{
+  constexpr int LB = BETA * (S - NHI);
+  const long long h = hi + (lo >> LB);
+  // h 2^LB + l as a signed 96-bit number, then its magnitude
+  const unsigned h0 = (unsigned)h, h1 = (unsigned)((unsigned long long)h >> 32), sg = (unsigned)((int)h1 >> 31);
+  unsigned w0 = (h0 << LB | ((unsigned)lo & ((1u << LB) - 1))) ^ sg;
+  unsigned w1 = __funnelshift_l(h0, h1, LB) ^ sg;
+  unsigned w2 = (unsigned)((int)h1 >> (32 - LB)) ^ sg;
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;" : "+r"(w0), "+r"(w1), "+r"(w2) : "r"(sg & 1u));
+  // leading one to bit 31 of w2
+  int e = X + 1022 + 95 - LB;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool z = w2 == 0;
+    e = z ? e - 32 : e;
+    w2 = z ? w1 : w2;
+    w1 = z ? w0 : w1;
+    w0 = z ? 0 : w0;
+  }
+  const int sh = __clz(w2) & 31;
+  const bool zero = w2 == 0;
+  w2 = __funnelshift_l(w1, w2, sh);
+  w1 = __funnelshift_l(w0, w1, sh);
+  w0 <<= sh;
+  // 53 bits of w2:w1; the leading one carries into the exponent field (and so does a carry out of rounding)
+  unsigned ml = __funnelshift_r(w1, w2, 11), mh = (w2 >> 11) + ((unsigned)(e - sh) << 20);
+  const unsigned tail = (w1 << 21) | (w0 != 0 ? 1u : 0u) | (ml & 1u);  // (low bits of w1 << 21 are 0)
+  asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(ml), "+r"(mh) : "r"(tail > 0x80000000u ? 1u : 0u));
+  return zero ? 0.0 : __hiloint2double((int)(mh | (sg & 0x80000000u)), (int)ml);
+}
+
+// Persistent kernel, one CTA per SM, each with its own run of tiles:
+//   warp 0: TMA producer; warp 1: tensor memory and MMA issue (one thread);
+//   warps 2-9: epilogue; warp 10: tile information.
+// A chunk's ten blocks (nine weights, magnitudes) are NP x 32 of the 512
+// columns of tensor memory.  Even chunks of a CTA start at column 0, odd ones
+// end at the last, so consecutive chunks share OV = 4 blocks; the epilogue
+// takes those first and releases them, and the next chunk's MMAs run under
+// the rest.  (168 registers a thread: eleven warps on four register files are three a file.)
+__global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_constant__ CUtensorMap mAA,
+                                                             const __grid_constant__ CUtensorMap mAB,
+                                                             const __grid_constant__ CUtensorMap mBA,
+                                                             const __grid_constant__ CUtensorMap mBB, DArgs g)
+{
+  constexpr int EPI_T = 32 * EPIW;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  // barriers: full[NSTAGE], empty[NSTAGE], acc_full[2], early, info_full[NINFO], info_empty[NINFO]; then the tensor-memory slot
+  unsigned long long* bars = (unsigned long long*)(smem + NSTAGE * STAGE);
+  unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 3 + 2 * NINFO);
+  __shared__ TileInfo s_info[NINFO];
+  __shared__ int s_err_, s_epi_err_;
+  volatile int& s_err = s_err_;
+  volatile int& s_epi_err = s_epi_err_;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned sbase = smem_u32(smem), bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (NSTAGE + s); };
+  auto acc_full = [&](int b) { return bar0 + 8u * (2 * NSTAGE + b); };
+  const unsigned acc_early = bar0 + 8u * (2 * NSTAGE + 2);
+  auto info_full = [&](int k) { return bar0 + 8u * (2 * NSTAGE + 3 + k); };
+  auto info_empty = [&](int k) { return bar0 + 8u * (2 * NSTAGE + 3 + NINFO + k); };
+  if (threadIdx.x == 0) {
+    s_err = 0;
+    s_epi_err = 0;
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(acc_full(0), 1);
+    mbar_init(acc_full(1), 1);
+    mbar_init(acc_early, EPI_T);
+    for (int k = 0; k < NINFO; ++k) {
+      mbar_init(info_full(k), 1);
+      mbar_init(info_empty(k), EPI_T + 2);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = *tmem_slot;
+  const int tbeg = g.cta_first[blockIdx.x], ntile = g.cta_first[blockIdx.x + 1] - tbeg;
+
+  if (warp == 2 + EPIW) {
+    // ------------------------------------------------ tile information
+    for (int t = 0; t < ntile && !s_err; ++t) {
+      const int k = t % NINFO;
+      const bool ok = mbar_wait(info_empty(k), (unsigned)((t / NINFO) & 1) ^ 1u);
+      if (!__all_sync(0xffffffffu, ok)) {
+        s_err = 1;
+        break;
+      }
+      const DTile tl = g.tiles[tbeg + t];
+      const DJob jb = g.jobs[tl.job];
+      TileInfo& f = s_info[k];
+      const int* ph = jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr;
+      const int sign = jb.sign != 0 ? jb.sign : g.gsign;
+      const int* ra = g.rexpA + jb.exp_base;
+      const int* rb = g.rexpB + jb.exp_base;
+      int x[2][TM / 32 + 1], p[TM / 32 + 1];
+#pragma unroll
+      for (int u = 0; u <= TM / 32; ++u) {
+        const int r = u < TM / 32 ? tl.I * TM + u * 32 + lane : tl.J * TN + lane;  // the last: the tile's columns
+        const int lim = u < TM / 32 ? jb.m : jb.n;
+        x[0][u] = r < lim ? (u < TM / 32 ? ra[r] : rb[r]) : 0;
+        x[1][u] = r < lim && !jb.nosym ? (u < TM / 32 ? rb[r] : ra[r]) : 0;
+        p[u] = ph && r < lim ? ph[r] : 1;
+      }
+#pragma unroll
+      for (int u = 0; u < TM / 32; ++u) {
+        f.rrow[0][u * 32 + lane] = x[0][u];
+        f.rrow[1][u * 32 + lane] = x[1][u];
+        f.prow[u * 32 + lane] = sign * p[u];
+      }
+      f.rcol[0][lane] = x[0][TM / 32];
+      f.rcol[1][lane] = x[1][TM / 32];
+      f.pcol[lane] = p[TM / 32];
+      if (lane == 0) {
+        f.O = g.out + jb.out_off;
+        f.m = jb.m;
+        f.n = jb.n;
+        f.K = jb.K;
+        f.ldo = jb.ldo;
+        f.nosym = jb.nosym;
+        f.nkb = jb.nkb;
+        f.nchunk = jb.nchunk;
+        f.m_pad = jb.m_pad;
+        f.row_base = jb.row_base;
+        f.accumulate = g.accum > 0 || (g.accum < 0 && jb.accumulate);
+        f.I = tl.I;
+        f.J = tl.J;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(info_full(k));
+    }
+  } else if (warp == 0) {
+    // ------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int it = 0;
+      for (int t = 0; t < ntile && !s_err; ++t) {
+        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) {
+          s_err = 1;
+          break;
+        }
+        const TileInfo& f = s_info[t % NINFO];
+        const int nkb = f.nkb, m_pad = f.m_pad, nhalf = f.nosym ? 1 : 2;
+        const int rA = f.row_base + f.I * TM, rB = f.row_base + f.J * TN;
+        mbar_arrive(info_empty(t % NINFO));
+        for (int k = 0; k < nhalf * nkb; ++k, ++it) {
+          const int st = it % NSTAGE;
+          if (!mbar_wait(empty_bar(st), (unsigned)((it / NSTAGE) & 1) ^ 1u)) {
+            s_err = 1;
+            break;
+          }
+          mbar_expect_tx(full_bar(st), STAGE);
+          const bool second = k >= nkb;
+          const int row = (second ? k - nkb : k) * m_pad;
+          const unsigned sA = sbase + st * STAGE;
+          tma_load_3d(sA, second ? &mAB : &mAA, 0, rA + row, full_bar(st));
+          tma_load_3d(sA + NP * A_SLICE, second ? &mBA : &mBB, 0, rB + row, full_bar(st));
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      constexpr int MAXT = 256 / TN;
+      int it = 0, cc = 0;
+      for (int t = 0; t < ntile && !s_err; ++t) {
+        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) {
+          s_err = 1;
+          break;
+        }
+        const TileInfo& f = s_info[t % NINFO];
+        const int nkb = f.nkb, nchunk = f.nchunk, nhalf = f.nosym ? 1 : 2;
+        mbar_arrive(info_empty(t % NINFO));
+        for (int hc = 0; hc < nhalf * nchunk && !s_err; ++hc, ++cc) {
+          const int c = hc >= nchunk ? hc - nchunk : hc;
+          const int len = chunk_begin(nkb, nchunk, c + 1) - chunk_begin(nkb, nchunk, c);
+          // the shared blocks of the chunk before have been taken (and so all of the one before that)
+          if (!mbar_wait(acc_early, (unsigned)((cc & 1) ^ 1))) {
+            s_err = 1;
+            break;
+          }
+          tc_fence_after();
+          const unsigned d = tmem + ((cc & 1) ? (NB - NP) * TN : 0);
+          for (int kb = 0; kb < len; ++kb, ++it) {
+            const int st = it % NSTAGE;
+            if (!mbar_wait(full_bar(st), (unsigned)((it / NSTAGE) & 1))) {
+              s_err = 1;
+              break;
+            }
+            tc_fence_after();
+            const unsigned sA = sbase + st * STAGE;
+            const unsigned long long a0 = sdesc_sw64(sA), b0 = sdesc_sw64(sA + NP * A_SLICE);
+            const unsigned first = kb == 0 ? 0u : 1u;
+            // the products (s, t) of one s over a run of t are one MMA: their
+            // weights s + t are consecutive blocks of tensor memory, their B
+            // tiles consecutive in shared memory
+#pragma unroll
+            for (int sub = 0; sub < KB / 16; ++sub) {
+#pragma unroll
+              for (int s = 0; s < S; ++s) {
+                const unsigned long long ad = a0 + (unsigned long long)((s * A_SLICE + sub * 32) >> 4);
+#pragma unroll
+                for (int t0 = 0; t0 < S - s; t0 += MAXT) {
+                  const int nt = (S - s - t0) < MAXT ? (S - s - t0) : MAXT;
+                  tc_mma(d + (s + t0) * TN, ad, b0 + (unsigned long long)((t0 * B_SLICE + sub * 32) >> 4),
+                         idesc_bf16(TM, nt * TN), (sub == 0 && s == 0) ? first : 1u);
+                }
+              }
+              tc_mma(d + S * TN, a0 + (unsigned long long)((S * A_SLICE + sub * 32) >> 4),
+                     b0 + (unsigned long long)((S * B_SLICE + sub * 32) >> 4), idesc_bf16(TM, TN),
+                     sub == 0 ? first : 1u);
+            }
+            tc_commit(empty_bar(st));
+          }
+          if (s_err) break;
+          tc_commit(acc_full(cc & 1));
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------ epilogue
+    const int q = warp & 3, cbeg = ((warp - 2) >> 2) * COLS_W, row = q * 32 + lane;
+    int cc = 0, t = 0;
+    for (; t < ntile; ++t) {
+      const TileInfo& f = s_info[t % NINFO];
+      if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) s_epi_err = 1;
+      asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
+      if (s_epi_err) break;
+      const int nosym = f.nosym, nkb = f.nkb, nchunk = f.nchunk, K = f.K;
+      const int i = f.I * TM + row, j0 = f.J * TN + cbeg;
+      unsigned bad = 0;  // this thread's columns that the digits cannot vouch for
+      double v1[COLS_W], v2[COLS_W];
+      for (int half = 0; half < (nosym ? 1 : 2); ++half) {
+        long long hi[COLS_W], lo[COLS_W];
+#pragma unroll
+        for (int c = 0; c < COLS_W; ++c) hi[c] = lo[c] = 0;
+        for (int c = 0; c < nchunk; ++c, ++cc) {
+          const int kb0 = chunk_begin(nkb, nchunk, c), kb1 = chunk_begin(nkb, nchunk, c + 1);
+          const float tau = 0.001953125f * __fsqrt_rn((float)(min(K, kb1 * KB) - kb0 * KB));
+          if (!mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1))) s_epi_err = 1;
+          // the epilogue warps decide together, so none waits at a barrier alone
+          asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
+          if (s_epi_err) break;
+          tc_fence_after();
+          const unsigned lane_base = tmem + ((unsigned)(q * 32) << 16) + cbeg;
+          if (cc & 1) {
+            const unsigned base = lane_base + (NB - NP) * TN;
+            take_run<0, OV>(base, hi, lo, tau, bad);
+            tc_fence_before();
+            mbar_arrive(acc_early);
+            take_run<OV, NP - OV>(base, hi, lo, tau, bad);
+          } else {
+            take_run<NP - OV, OV>(lane_base, hi, lo, tau, bad);
+            tc_fence_before();
+            mbar_arrive(acc_early);
+            take_run<0, NP - OV>(lane_base, hi, lo, tau, bad);
+          }
+        }
+        if (s_epi_err) break;
+        const int raw_i = f.rrow[half][row];
+        if (row_bad(raw_i)) bad = (1u << COLS_W) - 1;
+#pragma unroll
+        for (int c = 0; c < COLS_W; ++c) {
+          const int raw_j = f.rcol[half][cbeg + c];
+          bad |= (row_bad(raw_j) ? 1u : 0u) << c;
+          const double v = value_of(hi[c], lo[c], row_e(raw_i) + row_e(raw_j) - (2 * P - 2 * BETA * (S - 1) + BETA * (NHI - 1)));
+          if (half)
+            v2[c] = v;
+          else
+            v1[c] = v;
+        }
+      }
+      if (s_epi_err) {
+        s_err = 1;
+        break;
+      }
+      const int m = f.m, n = f.n, ldo = f.ldo;
+      const bool accumulate = f.accumulate, rowok = i < m;
+      double* O = f.O;
+      if (!rowok || (!nosym && i > j0 + COLS_W - 1)) bad = 0;
+      if (!nosym && i > j0) bad &= ~0u << min(i - j0, 31);  // columns below the diagonal are another element's mirror
+      bad &= j0 >= n ? 0u : n - j0 < COLS_W ? (1u << (n - j0)) - 1 : ~0u;
+      // the epilogue threads decide together whether the tile is listed
+      unsigned nbad;
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.popc.u32 %0, 2, %2, p;\n}"
+                   : "=r"(nbad)
+                   : "r"(bad), "r"(EPI_T)
+                   : "memory");
+      if (nbad > MAX_LISTED) {
+        if (threadIdx.x == 64) g.list[atomicAdd(g.nlist, 1)] = tbeg + t;
+        mbar_arrive(info_empty(t % NINFO));
+        continue;
+      }
+      for (unsigned b = bad; b; b &= b - 1)
+        g.elem[atomicAdd(g.nlist + 1, 1)] = {tbeg + t, row | ((cbeg + __ffs(b) - 1) << 16)};
+      if (!nosym) {
+        const int sp = f.prow[row];
+#pragma unroll
+        for (int c = 0; c < COLS_W; ++c) {
+          const bool neg = sp * f.pcol[cbeg + c] < 0;
+          v1[c] += neg ? -v2[c] : v2[c];
+          v2[c] = neg ? -v1[c] : v1[c];
+        }
+      }
+      mbar_arrive(info_empty(t % NINFO));
+      // columns this thread writes: in the matrix, on or above the diagonal, not listed
+      unsigned wd = !rowok || j0 >= n ? 0u : n - j0 < COLS_W ? (1u << (n - j0)) - 1 : (1u << COLS_W) - 1;
+      if (!nosym && i > j0) wd &= i - j0 < COLS_W ? ~0u << (i - j0) : 0u;
+      wd &= ~bad;
+      unsigned wm = nosym || g.nomirror ? 0u : wd;
+      if (i >= j0 && i < j0 + COLS_W) wm &= ~(1u << (i - j0));
+      double* od = O + (long long)j0 * ldo + i;
+      double* om = O + (long long)i * ldo + j0;
+      if (!accumulate) {
+#pragma unroll
+        for (int c = 0; c < COLS_W; ++c) {
+          if ((wd >> c) & 1) od[(long long)c * ldo] = v1[c];
+          if ((wm >> c) & 1) om[c] = v2[c];
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < COLS_W; h += 8) {
+          // all old values of eight columns before their first store
+          double x[8], y[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            x[c] = (wd >> (h + c)) & 1 ? __ldcg(od + (long long)(h + c) * ldo) : 0.0;
+            y[c] = (wm >> (h + c)) & 1 ? __ldcg(om + h + c) : 0.0;
+          }
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            if ((wd >> (h + c)) & 1) od[(long long)(h + c) * ldo] = x[c] + v1[h + c];
+            if ((wm >> (h + c)) & 1) om[h + c] = y[c] + v2[h + c];
+          }
+        }
+      }
+    }
+    // a wait that ran out: the tiles not written go to k_dgemm_exact
+    if (threadIdx.x == 64)
+      for (; t < ntile; ++t) g.list[atomicAdd(g.nlist, 1)] = tbeg + t;
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// out (+)= v at (i, j) and, for a symmetrised job, its mirror
+__device__ __forceinline__ void put_exact(const DJob& jb, double* O, const int* ph, double sgn, int i, int j, double p1,
+                                          double p2, bool accumulate, int nomirror)
+{
+  double* d = O + (long long)j * jb.ldo + i;
+  if (jb.nosym) {
+    *d = accumulate ? *d + p1 : p1;
+    return;
+  }
+  const double f = sgn * (ph ? (double)(ph[i] * ph[j]) : 1.0);
+  const double v = p1 + f * p2, w = p2 + f * p1;
+  *d = accumulate ? *d + v : v;
+  if (i != j && !nomirror) {
+    double* t = O + (long long)i * jb.ldo + j;
+    *t = accumulate ? *t + w : w;
+  }
+}
+
+// The listed tiles and elements with FP64 FMAs: tiles by 256 threads, each a
+// 4 x 4 block of both products, in the summation order of the FP64 kernel
+// (kernels_gemm.cu); elements by a warp each, lanes over K.  Bound by the
+// FP64 pipe; empty lists cost one short launch.
+__global__ void __launch_bounds__(256) k_dgemm_exact(const DJob* __restrict__ jobs, const DTile* __restrict__ tiles,
+                                                     const int* __restrict__ nlist, const int* __restrict__ list,
+                                                     const DElem* __restrict__ elem, const double* __restrict__ Abase,
+                                                     const double* __restrict__ B0, const double* __restrict__ B1,
+                                                     double* __restrict__ Obase, const int* __restrict__ kidx,
+                                                     const double* __restrict__ kw, const int* __restrict__ phase, int gsign,
+                                                     double gbscale, int accum, int nomirror)
+{
+  constexpr int TK = 8;
+  __shared__ double sAI[TK][TM], sBI[TK][TM], sAJ[TK][TN], sBJ[TK][TN];
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, lane = threadIdx.x & 31;
+  const int ntile = nlist[0], nelem = nlist[1];
+  for (int e = blockIdx.x; e < ntile; e += gridDim.x) {
+    const DTile tl = tiles[list[e]];
+    const DJob jb = jobs[tl.job];
+    const double* A = Abase + jb.a_off;
+    const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
+    const int i0 = tl.I * TM, j0 = tl.J * TN;
+    double acc1[4][4] = {}, acc2[4][4] = {};
+    for (int k0 = 0; k0 < jb.K; k0 += TK) {
+      const int nk = min(TK, jb.K - k0);
+      __syncthreads();
+      for (int x = threadIdx.x; x < nk * (TM + TN); x += 256) {
+        const int kk = x / (TM + TN), y = x % (TM + TN), t = k0 + kk;
+        const int r = y < TM ? i0 + y : j0 + y - TM;
+        const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
+        const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
+        const double a = r < jb.m ? A[col * jb.lda + r] : 0.0, b = r < jb.n ? sc * B[col * jb.ldb + r] : 0.0;
+        (y < TM ? sAI[kk][y] : sAJ[kk][y - TM]) = a;
+        (y < TM ? sBI[kk][y] : sBJ[kk][y - TM]) = b;
+      }
+      __syncthreads();
+      for (int kk = 0; kk < nk; ++kk)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            acc1[a][b] = fma(sAI[kk][ty * 4 + a], sBJ[kk][tx * 4 + b], acc1[a][b]);
+            if (!jb.nosym) acc2[a][b] = fma(sAJ[kk][tx * 4 + b], sBI[kk][ty * 4 + a], acc2[a][b]);
+          }
+    }
+    const int* ph = jb.phase_off >= 0 ? phase + jb.phase_off : nullptr;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int i = i0 + ty * 4 + a, j = j0 + tx * 4 + b;
+        if (i < jb.m && j < jb.n && (jb.nosym || i <= j))
+          put_exact(jb, Obase + jb.out_off, ph, jb.sign != 0 ? jb.sign : gsign, i, j, acc1[a][b], acc2[a][b],
+                    accum > 0 || (accum < 0 && jb.accumulate), nomirror);
+      }
+  }
+  for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < nelem; e += gridDim.x * 8) {
+    const DTile tl = tiles[elem[e].tile];
+    const DJob jb = jobs[tl.job];
+    const double* A = Abase + jb.a_off;
+    const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
+    const int i = tl.I * TM + (elem[e].ij & 0xFFFF), j = tl.J * TN + (elem[e].ij >> 16);
+    double p1 = 0.0, p2 = 0.0;
+    for (int t = lane; t < jb.K; t += 32) {
+      const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
+      const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
+      p1 = fma(A[col * jb.lda + i], sc * B[col * jb.ldb + j], p1);
+      if (!jb.nosym) p2 = fma(A[col * jb.lda + j], sc * B[col * jb.ldb + i], p2);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+      p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+    }
+    if (lane == 0)
+      put_exact(jb, Obase + jb.out_off, jb.phase_off >= 0 ? phase + jb.phase_off : nullptr, jb.sign != 0 ? jb.sign : gsign, i,
+                j, p1, p2, accum > 0 || (accum < 0 && jb.accumulate), nomirror);
+  }
+}
+
+// a plane array as (K element, row, plane); a box is one K block x rows x all planes
+void plane_map(CUtensorMap* m, void* base, long long rows, int box_rows)
+{
+  cuuint64_t dims[3] = {(cuuint64_t)KB, (cuuint64_t)rows, (cuuint64_t)NP};
+  cuuint64_t strides[2] = {(cuuint64_t)KB * 2, (cuuint64_t)KB * 2 * (cuuint64_t)rows};
+  cuuint32_t box[3] = {(cuuint32_t)KB, (cuuint32_t)box_rows, (cuuint32_t)NP};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = get_encode()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed");
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ host
+DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
+{
+  DgemmPlan* p = new DgemmPlan();
+  p->family = family;
+  std::vector<DJob> jobs;
+  std::vector<DTile> tiles;
+  std::vector<long long> cost;
+  long long erow = 0, prow = 0;
+  for (const GemmJobDev& j : jobs_in) {
+    DJob d{};
+    d.a_off = j.a_off;
+    d.b_off = j.b_off;
+    d.out_off = j.out_off;
+    d.bscale = j.bscale;
+    d.m = j.m;
+    d.n = j.nosym ? j.n : j.m;
+    d.K = j.K;
+    d.lda = j.lda;
+    d.ldb = j.ldb;
+    d.ldo = j.ldo;
+    d.kidx_off = j.kidx_off;
+    d.w_off = j.w_off;
+    d.phase_off = j.phase_off;
+    d.bsel = j.bsel;
+    d.sign = j.sign;
+    d.accumulate = j.accumulate;
+    d.nosym = j.nosym ? 1 : 0;
+    d.m_pad = (std::max(d.m, d.n) + TM - 1) / TM * TM;
+    d.nkb = std::max(1, (j.K + KB - 1) / KB);
+    d.nchunk = (d.nkb + CH - 1) / CH;
+    d.exp_base = (int)erow;
+    d.row_base = (int)prow;
+    erow += d.m_pad;
+    prow += (long long)d.m_pad * d.nkb;
+    if (prow > (1ll << 31) - TM || erow > (1ll << 31) - TM) {
+      delete p;
+      throw std::runtime_error("digit planes exceed 2^31 rows");
+    }
+    const int jix = (int)jobs.size();
+    jobs.push_back(d);
+    if (d.m == 0 || d.n == 0 || d.K == 0) continue;
+    // a tile costs its K blocks and, per chunk, about three of them in the epilogue, plus its stores
+    const long long c = (d.nosym ? 1 : 2) * (d.nkb + 3 * d.nchunk) + 4;
+    for (int I = 0; I * TM < d.m; ++I)
+      for (int J = d.nosym ? 0 : I * (TM / TN); J * TN < d.n; ++J) {
+        tiles.push_back({jix, I, J});
+        cost.push_back(c);
+      }
+  }
+  p->njobs = (int)jobs.size();
+  p->ntiles = (int)tiles.size();
+  p->rows = std::max<long long>(prow, TM);
+  p->exp_rows = std::max<long long>(erow, TM);
+  if (tiles.empty()) return p;
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  p->grid = std::max(1, std::min(nsm, p->ntiles));
+  // longest first, each to the least loaded CTA; a CTA's tiles in that order
+  std::vector<int> ord(tiles.size());
+  for (size_t t = 0; t < ord.size(); ++t) ord[t] = (int)t;
+  std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  std::vector<std::pair<long long, int>> heap;
+  for (int b = 0; b < p->grid; ++b) heap.push_back({0, b});
+  auto gt = [](const std::pair<long long, int>& x, const std::pair<long long, int>& y) { return x > y; };
+  std::make_heap(heap.begin(), heap.end(), gt);
+  std::vector<std::vector<int>> lists(p->grid);
+  for (int t : ord) {
+    std::pop_heap(heap.begin(), heap.end(), gt);
+    heap.back().first += cost[t];
+    lists[heap.back().second].push_back(t);
+    std::push_heap(heap.begin(), heap.end(), gt);
+  }
+  std::vector<DTile> sorted;
+  std::vector<int> first(p->grid + 1, 0);
+  for (int b = 0; b < p->grid; ++b) {
+    for (int t : lists[b]) sorted.push_back(tiles[t]);
+    first[b + 1] = (int)sorted.size();
+  }
+  std::vector<int4> rb, db;
+  for (int j = 0; j < p->njobs; ++j) {
+    const DJob& d = jobs[j];
+    if (d.m == 0 || d.n == 0 || d.K == 0) continue;
+    for (int y = 0; y < d.m_pad / 32; ++y)
+      for (int x = 0; x < (d.K + 255) / 256; ++x) rb.push_back(make_int4(j, y, x, 0));
+  }
+  // the digit pass starts on the operands that the exponent pass read last
+  for (int j = p->njobs - 1; j >= 0; --j) {
+    const DJob& d = jobs[j];
+    if (d.m == 0 || d.n == 0 || d.K == 0) continue;
+    for (int x = 0; x < d.nkb; ++x)
+      for (int y = 0; y < d.m_pad / 32; ++y) db.push_back(make_int4(j, y, x, 0));
+  }
+  p->n_rblk = (int)rb.size();
+  p->n_dblk = (int)db.size();
+  try {
+    auto dm = [](size_t bytes) {
+      void* q = nullptr;
+      if (cudaMalloc(&q, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+        cudaGetLastError();
+        throw std::runtime_error("cudaMalloc");
+      }
+      return q;
+    };
+    auto up = [&](const void* src, size_t bytes) {
+      void* q = dm(bytes);
+      if (cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaFree(q);
+        throw std::runtime_error("cudaMemcpy");
+      }
+      return q;
+    };
+    for (int a = 0; a < 2; ++a) p->arr[a] = (__nv_bfloat16*)dm((size_t)NP * p->rows * KB * 2);
+    p->d_exp = (int*)dm(sizeof(int) * (2 * p->exp_rows + 2));
+    p->d_list = (int*)dm(sizeof(int) * p->ntiles);
+    p->d_elem = (DElem*)dm(sizeof(DElem) * MAX_LISTED * COLS_W * (size_t)p->ntiles);
+    p->d_jobs = (DJob*)up(jobs.data(), sizeof(DJob) * jobs.size());
+    p->d_tiles = (DTile*)up(sorted.data(), sizeof(DTile) * sorted.size());
+    p->d_cta = (int*)up(first.data(), sizeof(int) * first.size());
+    p->d_rblk = (int4*)up(rb.data(), sizeof(int4) * rb.size());
+    p->d_dblk = (int4*)up(db.data(), sizeof(int4) * db.size());
+    for (int a = 0; a < 2; ++a) {
+      plane_map(&p->maps[a], p->arr[a], p->rows, TM);
+      plane_map(&p->maps[2 + a], p->arr[a], p->rows, TN);
+    }
+    int maxsm = 0;
+    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    p->smem = 1024 + NSTAGE * STAGE + (2 * NSTAGE + 3 + 2 * NINFO) * 8 + 16;
+    if (p->smem + sizeof(TileInfo) * NINFO + 64 > (size_t)maxsm) throw std::runtime_error("not enough shared memory for the FP64 product's pipeline");
+    if (cudaFuncSetAttribute(k_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem) != cudaSuccess) {
+      cudaGetLastError();
+      throw std::runtime_error("cudaFuncSetAttribute");
+    }
+  } catch (...) {
+    dgemm_plan_destroy(p);
+    throw;
+  }
+  return p;
+}
+
+void dgemm_plan_destroy(DgemmPlan* p)
+{
+  if (!p) return;
+  for (void* q : {(void*)p->arr[0], (void*)p->arr[1], (void*)p->d_exp, (void*)p->d_list, (void*)p->d_elem, (void*)p->d_jobs, (void*)p->d_tiles,
+                  (void*)p->d_cta, (void*)p->d_rblk, (void*)p->d_dblk})
+    if (q) cudaFree(q);
+  delete p;
+}
+
+cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, const double* B1, double* O, const int* kidx,
+                         const double* kw, const int* phase, int gsign, double gbscale, int accum, bool mirror,
+                         cudaStream_t st)
+{
+  if (p->ntiles == 0) return cudaSuccess;
+  int *rexpA = p->d_exp, *rexpB = p->d_exp + p->exp_rows, *nlist = p->d_exp + 2 * p->exp_rows;
+  cudaError_t e;
+  {
+    ProfScope ps(p->family == 0 ? "dgemm_slice_ladder" : "dgemm_slice_zbar", st);
+    if ((e = cudaMemsetAsync(p->d_exp, 0, sizeof(int) * (2 * p->exp_rows + 2), st)) != cudaSuccess) return e;
+    k_dgemm_rowexp<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB);
+    k_dgemm_digits<<<p->n_dblk, 256, 0, st>>>(p->d_jobs, p->d_dblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
+                                              p->arr[0], p->arr[1]);
+    count_launch(2);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  ProfScope ps(p->family == 0 ? "dgemm_ladder" : "dgemm_zbar", st);
+  DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA, rexpB, phase, O, nlist, p->d_list, p->d_elem, gsign, accum, mirror ? 0 : 1};
+  k_dgemm<<<p->grid, 96 + 32 * EPIW, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], a);
+  k_dgemm_exact<<<std::min(p->ntiles, 2 * p->grid), 256, 0, st>>>(p->d_jobs, p->d_tiles, nlist, p->d_list, p->d_elem, A, B0, B1, O, kidx,
+                                                                 kw, phase, gsign, gbscale, accum, a.nomirror);
+  count_launch(2);
+  return cudaGetLastError();
+}
+
+}  // namespace imsrg

@@ -412,6 +412,10 @@ int ensure_scratch(imsrg_space* sp, bool pandya, bool w2)
       sp->d_yt = sp->track(dmalloc<double>(s.xb_total));
       sp->d_yf = sp->track(dmalloc<double>(s.xb_total));
       sp->d_zb = sp->track(dmalloc<double>(s.zb_total));
+      // the blocks of channels without ph kets: zero for good (no product writes them)
+      for (auto& zr : sp->zbar_zero)
+        if (cudaMemset(sp->d_zb + zr.first, 0, zr.second * sizeof(double)) != cudaSuccess) throw std::runtime_error("cudaMemset");
+      if (cudaStreamSynchronize(nullptr) != cudaSuccess) throw std::runtime_error("cudaStreamSynchronize");
     }
     if (w2 && !sp->d_w2) sp->d_w2 = sp->track(dmalloc<double>(s.arena));
   } catch (std::exception& e) {
@@ -537,28 +541,14 @@ int check_ops(const imsrg_op* X, const imsrg_op* Y, const imsrg_op* Z)
 cudaStream_t S_(void* st) { return (cudaStream_t)st; }
 
 // ---------------------------------------------------------------- the terms
-int do_111_110(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, bool do111, bool do110, cudaStream_t st)
+// the zero- and one-body terms of todo (OB_*); comm110ss and comm220ss return
+// early when X and Y have the same hermiticity (src/Commutator.cc:567-570, 606-609)
+int do_onebody(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int todo, const char* name, cudaStream_t st)
 {
-  // comm110ss returns early when X and Y have the same hermiticity (src/Commutator.cc:567-570)
-  if (do110 && X->herm == Y->herm) do110 = false;
-  if (!do111 && !do110) return IMSRG_OK;
-  ProfScope ps(do111 ? (do110 ? "comm111ss+comm110ss" : "comm111ss") : "comm110ss", st);
-  CUDA_TRY(launch_comm111_110(*X->sp->s, X->d, Y->d, Z->d, do111, do110, st));
-  return IMSRG_OK;
-}
-
-int do_220(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
-{
-  if (X->herm == Y->herm) return IMSRG_OK;  // src/Commutator.cc:606-609
-  ProfScope ps("comm220ss", st);
-  CUDA_TRY(launch_comm220(*X->sp->s, X->d, Y->d, Z->d, X->herm, st));
-  return IMSRG_OK;
-}
-
-int do_121(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
-{
-  ProfScope ps("comm121ss", st);
-  CUDA_TRY(launch_comm121(*X->sp->s, X->sp->d_holes, X->d, Y->d, Z->d, Z->herm, st));
+  if (X->herm == Y->herm) todo &= ~(OB_110 | OB_220);
+  if (!todo) return IMSRG_OK;
+  ProfScope ps(name, st);
+  CUDA_TRY(launch_onebody(*X->sp->s, X->d, Y->d, Z->d, X->herm, Z->herm, todo, st));
   return IMSRG_OK;
 }
 
@@ -607,12 +597,10 @@ int do_122(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st, i
   return IMSRG_OK;
 }
 
-// Mz: the two-body blocks of Mpp - Mhh when already available (the ladder
-// product accumulated onto a zeroed Z), else nullptr (dot products)
-int do_221_1b(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st, const double* Mz = nullptr)
+int do_221_1b(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
 {
   ProfScope ps("comm221ss", st);
-  CUDA_TRY(launch_comm221_1b(*X->sp->s, X->d, Y->d, Z->d, X->herm, Z->herm, Mz, st));
+  CUDA_TRY(launch_comm221_1b(*X->sp->s, X->d, Y->d, Z->d, X->herm, Z->herm, st));
   return IMSRG_OK;
 }
 
@@ -676,12 +664,12 @@ int ladder_term_fp64(imsrg_space* sp, const imsrg_op* X, const imsrg_op* Y, imsr
     return IMSRG_OK;
   }
   CUDA_TRY(launch_symgemm_fp64(sp->d_ladder_jobs, sp->d_ladder_pairs, sp->n_ladder_pairs, X->d, Y->d, Y->d, Z->d,
-                               s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, st));
+                               s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, -1, st));
   return IMSRG_OK;
 }
 
-// overwrite: Z2 is known to be zero (fresh commutator), so the product
-// writes its blocks instead of read-modify-write
+// overwrite: the product writes Z2's blocks (a fresh commutator) instead of
+// adding to them
 int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st, bool overwrite = false)
 {
   imsrg_space* sp = X->sp;
@@ -703,12 +691,12 @@ int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaS
     return IMSRG_OK;
   }
   CUDA_TRY(launch_symgemm_fp64(sp->d_ladder_jobs, sp->d_ladder_pairs, sp->n_ladder_pairs, X->d, Y->d, Y->d, Z->d,
-                               s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, st));
+                               s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, (double)Y->herm, 0, st));
   return IMSRG_OK;
 }
 
 // comm222_phss, first half: the Pandya-transformed operands (X bar, Y bar,
-// Y bar flipped) and the zero blocks of Z bar
+// Y bar flipped)
 int prep_ph(const imsrg_op* X, const imsrg_op* Y, int prec, cudaStream_t st)
 {
   imsrg_space* sp = X->sp;
@@ -717,7 +705,6 @@ int prep_ph(const imsrg_op* X, const imsrg_op* Y, int prec, cudaStream_t st)
   if (rc) return rc;
   ProfScope ps("Pandya transform of X, Y", st);
   CUDA_TRY(launch_pandya_fwd(s, X->d, Y->d, Y->herm, sp->d_xb, sp->d_yt, sp->d_yf, prec == IMSRG_PREC_SPLIT, st));
-  for (auto& zr : sp->zbar_zero) CUDA_TRY(cudaMemsetAsync(sp->d_zb + zr.first, 0, zr.second * sizeof(double), st));
   return IMSRG_OK;
 }
 
@@ -747,7 +734,7 @@ int do_ph(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStrea
                             Z->herm, 1.0, 0, sp->inv_fp64 == 0, st));
     else
       CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
-                                   sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, 1.0, st));
+                                   sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, 1.0, 0, st));
   } else {
     return fail(IMSRG_ERR_ARG, "unknown precision");
   }
@@ -779,31 +766,39 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   }
   cudaStream_t sd = sp->side;
   ProfScope ps("CommutatorScalarScalar", st);
-  CUDA_TRY(cudaMemsetAsync(Z->d, 0, sp->s->arena * sizeof(double), st));
+  const bool ladder_first = on[T222PPHH];
+  if (ladder_first)
+    CUDA_TRY(launch_zero_gaps(*sp->s, Z->d, st));  // the ladder product writes the rest
+  else
+    CUDA_TRY(cudaMemsetAsync(Z->d, 0, sp->s->arena * sizeof(double), st));
   // The terms add into Z in an order of our own (the sum is the same up to
-  // rounding): the ladder product goes first, onto the zeroed two-body blocks,
+  // rounding): the ladder product goes first and overwrites the two-body blocks,
   // so the one-body part of comm221ss can read Mpp - Mhh straight from Z2
   // instead of recomputing the pp dot products (ConstructScalarMpp_Mhh is
   // shared the same way by the reference's comm222_pp_hh_221ss).
   //
   // While the ladder product runs on st, a second stream does what does not
   // depend on it: the operand preparation of comm122ss and comm222_phss and
-  // the zero- and one-body terms 111/110, 220, 121 (they write only Z0 and Z1,
-  // the ladder only Z2).  The streams join before comm221ss, which reads Z2
-  // and writes Z1.
+  // the zero- and one-body terms (they write only Z0 and Z1, the ladder only
+  // Z2).  The streams join before comm221ss's last part, which reads Z2 and
+  // writes Z1.
   CUDA_TRY(cudaEventRecord(sp->ev_fork, st));
   CUDA_TRY(cudaStreamWaitEvent(sd, sp->ev_fork, 0));
   const bool split = prec == IMSRG_PREC_SPLIT;
   if (on[T122] && split && (rc = prep_122_df(X, Y, sd))) return rc;
   if (on[T222PH] && (rc = prep_ph(X, Y, prec, sd))) return rc;
-  if ((rc = do_111_110(X, Y, Z, on[T111], on[T110], sd))) return rc;
-  if (on[T220] && (rc = do_220(X, Y, Z, sd))) return rc;
-  if (on[T121] && (rc = do_121(X, Y, Z, sd))) return rc;
+  const int todo = (on[T111] ? OB_111 : 0) | (on[T110] ? OB_110 : 0) | (on[T121] ? OB_121 : 0) | (on[T220] ? OB_220 : 0) |
+                   (on[T221] && ladder_first ? OB_221 : 0);
+  if ((rc = do_onebody(X, Y, Z, todo, "zero- and one-body terms", sd))) return rc;
   CUDA_TRY(cudaEventRecord(sp->ev_join, sd));
-  bool ladder_first = on[T222PPHH];
   if (ladder_first && (rc = do_ladder(X, Y, Z, prec, st, true))) return rc;
   CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join, 0));
-  if (on[T221] && (rc = do_221_1b(X, Y, Z, st, ladder_first ? Z->d : nullptr))) return rc;
+  if (on[T221] && ladder_first) {
+    ProfScope p221("comm221ss", st);
+    CUDA_TRY(launch_comm221_z(*sp->s, Z->d, Z->herm, Z->d, st));
+  } else if (on[T221] && (rc = do_221_1b(X, Y, Z, st))) {
+    return rc;
+  }
   // comm122ss's final Z -= W2 + hZ W2^T rides in the inverse Pandya kernel,
   // which reads and writes every upper-triangle element of Z and its mirror
   // anyway, when that kernel is the descriptor one and lists every element
@@ -1236,25 +1231,25 @@ int imsrg_op_fill_random(imsrg_op* op, unsigned long long seed, void* stream)
 int imsrg_comm110ss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, void* stream)
 {
   TERM_PROLOGUE
-  return do_111_110(X, Y, Z, false, true, st);
+  return do_onebody(X, Y, Z, OB_110, "comm110ss", st);
 }
 
 int imsrg_comm220ss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, void* stream)
 {
   TERM_PROLOGUE
-  return do_220(X, Y, Z, st);
+  return do_onebody(X, Y, Z, OB_220, "comm220ss", st);
 }
 
 int imsrg_comm111ss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, void* stream)
 {
   TERM_PROLOGUE
-  return do_111_110(X, Y, Z, true, false, st);
+  return do_onebody(X, Y, Z, OB_111, "comm111ss", st);
 }
 
 int imsrg_comm121ss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, void* stream)
 {
   TERM_PROLOGUE
-  return do_121(X, Y, Z, st);
+  return do_onebody(X, Y, Z, OB_121, "comm121ss", st);
 }
 
 int imsrg_comm122ss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, void* stream)
@@ -1498,7 +1493,7 @@ int end_status(imsrg_space* sp, cudaStream_t st) { return sp->defer_status ? IMS
 // ------------------------------------------------------------- batch phases
 // CommutatorScalarScalar in the split form for a group of pairs of the same
 // structure, every kernel launched once for all of them (see capi_batch.cu):
-// pre (Z zeroed, operand preparation, the zero- and one-body terms), the
+// pre (what the ladder leaves of Z zeroed, operand preparation, the zero- and one-body terms), the
 // ladder product, mid (comm221ss, comm122ss), the Zbar product, post (inverse
 // Pandya transform).  Every term must be on.
 namespace imsrg {
@@ -1656,26 +1651,21 @@ GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, 
 int group_pre(GroupedProducts* g, cudaStream_t st)
 {
   const int nz = (int)g->X.size();
-  for (int p = 0; p < nz; ++p) {
-    imsrg_space* sp = g->X[p]->sp;
-    g->Z[p]->herm = z_herm(g->X[p]->herm, g->Y[p]->herm);
-    CUDA_TRY(cudaMemsetAsync(g->Z[p]->d, 0, sp->s->arena * sizeof(double), st));
-    for (auto& zr : sp->zbar_zero) CUDA_TRY(cudaMemsetAsync(sp->d_zb + zr.first, 0, zr.second * sizeof(double), st));
-  }
+  for (int p = 0; p < nz; ++p) g->Z[p]->herm = z_herm(g->X[p]->herm, g->Y[p]->herm);
   const imsrg_op *X = g->X[0], *Y = g->Y[0];
   imsrg_op* Z = g->Z[0];
   imsrg_space* sp = X->sp;
   const Space& s = *sp->s;
   const long long* zo = g->d_zoff;
+  CUDA_TRY(launch_zero_gaps(s, Z->d, st, zo, nz));  // the ladder product writes the rest of Z
   if (g->prec == IMSRG_PREC_SPLIT) {
     CUDA_TRY(launch_to_ff(s, X->d, sp->d_xf, st, zo, nz, ZR_X, ZR_XF));
     CUDA_TRY(launch_to_ff(s, Y->d, sp->d_yff, st, zo, nz, ZR_Y, ZR_YF));
   }
   CUDA_TRY(launch_pandya_fwd(s, X->d, Y->d, Y->herm, sp->d_xb, sp->d_yt, sp->d_yf, g->prec == IMSRG_PREC_SPLIT, st,
                              zo, nz));
-  CUDA_TRY(launch_comm111_110(s, X->d, Y->d, Z->d, true, X->herm != Y->herm, st, zo, nz));
-  if (X->herm != Y->herm) CUDA_TRY(launch_comm220(s, X->d, Y->d, Z->d, X->herm, st, zo, nz));
-  CUDA_TRY(launch_comm121(s, sp->d_holes, X->d, Y->d, Z->d, Z->herm, st, zo, nz));
+  CUDA_TRY(launch_onebody(s, X->d, Y->d, Z->d, X->herm, Z->herm,
+                          OB_111 | OB_121 | OB_221 | (X->herm != Y->herm ? OB_110 | OB_220 : 0), st, zo, nz));
   return IMSRG_OK;
 }
 
@@ -1687,7 +1677,7 @@ int group_mid(GroupedProducts* g, cudaStream_t st)
   imsrg_space* sp = X->sp;
   const Space& s = *sp->s;
   const long long* zo = g->d_zoff;
-  CUDA_TRY(launch_comm221_1b(s, X->d, Y->d, Z->d, X->herm, Z->herm, Z->d, st, zo, nz));
+  CUDA_TRY(launch_comm221_z(s, Z->d, Z->herm, Z->d, st, zo, nz));
   if (g->prec == IMSRG_PREC_FP64)
     CUDA_TRY(launch_comm122(s, X->d, Y->d, Z->d, sp->d_w2, Z->herm, sp->d_sym122, sp->n_sym122, st, zo, nz));
   else if (sp->comm122_fused)
@@ -1723,7 +1713,7 @@ int grouped_ladder(GroupedProducts* g, cudaStream_t st)
 {
   imsrg_space* s0 = g->X[0]->sp;
   const Space& s = *s0->s;
-  if (g->fp64_ladder) {  // Z was zeroed in the pre phase
+  if (g->fp64_ladder) {
     CUDA_TRY(launch_dgemm(g->fp64_ladder, g->X[0]->d, g->Y[0]->d, g->Y[0]->d, g->Z[0]->d, s.work.kidx, s.work.kweight,
                           s.work.phase_tab, g->Z[0]->herm, (double)g->Y[0]->herm, 0, true, st));
     return IMSRG_OK;
@@ -1731,10 +1721,10 @@ int grouped_ladder(GroupedProducts* g, cudaStream_t st)
   if (g->prec == IMSRG_PREC_FP64) {
     CUDA_TRY(launch_symgemm_fp64(g->d_lj, g->d_lp, g->n_lp, g->X[0]->d, g->Y[0]->d, g->Y[0]->d, g->Z[0]->d,
                                  s.work.kidx, s.work.kweight, s.work.phase_tab, g->Z[0]->herm,
-                                 (double)g->Y[0]->herm, st));
+                                 (double)g->Y[0]->herm, 0, st));
     return IMSRG_OK;
   }
-  split_plan_set_accumulate(g->ladder, 0);  // Z was zeroed in the pre phase
+  split_plan_set_accumulate(g->ladder, 0);  // the pre phase zeroed only the rest of Z
   CUDA_TRY(launch_symgemm_split(g->ladder, g->X[0]->d, g->Y[0]->d, g->Y[0]->d, g->Z[0]->d, s.work.kidx,
                                 s.work.kweight, s.work.phase_tab, s0->d_status, g->Z[0]->herm,
                                 (double)g->Y[0]->herm, st));
@@ -1752,7 +1742,7 @@ int grouped_zbar(GroupedProducts* g, cudaStream_t st)
   }
   if (g->prec == IMSRG_PREC_FP64) {
     CUDA_TRY(launch_symgemm_fp64(g->d_zj, g->d_zp, g->n_zp, s0->d_xb, s0->d_yt, s0->d_yf, s0->d_zb, s.work.kidx,
-                                 s.work.kweight, s.work.phase_tab, g->Z[0]->herm, 1.0, st));
+                                 s.work.kweight, s.work.phase_tab, g->Z[0]->herm, 1.0, 0, st));
     return IMSRG_OK;
   }
   split_plan_set_mirror(g->zbar, s0->inv_split == 0 ? 1 : 0);  // as group_post reads Zbar

@@ -56,7 +56,31 @@ struct PfOut {
   double xs;       // normfactor * (n_a - n_b)
 };
 
+// comm121ss and comm221ss for one one-body pair (i <= j) as sums over arena
+// elements, from per-space descriptors (build_onebody, space.cpp)
+struct T121 {  // w (X[u] Y[v] - Y[u] X[v])
+  long long v;
+  double w;
+  int u, pad;
+};
+struct T221 {  // w sum_k nn_k (X[r + k] Y[s + k] + h_Z X[s + k] Y[r + k]), k over hh_list[hh .. hh + nhh)
+  long long r, s;
+  double w;
+  int hh, nhh;
+  int kofs, pad;
+};
+struct T221Z {  // w (Mpp - Mhh)[v]
+  long long v;
+  double w;
+};
+
 struct DevWork {
+  const T121* t121;
+  const T221* t221;
+  const T221Z* t221z;
+  const int3* ob_off;       // per pair (and one past): first t121, t221, t221z
+  const longlong2* gaps;    // what the ladder product does not write of an arena: (offset, length)
+  int ngaps;
   const double* ket_wpp;  // flat over 2b channel kets (ch_kofs order)
   const double* ket_nn;
   const int* hh_off;      // per channel, into hh_list

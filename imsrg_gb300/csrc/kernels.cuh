@@ -28,18 +28,18 @@ struct GemmJobDev {
 // (batches): pair z's operands sit at byte offsets zo[z * kZRoles + role] from
 // the pointers passed (pair 0's); zo = nullptr, nz = 1 is one pair.
 enum ZRole { ZR_X, ZR_Y, ZR_Z, ZR_XF, ZR_YF, ZR_W2, ZR_XB, ZR_YT, ZR_YFL, ZR_ZB, kZRoles };
-// (grouped)
-cudaError_t launch_comm111_110(const Space& s, const double* X, const double* Y, double* Z, bool do111, bool do110,
-                               cudaStream_t st, const long long* zo = nullptr, int nz = 1);
-// (grouped)
-cudaError_t launch_comm220(const Space& s, const double* X, const double* Y, double* Z, int hX, cudaStream_t st,
-                           const long long* zo = nullptr, int nz = 1);
-// (grouped)
-cudaError_t launch_comm121(const Space& s, const int* dev_holes, const double* X, const double* Y, double* Z, int hZ,
+// zeroes what the ladder product does not write of an arena; (grouped)
+cudaError_t launch_zero_gaps(const Space& s, double* Z, cudaStream_t st, const long long* zo = nullptr, int nz = 1);
+// the zero- and one-body terms of todo: OB_221 is comm221ss without its
+// Mpp - Mhh part, which launch_comm221_z adds; (grouped)
+enum { OB_111 = 1, OB_110 = 2, OB_121 = 4, OB_221 = 8, OB_220 = 16 };
+cudaError_t launch_onebody(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ, int todo,
                            cudaStream_t st, const long long* zo = nullptr, int nz = 1);
-// (grouped with Mz)
-cudaError_t launch_comm221_1b(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ,
-                              const double* Mz, cudaStream_t st, const long long* zo = nullptr, int nz = 1);
+// Mz: the two-body blocks of Mpp - Mhh, in Z's layout (grouped: Z itself)
+cudaError_t launch_comm221_z(const Space& s, double* Z, int hZ, const double* Mz, cudaStream_t st,
+                             const long long* zo = nullptr, int nz = 1);
+// comm221ss on its own
+cudaError_t launch_comm221_1b(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ, cudaStream_t st);
 // (grouped)
 cudaError_t launch_comm122(const Space& s, const double* X, const double* Y, double* Z, double* W2, int hZ,
                            const int* sym_tiles, int nsym_tiles, cudaStream_t st, const long long* zo = nullptr,
@@ -171,9 +171,10 @@ cudaError_t launch_tensor_inverse_pandya(const Space& s, const TensorLayout& t, 
 
 // kernels_gemm.cu
 int symgemm_fp64_tile();
+// accum: -1 each job's own flag, 0 overwrite, 1 accumulate
 cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int npairs, const double* A,
                                 const double* B0, const double* B1, double* O, const int* kidx, const double* kw,
-                                const int* phase, int gsign, double gbscale, cudaStream_t st);
+                                const int* phase, int gsign, double gbscale, int accum, cudaStream_t st);
 
 // kernels_dgemm.cu: the same products, and plain ones (nosym), to FP64 accuracy
 // on the tensor cores.  create throws when its planes do not fit in device

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256) k_symgemm_fp64(const GemmJobDev* __restri
                                                       const double* __restrict__ B0, const double* __restrict__ B1,
                                                       double* __restrict__ Obase, const int* __restrict__ kidx,
                                                       const double* __restrict__ kw, const int* __restrict__ phase,
-                                                      int gsign, double gbscale)
+                                                      int gsign, double gbscale, int accum)
 {
   extern __shared__ double smem[];
   int pid = blockIdx.x;
@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(256) k_symgemm_fp64(const GemmJobDev* __restri
   const int* ph = jb.phase_off >= 0 ? phase + jb.phase_off : nullptr;
   double* O = Obase + jb.out_off;
   const double sgn = (double)(jb.sign != 0 ? jb.sign : gsign);
+  const bool accumulate = accum > 0 || (accum < 0 && jb.accumulate);
   for (int e = tid; e < TM * TM; e += 256) {
     int r = e & 63, c = e >> 6;  // r fastest -> coalesced column-major stores
     int i = I0 + r, j = J0 + c;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(256) k_symgemm_fp64(const GemmJobDev* __restri
       double f = ph ? (double)(ph[i] * ph[j]) : 1.0;
       double v = S1[r * LDS + c] + sgn * f * p;
       long long o = (long long)j * jb.ldo + i;
-      O[o] = jb.accumulate ? O[o] + v : v;
+      O[o] = accumulate ? O[o] + v : v;
     }
     if (!diag) {
       // Out(J, I): rows from J, cols from I
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(256) k_symgemm_fp64(const GemmJobDev* __restri
         double f = ph ? (double)(ph[i2] * ph[j2]) : 1.0;
         double v = S2[r * LDS + c] + sgn * f * S1[c * LDS + r];
         long long o = (long long)j2 * jb.ldo + i2;
-        O[o] = jb.accumulate ? O[o] + v : v;
+        O[o] = accumulate ? O[o] + v : v;
       }
     }
   }
@@ -149,7 +150,7 @@ int symgemm_fp64_tile() { return TM; }
 
 cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int npairs, const double* A,
                                 const double* B0, const double* B1, double* O, const int* kidx, const double* kw,
-                                const int* phase, int gsign, double gbscale, cudaStream_t st)
+                                const int* phase, int gsign, double gbscale, int accum, cudaStream_t st)
 {
   if (npairs == 0) return cudaSuccess;
   static bool attr = false;
@@ -159,7 +160,8 @@ cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int np
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  k_symgemm_fp64<<<npairs, 256, sm, st>>>(jobs, pairs, npairs, A, B0, B1, O, kidx, kw, phase, gsign, gbscale);
+  k_symgemm_fp64<<<npairs, 256, sm, st>>>(jobs, pairs, npairs, A, B0, B1, O, kidx, kw, phase, gsign, gbscale,
+                                           accum);
   count_launch();
   return cudaGetLastError();
 }

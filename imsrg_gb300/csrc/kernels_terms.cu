@@ -31,63 +31,157 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
-// ---------------------------------------------------------------- 111 + 110
-// Z1 += X1 Y1 - Y1 X1  (comm111ss, src/Commutator.cc:644-649) and
-// Z0 += sum_a (2j_a+1) n_a (X1 Y1 - Y1 X1)_aa over holes (comm110ss, :564-581)
-__global__ void k_comm111_110(DevSpace S, const double* __restrict__ X, const double* __restrict__ Y,
-                              double* __restrict__ Z, int do111, int do110, const long long* __restrict__ zo)
+// ------------------------------------------- zero- and one-body terms, zeroing
+// The arena but for the blocks the ladder product overwrites (a commutator's
+// Z): a block per piece.  emax=10: 3 us, where clearing the whole arena took 50.
+__global__ void k_zero_gaps(DevWork W, double* __restrict__ Z, const long long* __restrict__ zo)
 {
-  X = zsh(X, zo, ZR_X);
-  Y = zsh(Y, zo, ZR_Y);
   Z = zsh(Z, zo, ZR_Z);
-  int N = S.norb;
-  int i = blockIdx.x;
-  const double* X1 = X + 32;
-  const double* Y1 = Y + 32;
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    double xy = 0.0, yx = 0.0;
-    for (int b = 0; b < N; ++b) {
-      xy = fma(X1[(size_t)b * N + i], Y1[(size_t)j * N + b], xy);
-      yx = fma(Y1[(size_t)b * N + i], X1[(size_t)j * N + b], yx);
-    }
-    double v = xy - yx;
-    if (do111) Z[32 + (size_t)j * N + i] += v;
-    if (do110 && j == i) {
-      double oc = S.occ[i];
-      if (oc >= 1e-6) atomicAdd(Z, (S.j2[i] + 1) * oc * v);
-    }
-  }
+  const longlong2 g = W.gaps[blockIdx.x];
+  for (int t = threadIdx.x; t < (int)g.y; t += blockDim.x) Z[g.x + t] = 0.0;
 }
 
-// ---------------------------------------------------------------------- 220
-// Z0 += 2 sum_ch (2J+1) sum_{h in hh} n_h n_h' (X_{h,nbar} (nbar nbar) Y_{nbar,h})
-// (comm220ss, src/Commutator.cc:601-631); one warp per hh ket.
-__global__ void k_comm220(DevSpace S, DevWork W, const double* __restrict__ X, const double* __restrict__ Y,
-                          double* __restrict__ Z, int hX, const long long* __restrict__ zo)
+// One launch for the terms that read X and Y only and write Z0 and Z1 (do: a
+// mask of OB_*); a block's role is its index:
+//  - a one-body pair (i <= j): comm121ss (src/Commutator.cc:670-728) and the
+//    hole-hole part of comm221ss (:1250-1294), threads over the space's
+//    descriptors (build_onebody, space.cpp);
+//  - a 16 x 16 tile of Z1 += X1 Y1 - Y1 X1 (comm111ss, :644-649), with
+//    Z0 += sum_a (2j_a+1) n_a (X1 Y1 - Y1 X1)_aa (comm110ss, :564-581) on the
+//    diagonal tiles;
+//  - an hh ket of comm220ss (:601-631):
+//    Z0 += 2 (2J+1) n_h n_h' X_{h,k} nbar_k nbar_k' Y_{k,h}.
+// Bound by latency: a pair's threads make one or two dependent loads a
+// descriptor.  The four kernels it replaces (a warp or block a pair working
+// the elements out, a thread an element of Z1) took 17 + 22 + 5 + 5 us one
+// after the other at emax=2 and 29 + 42 + 38 + 20 at emax=10.
+constexpr int kObThreads = 256;
+
+__device__ __forceinline__ double block_sum(double v, double* red)
+{
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = threadIdx.x < kObThreads / 32 ? red[threadIdx.x] : 0.0;
+  return threadIdx.x < 32 ? warp_sum(v) : 0.0;
+}
+
+__global__ void __launch_bounds__(kObThreads) k_onebody(DevSpace S, DevWork W, const double* __restrict__ X,
+                                                        const double* __restrict__ Y, double* __restrict__ Z, int hX,
+                                                        int hZ, int todo, const long long* __restrict__ zo)
 {
   X = zsh(X, zo, ZR_X);
   Y = zsh(Y, zo, ZR_Y);
   Z = zsh(Z, zo, ZR_Z);
-  int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  if (item >= W.n220) return;
-  int ch = W.items220[2 * item], h = W.items220[2 * item + 1];
-  int n = S.ch_n[ch];
-  long long off = S.ch_off[ch];
-  const double* xc = X + off + (long long)h * n;  // X(h,k) = hX X(k,h)
-  const double* yc = Y + off + (long long)h * n;  // Y(k,h)
+  __shared__ double red[kObThreads / 32];
+  constexpr int T = 16, TK = 32;
+  __shared__ double xi[TK][T + 1], yi[TK][T + 1], xj[T][TK + 1], yj[T][TK + 1];
+  const int N = S.norb, tid = threadIdx.x;
+  int item = blockIdx.x;
+  if (todo & (OB_121 | OB_221)) {
+    if (item < W.npairs1b) {
+      const int3 b0 = W.ob_off[item], b1 = W.ob_off[item + 1];
+      double z = 0.0;
+      if (todo & OB_121)
+        for (int t = b0.x + tid; t < b1.x; t += kObThreads) {
+          const T121 d = W.t121[t];
+          z = fma(d.w, X[d.u] * Y[d.v] - Y[d.u] * X[d.v], z);
+        }
+      if (todo & OB_221) {
+        double h = 0.0;
+        for (int t = b0.y + tid; t < b1.y; t += kObThreads) {
+          const T221 d = W.t221[t];
+          double rs = 0.0, sr = 0.0;
+          for (int x = 0; x < d.nhh; ++x) {
+            const int k = W.hh_list[d.hh + x];
+            const double nn = W.ket_nn[d.kofs + k];
+            rs = fma(X[d.r + k] * nn, Y[d.s + k], rs);
+            sr = fma(X[d.s + k] * nn, Y[d.r + k], sr);
+          }
+          h = fma(d.w, hZ > 0 ? rs + sr : rs - sr, h);
+        }
+        z += hX > 0 ? h : -h;
+      }
+      z = block_sum(z, red);
+      if (tid == 0) {
+        const int i = W.pairs1b[2 * item], j = W.pairs1b[2 * item + 1];
+        atomicAdd(Z + 32 + (size_t)j * N + i, z);  // comm111ss's block adds there too
+        if (i != j) atomicAdd(Z + 32 + (size_t)i * N + j, hZ * z);
+      }
+      return;
+    }
+    item -= W.npairs1b;
+  }
+  if (todo & (OB_111 | OB_110)) {
+    const int nt = (N + T - 1) / T;
+    if (item < nt * nt) {
+      const int i0 = item % nt * T, j0 = item / nt * T;
+      const int r = tid & 15, c = tid >> 4, i = i0 + r, j = j0 + c;
+      const double* X1 = X + 32;
+      const double* Y1 = Y + 32;
+      double xy = 0.0, yx = 0.0;
+      for (int b0 = 0; b0 < N; b0 += TK) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < T * TK / kObThreads; ++u) {
+          const int b = b0 + c + u * (kObThreads / T);  // 16 rows i, 32 columns b
+          const bool ok = b < N && i < N;
+          xi[b - b0][r] = ok ? X1[(size_t)b * N + i] : 0.0;
+          yi[b - b0][r] = ok ? Y1[(size_t)b * N + i] : 0.0;
+          const int e = tid + u * kObThreads, bb = e & 31, jj = e >> 5;  // 32 rows b, 16 columns j
+          const bool ok2 = b0 + bb < N && j0 + jj < N;
+          xj[jj][bb] = ok2 ? X1[(size_t)(j0 + jj) * N + b0 + bb] : 0.0;
+          yj[jj][bb] = ok2 ? Y1[(size_t)(j0 + jj) * N + b0 + bb] : 0.0;
+        }
+        __syncthreads();
+        const int nb = min(TK, N - b0);
+        for (int b = 0; b < nb; ++b) {
+          xy = fma(xi[b][r], yj[c][b], xy);
+          yx = fma(yi[b][r], xj[c][b], yx);
+        }
+      }
+      if (i < N && j < N) {
+        const double v = xy - yx;
+        if (todo & OB_111) atomicAdd(Z + 32 + (size_t)j * N + i, v);
+        if ((todo & OB_110) && j == i) {
+          const double oc = S.occ[i];
+          if (oc >= 1e-6) atomicAdd(Z, (S.j2[i] + 1) * oc * v);
+        }
+      }
+      return;
+    }
+    item -= nt * nt;
+  }
+  // comm220ss
+  const int ch = W.items220[2 * item], h = W.items220[2 * item + 1];
+  const int n = S.ch_n[ch];
+  const long long off = S.ch_off[ch] + (long long)h * n;  // X(h,k) = hX X(k,h)
   const double* w = W.ket_wpp + S.ch_kofs[ch];
   double d = 0.0;
-  for (int k = lane; k < n; k += 32) d = fma(xc[k] * w[k], yc[k], d);
-  d = warp_sum(d);
+  for (int k = tid; k < n; k += kObThreads) d = fma(X[off + k] * w[k], Y[off + k], d);
+  d = block_sum(d, red);
+  if (tid == 0) atomicAdd(Z, 2.0 * (2 * (ch / 6) + 1) * hX * d * W.ket_nn[S.ch_kofs[ch] + h]);
+}
+
+// The rest of comm221ss, once the ladder product's Mpp - Mhh is in Z2 (Mz = Z
+// there): a warp per pair over the holes' elements.
+__global__ void __launch_bounds__(256) k_comm221_z(DevSpace S, DevWork W, double* __restrict__ Z, int hZ,
+                                                   const double* __restrict__ Mz, const long long* __restrict__ zo)
+{
+  Z = zsh(Z, zo, ZR_Z);
+  Mz = zsh(Mz, zo, ZR_Z);
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= W.npairs1b) return;
+  double z = 0.0;
+  for (int t = W.ob_off[item].z + lane; t < W.ob_off[item + 1].z; t += 32) z = fma(W.t221z[t].w, Mz[W.t221z[t].v], z);
+  z = warp_sum(z);
   if (lane == 0) {
-    int J = ch / 6;
-    double nn = W.ket_nn[S.ch_kofs[ch] + h];
-    atomicAdd(Z, 2.0 * (2 * J + 1) * hX * d * nn);
+    const int i = W.pairs1b[2 * item], j = W.pairs1b[2 * item + 1], N = S.norb;
+    Z[32 + (size_t)j * N + i] += z;
+    if (i != j) Z[32 + (size_t)i * N + j] += hZ * z;
   }
 }
 
-// ---------------------------------------------------------------------- 121
 // TwoBodyME::GetTBMEmonopole (src/TwoBodyME.cc:615-682)
 __device__ double dev_monopole(const DevSpace& S, const double* op, int a, int b, int c, int d)
 {
@@ -102,51 +196,6 @@ __device__ double dev_monopole(const DevSpace& S, const double* op, int a, int b
   if (a == b) mon *= kSqrt2;
   if (c == d) mon *= kSqrt2;
   return mon;
-}
-
-// comm121ss, src/Commutator.cc:670-728: one warp per (i <= j) pair, lanes over
-// (hole a, b in the one-body channel of a).
-__global__ void k_comm121(DevSpace S, DevWork W, const int* __restrict__ holes, int nholes,
-                          const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ Z, int hZ,
-                          const long long* __restrict__ zo)
-{
-  X = zsh(X, zo, ZR_X);
-  Y = zsh(Y, zo, ZR_Y);
-  Z = zsh(Z, zo, ZR_Z);
-  int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  if (item >= W.npairs1b) return;
-  int i = W.pairs1b[2 * item], j = W.pairs1b[2 * item + 1];
-  int N = S.norb;
-  const double* X1 = X + 32;
-  const double* Y1 = Y + 32;
-  double z = 0.0;
-  // enumerate (a, b) pairs: a = holes[ia], b = ob_list[ob_start[a] + ib]
-  int total = 0;
-  for (int ia = 0; ia < nholes; ++ia) total += S.ob_count[holes[ia]];
-  for (int t = lane; t < total; t += 32) {
-    int ia = 0, rem = t;
-    while (rem >= S.ob_count[holes[ia]]) {
-      rem -= S.ob_count[holes[ia]];
-      ++ia;
-    }
-    int a = holes[ia];
-    int b = S.ob_list[S.ob_start[a] + rem];
-    double nanb = S.occ[a] * (1.0 - S.occ[b]);
-    if (fabs(nanb) < 1e-6) continue;
-    int jja = S.j2[a], jjb = S.j2[b];
-    double ybiaj = dev_monopole(S, Y, b, i, a, j);
-    double yaibj = dev_monopole(S, Y, a, i, b, j);
-    z += (jjb + 1) * nanb * X1[(size_t)b * N + a] * ybiaj;
-    z -= (jja + 1) * nanb * X1[(size_t)a * N + b] * yaibj;
-    z -= (jjb + 1) * nanb * Y1[(size_t)b * N + a] * dev_monopole(S, X, b, i, a, j);
-    z += (jja + 1) * nanb * Y1[(size_t)a * N + b] * dev_monopole(S, X, a, i, b, j);
-  }
-  z = warp_sum(z);
-  if (lane == 0) {
-    Z[32 + (size_t)j * N + i] += z;
-    if (i != j) Z[32 + (size_t)i * N + j] += hZ * z;
-  }
 }
 
 // -------------------------------------------------------------- 221 (1b)
@@ -173,11 +222,10 @@ __device__ __forceinline__ double warp_dot_list(const double* a, const double* b
   return warp_sum(d);
 }
 
-// With Mz != nullptr, Mz holds the two-body blocks of Mpp - Mhh (symmetrised),
-// i.e. exactly what the ladder product added to a zeroed Z, and
-// Mpp = Mz + Mhh needs only the short hh dot products.
+// (The term on its own; a commutator reads Mpp - Mhh from the ladder product
+// instead: k_onebody and k_comm221_z.)
 __global__ void k_comm221_1b(DevSpace S, DevWork W, const double* __restrict__ X, const double* __restrict__ Y,
-                             double* __restrict__ Z, int hX, int hZ, const double* __restrict__ Mz)
+                             double* __restrict__ Z, int hX, int hZ)
 {
   int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
@@ -210,7 +258,7 @@ __global__ void k_comm221_1b(DevSpace S, DevWork W, const double* __restrict__ X
     double fac = (2 * J + 1) * ph * nrm;
     const bool need_pp = fabs(nc) > 1e-9, need_hh = fabs(nbarc) > 1e-9;
     double mhh = 0.0;
-    if (need_hh || (need_pp && Mz)) {
+    if (need_hh) {
       const double* w = W.ket_nn + S.ch_kofs[ch];
       const int* hh = W.hh_list + W.hh_off[ch];
       int nhh = W.hh_off[ch + 1] - W.hh_off[ch];
@@ -219,16 +267,10 @@ __global__ void k_comm221_1b(DevSpace S, DevWork W, const double* __restrict__ X
       mhh = m_rs + hZ * m_sr;
     }
     if (need_pp) {
-      double mpp;
-      if (Mz) {
-        mpp = Mz[off + (long long)s * n + r] + mhh;
-      } else {
-        const double* w = W.ket_wpp + S.ch_kofs[ch];
-        double m_rs = hX * warp_dot_w(xr, ys, w, n, lane);
-        double m_sr = (r == s) ? m_rs : hX * warp_dot_w(xs, yr, w, n, lane);
-        mpp = m_rs + hZ * m_sr;
-      }
-      z += fac * nc * mpp;
+      const double* w = W.ket_wpp + S.ch_kofs[ch];
+      double m_rs = hX * warp_dot_w(xr, ys, w, n, lane);
+      double m_sr = (r == s) ? m_rs : hX * warp_dot_w(xs, yr, w, n, lane);
+      z += fac * nc * (m_rs + hZ * m_sr);
     }
     if (need_hh) z += fac * nbarc * mhh;
   }
@@ -371,79 +413,6 @@ __global__ void k_sym_subtract_ff(DevSpace S, const float2* __restrict__ W2, dou
       df_add(w[k].x, w[k].y, u.x, u.y, hi, lo);
       Z[off + (long long)c * n + r] = zo4[k] - ff2d(hi, lo);
     }
-  }
-}
-
-// Same one-body part when Mpp - Mhh is already in Mz (the ladder product added
-// to a zeroed Z): one block of 128 threads per (i <= j) pair, threads over c;
-// each thread forms the short Mhh dot products (hh kets only) itself, and the
-// block reduces once.  (A warp per pair left 5% of the warps of the GPU
-// active: there are only a few hundred pairs.)
-__global__ void k_comm221_1b_mz(DevSpace S, DevWork W, const double* __restrict__ X, const double* __restrict__ Y,
-                                double* __restrict__ Z, int hX, int hZ, const double* __restrict__ Mz,
-                                const long long* __restrict__ zo)
-{
-  X = zsh(X, zo, ZR_X);
-  Y = zsh(Y, zo, ZR_Y);
-  Z = zsh(Z, zo, ZR_Z);
-  Mz = zsh(Mz, zo, ZR_Z);
-  __shared__ double red[4];
-  const int item = blockIdx.x;
-  const int lane = threadIdx.x & 31;
-  if (item >= W.npairs1b) return;
-  const int i = W.pairs1b[2 * item], j = W.pairs1b[2 * item + 1];
-  const int N = S.norb;
-  const int ji = S.j2[i], jj = S.j2[j];
-  double z = 0.0;
-  for (int c = threadIdx.x; c < N; c += blockDim.x) {
-    const double nc = S.occ[c], nbarc = 1.0 - nc;
-    const bool need_pp = fabs(nc) > 1e-9, need_hh = fabs(nbarc) > 1e-9;
-    const int jc = S.j2[c];
-    const int Jmin = max(abs(jc - ji), abs(jc - jj)) / 2;
-    const int Jmax = (jc + min(ji, jj)) / 2;
-    const int par = (S.l[c] + S.l[i]) & 1, tz = (S.tz2[c] + S.tz2[i]) / 2;
-    const int kci = ket_index(N, min(c, i), max(c, i)), kcj = ket_index(N, min(c, j), max(c, j));
-    for (int J = Jmin; J <= Jmax; ++J) {
-      int r = S.ketJ_loc[J * S.nkets + kci], s = S.ketJ_loc[J * S.nkets + kcj];
-      if (r < 0 || s < 0) continue;
-      int ch = chan_index(J, par, tz);
-      int n = S.ch_n[ch];
-      long long off = S.ch_off[ch];
-      const double* xr = X + off + (long long)r * n;
-      const double* xs = X + off + (long long)s * n;
-      const double* yr = Y + off + (long long)r * n;
-      const double* ys = Y + off + (long long)s * n;
-      const double* w = W.ket_nn + S.ch_kofs[ch];
-      const int* hh = W.hh_list + W.hh_off[ch];
-      const int nhh = W.hh_off[ch + 1] - W.hh_off[ch];
-      double m_rs = 0.0, m_sr = 0.0;
-      for (int t = 0; t < nhh; ++t) {
-        int k = hh[t];
-        double wk = w[k];
-        m_rs = fma(xr[k] * wk, ys[k], m_rs);
-        m_sr = fma(xs[k] * wk, yr[k], m_sr);
-      }
-      if (r == s) m_sr = m_rs;
-      double mhh = hX * (m_rs + hZ * m_sr);
-      double ph = 1.0;
-      if (c > i) ph *= iphase((jc + ji) / 2 + 1 + J);
-      if (c > j) ph *= iphase((jc + jj) / 2 + 1 + J);
-      double nrm = 1.0;
-      if (c == i) nrm *= kSqrt2;
-      if (c == j) nrm *= kSqrt2;
-      double fac = (2 * J + 1) * ph * nrm;
-      if (need_pp) z += fac * nc * (Mz[off + (long long)s * n + r] + mhh);
-      if (need_hh) z += fac * nbarc * mhh;
-    }
-  }
-  z = warp_sum(z);
-  if (lane == 0) red[threadIdx.x >> 5] = z;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    z = red[0] + red[1] + red[2] + red[3];
-    double v = z / (ji + 1.0);
-    Z[32 + (size_t)j * N + i] += v;
-    if (i != j) Z[32 + (size_t)i * N + j] += hZ * v;
   }
 }
 
@@ -1317,48 +1286,40 @@ __global__ void k_norm_onebody(DevSpace S, const double* __restrict__ A, double*
 }
 
 // ------------------------------------------------------------------ launchers
-cudaError_t launch_comm111_110(const Space& s, const double* X, const double* Y, double* Z, bool do111, bool do110,
-                               cudaStream_t st, const long long* zo, int nz)
+cudaError_t launch_zero_gaps(const Space& s, double* Z, cudaStream_t st, const long long* zo, int nz)
 {
-  int threads = s.norb <= 128 ? 128 : 256;
-  k_comm111_110<<<dim3(s.norb, 1, nz), threads, 0, st>>>(s.dev, X, Y, Z, do111, do110, zo);
+  if (s.work.ngaps == 0) return cudaSuccess;
+  k_zero_gaps<<<dim3(s.work.ngaps, 1, nz), 256, 0, st>>>(s.work, Z, zo);
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_comm220(const Space& s, const double* X, const double* Y, double* Z, int hX, cudaStream_t st,
-                           const long long* zo, int nz)
+cudaError_t launch_onebody(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ, int todo,
+                           cudaStream_t st, const long long* zo, int nz)
 {
-  if (s.work.n220 == 0) return cudaSuccess;
-  int wpb = 8;
-  k_comm220<<<dim3((s.work.n220 + wpb - 1) / wpb, 1, nz), 32 * wpb, 0, st>>>(s.dev, s.work, X, Y, Z, hX, zo);
+  const int nt = (s.norb + 15) / 16;
+  const int blocks = (todo & (OB_121 | OB_221) ? s.work.npairs1b : 0) + (todo & (OB_111 | OB_110) ? nt * nt : 0) +
+                     (todo & OB_220 ? s.work.n220 : 0);
+  if (blocks == 0) return cudaSuccess;
+  k_onebody<<<dim3(blocks, 1, nz), kObThreads, 0, st>>>(s.dev, s.work, X, Y, Z, hX, hZ, todo, zo);
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_comm121(const Space& s, const int* dev_holes, const double* X, const double* Y, double* Z,
-                           int hZ, cudaStream_t st, const long long* zo, int nz)
+cudaError_t launch_comm221_z(const Space& s, double* Z, int hZ, const double* Mz, cudaStream_t st, const long long* zo,
+                             int nz)
 {
   if (s.work.npairs1b == 0) return cudaSuccess;
-  int wpb = 4;
-  k_comm121<<<dim3((s.work.npairs1b + wpb - 1) / wpb, 1, nz), 32 * wpb, 0, st>>>(
-      s.dev, s.work, dev_holes, (int)s.holes.size(), X, Y, Z, hZ, zo);
+  k_comm221_z<<<dim3((s.work.npairs1b + 7) / 8, 1, nz), 256, 0, st>>>(s.dev, s.work, Z, hZ, Mz, zo);
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_comm221_1b(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ,
-                              const double* Mz, cudaStream_t st, const long long* zo, int nz)
+cudaError_t launch_comm221_1b(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ, cudaStream_t st)
 {
   if (s.work.n221 == 0) return cudaSuccess;
-  int wpb = 8;
-  if (Mz) {
-    // no other kernel writes Z1 concurrently: plain stores per (i, j) pair
-    k_comm221_1b_mz<<<dim3(s.work.npairs1b, 1, nz), 128, 0, st>>>(s.dev, s.work, X, Y, Z, hX, hZ, Mz, zo);
-    count_launch();
-    return cudaGetLastError();
-  }
-  k_comm221_1b<<<(s.work.n221 + wpb - 1) / wpb, 32 * wpb, 0, st>>>(s.dev, s.work, X, Y, Z, hX, hZ, Mz);
+  const int wpb = 8;
+  k_comm221_1b<<<(s.work.n221 + wpb - 1) / wpb, 32 * wpb, 0, st>>>(s.dev, s.work, X, Y, Z, hX, hZ);
   count_launch();
   return cudaGetLastError();
 }

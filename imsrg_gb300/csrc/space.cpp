@@ -182,6 +182,92 @@ static void build_pandya_fwd(Space& s)
   }
 }
 
+// One-body parts of comm121ss (src/Commutator.cc:670-728) and comm221ss
+// (:1250-1294) for every pair (i <= j) of one one-body channel.  Which
+// elements of X, Y and Mpp - Mhh they read, with what phase, norm, occupation
+// and angular weight, is a property of the space: listed here once, so the
+// kernel does nothing but loads and FMAs.  (Worked out per call, a warp or
+// block a pair, they took 17-52 us each at every size.)
+static void build_onebody(Space& s)
+{
+  const double SQ2 = 1.4142135623730950488;
+  const int N = s.norb;
+  struct El {
+    long long e;
+    double f;
+    int ch, r, s;
+  };
+  // normalised element <ab|O|cd>_J of a scalar operator: arena index and the
+  // phases of the swaps to the kets' order (TwoBodyME::GetTBME_J_norm); f = 0 if none
+  auto elem = [&](int J, int a, int b, int c, int d) {
+    El x{0, 0.0, 0, 0, 0};
+    if (((s.l[a] + s.l[b] + s.l[c] + s.l[d]) & 1) || s.tz2[a] + s.tz2[b] != s.tz2[c] + s.tz2[d] || J >= s.NJ) return x;
+    x.r = s.ketJ_loc[(size_t)J * s.nkets + ket_index(N, std::min(a, b), std::max(a, b))];
+    x.s = s.ketJ_loc[(size_t)J * s.nkets + ket_index(N, std::min(c, d), std::max(c, d))];
+    if (x.r < 0 || x.s < 0) return x;
+    x.ch = chan_index(J, (s.l[a] + s.l[b]) & 1, (s.tz2[a] + s.tz2[b]) / 2);
+    x.e = s.ch[x.ch].off + (long long)x.s * s.ch[x.ch].n() + x.r;
+    x.f = 1.0;
+    if (a > b) x.f *= iphase((s.j2[a] + s.j2[b]) / 2 + 1 + J);
+    if (c > d) x.f *= iphase((s.j2[c] + s.j2[d]) / 2 + 1 + J);
+    return x;
+  };
+  std::vector<int> kofs(s.nch + 1, 0);
+  for (int c = 0; c < s.nch; ++c) kofs[c + 1] = kofs[c] + s.ch[c].n();
+  // w times the monopole sum_J (2J+1) <ab|O|cd>_J / ((2j_a+1)(2j_b+1)), times element u of the other operator
+  auto monopole = [&](double w, int u, int a, int b, int c, int d) {
+    w /= (double)((s.j2[a] + 1) * (s.j2[b] + 1));
+    if (a == b) w *= SQ2;
+    if (c == d) w *= SQ2;
+    for (int J = std::abs(s.j2[a] - s.j2[b]) / 2; J <= (s.j2[a] + s.j2[b]) / 2; ++J) {
+      const El x = elem(J, a, b, c, d);
+      if (x.f != 0.0) s.t121.push_back({x.e, w * (2 * J + 1) * x.f, u, 0});
+    }
+  };
+  for (size_t p = 0; p < s.pairs1b.size(); p += 2) {
+    const int i = s.pairs1b[p], j = s.pairs1b[p + 1];
+    s.ob_off.push_back(make_int3((int)s.t121.size(), (int)s.t221.size(), (int)s.t221z.size()));
+    for (int a : s.holes)
+      for (int k = 0; k < s.ob_count[a]; ++k) {
+        const int b = s.ob_list[s.ob_start[a] + k];
+        const double nanb = s.occ[a] * (1.0 - s.occ[b]);
+        if (std::fabs(nanb) < OCC_CUT) continue;
+        monopole((s.j2[b] + 1) * nanb, 32 + b * N + a, b, i, a, j);
+        monopole(-(s.j2[a] + 1) * nanb, 32 + a * N + b, a, i, b, j);
+      }
+    for (int c = 0; c < N; ++c) {
+      const double nc = s.occ[c], nbar = 1.0 - nc;
+      const double wz = std::fabs(nc) > 1e-9 ? nc : 0.0, wh = wz + (std::fabs(nbar) > 1e-9 ? nbar : 0.0);
+      const int Jmin = std::max(std::abs(s.j2[c] - s.j2[i]), std::abs(s.j2[c] - s.j2[j])) / 2;
+      const int Jmax = (s.j2[c] + std::min(s.j2[i], s.j2[j])) / 2;
+      for (int J = Jmin; J <= Jmax; ++J) {
+        const El x = elem(J, c, i, c, j);
+        if (x.f == 0.0) continue;
+        double f = (2 * J + 1) * x.f / (s.j2[i] + 1.0);
+        if (c == i) f *= SQ2;
+        if (c == j) f *= SQ2;
+        const Chan& C = s.ch[x.ch];
+        const int nhh = s.hh_off[x.ch + 1] - s.hh_off[x.ch];
+        if (wh != 0.0 && nhh)
+          s.t221.push_back({C.off + (long long)x.r * C.n(), C.off + (long long)x.s * C.n(), wh * f, s.hh_off[x.ch], nhh, kofs[x.ch], 0});
+        if (wz != 0.0) s.t221z.push_back({x.e, wz * f});
+      }
+    }
+  }
+  s.ob_off.push_back(make_int3((int)s.t121.size(), (int)s.t221.size(), (int)s.t221z.size()));
+  // the arena but for the blocks the ladder product overwrites (pieces of at
+  // most 4096, one block of the zeroing kernel each)
+  std::vector<std::pair<int64_t, int64_t>> written;
+  for (const SymGemmJob& j : s.ladder_jobs) written.push_back({j.out_off, j.out_off + (int64_t)j.m * j.m});
+  std::sort(written.begin(), written.end());
+  written.push_back({s.arena, s.arena});
+  int64_t at = 0;
+  for (auto& w : written) {
+    for (; at < w.first; at += 4096) s.gaps.push_back({at, std::min<int64_t>(4096, w.first - at)});
+    at = w.second;
+  }
+}
+
 Space* build_space(int emax, const std::vector<int>& n, const std::vector<int>& l, const std::vector<int>& j2,
                    const std::vector<int>& tz2, const std::vector<double>& occ)
 {
@@ -378,6 +464,7 @@ Space* build_space(int emax, const std::vector<int>& n, const std::vector<int>& 
         s.items221.push_back(c);
       }
     }
+  build_onebody(s);
   // comm122ss gathers (src/Commutator.cc:862-903)
   const double SQ2 = 1.4142135623730950488;
   for (int c = 0; c < s.nch; ++c) {
@@ -476,6 +563,12 @@ void upload_space(Space& s)
 
   DevWork& w = s.work;
   w.ket_wpp = dev_copy(s, s.ket_wpp);
+  w.t121 = dev_copy(s, s.t121);
+  w.t221 = dev_copy(s, s.t221);
+  w.t221z = dev_copy(s, s.t221z);
+  w.ob_off = dev_copy(s, s.ob_off);
+  w.gaps = dev_copy(s, s.gaps);
+  w.ngaps = (int)s.gaps.size();
   w.ket_nn = dev_copy(s, s.ket_nn);
   w.hh_off = dev_copy(s, s.hh_off);
   w.hh_list = dev_copy(s, s.hh_list);

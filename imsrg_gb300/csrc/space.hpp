@@ -78,6 +78,11 @@ struct Space {
   std::vector<double> ket_wpp, ket_nn;  // per 2b channel ket (flat, channel-major): Mpp / Mhh weights
   std::vector<int> hh_off, hh_list;     // per 2b channel: local indices of its hh kets
   std::vector<int> items220;            // (ch, hh local) pairs, flattened
+  std::vector<T121> t121;               // one-body parts of comm121ss and comm221ss, by pair
+  std::vector<T221> t221;
+  std::vector<T221Z> t221z;
+  std::vector<int3> ob_off;
+  std::vector<longlong2> gaps;          // arena ranges the ladder product does not write
   std::vector<int> pairs1b;             // (i, j), i <= j in one one-body channel, flattened
   std::vector<int> items221;            // (i, j, c), flattened
   std::vector<int> cols122;             // (ch, column, first item, item count), flattened

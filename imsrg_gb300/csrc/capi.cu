@@ -79,6 +79,11 @@ T* dcopy(const std::vector<T>& v)
 
 namespace imsrg {
 int set_error(int code, const char* msg) { return fail(code, msg); }
+bool capturing(cudaStream_t st)
+{
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
 }  // namespace imsrg
 
 // struct imsrg_space / imsrg_op: capi_internal.hpp
@@ -625,12 +630,6 @@ int ensure_split(imsrg_space* sp)
     return fail(IMSRG_ERR_NOMEM, std::string("split-precision plan: ") + e.what());
   }
   return IMSRG_OK;
-}
-
-bool capturing(cudaStream_t st)
-{
-  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
 
 // the plan in *slot, made on first use outside a capture; null where it

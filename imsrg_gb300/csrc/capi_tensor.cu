@@ -2,8 +2,8 @@
 // Commutator::CommutatorScalarTensor (src/Commutator.cc:432-500) and its
 // IMSRG(2) terms on device operators.  X is a scalar operator, Y and Z are
 // reduced tensors of the same rank (imsrg_op_create_tensor).  The ladder and
-// Z bar products run in FP64 on the CUDA cores, or in the split form on the
-// tensor cores (plain rectangular split products, kernels_split.cu).
+// Z bar products run on the tensor cores as plain rectangular products: to
+// FP64 accuracy (kernels_dgemm.cu), or in the split form (kernels_split.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -68,8 +68,8 @@ int scratch(imsrg_space* sp, TensorLayout* tl)
   return IMSRG_OK;
 }
 
-// ---------------------------------------------------------- split form
-// plain split products of the ladder: term 1, D = Xb w Yc (A = X of the bra
+// ---------------------------------------------------------- products
+// plain products of the ladder: term 1, D = Xb w Yc (A = X of the bra
 // channel gathered by its ladder list, B = Y's block transposed), overwrite;
 // term 2, D -= Yc w Xk (A = Y's block gathered by the ket channel's list,
 // B = Xk, taken as hX Xk^T: the launch scale is hX), accumulate
@@ -109,7 +109,7 @@ std::vector<GemmJobDev> ladder_jobs(const Space& s, const TensorLayout& t, int t
   return v;
 }
 
-// plain split products of Z bar (lo, hi) = M_left M_right, columns [0, n_hi)
+// plain products of Z bar (lo, hi) = M_left M_right, columns [0, n_hi)
 // (head) and [n_hi, 2 n_hi) (tail), src/TensorCommutators.cc:1130-1190:
 // part 1, K over the 2 nph_lo rows of X bar (lo): A = X bar (lo), B = the
 // transposed panel Ybar(lo, hi) (head) or its half-swapped copy (tail, which
@@ -159,15 +159,24 @@ std::vector<GemmJobDev> zbar_jobs(const Space& s, const TensorLayout& t, int par
   return v;
 }
 
-int split_ready(imsrg_space* sp, TensorLayout* tl)
+// scratch of the product operands (Y transposed, Pandya panels), both forms
+int product_scratch(imsrg_space* sp, TensorLayout* tl)
 {
   int rc = scratch(sp, tl);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(sp->mu);
-  const Space& s = *sp->s;
-  if ((rc = alloc(tl, tl->d_ybt, tl->yb_total)) ||
-      (rc = alloc(tl, tl->d_ybtf, tl->yb_total)) || (rc = alloc(tl, tl->d_xbf, s.xb_total)))
+  if ((rc = alloc(tl, tl->d_ybt, tl->yb_total)) || (rc = alloc(tl, tl->d_ybtf, tl->yb_total)) ||
+      (rc = alloc(tl, tl->d_xbf, sp->s->xb_total)))
     return rc;
+  return IMSRG_OK;
+}
+
+int split_ready(imsrg_space* sp, TensorLayout* tl)
+{
+  int rc = product_scratch(sp, tl);
+  if (rc) return rc;
+  std::lock_guard<std::mutex> g(sp->mu);
+  const Space& s = *sp->s;
   try {
     if (!tl->sp_lad1) tl->sp_lad1 = split_plan_create(s, ladder_jobs(s, *tl, 1), 0);
     if (!tl->sp_lad2) tl->sp_lad2 = split_plan_create(s, ladder_jobs(s, *tl, 2), 0);
@@ -179,8 +188,35 @@ int split_ready(imsrg_space* sp, TensorLayout* tl)
   return IMSRG_OK;
 }
 
-// X bar and the split products' operands (Y transposed, Pandya panels)
-int split_operands(const imsrg_op* X, const imsrg_op* Y, cudaStream_t st)
+// the FP64 form's product plans, made on first use outside a capture; false
+// where they cannot be (the FP64-pipe kernels run then).  Rank (1, 1, +) at
+// emax 6: 0.45 ms for the ladder and Z bar products, slicing included, against
+// 1.58 ms with the FP64-pipe kernels
+bool fp64_ready(imsrg_space* sp, TensorLayout* tl, cudaStream_t st)
+{
+  if (!tl->dg_tried && !capturing(st)) {
+    if (product_scratch(sp, tl) != IMSRG_OK) return false;
+    std::lock_guard<std::mutex> g(sp->mu);
+    const Space& s = *sp->s;
+    DgemmPlan* p[4] = {};
+    tl->dg_tried = true;
+    try {
+      for (int k = 0; k < 4; ++k)
+        p[k] = k < 2 ? dgemm_plan_create(ladder_jobs(s, *tl, k + 1), 0) : dgemm_plan_create(zbar_jobs(s, *tl, k - 1), 1);
+    } catch (std::exception&) {
+      for (DgemmPlan* q : p) dgemm_plan_destroy(q);
+      return false;
+    }
+    tl->dg_lad1 = p[0];
+    tl->dg_lad2 = p[1];
+    tl->dg_zb1 = p[2];
+    tl->dg_zb2 = p[3];
+  }
+  return tl->dg_zb2 != nullptr;
+}
+
+// X bar and the products' operands (Y transposed, Pandya panels)
+int product_operands(const imsrg_op* X, const imsrg_op* Y, cudaStream_t st)
 {
   TensorLayout* tl = Y->tl;
   const Space& s = *X->sp->s;
@@ -190,32 +226,38 @@ int split_operands(const imsrg_op* X, const imsrg_op* Y, cudaStream_t st)
   return IMSRG_OK;
 }
 
-int t222_split(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
+// one of the four plain products in either form
+cudaError_t product(imsrg_space* sp, SplitPlan* split, const DgemmPlan* fp64, int prec, const double* A, const double* B0,
+                    const double* B1, double* O, double scale, cudaStream_t st)
+{
+  const DevWork& w = sp->s->work;
+  if (prec == IMSRG_PREC_FP64)
+    return launch_dgemm(fp64, A, B0, B1, O, w.kidx, w.kweight, w.phase_tab, 1, scale, -1, true, st);
+  return launch_symgemm_split(split, A, B0, B1, O, w.kidx, w.kweight, w.phase_tab, sp->d_status, 1, scale, st);
+}
+
+int t222_product(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st)
 {
   TensorLayout* tl = Y->tl;
   const Space& s = *X->sp->s;
   ProfScope ps("comm222_pp_hh_221st", st);
   T_CUDA(cudaMemsetAsync(tl->d_mpp, 0, std::max<long long>(1, tl->total) * sizeof(double), st));
-  T_CUDA(launch_symgemm_split(tl->sp_lad1, X->d, tl->d_yt, tl->d_yt, tl->d_mpp, s.work.kidx, s.work.kweight,
-                              s.work.phase_tab, X->sp->d_status, 1, 1.0, st));
-  T_CUDA(launch_symgemm_split(tl->sp_lad2, Y->d, X->d, X->d, tl->d_mpp, s.work.kidx, s.work.kweight,
-                              s.work.phase_tab, X->sp->d_status, 1, (double)X->herm, st));
+  T_CUDA(product(X->sp, tl->sp_lad1, tl->dg_lad1, prec, X->d, tl->d_yt, tl->d_yt, tl->d_mpp, 1.0, st));
+  T_CUDA(product(X->sp, tl->sp_lad2, tl->dg_lad2, prec, Y->d, X->d, X->d, tl->d_mpp, (double)X->herm, st));
   T_CUDA(launch_tensor_222_221_split(s, *tl, X->d, Y->d, tl->d_mpp, tl->d_mhh, Z->d, Z->herm, st));
   return IMSRG_OK;
 }
 
-int tph_split(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st)
+int tph_product(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st)
 {
   TensorLayout* tl = Y->tl;
   const Space& s = *X->sp->s;
   ProfScope ps("comm222_phst", st);
   T_CUDA(cudaMemsetAsync(tl->d_zbar, 0, std::max<long long>(1, tl->zb_total) * sizeof(double), st));
-  T_CUDA(launch_symgemm_split(tl->sp_zb1, tl->d_xbar, tl->d_ybt, tl->d_ybtf, tl->d_zbar, s.work.kidx,
-                              s.work.kweight, s.work.phase_tab, X->sp->d_status, 1, 1.0, st));
-  T_CUDA(launch_symgemm_split(tl->sp_zb2, tl->d_ybt, tl->d_xbar, tl->d_xbf, tl->d_zbar, s.work.kidx,
-                              s.work.kweight, s.work.phase_tab, X->sp->d_status, 1, (double)(X->herm * Y->herm),
-                              st));
-  T_CUDA(launch_tensor_inverse_pandya(s, *tl, tl->d_zbar, Z->d, Z->herm, st));
+  T_CUDA(product(X->sp, tl->sp_zb1, tl->dg_zb1, prec, tl->d_xbar, tl->d_ybt, tl->d_ybtf, tl->d_zbar, 1.0, st));
+  T_CUDA(product(X->sp, tl->sp_zb2, tl->dg_zb2, prec, tl->d_ybt, tl->d_xbar, tl->d_xbf, tl->d_zbar,
+                 (double)(X->herm * Y->herm), st));
+  T_CUDA(launch_tensor_inverse_pandya(s, *tl, tl->d_zbar, Z->d, Z->herm, prec == IMSRG_PREC_SPLIT, st));
   return IMSRG_OK;
 }
 
@@ -312,10 +354,12 @@ int imsrg_comm222_pp_hh_221st(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z,
   int rc = check_st(X, Y, Z);
   if (rc || (rc = check_prec(precision))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == IMSRG_PREC_FP64) return t222(X, Y, Z, st);
-  if ((rc = split_ready(X->sp, Y->tl)) || (rc = split_operands(X, Y, st)) || (rc = t222_split(X, Y, Z, st)))
+  const bool split = precision == IMSRG_PREC_SPLIT;
+  if (!split && !fp64_ready(X->sp, Y->tl, st)) return t222(X, Y, Z, st);
+  if ((split && (rc = split_ready(X->sp, Y->tl))) || (rc = product_operands(X, Y, st)) ||
+      (rc = t222_product(X, Y, Z, precision, st)))
     return rc;
-  return end_status(X->sp, st);
+  return split ? end_status(X->sp, st) : IMSRG_OK;
 }
 
 int imsrg_comm222_phst(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int precision, void* stream)
@@ -323,10 +367,12 @@ int imsrg_comm222_phst(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int pr
   int rc = check_st(X, Y, Z);
   if (rc || (rc = check_prec(precision))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == IMSRG_PREC_FP64) return tph(X, Y, Z, st);
-  if ((rc = split_ready(X->sp, Y->tl)) || (rc = split_operands(X, Y, st)) || (rc = tph_split(X, Y, Z, st)))
+  const bool split = precision == IMSRG_PREC_SPLIT;
+  if (!split && !fp64_ready(X->sp, Y->tl, st)) return tph(X, Y, Z, st);
+  if ((split && (rc = split_ready(X->sp, Y->tl))) || (rc = product_operands(X, Y, st)) ||
+      (rc = tph_product(X, Y, Z, precision, st)))
     return rc;
-  return end_status(X->sp, st);
+  return split ? end_status(X->sp, st) : IMSRG_OK;
 }
 
 int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int precision, void* stream)
@@ -346,15 +392,15 @@ int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_o
   if ((on[0] && (rc = t111(X, Y, Z, st))) || (on[1] && (rc = t121(X, Y, Z, st))) ||
       (on[2] && (rc = t122(X, Y, Z, st))))
     return rc;
-  if (precision == IMSRG_PREC_FP64) {
+  if (!on[3] && !on[4]) return IMSRG_OK;
+  if (precision == IMSRG_PREC_FP64 && !fp64_ready(X->sp, Y->tl, st)) {
     if ((on[3] && (rc = t222(X, Y, Z, st))) || (on[4] && (rc = tph(X, Y, Z, st)))) return rc;
-  } else if (on[3] || on[4]) {
-    if ((rc = split_operands(X, Y, st)) || (on[3] && (rc = t222_split(X, Y, Z, st))) ||
-        (on[4] && (rc = tph_split(X, Y, Z, st))))
-      return rc;
-    return end_status(X->sp, st);
+    return IMSRG_OK;
   }
-  return IMSRG_OK;
+  if ((rc = product_operands(X, Y, st)) || (on[3] && (rc = t222_product(X, Y, Z, precision, st))) ||
+      (on[4] && (rc = tph_product(X, Y, Z, precision, st))))
+    return rc;
+  return precision == IMSRG_PREC_SPLIT ? end_status(X->sp, st) : IMSRG_OK;
 }
 
 }  // extern "C"

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 
+#include "dfloat.cuh"
 #include "kernels.cuh"
 #include "prof.hpp"
 #include "tensor.hpp"
@@ -757,156 +758,223 @@ __global__ void k_tzbar(DevSpace S, DevWork W, DevTensor T, const double* __rest
   Zb[T.zb_off[p] + (long long)col * nlo + r] = s;
 }
 
-// Zbar(al | kb) at (J3, J4) as the inverse transform reads it: the element's
-// place and phase follow the reference's four cases (src/TensorCommutators.cc:
-// 830-852); 0 when the Zbar block is not stored
-__device__ __forceinline__ double zbar_val(const DevSpace& S, const DevTensor& T, const double* Zb, int hZ, int a,
-                                           int b, int k, int l, int J3, int J4)
+// What the Zbar values Zbar_(J3, J4)(a l, k b) of one sum have in common: the
+// global indices of their cross-coupled kets, the parity / |dTz| parts of their
+// channels, the orders of their orbits and (-1)^(j_a + j_b + j_k + j_l)
+struct ZbarKets {
+  int il, kj;
+  int code;  // bra class (0..5) | ket class << 4 | a > l << 8 | k > b << 9 | phase << 10
+};
+
+__device__ __forceinline__ ZbarKets zbar_kets(const DevSpace& S, int a, int b, int k, int l)
 {
-  const int pbc = (S.l[a] + S.l[l]) & 1, pkc = (S.l[k] + S.l[b]) & 1;
-  const int tbc = abs(S.tz2[a] - S.tz2[l]) / 2, tkc = abs(S.tz2[k] - S.tz2[b]) / 2;
-  const int cbra = chan_index(J3, pbc, tbc), cket = chan_index(J4, pkc, tkc);
-  const int lo = min(cbra, cket), hi = max(cbra, cket);
-  const long long off = T.zb_lookup[lo * S.nch + hi];
+  ZbarKets z;
+  z.il = ket_index(S.norb, min(a, l), max(a, l));
+  z.kj = ket_index(S.norb, min(b, k), max(b, k));
+  const int cb = chan_index(0, (S.l[a] + S.l[l]) & 1, abs(S.tz2[a] - S.tz2[l]) / 2);
+  const int ck = chan_index(0, (S.l[k] + S.l[b]) & 1, abs(S.tz2[k] - S.tz2[b]) / 2);
+  z.code = cb | ck << 4 | (a > l) << 8 | (k > b) << 9 | (((S.j2[a] + S.j2[b] + S.j2[k] + S.j2[l]) >> 1) & 1) << 10;
+  return z;
+}
+
+// the value at (J3, J4), times (-1)^odd: its place and phase follow the
+// reference's four cases (src/TensorCommutators.cc:830-852); 0 when the Zbar
+// block is not stored
+__device__ __forceinline__ double zbar_val(const DevSpace& S, const DevTensor& T, const double* Zb, int hZ, const ZbarKets& z,
+                                           int J3, int J4, int odd)
+{
+  const int cbra = 6 * J3 + (z.code & 15), cket = 6 * J4 + ((z.code >> 4) & 15);
+  const bool up = cbra <= cket;
+  const int lo = up ? cbra : cket, hi = up ? cket : cbra;
+  const long long off = __ldg(T.zb_lookup + lo * S.nch + hi);
+  const int il = __ldg(S.ccJ_loc + J3 * S.nkets + z.il), kj = __ldg(S.ccJ_loc + J4 * S.nkets + z.kj);
+  const int nrow = __ldg(S.cc_n + lo), ncol = __ldg(S.cc_n + hi);
   if (off < 0) return 0.0;
-  const int ixil = S.ccJ_loc[J3 * S.nkets + ket_index(S.norb, min(a, l), max(a, l))];
-  const int ixkj = S.ccJ_loc[J4 * S.nkets + ket_index(S.norb, min(b, k), max(b, k))];
-  const double* M = Zb + off;
-  const int nrow = S.cc_n[lo];
-  const int sum4 = (S.j2[a] + S.j2[b] + S.j2[k] + S.j2[l]) >> 1, hneg = hZ < 0;
-  if (cbra <= cket) {
-    if (a <= l) return M[(long long)(ixkj + (k > b ? S.cc_n[cket] : 0)) * nrow + ixil];
-    return flip(M[(long long)(ixkj + (k > b ? 0 : S.cc_n[cket])) * nrow + ixil], hneg + J3 - J4 + sum4);
-  }
-  if (k <= b) return flip(M[(long long)(ixil + (a > l ? S.cc_n[cbra] : 0)) * nrow + ixkj], hneg + J3 - J4);
-  return flip(M[(long long)(ixil + (a > l ? 0 : S.cc_n[cbra])) * nrow + ixkj], sum4);
-}
-
-// the Zbar values one sum of the inverse transform reads for the quadruple
-// (a, b, k, l): slot (J3 - J3min) w + (J4 - J3 + lam), lanes over slots
-__device__ __forceinline__ void tinv_gather(const DevSpace& S, const DevTensor& T, const double* Zb, int hZ, int a,
-                                            int b, int k, int l, double* in, int lane)
-{
-  const int ja = S.j2[a], jb = S.j2[b], jk = S.j2[k], jl = S.j2[l], Lam = T.lam, w = 2 * Lam + 1;
-  const int J3min = abs(ja - jl) >> 1, nJ3 = ((ja + jl) >> 1) - J3min + 1;
-  const int J4lo = abs(jk - jb) >> 1, J4hi = (jk + jb) >> 1;
-  for (int s = lane; s < nJ3 * w; s += 32) {
-    const int J3 = J3min + s / w, J4 = J3 - Lam + s % w;
-    in[s] = (J4 < J4lo || J4 > J4hi) ? 0.0 : zbar_val(S, T, Zb, hZ, a, b, k, l, J3, J4);
-  }
-}
-
-// one sum over the gathered values: sum_{J3, J4} hat 9j (-1)^(jb + jl + J2 + J4)
-// Zbar (the 9j {ja jb J1; ...} row of (J1, J2))
-__device__ __forceinline__ double tinv_dot(const DevSpace& S, const DevTensor& T, int a, int b, int k, int l, int J1,
-                                           int J2, const double* in)
-{
-  const int ja = S.j2[a], jb = S.j2[b], jk = S.j2[k], jl = S.j2[l], Lam = T.lam, w = 2 * Lam + 1;
-  const NineJRow nj = ninej_row(T, ja, jb, jk, jl, J1, J2);
-  if (!nj.p) return 0.0;
-  // the row's J1 window is this sum's J3 range (both |ja - jl| .. ja + jl),
-  // and J4 - J3 + lam stays in [0, w): every slot below is in the table
-  const int J3min = abs(ja - jl) >> 1, J3max = (ja + jl) >> 1;
-  const int J4lo = abs(jk - jb) >> 1, J4hi = (jk + jb) >> 1;
-  const long long st = nj.stride;
-  double acc = 0.0;
-  for (int J3 = J3min; J3 <= J3max; ++J3) {
-    const int J4min = max(J4lo, abs(J3 - Lam)), J4max = min(J4hi, J3 + Lam);
-    if (J4min > J4max) continue;
-    long long k9 = ((long long)(J3 - J3min) * w + (J4min - J3 + Lam)) * st;
-    int e = (J3 - J3min) * w + (J4min - J3 + Lam);
-    int odd = ((jb + jl) >> 1) + J2 + J4min;
-    // the table's zeros (the reference's skipped terms) add exactly 0: no
-    // branch, so the loads of consecutive terms can be in flight together
-    for (int J4 = J4min; J4 <= J4max; ++J4, k9 += st, ++e, ++odd) acc = fma(flip(nj.p[k9], odd), in[e], acc);
-  }
-  return acc;
+  const bool al = (z.code >> 8) & 1, kb = (z.code >> 9) & 1;
+  // stored with the smaller channel's ket as row; a swapped row pair moves the
+  // column to the other half and brings the ket phases
+  const bool swap = up ? al : kb, tail = up ? kb : al;
+  const int r = up ? il : kj, c = (up ? kj : il) + (tail != swap ? ncol : 0);
+  if (swap != !up) odd += (hZ < 0) + J3 - J4;
+  if (swap) odd += z.code >> 10;
+  return flip(__ldg(Zb + off + (long long)c * nrow + r), odd);
 }
 
 // Inverse tensor Pandya transform by orbit quadruple (AddInverseTensor-
-// PandyaTransformation, src/TensorCommutators.cc:754-920): a warp per (i <= j,
-// k <= l) of the layout's quadruple list.  The Zbar values of both sums (over
-// J3, J4) are gathered once into shared memory; then the lanes take the
-// (J1, J2) slots whose element the quadruple owns (a stored block, the upper
-// triangle of a diagonal one) and sum over them.  Each stored element is owned
-// by exactly one quadruple and slot, so there are no write conflicts.
-constexpr int kTqWarps = 8;
+// PandyaTransformation, src/TensorCommutators.cc:754-920): z(J1, J2) of a
+// quadruple (i <= j, k <= l) is two sums over (J3, J4) of the hat-weighted 9j
+// times Zbar values that do not depend on (J1, J2).  A block takes a batch of
+// quadruples of one class (j_i, j_j, j_k, j_l), which share the 9j matrix:
+//   1. the Zbar values of both sums, all quadruples, into shared memory, with
+//      the signs that do not depend on (J1, J2);
+//   2. a thread per (J1, J2) slot and four quadruples: one 9j load (lanes run
+//      over slots, consecutive in the table) serves four FMAs, and loop and
+//      index work is shared by them;
+//   3. each result whose element the quadruple owns (a stored block, the
+//      upper triangle of a diagonal one; exactly one quadruple owns each)
+//      updates Z.
+// DF: the sums in double-float on the FP32 pipe, each quadruple's values
+// scaled by their largest exponent; else in FP64, bound by its pipe.
+// A warp per quadruple and FP64 sums took 6.43 ms at emax 8, rank (2, 0, +),
+// and 1.00 ms at emax 6, rank (1, 1, +); this takes 2.70 ms (DF) and 0.31 ms
+// (FP64).
+constexpr int kTqThreads = 256;
 
-__global__ void __launch_bounds__(32 * kTqWarps, 6) k_tinv_q(DevSpace S, DevTensor T, const double* __restrict__ Zb,
-                                                         int hZ, double* __restrict__ Z,
-                                                         const int2* __restrict__ tq, long long nq, int slots)
+// floor(x / n) for 0 <= x < 2^16, 1 <= n <= 128 and r = 1.0f / n: (x + 1/2) / n is
+// at least 1 / 256 from an integer, more than the product rounds by (checked over the range)
+__device__ __forceinline__ int small_div(int x, float r) { return __float2int_rz(__fmul_rn((float)x + 0.5f, r)); }
+
+template <bool DF>
+__global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
+                                                       double* __restrict__ Z, const int2* __restrict__ tq,
+                                                       const int2* __restrict__ batches)
 {
-  extern __shared__ double s_in[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long qi = blockIdx.x * (long long)kTqWarps + warp;
-  if (qi >= nq) return;
-  // per warp: the two sums' gathered values, then the owned output slots
-  double* in1 = s_in + (size_t)warp * 3 * slots;
-  double* in2 = in1 + slots;
-  int* own = reinterpret_cast<int*>(in2 + slots);
-  const int2 v = tq[qi];
-  const int i = v.x & 0xFFFF, j = v.x >> 16, k = v.y & 0xFFFF, l = v.y >> 16;
-  tinv_gather(S, T, Zb, hZ, i, j, k, l, in1, lane);
-  if (i != j) tinv_gather(S, T, Zb, hZ, j, i, k, l, in2, lane);
-  __syncwarp();
-  const int ji = S.j2[i], jj = S.j2[j], jk = S.j2[k], jl = S.j2[l], Lam = T.lam, w = 2 * Lam + 1;
-  const int pb = (S.l[i] + S.l[j]) & 1, tb = (S.tz2[i] + S.tz2[j]) / 2;
-  const int pk = (S.l[k] + S.l[l]) & 1, tk = (S.tz2[k] + S.tz2[l]) / 2;
-  const int kb = ket_index(S.norb, i, j), kk = ket_index(S.norb, k, l);
-  const int J1min = abs(ji - jj) >> 1, nJ1 = ((ji + jj) >> 1) - J1min + 1;
-  const int J2lo = abs(jk - jl) >> 1, J2hi = (jk + jl) >> 1;
-  // the slots this quadruple owns, compacted (ballot) so every lane of the
-  // sums below has one
-  int nown = 0;
-  for (int c0 = 0; c0 < nJ1 * w; c0 += 32) {
-    const int t = c0 + lane;
-    bool ok = false;
-    if (t < nJ1 * w) {
-      const int J1 = J1min + t / w, J2 = J1 - Lam + t % w;
-      if (J2 >= J2lo && J2 <= J2hi && J1 < S.NJ && J2 < S.NJ) {
-        const int ib = S.ketJ_loc[J1 * S.nkets + kb], ik = S.ketJ_loc[J2 * S.nkets + kk];
-        const int chb = chan_index(J1, pb, tb), chk = chan_index(J2, pk, tk);
-        ok = ib >= 0 && ik >= 0 && !(chb > chk || (chb == chk && ik < ib)) && T.lookup[chb * S.nch + chk] >= 0;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* in = (double*)smem;  // [value of sum 1, then of sum 2][quadruple]
+  __shared__ int2 s_q[kTqBatch];
+  __shared__ ZbarKets s_z[2][kTqBatch];
+  __shared__ int s_e[kTqBatch];
+  const int tid = threadIdx.x;
+  const int2 bt = batches[blockIdx.x];
+  const int nq = bt.y, QP = (nq + 3) & ~3;
+  if (tid < QP) {
+    const int2 v = tq[bt.x + min(tid, nq - 1)];
+    const int i = v.x & 0xFFFF, j = v.x >> 16, k = v.y & 0xFFFF, l = v.y >> 16;
+    s_q[tid] = v;
+    s_z[0][tid] = zbar_kets(S, i, j, k, l);
+    s_z[1][tid] = zbar_kets(S, j, i, k, l);
+    s_e[tid] = 0;
+  }
+  __syncthreads();
+  const int ji = S.j2[s_q[0].x & 0xFFFF], jj = S.j2[s_q[0].x >> 16], jk = S.j2[s_q[0].y & 0xFFFF], jl = S.j2[s_q[0].y >> 16];
+  const int Lam = T.lam, w = 2 * Lam + 1;
+  // sum 1 reads (i, j, k, l), sum 2 (j, i, k, l): J3 from lo3, n3 values; J4 in [lo4, hi4]
+  const int lo3[2] = {abs(ji - jl) >> 1, abs(jj - jl) >> 1};
+  const int n3[2] = {((ji + jl) >> 1) - lo3[0] + 1, ((jj + jl) >> 1) - lo3[1] + 1};
+  const int lo4[2] = {abs(jk - jj) >> 1, abs(jk - ji) >> 1}, hi4[2] = {(jk + jj) >> 1, (jk + ji) >> 1};
+  const int nval = (n3[0] + n3[1]) * w;
+  const float rq = 1.0f / QP, rw = 1.0f / w;  // exact quotients of the small indices below
+  for (int e = tid; e < nval * QP; e += kTqThreads) {
+    int v = small_div(e, rq);
+    const int q = e - v * QP, sum = v >= n3[0] * w;
+    if (sum) v -= n3[0] * w;
+    const int a = small_div(v, rw), J3 = lo3[sum] + a, J4 = J3 - Lam + v - a * w;
+    double x = 0.0;
+    if (q < nq && J4 >= lo4[sum] && J4 <= hi4[sum])
+      x = zbar_val(S, T, Zb, hZ, s_z[sum][q], J3, J4, (((sum ? ji : jj) + jl) >> 1) + J4);
+    in[e] = x;
+    if (DF) {
+      const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
+      if (ex) atomicMax(&s_e[q], ex);
+    }
+  }
+  __syncthreads();
+  if (DF) {
+    // v 2^(1023 - e) of the quadruple's largest exponent e, as float pairs in place
+    for (int e = tid; e < nval * QP; e += kTqThreads) {
+      const long long b = __double_as_longlong(in[e]);
+      const int ex = (int)((b >> 52) & 0x7FF), es = ex - s_e[e - small_div(e, rq) * QP] + 1023;
+      const double x = ex == 0x7FF ? in[e] : ex == 0 || es <= 0 ? 0.0 : __longlong_as_double((b & ~(0x7FFll << 52)) | ((long long)es << 52));
+      ((float2*)in)[e] = d2ff(x);
+    }
+    __syncthreads();
+  }
+  const int J1min = abs(ji - jj) >> 1, nslot = (((ji + jj) >> 1) - J1min + 1) * w;
+  const int d1 = T.d1, ci = (ji - 1) >> 1, cj = (jj - 1) >> 1, ck = (jk - 1) >> 1, cl = (jl - 1) >> 1;
+  const long long base[2] = {T.nj_base[((ci * d1 + cj) * d1 + ck) * d1 + cl], T.nj_base[((cj * d1 + ci) * d1 + ck) * d1 + cl]};
+  // only J2 >= J1: an element with J1 > J2 has its bra channel above its ket
+  // channel, and is stored as its conjugate (another quadruple's)
+  const int nown = nslot / w * (Lam + 1);
+  for (int x = tid; x < nown * (QP >> 2); x += kTqThreads) {
+    const int g4 = x / nown, y = x - g4 * nown, a = y / (Lam + 1), q0 = 4 * g4;
+    const int J1 = J1min + a, J2 = J1 + y - a * (Lam + 1), t = a * w + Lam + J2 - J1;
+    double sum[2][4];
+    if (J2 < (abs(jk - jl) >> 1) || J2 > ((jk + jl) >> 1) || J1 >= S.NJ || J2 >= S.NJ) continue;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
+      double sd[4] = {0.0, 0.0, 0.0, 0.0};
+      const int v0 = u ? n3[0] * w : 0;
+      for (int a = 0; a < n3[u]; ++a) {
+        const int J3 = lo3[u] + a;
+        const int b0 = max(lo4[u], abs(J3 - Lam)) - J3 + Lam, b1 = min(hi4[u], J3 + Lam) - J3 + Lam;
+        for (int b = b0; b <= b1; ++b) {
+          const int v = a * w + b;
+          if (DF) {
+            const float2 c = __ldg(T.nj_hatf + base[u] + (long long)v * nslot + t);
+            const float4* y = (const float4*)((const float2*)in + (v0 + v) * QP + q0);
+            const float4 y0 = y[0], y1 = y[1];
+            df_fma(c, make_float2(y0.x, y0.y), sh[0], sl[0]);
+            df_fma(c, make_float2(y0.z, y0.w), sh[1], sl[1]);
+            df_fma(c, make_float2(y1.x, y1.y), sh[2], sl[2]);
+            df_fma(c, make_float2(y1.z, y1.w), sh[3], sl[3]);
+          } else {
+            const double c = __ldg(T.nj_hat + base[u] + (long long)v * nslot + t);
+            const double2* y = (const double2*)(in + (v0 + v) * QP + q0);
+            const double2 y0 = y[0], y1 = y[1];
+            sd[0] = fma(c, y0.x, sd[0]);
+            sd[1] = fma(c, y0.y, sd[1]);
+            sd[2] = fma(c, y1.x, sd[2]);
+            sd[3] = fma(c, y1.y, sd[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        if (DF) {
+          const float hi = __fadd_rn(sh[h], sl[h]);
+          sum[u][h] = ff2d(hi, __fsub_rn(sl[h], __fsub_rn(hi, sh[h])));
+        } else {
+          sum[u][h] = sd[h];
+        }
       }
     }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (ok) own[nown + __popc(m & ((1u << lane) - 1))] = t;
-    nown += __popc(m);
-  }
-  __syncwarp();
-  for (int x = lane; x < nown; x += 32) {
-    const int t = own[x];
-    const int J1 = J1min + t / w, J2 = J1 - Lam + t % w;
-    const int ib = S.ketJ_loc[J1 * S.nkets + kb], ik = S.ketJ_loc[J2 * S.nkets + kk];
-    const int chb = chan_index(J1, pb, tb), chk = chan_index(J2, pk, tk);
-    const int blk = T.lookup[chb * S.nch + chk];
-    const double commij = tinv_dot(S, T, i, j, k, l, J1, J2, in1);
-    const double commji = i == j ? commij : tinv_dot(S, T, j, i, k, l, J1, J2, in2);
-    const double z = unnorm(commij + flip(commji, 1 + ((ji + jj) >> 1) - J1), i == j, k == l);
-    const int nb = S.ch_n[chb];
-    Z[T.off[blk] + (long long)ik * nb + ib] += z;
-    if (chb == chk && ik != ib) Z[T.off[blk] + (long long)ib * nb + ik] += flip(z, hZ < 0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int q = q0 + h;
+      if (q >= nq) break;
+      const int i = s_q[q].x & 0xFFFF, j = s_q[q].x >> 16, k = s_q[q].y & 0xFFFF, l = s_q[q].y >> 16;
+      const int ib = S.ketJ_loc[J1 * S.nkets + ket_index(S.norb, i, j)], ik = S.ketJ_loc[J2 * S.nkets + ket_index(S.norb, k, l)];
+      const int chb = chan_index(J1, (S.l[i] + S.l[j]) & 1, (S.tz2[i] + S.tz2[j]) / 2);
+      const int chk = chan_index(J2, (S.l[k] + S.l[l]) & 1, (S.tz2[k] + S.tz2[l]) / 2);
+      if (ib < 0 || ik < 0 || chb > chk || (chb == chk && ik < ib)) continue;
+      const int blk = T.lookup[chb * S.nch + chk];
+      if (blk < 0) continue;
+      // both sums carry (-1)^J2
+      double z = flip(sum[0][h] + flip(sum[1][h], 1 + ((ji + jj) >> 1) - J1), J2);
+      if (DF) {
+        const int e = s_e[q] - 1023;
+        z *= __longlong_as_double((long long)(1023 + e / 2) << 52);
+        z *= __longlong_as_double((long long)(1023 + e - e / 2) << 52);
+      }
+      z = unnorm(z, i == j, k == l);
+      const int nb = S.ch_n[chb];
+      Z[T.off[blk] + (long long)ik * nb + ib] += z;
+      if (chb == chk && ik != ib) Z[T.off[blk] + (long long)ib * nb + ik] += flip(z, hZ < 0);
+    }
   }
 }
 
 unsigned grid_for(long long n) { return (unsigned)std::max(1LL, (n + 255) / 256); }
 
-cudaError_t launch_tinv_q(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ,
-                          cudaStream_t st)
+cudaError_t launch_tinv(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ, bool df,
+                        cudaStream_t st)
 {
-  const long long nq = (long long)t.tq.size();
-  if (nq == 0) return cudaSuccess;
-  // slots bounds a sum's gathered values and the output slots alike
-  const int slots = t.tq_max_j3 * (2 * t.lam + 1);
-  const size_t smem = (size_t)kTqWarps * 3 * slots * sizeof(double);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_tinv_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (t.tqb.empty()) return cudaSuccess;
+  auto kern = df && t.dev.nj_hatf ? k_tinv_b<true> : k_tinv_b<false>;
+  if (t.tqb_smem > 40 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, t.tqb_smem);
     if (e != cudaSuccess) return e;
   }
-  k_tinv_q<<<(unsigned)((nq + kTqWarps - 1) / kTqWarps), 32 * kTqWarps, smem, st>>>(s.dev, t.dev, Zbar, hZ, Z, t.d_tq,
-                                                                                     nq, slots);
+  kern<<<(unsigned)t.tqb.size(), kTqThreads, t.tqb_smem, st>>>(s.dev, t.dev, Zbar, hZ, Z, t.d_tq, t.d_tqb);
   count_launch();
   return cudaGetLastError();
+}
+
+__global__ void k_ff_table(const double* __restrict__ src, float2* __restrict__ dst, long long n)
+{
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    dst[i] = d2ff(src[i]);
 }
 
 }  // namespace
@@ -994,7 +1062,7 @@ cudaError_t launch_tensor_ph(const Space& s, const TensorLayout& t, const double
   k_tzbar<<<gz, 256, 0, st>>>(s.dev, s.work, t.dev, Xbar, Ybar, hX, hY, Zbar, s.work.phase_tab);
   count_launch();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  return launch_tinv_q(s, t, Zbar, Z, hZ, st);
+  return launch_tinv(s, t, Zbar, Z, hZ, false, st);
 }
 
 // ---------------------------------------------------------- split form
@@ -1041,9 +1109,17 @@ cudaError_t launch_tensor_222_221_split(const Space& s, const TensorLayout& t, c
 }
 
 cudaError_t launch_tensor_inverse_pandya(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ,
-                                         cudaStream_t st)
+                                         bool df, cudaStream_t st)
 {
-  return launch_tinv_q(s, t, Zbar, Z, hZ, st);
+  return launch_tinv(s, t, Zbar, Z, hZ, df, st);
+}
+
+cudaError_t launch_ff_table(const double* src, float2* dst, long long n, cudaStream_t st)
+{
+  if (n <= 0) return cudaSuccess;
+  k_ff_table<<<(unsigned)std::min<long long>((n + 255) / 256, 65536), 256, 0, st>>>(src, dst, n);
+  count_launch();
+  return cudaGetLastError();
 }
 
 // Operator::Norm of a tensor operator: blocks 0 .. n2-1 sum their chunk's

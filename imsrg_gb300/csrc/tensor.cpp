@@ -75,10 +75,11 @@ TensorLayout::~TensorLayout()
 {
   for (SplitPlan* p : {sp_lad1, sp_lad2, sp_zb1, sp_zb2})
     if (p) split_plan_destroy(p);
+  for (DgemmPlan* p : {dg_lad1, dg_lad2, dg_zb1, dg_zb2}) dgemm_plan_destroy(p);
   for (void* p : dev_allocs) cudaFree(p);
 }
 
-// The orbit quadruples of the inverse tensor Pandya transform (k_tinv_q): a
+// The orbit quadruples of the inverse tensor Pandya transform (k_tinv_b): a
 // bra ket (i <= j) and a ket ket (k <= l) with the rank's parity and |dTz|,
 // kept when some (J1, J2) gives a stored element it owns: block (chb, chk)
 // with chb <= chk and, within a diagonal block, ket index >= bra index.
@@ -96,8 +97,6 @@ static void build_quadruples(const Space& s, TensorLayout& t)
     int2 v;
   };
   std::vector<std::vector<Item>> part(nk);
-  int maxj = 0;
-  for (int p = 0; p < N; ++p) maxj = std::max(maxj, s.j2[p]);
 #pragma omp parallel for schedule(dynamic, 16)
   for (int kb = 0; kb < nk; ++kb) {
     const int i = kp[kb], j = kq[kb];
@@ -138,7 +137,30 @@ static void build_quadruples(const Space& s, TensorLayout& t)
   t.tq.assign((size_t)cnt[nkey], make_int2(0, 0));
   for (const auto& v : part)
     for (const Item& it : v) t.tq[(size_t)cnt[it.key]++] = it.v;
-  t.tq_max_j3 = maxj + 1;
+  // batches: as many quadruples as give each of 256 threads about one slot of
+  // four quadruples, within the shared memory of the gathered values
+  t.tqb.clear();
+  t.tqb_smem = 0;
+  const int w = 2 * lam + 1;
+  for (size_t a = 0; a < t.tq.size();) {
+    auto cls = [&](size_t x) {
+      return make_int4(s.j2[t.tq[x].x & 0xFFFF], s.j2[t.tq[x].x >> 16], s.j2[t.tq[x].y & 0xFFFF], s.j2[t.tq[x].y >> 16]);
+    };
+    const int4 j = cls(a);
+    size_t b = a;
+    while (b < t.tq.size()) {
+      const int4 k = cls(b);
+      if (k.x != j.x || k.y != j.y || k.z != j.z || k.w != j.w) break;
+      ++b;
+    }
+    const int nslot = (std::min(j.x, j.y) + 1) * (lam + 1);
+    const int nval = (std::min(j.x, j.w) + 1 + std::min(j.y, j.w) + 1) * w;
+    int q = std::min({kTqBatch, (1024 + nslot - 1) / nslot, kTqValues / nval});
+    q = std::max(4, q / 4 * 4);
+    for (size_t x = a; x < b; x += q) t.tqb.push_back(make_int2((int)x, (int)std::min<size_t>(q, b - x)));
+    t.tqb_smem = std::max(t.tqb_smem, q * nval * 8);
+    a = b;
+  }
 }
 
 TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity)
@@ -418,6 +440,19 @@ void tensor_upload(TensorLayout& t)
   d.tob_off = dev_copy(t, t.tob_off);
   d.tob_list = dev_copy(t, t.tob_list);
   t.d_tq = dev_copy(t, t.tq);
+  t.d_tqb = dev_copy(t, t.tqb);
+  // the split form's float pairs of the 9j table; without room for them it reads the FP64 table
+  d.nj_hatf = nullptr;
+  void* f = nullptr;
+  if (!t.nj_hat.empty() && cudaMalloc(&f, t.nj_hat.size() * sizeof(float2)) == cudaSuccess) {
+    t.dev_allocs.push_back(f);
+    if (launch_ff_table(d.nj_hat, (float2*)f, (long long)t.nj_hat.size(), nullptr) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess)
+      throw std::runtime_error("9j float-pair table");
+    d.nj_hatf = (const float2*)f;
+  } else {
+    cudaGetLastError();
+  }
   d.lad_koff = dev_copy(t, t.lad_koff);
   d.lad_woff = dev_copy(t, t.lad_woff);
   d.lad_n = dev_copy(t, t.lad_n);

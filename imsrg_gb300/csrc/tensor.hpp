@@ -57,6 +57,7 @@ struct DevTensor {
   const long long* nj_base = nullptr;
   const double* nj_val = nullptr;
   const double* nj_hat = nullptr;
+  const float2* nj_hatf = nullptr;  // nj_hat as (hi, lo) float pairs (split form; null: none)
   int d1 = 0;
   const double* hat2 = nullptr;  // [J1 * NJ + J2] = sqrt((2J1+1)(2J2+1))
   // per orbit i: the orbits j with <i||T||j> allowed (tob_list[tob_off[i] ..
@@ -71,6 +72,7 @@ struct DevTensor {
 };
 
 struct SplitPlan;
+struct DgemmPlan;
 
 struct TensorLayout {
   int lam = 0, trank = 0, parity = 0;
@@ -125,13 +127,19 @@ struct TensorLayout {
   // first K half (overwrite) and second K half (accumulate)
   double *d_yt = nullptr, *d_ybt = nullptr, *d_ybtf = nullptr, *d_xbf = nullptr;
   SplitPlan *sp_lad1 = nullptr, *sp_lad2 = nullptr, *sp_zb1 = nullptr, *sp_zb2 = nullptr;
+  // the FP64 form's plans of the same products (on the same operands); tried
+  // once: without them (their planes do not fit) the FP64-pipe kernels run
+  DgemmPlan *dg_lad1 = nullptr, *dg_lad2 = nullptr, *dg_zb1 = nullptr, *dg_zb2 = nullptr;
+  bool dg_tried = false;
   int max_tiles32 = 0;        // largest block in 32 x 32 tiles (transpose grid)
   // orbit quadruples of the inverse tensor Pandya transform: (i | j << 16,
   // k | l << 16) for every bra ket i <= j and ket ket k <= l that own at
   // least one stored element, ordered by the class (ji, jj, jk, jl)
   std::vector<int2> tq;
-  int tq_max_j3 = 0;          // largest J3 (or J1) range of a quadruple
-  int2* d_tq = nullptr;
+  // batches of k_tinv_b: (first quadruple, count), the quadruples of one class
+  std::vector<int2> tqb;
+  int tqb_smem = 0;           // shared memory of the largest batch
+  int2 *d_tq = nullptr, *d_tqb = nullptr;
   long long max_xbf = 0;      // largest X bar panel (2 nph x n_cc)
   DevTensor dev;
   bool dev_ready = false;
@@ -141,6 +149,8 @@ struct TensorLayout {
 
 // the space's layout of rank (lam, trank, parity), built on first use
 // (host tables only; tensor_upload copies them to the device)
+// quadruples a batch holds at most, and the gathered values (8 bytes each)
+constexpr int kTqBatch = 128, kTqValues = 5120;
 TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity);
 void tensor_upload(TensorLayout& t);
 // the same view with host pointers (host-side 9j and 6j evaluation)

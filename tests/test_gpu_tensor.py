@@ -234,3 +234,23 @@ def test_tensor_term_switches(off, dropped):
     finally:
         ig.Commutator.TurnOnTerm(off)
     assert ig.Commutator.IsTermOn(off)
+
+
+@pytest.mark.parametrize("rank", [(2, 0, 0), (1, 1, 1), (0, 1, 0), (4, 0, 0)])
+@pytest.mark.parametrize("exponent", [-500, 500])
+def test_split_inverse_transform_far_scales(rank, exponent):
+    """The inverse transform's double-float sums are scaled per quadruple, so
+    values far outside the FP32 range keep their precision: 2^e times Y gives
+    2^e times Z (every step is exact under a power of two; 1e-14 allows for
+    the order in which the one-body sums meet)."""
+    emax = 4
+    ref = ref_space(emax)
+    ms = ig.ModelSpace(emax, "O16", "O16")
+    X = ref.random_operator(5, True)
+    Y = ref.random_tensor(6, *rank)
+    out = []
+    for s in (1.0, 2.0**exponent):
+        Z = ig.Commutator.CommutatorScalarTensor(ig.Operator(ms, arena=X), ig.Operator(ms, *rank, arena=Y * s), "split")
+        out.append(Z.arena / s)
+    assert np.linalg.norm(out[0]) > 0
+    assert np.linalg.norm(out[1] - out[0]) <= 1e-14 * np.linalg.norm(out[0])

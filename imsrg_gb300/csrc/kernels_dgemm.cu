@@ -978,7 +978,9 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     p->smem = 1024 + NSTAGE * STAGE + (2 * NSTAGE + 3 + 2 * NINFO) * 8 + 16;
     if (p->smem + sizeof(TileInfo) * NINFO + 64 > (size_t)maxsm) throw std::runtime_error("not enough shared memory for the FP64 product's pipeline");
-    if (cudaFuncSetAttribute(k_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem) != cudaSuccess) {
+    // (the whole shared memory, so that a second stream's kernels find some beside the CTA)
+    if (cudaFuncSetAttribute(k_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_dgemm, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
       cudaGetLastError();
       throw std::runtime_error("cudaFuncSetAttribute");
     }

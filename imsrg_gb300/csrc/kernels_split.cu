@@ -7,9 +7,9 @@
 //
 //  * Digits.  Each row i gets one exponent a_i for its A row and b_i = a_i + c
 //    for its B row (c is one per job), chosen so both rows fit below the
-//    exponent.  Every element is rounded to an integer q = v * 2^(beta*S - e)
-//    (|q| <= 2^(beta*S)) and split into S balanced base-2^beta digits
-//    (|d_1| <= 2^beta, |d_s| <= 2^(beta-1)), all exact in BF16.  Only integer
+//    exponent.  Every element is rounded to an integer q = v * 2^(P - e)
+//    (|q| <= 2^P, P = beta*S, or 37 for five 8-bit digits) and split
+//    into S balanced base-2^beta digits, all exact in BF16.  Only integer
 //    instructions are used (FP64 runs at 1/57 of the FP32 rate on this part).
 //  * Symmetrisation folded into K.  With the shared-exponent choice both
 //    A_i.B_j and B_i.A_j carry the scale 2^(a_i + a_j + c), so
@@ -20,7 +20,8 @@
 //  * Products.  The digit products with s + t <= S + 1 are issued as
 //    tcgen05.mma kind::f16 (BF16 in, FP32 accumulate in tensor memory), one
 //    TMEM accumulator per weight group T = s + t.  beta is chosen from K so
-//    that the FP32 sums of the leading groups stay exact integers.
+//    that the FP32 sums of the leading groups stay exact integers, over the
+//    whole reduction or over chunks of it.
 //  * Recombination.  The epilogue reads the S group sums (tcgen05.ld), merges
 //    them exactly as int64, converts once to FP64 and applies the power-of-two
 //    scale by exponent arithmetic.  Tensor memory is a ring of accumulator
@@ -83,6 +84,8 @@ struct SplitTile {
 struct SplitPlan {
   int family = 0;
   int S = 6, beta = 6;
+  int P = 36;      // bits of the fixed point below a row's exponent
+  int chunk = 0;   // K blocks whose group sums stay exact (0: the whole reduction)
   int K_stride = 0;
   long long total_exp_rows = 0;   // rows of one digit plane (and of the exponent arrays)
   int njobs = 0, ntiles = 0;
@@ -118,7 +121,7 @@ namespace {
 // biased exponent field of a double (0 for zero / subnormal)
 __device__ __forceinline__ int dexp(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7FF); }
 
-// q = round(v * 2^(P - e)) for |v| < 2^e, P = beta*S <= 42; integer only
+// q = round(v * 2^(P - e)) for |v| < 2^e, P <= 42; integer only
 __device__ __forceinline__ long long to_fixed(double v, int e, int P)
 {
   long long bits = __double_as_longlong(v);
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(256) k_split_digits(const SplitJob* __restrict
                                                      const int* __restrict__ phase, double gbscale, int gsign,
                                                      const int* __restrict__ rexpA, const int* __restrict__ rexpB,
                                                      const int* __restrict__ jobmax, const int* __restrict__ flags,
-                                                     int beta, int K_stride, long long plane_rows,
+                                                     int beta, int P, int K_stride, long long plane_rows,
                                                      __nv_bfloat16* __restrict__ alpha, __nv_bfloat16* __restrict__ bet,
                                                      __nv_bfloat16* __restrict__ gam, __nv_bfloat16* __restrict__ del)
 {
@@ -354,7 +357,6 @@ __global__ void __launch_bounds__(256) k_split_digits(const SplitJob* __restrict
   __syncthreads();
   const double* A = Abase + jb.a_off;
   const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
-  const int P = beta * S;
   const long long half = 1ll << (beta - 1), mask = (1ll << beta) - 1;
   long long bias = 0;
 #pragma unroll
@@ -478,7 +480,7 @@ struct GemmArgs {
   const int* phase;
   double* out;
   int* status;
-  int S, beta, nstages, gsign;
+  int S, beta, P, chunk, nstages, gsign;
   int accum;  // -1: each job's flag; 0: overwrite; 1: accumulate
   int nomirror;  // 1: symmetrised jobs skip the mirror (lower-triangle) stores
 };
@@ -490,6 +492,11 @@ struct GemmArgs {
 // an even tile, the first OV groups of an odd one.  The epilogue folds those
 // groups into a per-column int64 partial sum first and releases them, and the
 // next tile's MMAs run under the rest of the epilogue.
+// (A tile whose reduction is cut into chunks goes through this chunk by chunk:
+// "tile" above then reads "chunk".)
+__host__ __device__ __forceinline__ int split_chunks(int nkt, int chunk) { return chunk ? (nkt + chunk - 1) / chunk : 1; }
+__host__ __device__ __forceinline__ int split_chunk_begin(int nkt, int n, int c) { return nkt * c / n; }
+
 template <int S, int TN>
 struct AccPair {
   static constexpr int NB = 512 / TN;
@@ -509,7 +516,9 @@ struct AccPair {
 // a second stream still fit beside the product on every SM; uncapped, the
 // epilogue's per-column partial sums take it to 168 and the commutator's two
 // streams stop overlapping.
-template <int S, int TN, int EPIW>
+// CHUNKED: reductions longer than g.chunk K blocks are cut (a plan of its
+// own kernel: the loop over chunks costs the short products 4%).
+template <int S, int TN, int EPIW, bool CHUNKED>
 __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMap mAlphaA,
                                                                  const __grid_constant__ CUtensorMap mBetaA,
                                                                  const __grid_constant__ CUtensorMap mGammaA,
@@ -619,65 +628,70 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
       constexpr int MAXT = 256 / TN;  // B digit tiles per MMA (UMMA N <= 256)
       int it = 0, tc = 0;
       const int tend = g.cta_first[blockIdx.x + 1];
-      for (int tix = g.cta_first[blockIdx.x]; tix < tend && !s_err; ++tix, ++tc) {
+      for (int tix = g.cta_first[blockIdx.x]; tix < tend && !s_err; ++tix) {
         const int job = g.tiles[tix].job;
         const int nkt = g.jobs[job].nkt, nkb = g.jobs[job].nkb;
         const unsigned neg2 = g.flags[2 * job] == 2 ? (1u << 13) : 0u;  // negate A in the second K half
-        // the blocks of this tile are free: the tile before last is done, and
-        // the shared blocks of the previous tile have been read (the
-        // epilogue works through the tiles in order, so the second implies
-        // the first)
-        const bool waited = OV > 0 ? mbar_wait(acc_early, (unsigned)((tc & 1) ^ 1))
-                                   : mbar_wait(acc_done(tc & 1), (unsigned)(((tc >> 1) & 1) ^ 1));
-        if (!waited) {
-          set_status(g.status, 102);
-          s_err = 1;
-          break;
-        }
-        tc_fence_after();
-        const unsigned dbase = tmem + Acc::base(tc);
+        const int nch = CHUNKED ? split_chunks(nkt, g.chunk) : 1;
         bool ok = true;
-        for (int kb = 0; kb < nkt; ++kb, ++it) {
-          int st = it % NST;
-          unsigned ph = (unsigned)((it / NST) & 1);
-          if (!mbar_wait(full_bar(st), ph)) {
-            set_status(g.status, 103);
+        for (int c = 0; c < nch && ok; ++c, ++tc) {
+          // the blocks of this chunk are free: the chunk before last is done,
+          // and the shared blocks of the previous one have been read (the
+          // epilogue works through them in order, so the second implies the
+          // first)
+          const bool waited = OV > 0 ? mbar_wait(acc_early, (unsigned)((tc & 1) ^ 1))
+                                     : mbar_wait(acc_done(tc & 1), (unsigned)(((tc >> 1) & 1) ^ 1));
+          if (!waited) {
+            set_status(g.status, 102);
             s_err = 1;
             ok = false;
             break;
           }
           tc_fence_after();
-          // descriptors of this stage: a base each, every operand tile a
-          // compile-time offset from it (the start-address field is addr >> 4,
-          // and the stage never crosses its 14 bits); each group is written
-          // (not accumulated) by the first K16 step of the tile, whose s = 0
-          // products are the first ones issued into every group
-          const unsigned sA = sbase + st * STAGE;
-          const unsigned long long a0 = sdesc_sw64(sA), b0 = sdesc_sw64(sA + S * A_SLICE);
-          const unsigned first = kb == 0 ? 0u : 1u;
-          const unsigned neg = kb >= nkb ? neg2 : 0u;
-          // The products (s, t) of one A digit s go to the weight groups s + t,
-          // which are consecutive TN-column blocks of tensor memory, and the B
-          // digit tiles t are consecutive TN-row blocks of shared memory with
-          // the same 512-byte swizzle-atom stride: so the products of one s
-          // over a run of t are one MMA with N = (run length) x TN, up to 256
+          const unsigned dbase = tmem + Acc::base(tc);
+          const int kb0 = split_chunk_begin(nkt, nch, c), kb1 = split_chunk_begin(nkt, nch, c + 1);
+          for (int kb = kb0; kb < kb1; ++kb, ++it) {
+            int st = it % NST;
+            unsigned ph = (unsigned)((it / NST) & 1);
+            if (!mbar_wait(full_bar(st), ph)) {
+              set_status(g.status, 103);
+              s_err = 1;
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            // descriptors of this stage: a base each, every operand tile a
+            // compile-time offset from it (the start-address field is addr >> 4,
+            // and the stage never crosses its 14 bits); each group is written
+            // (not accumulated) by the first K16 step of the chunk, whose s = 0
+            // products are the first ones issued into every group
+            const unsigned sA = sbase + st * STAGE;
+            const unsigned long long a0 = sdesc_sw64(sA), b0 = sdesc_sw64(sA + S * A_SLICE);
+            const unsigned first = kb == kb0 ? 0u : 1u;
+            const unsigned neg = kb >= nkb ? neg2 : 0u;
+            // The products (s, t) of one A digit s go to the weight groups s + t,
+            // which are consecutive TN-column blocks of tensor memory, and the B
+            // digit tiles t are consecutive TN-row blocks of shared memory with
+            // the same 512-byte swizzle-atom stride: so the products of one s
+            // over a run of t are one MMA with N = (run length) x TN, up to 256
 #pragma unroll
-          for (int sub = 0; sub < KB / 16; ++sub) {
+            for (int sub = 0; sub < KB / 16; ++sub) {
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-              const unsigned long long ad = a0 + (unsigned long long)((s * A_SLICE + sub * 32) >> 4);
+              for (int s = 0; s < S; ++s) {
+                const unsigned long long ad = a0 + (unsigned long long)((s * A_SLICE + sub * 32) >> 4);
 #pragma unroll
-              for (int t0 = 0; t0 < S - s; t0 += MAXT) {
-                const int nt = (S - s - t0) < MAXT ? (S - s - t0) : MAXT;
-                const unsigned long long bd = b0 + (unsigned long long)((t0 * B_SLICE + sub * 32) >> 4);
-                tc_mma(dbase + (s + t0) * TN, ad, bd, idesc_bf16(TILE_M, nt * TN) | neg, (sub == 0 && s == 0) ? first : 1u);
+                for (int t0 = 0; t0 < S - s; t0 += MAXT) {
+                  const int nt = (S - s - t0) < MAXT ? (S - s - t0) : MAXT;
+                  const unsigned long long bd = b0 + (unsigned long long)((t0 * B_SLICE + sub * 32) >> 4);
+                  tc_mma(dbase + (s + t0) * TN, ad, bd, idesc_bf16(TILE_M, nt * TN) | neg, (sub == 0 && s == 0) ? first : 1u);
+                }
               }
             }
+            tc_commit(empty_bar(st));
           }
-          tc_commit(empty_bar(st));
+          if (!ok) break;
+          tc_commit(acc_full(tc & 1));
         }
-        if (!ok) break;
-        tc_commit(acc_full(tc & 1));
       }
     }
   } else {
@@ -685,21 +699,22 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
     const int q = warp & 3;                  // TMEM lane quarter of this warp
     const int cbeg = ((warp - 2) >> 2) * COLS_W;  // first column of this warp
     const int et = threadIdx.x - 64;         // 0 .. EPI_T-1
-    int tc = 0;
-    const int tend = g.cta_first[blockIdx.x + 1];
-    for (int tix = g.cta_first[blockIdx.x]; tix < tend; ++tix, ++tc) {
+    int tc = 0;  // chunks
+    const int tbeg = g.cta_first[blockIdx.x], tend = g.cta_first[blockIdx.x + 1];
+    for (int tix = tbeg; tix < tend; ++tix) {
       const SplitTile tl = g.tiles[tix];
+      const int tp = (tix - tbeg) & 1;
       // the job's fields in registers (a reference would be re-read after
       // every store to the output, which the compiler cannot tell apart)
       const SplitJob* jp = g.jobs + tl.job;
       const int jm = jp->m, jn = jp->n, ldo = jp->ldo, nosym = jp->nosym, phase_off = jp->phase_off;
-      const int jsign = jp->sign, jacc = jp->accumulate;
+      const int jsign = jp->sign, jacc = jp->accumulate, nch = CHUNKED ? split_chunks(jp->nkt, g.chunk) : 1;
       const long long exp_base = jp->exp_base, out_off = jp->out_off;
       // the tile's row and column exponents and phases come from the
       // exponent pass (before this kernel), not from the MMAs: they are read
-      // while the tile's products still run.  (s_colexp[tc & 1] was last read
-      // for tile tc - 2, which every epilogue warp finished before the
-      // barrier of tile tc - 1.)
+      // while the tile's products still run.  (s_colexp[tp] was last read
+      // two tiles before, which every epilogue warp finished before the
+      // barriers of the last.)
       const int c = nosym ? 0 : job_c(g.jobmax, tl.job);
       const int* ph = phase_off >= 0 ? g.phase + phase_off : nullptr;
       // column exponents and phases of this tile (a plain job's columns are
@@ -707,10 +722,10 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
       if (et < TN) {
         const int j = tl.J * TN + et;
         const bool ok = j < jn;
-        s_colexp[tc & 1][et] = !ok ? EXP_NONE
+        s_colexp[tp][et] = !ok ? EXP_NONE
                                : nosym ? own_exp(g.rexpB[exp_base + j])
                                           : row_exp(g.rexpA[exp_base + j], g.rexpB[exp_base + j], c);
-        s_colph[tc & 1][et] = (ph && ok) ? ph[j] : 1;
+        s_colph[tp][et] = (ph && ok) ? ph[j] : 1;
       }
       const int sign = jsign != 0 ? jsign : g.gsign;
       const int i = tl.I * TILE_M + q * 32 + lane;
@@ -719,52 +734,73 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
                      : nosym ? own_exp(g.rexpA[exp_base + i])
                                 : row_exp(g.rexpA[exp_base + i], g.rexpB[exp_base + i], c);
       const int phi_i = (ph && rowok) ? ph[i] : 1;
-      // the epilogue warps decide together (named barrier 1), so a timeout
-      // never leaves one of them waiting at a barrier alone
-      if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1))) {
-        set_status(g.status, 104);
-        s_epi_err = 1;
+      double* O = g.out + out_off;
+      const int Xi = ai + c - 2 * g.P + g.beta * (S - 1);
+      const bool accumulate = g.accum > 0 || (g.accum < 0 && jacc);
+      // exact merge of the weight groups (group t counts 2^(beta (S-1-t))),
+      // per column, over the chunks of the reduction.  Of each chunk the
+      // groups that the next one overwrites (e0 .. e0+OV-1) are added first
+      // for all this warp's columns, then released; then the others
+      // (l0 .. l0+S-OV-1), those of the last chunk together with the stores
+      long long P[COLS_W];
+#pragma unroll
+      for (int cc = 0; cc < COLS_W; ++cc) P[cc] = 0;
+      unsigned lane_base = 0;
+      int l0 = 0;
+      for (int ch = 0; ch < nch; ++ch, ++tc) {
+        if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1))) {
+          set_status(g.status, 104);
+          s_epi_err = 1;
+        }
+        // the epilogue warps decide together (named barrier 1), so a timeout
+        // never leaves one of them waiting at a barrier alone
+        asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
+        if (s_epi_err) break;
+        tc_fence_after();
+        lane_base = tmem + ((unsigned)(q * 32) << 16) + Acc::base(tc);
+        const int e0 = Acc::early_lo(tc);
+        l0 = (tc & 1) ? OV : 0;
+        if (OV > 0) {
+#pragma unroll
+          for (int c0 = 0; c0 < COLS_W; c0 += EPI_COLS) {
+            unsigned r[OV > 0 ? OV : 1][EPI_COLS];
+#pragma unroll
+            for (int gi = 0; gi < OV; ++gi) tmem_ld8(lane_base + (unsigned)((e0 + gi) * TN + cbeg + c0), r[gi]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int cc = 0; cc < EPI_COLS; ++cc) {
+              long long E = 0;
+#pragma unroll
+              for (int gi = 0; gi < OV; ++gi) E = E * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
+              P[c0 + cc] += E * (1ll << (g.beta * (S - OV - e0)));
+            }
+          }
+          tc_fence_before();
+          mbar_arrive(acc_early);
+        }
+        if (ch + 1 == nch) break;  // the rest with the stores
+#pragma unroll
+        for (int c0 = 0; c0 < COLS_W; c0 += EPI_COLS) {
+          unsigned r[S - OV][EPI_COLS];
+#pragma unroll
+          for (int gi = 0; gi < S - OV; ++gi) tmem_ld8(lane_base + (unsigned)((l0 + gi) * TN + cbeg + c0), r[gi]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int cc = 0; cc < EPI_COLS; ++cc) {
+            long long L = 0;
+#pragma unroll
+            for (int gi = 0; gi < S - OV; ++gi) L = L * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
+            P[c0 + cc] += L * (1ll << (g.beta * (OV - l0)));
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(acc_done(tc & 1));
       }
-      asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
       if (s_epi_err) {
         s_err = 1;
         break;
       }
-      tc_fence_after();
-      double* O = g.out + out_off;
-      const int Xi = ai + c - g.beta * (S + 1);
-      const bool accumulate = g.accum > 0 || (g.accum < 0 && jacc);
-      const unsigned lane_base = tmem + ((unsigned)(q * 32) << 16) + Acc::base(tc);
-      // exact merge of the weight groups: Horner in base 2^beta, per column,
-      // in two parts.  The groups the next tile overwrites (e0 .. e0+OV-1)
-      // are read first for all this warp's columns into P, then released;
-      // per chunk of columns the other groups (l0 .. l0+S-OV-1) give the rest:
-      //   odd tile  (e0 = 0, the leading groups):  I = P 2^(beta (S-OV)) + L
-      //   even tile (e0 = S-OV, the trailing ones): I = L 2^(beta OV) + P
-      const int e0 = Acc::early_lo(tc);
-      const int l0 = (tc & 1) ? OV : 0;
-      const long long mulP = (tc & 1) ? (1ll << (g.beta * (S - OV))) : 1ll;
-      const long long mulL = (tc & 1) ? 1ll : (1ll << (g.beta * OV));
-      long long P[COLS_W];
-#pragma unroll
-      for (int cc = 0; cc < COLS_W; ++cc) P[cc] = 0;
-      if (OV > 0) {
-#pragma unroll
-        for (int c0 = 0; c0 < COLS_W; c0 += EPI_COLS) {
-          unsigned r[OV > 0 ? OV : 1][EPI_COLS];
-#pragma unroll
-          for (int gi = 0; gi < OV; ++gi)
-            tmem_ld8(lane_base + (unsigned)((e0 + gi) * TN + cbeg + c0), r[gi]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int gi = 0; gi < OV; ++gi)
-#pragma unroll
-            for (int cc = 0; cc < EPI_COLS; ++cc)
-              P[c0 + cc] = P[c0 + cc] * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
-        }
-        tc_fence_before();
-        mbar_arrive(acc_early);
-      }
+      const long long mulL = 1ll << (g.beta * (OV - l0));
 #pragma unroll
       for (int c0 = 0; c0 < COLS_W; c0 += EPI_COLS) {
         unsigned r[S - OV][EPI_COLS];
@@ -784,10 +820,10 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           long long L = 0;
 #pragma unroll
           for (int gi = 0; gi < S - OV; ++gi) L = L * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
-          const long long I64 = P[c0 + cc] * mulP + L * mulL;
-          v[cc] = i64_ldexp(I64, Xi + s_colexp[tc & 1][jc]);
+          const long long I64 = P[c0 + cc] + L * mulL;
+          v[cc] = i64_ldexp(I64, Xi + s_colexp[tp][jc]);
           mv[cc] = __longlong_as_double(__double_as_longlong(v[cc]) ^
-                                        ((sign * phi_i * s_colph[tc & 1][jc]) < 0 ? (long long)0x8000000000000000ull
+                                        ((sign * phi_i * s_colph[tp][jc]) < 0 ? (long long)0x8000000000000000ull
                                                                                    : 0ll));
           od[cc] = 0.0;
           om[cc] = 0.0;
@@ -818,6 +854,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
       // every TMEM load of this tile has completed (tcgen05.wait::ld)
       tc_fence_before();
       mbar_arrive(acc_done(tc & 1));
+      ++tc;
     }
   }
   // every role has left its loop: all MMAs this CTA issued have been drained
@@ -894,6 +931,18 @@ static void choose_digits(int Kmax, int& beta, int& S)
   if (S > MAX_S) S = MAX_S;
 }
 
+// Where that takes six digits for 36 bits (any K above 58), five of 8 bits
+// (5 in the leading one) give 37: 15 products and five planes instead of 21
+// and six.  Their leading three weight groups are exact over WIDE_CHUNK K
+// blocks ((2 x 33 x 128 + 128^2) x 672 < 2^24), so the reduction is cut into
+// chunks of that, whose sums are added as integers; what the other groups
+// round is below 2^-38 of the rows' maxima.  A chunk costs the MMAs the time
+// in which the epilogue takes the blocks that consecutive chunks share: 39
+// bits need chunks of 10 blocks.  emax=10 ladder product (beside the second
+// stream's kernels): 1135 us with six digits, 1062 with chunks of 10 blocks,
+// 945 so, 898 uncut.
+constexpr int WIDE_BETA = 8, WIDE_S = 5, WIDE_P = 37, WIDE_CHUNK = 21;
+
 SplitOpts split_plan_opts(const SplitPlan* p)
 {
   SplitOpts o;
@@ -938,6 +987,13 @@ SplitPlan* split_plan_create(const Space& s, const std::vector<GemmJobDev>& jobs
   int Kmax = 1;
   for (const GemmJobDev& j : jobs_in) Kmax = std::max(Kmax, j.K);
   choose_digits(Kmax, p->beta, p->S);
+  p->P = p->beta * p->S;
+  if (opts.digits == 0 && p->P < WIDE_P && Kmax <= 40000) {  // (the chunks' integer sums stay below 2^63)
+    p->beta = WIDE_BETA;
+    p->S = WIDE_S;
+    p->P = WIDE_P;
+    p->chunk = WIDE_CHUNK;
+  }
   // a requested digit count keeps the digit width (set by exactness) and
   // changes the precision: beta * S bits per operand row
   if (opts.digits != 0) {
@@ -950,6 +1006,7 @@ SplitPlan* split_plan_create(const Space& s, const std::vector<GemmJobDev>& jobs
       throw std::invalid_argument("split plan: digits x digit width above 42 bits");
     }
     p->S = opts.digits;
+    p->P = p->beta * p->S;
   }
   long long erow = 0;
   int kstride = KB;
@@ -1032,7 +1089,10 @@ SplitPlan* split_plan_create(const Space& s, const std::vector<GemmJobDev>& jobs
     } else {
       std::vector<int> ord(tiles.size());
       for (size_t t = 0; t < ord.size(); ++t) ord[t] = (int)t;
-      auto cost = [&](int t) { return (long long)p->jobs[tiles[t].job].nkt + 4; };
+      auto cost = [&](int t) {
+        const int nkt = p->jobs[tiles[t].job].nkt;
+        return (long long)nkt + 2 + 2 * split_chunks(nkt, p->chunk);
+      };
       std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost(a) > cost(b); });
       std::vector<std::pair<long long, int>> heap;  // (load, cta), min-heap
       for (int b = 0; b < G; ++b) heap.push_back({0, b});
@@ -1188,7 +1248,7 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
       auto kd = p->plain ? k_split_digits<S, true> : k_split_digits<S, false>;
       kd<<<p->n_dblk, 256, 0, st>>>(p->d_jobs, p->d_dblk, A, B0, B1, kidx, kw, phase, gbscale, gsign,
                                                     p->d_rexpA, p->d_rexpB, p->d_jobmax, flags_for(p, gsign),
-                                                    p->beta, p->K_stride, p->total_exp_rows, p->arr[0],
+                                                    p->beta, p->P, p->K_stride, p->total_exp_rows, p->arr[0],
                                                     p->arr[1], p->arr[2], p->arr[3]);
       count_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1210,23 +1270,19 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
     ga.status = status;
     ga.S = S;
     ga.beta = p->beta;
+    ga.P = p->P;
+    ga.chunk = p->chunk;
     ga.nstages = p->nstages;
     ga.gsign = gsign;
     ga.accum = p->accum_override;
     ga.nomirror = p->mirror ? 0 : 1;
-    if (p->tn == 64) {
-      auto kern = k_split_gemm<S, 64, 8>;
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
-      if (e != cudaSuccess) return e;
-      kern<<<p->grid, 64 + 32 * 8, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], p->maps[4],
-                                                   p->maps[5], ga);
-    } else {
-      auto kern = k_split_gemm<S, 32, 8>;
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
-      if (e != cudaSuccess) return e;
-      kern<<<p->grid, 64 + 32 * 8, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], p->maps[4],
-                                                   p->maps[5], ga);
-    }
+    auto kern = p->chunk ? (p->tn == 64 ? k_split_gemm<S, 64, 8, true> : k_split_gemm<S, 32, 8, true>)
+                         : (p->tn == 64 ? k_split_gemm<S, 64, 8, false> : k_split_gemm<S, 32, 8, false>);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+    // the whole shared memory, so that the second stream's kernels find some beside the product's CTA
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    kern<<<p->grid, 64 + 32 * 8, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], p->maps[4], p->maps[5], ga);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }

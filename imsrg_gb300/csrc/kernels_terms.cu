@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kObThreads) k_onebody(DevSpace S, DevWork W, c
   Y = zsh(Y, zo, ZR_Y);
   Z = zsh(Z, zo, ZR_Z);
   __shared__ double red[kObThreads / 32];
-  constexpr int T = 16, TK = 32;
+  constexpr int T = 16, TK = 16;  // 9 KB in all: more does not fit beside a product's CTA, and the kernel then waits for its end
   __shared__ double xi[TK][T + 1], yi[TK][T + 1], xj[T][TK + 1], yj[T][TK + 1];
   const int N = S.norb, tid = threadIdx.x;
   int item = blockIdx.x;
@@ -122,17 +122,11 @@ __global__ void __launch_bounds__(kObThreads) k_onebody(DevSpace S, DevWork W, c
       double xy = 0.0, yx = 0.0;
       for (int b0 = 0; b0 < N; b0 += TK) {
         __syncthreads();
-#pragma unroll
-        for (int u = 0; u < T * TK / kObThreads; ++u) {
-          const int b = b0 + c + u * (kObThreads / T);  // 16 rows i, 32 columns b
-          const bool ok = b < N && i < N;
-          xi[b - b0][r] = ok ? X1[(size_t)b * N + i] : 0.0;
-          yi[b - b0][r] = ok ? Y1[(size_t)b * N + i] : 0.0;
-          const int e = tid + u * kObThreads, bb = e & 31, jj = e >> 5;  // 32 rows b, 16 columns j
-          const bool ok2 = b0 + bb < N && j0 + jj < N;
-          xj[jj][bb] = ok2 ? X1[(size_t)(j0 + jj) * N + b0 + bb] : 0.0;
-          yj[jj][bb] = ok2 ? Y1[(size_t)(j0 + jj) * N + b0 + bb] : 0.0;
-        }
+        const bool oki = b0 + c < N && i < N, okj = b0 + r < N && j < N;
+        xi[c][r] = oki ? X1[(size_t)(b0 + c) * N + i] : 0.0;
+        yi[c][r] = oki ? Y1[(size_t)(b0 + c) * N + i] : 0.0;
+        xj[c][r] = okj ? X1[(size_t)j * N + b0 + r] : 0.0;
+        yj[c][r] = okj ? Y1[(size_t)j * N + b0 + r] : 0.0;
         __syncthreads();
         const int nb = min(TK, N - b0);
         for (int b = 0; b < nb; ++b) {

@@ -531,6 +531,15 @@ int inverse_pandya(imsrg_space* sp, const double* zb, double* Z, int hZ, int pre
   return IMSRG_OK;
 }
 
+// whether the form's inverse Pandya kernel can apply comm122ss's update too
+bool inverse_folds(imsrg_space* sp, int prec, int& rc)
+{
+  const int variant = prec == IMSRG_PREC_SPLIT ? sp->inv_split : (sp->inv_fp64 ? 2 : 0);
+  if (variant != 1 && variant != 2) return false;
+  rc = ensure_invd(sp);
+  return rc == IMSRG_OK && sp->invd.covers_all;
+}
+
 int check_ops(const imsrg_op* X, const imsrg_op* Y, const imsrg_op* Z)
 {
   if (!X || !Y || !Z) return fail(IMSRG_ERR_ARG, "null operator");
@@ -578,9 +587,9 @@ int prep_122_df(const imsrg_op* X, const imsrg_op* Y, cudaStream_t st)
 // FP64 form: FP64 gathers (the plain form keeps every term in FP64).
 // Split form: the same gathers in double-float on the FP32 pipe (prepared:
 // the float-pair copies are already made, on a stream ordered before st).
-// fold_sym: only W2 here; the inverse Pandya kernel applies Z -= W2 + hZ W2^T
+// part: W2, its subtraction from Z, or both
 int do_122(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st, int prec = IMSRG_PREC_FP64,
-           bool prepared = false, bool fold_sym = false)
+           bool prepared = false, int part = W2_MAKE | W2_SUBTRACT)
 {
   imsrg_space* sp = X->sp;
   int rc = ensure_scratch(sp, false, true);
@@ -593,12 +602,12 @@ int do_122(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t st, i
                                        sp->n_sym122u, st));
     else
       CUDA_TRY(launch_comm122_df(*sp->s, X->d, Y->d, Z->d, sp->d_xf, sp->d_yff, (float2*)sp->d_w2, Z->herm,
-                                 sp->d_sym122, sp->n_sym122, st, nullptr, 1, !fold_sym));
+                                 sp->d_sym122, sp->n_sym122, st, nullptr, 1, part));
     return IMSRG_OK;
   }
   ProfScope ps("comm122ss", st);
   CUDA_TRY(launch_comm122(*sp->s, X->d, Y->d, Z->d, sp->d_w2, Z->herm, sp->d_sym122, sp->n_sym122, st, nullptr, 1,
-                          !fold_sym));
+                          part));
   return IMSRG_OK;
 }
 
@@ -694,7 +703,7 @@ int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaS
   return IMSRG_OK;
 }
 
-// comm222_phss, first half: the Pandya-transformed operands (X bar, Y bar,
+// comm222_phss, first part: the Pandya-transformed operands (X bar, Y bar,
 // Y bar flipped)
 int prep_ph(const imsrg_op* X, const imsrg_op* Y, int prec, cudaStream_t st)
 {
@@ -707,40 +716,48 @@ int prep_ph(const imsrg_op* X, const imsrg_op* Y, int prec, cudaStream_t st)
   return IMSRG_OK;
 }
 
-// prepared: prep_ph already ran, on a stream ordered before st
-// fold_w2: also apply comm122ss's Z -= W2 + hZ W2^T (W2 already computed on st)
-int do_ph(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st, bool prepared = false,
-          bool fold_w2 = false)
+// comm222_phss, second part: Z bar of the transformed operands (prep_ph) for
+// a Z of hermiticity hZ
+int zbar_product(imsrg_space* sp, int hZ, int prec, cudaStream_t st)
 {
-  imsrg_space* sp = X->sp;
   Space& s = *sp->s;
-  int rc = ensure_scratch(sp, true, false);
-  if (rc) return rc;
-  if (!prepared && (rc = prep_ph(X, Y, prec, st))) return rc;
-  ProfScope ps("comm222_phss", st);
-  int slot = prof_begin("Build Z_bar", st);
+  ProfScope ps("Build Z_bar", st);
   if (prec == IMSRG_PREC_SPLIT) {
-    rc = ensure_split(sp);
+    int rc = ensure_split(sp);
     if (rc) return rc;
     // the descriptor inverse kernels read only Zbar's upper triangle
     split_plan_set_mirror(sp->split_zbar, sp->inv_split == 0 ? 1 : 0);
     CUDA_TRY(launch_symgemm_split(sp->split_zbar, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx,
-                                  s.work.kweight, s.work.phase_tab, sp->d_status, Z->herm, 1.0, st));
-  } else if (prec == IMSRG_PREC_FP64) {
-    if (DgemmPlan* p = fp64_plan(&sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
-      // the descriptor inverse kernel reads only Zbar's upper triangle
-      CUDA_TRY(launch_dgemm(p, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab,
-                            Z->herm, 1.0, 0, sp->inv_fp64 == 0, st));
-    else
-      CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
-                                   sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm, 1.0, 0, st));
-  } else {
-    return fail(IMSRG_ERR_ARG, "unknown precision");
+                                  s.work.kweight, s.work.phase_tab, sp->d_status, hZ, 1.0, st));
+    return IMSRG_OK;
   }
-  prof_end(slot, st);
+  if (prec != IMSRG_PREC_FP64) return fail(IMSRG_ERR_ARG, "unknown precision");
+  if (DgemmPlan* p = fp64_plan(&sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
+    // the descriptor inverse kernel reads only Zbar's upper triangle
+    CUDA_TRY(launch_dgemm(p, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, hZ,
+                          1.0, 0, sp->inv_fp64 == 0, st));
+  else
+    CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
+                                 sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, hZ, 1.0, 0, st));
+  return IMSRG_OK;
+}
+
+// comm222_phss, last part: the inverse Pandya transform of Z bar into Z
+// (fold_w2: with comm122ss's Z -= W2 + hZ W2^T, W2 already computed)
+int ph_inverse(imsrg_op* Z, int prec, cudaStream_t st, bool fold_w2)
+{
+  imsrg_space* sp = Z->sp;
   ProfScope pinv("InversePandyaTransformation", st);
   return inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, prec, st, nullptr, 1, fold_w2 ? (const void*)sp->d_w2 : nullptr,
                         fold_w2 ? (prec == IMSRG_PREC_SPLIT ? 1 : 2) : 0);
+}
+
+int do_ph(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st)
+{
+  ProfScope ps("comm222_phss", st);
+  int rc;
+  if ((rc = prep_ph(X, Y, prec, st)) || (rc = zbar_product(X->sp, Z->herm, prec, st))) return rc;
+  return ph_inverse(Z, prec, st, false);
 }
 
 int z_herm(int hx, int hy) { return (hx == hy) ? -1 : 1; }
@@ -770,6 +787,19 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
     CUDA_TRY(launch_zero_gaps(*sp->s, Z->d, st));  // the ladder product writes the rest
   else
     CUDA_TRY(cudaMemsetAsync(Z->d, 0, sp->s->arena * sizeof(double), st));
+  const bool split = prec == IMSRG_PREC_SPLIT;
+  // comm122ss's W2 reads only X and Y (not so the fused split form, which
+  // updates Z): it is formed on the second stream.  Its Z -= W2 + hZ W2^T
+  // rides in the inverse Pandya kernel, which reads and writes every
+  // upper-triangle element of Z and its mirror anyway, when that kernel is
+  // the descriptor one and lists every element
+  const bool w2 = on[T122] && !(split && sp->comm122_fused);
+  bool fold = false;
+  if (w2 && on[T222PH]) {
+    int rf = IMSRG_OK;
+    fold = inverse_folds(sp, prec, rf);
+    if (rf) return rf;
+  }
   // The terms add into Z in an order of our own (the sum is the same up to
   // rounding): the ladder product goes first and overwrites the two-body blocks,
   // so the one-body part of comm221ss can read Mpp - Mhh straight from Z2
@@ -777,18 +807,21 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   // shared the same way by the reference's comm222_pp_hh_221ss).
   //
   // While the ladder product runs on st, a second stream does what does not
-  // depend on it: the operand preparation of comm122ss and comm222_phss and
-  // the zero- and one-body terms (they write only Z0 and Z1, the ladder only
-  // Z2).  The streams join before comm221ss's last part, which reads Z2 and
-  // writes Z1.
+  // depend on it: comm122ss's W2, the zero- and one-body terms (they write
+  // only Z0 and Z1, the ladder only Z2) and comm222_phss up to Z bar, whose
+  // product takes the SMs that the ladder leaves (small spaces) or has left.
+  // The streams join before comm221ss's last part, which reads Z2 and writes
+  // Z1.  (W2 and Z bar after the ladder instead: 100 against 78 us at emax 2
+  // FP64, 310 against 279 at emax 6, 3.31 against 3.22 ms at emax 10 split.)
   CUDA_TRY(cudaEventRecord(sp->ev_fork, st));
   CUDA_TRY(cudaStreamWaitEvent(sd, sp->ev_fork, 0));
-  const bool split = prec == IMSRG_PREC_SPLIT;
   if (on[T122] && split && (rc = prep_122_df(X, Y, sd))) return rc;
   if (on[T222PH] && (rc = prep_ph(X, Y, prec, sd))) return rc;
   const int todo = (on[T111] ? OB_111 : 0) | (on[T110] ? OB_110 : 0) | (on[T121] ? OB_121 : 0) | (on[T220] ? OB_220 : 0) |
                    (on[T221] && ladder_first ? OB_221 : 0);
   if ((rc = do_onebody(X, Y, Z, todo, "zero- and one-body terms", sd))) return rc;
+  if (w2 && (rc = do_122(X, Y, Z, sd, prec, split, W2_MAKE))) return rc;
+  if (on[T222PH] && (rc = zbar_product(sp, Z->herm, prec, sd))) return rc;
   CUDA_TRY(cudaEventRecord(sp->ev_join, sd));
   if (ladder_first && (rc = do_ladder(X, Y, Z, prec, st, true))) return rc;
   CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join, 0));
@@ -798,19 +831,8 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   } else if (on[T221] && (rc = do_221_1b(X, Y, Z, st))) {
     return rc;
   }
-  // comm122ss's final Z -= W2 + hZ W2^T rides in the inverse Pandya kernel,
-  // which reads and writes every upper-triangle element of Z and its mirror
-  // anyway, when that kernel is the descriptor one and lists every element
-  bool fold = false;
-  if (on[T122] && on[T222PH] && !(split && sp->comm122_fused)) {
-    const int variant = split ? sp->inv_split : (sp->inv_fp64 ? 2 : 0);
-    if (variant == 1 || variant == 2) {
-      if ((rc = ensure_invd(sp))) return rc;
-      fold = sp->invd.covers_all;
-    }
-  }
-  if (on[T122] && (rc = do_122(X, Y, Z, st, prec, split, fold))) return rc;
-  if (on[T222PH] && (rc = do_ph(X, Y, Z, prec, st, true, fold))) return rc;
+  if (on[T122] && !fold && (rc = do_122(X, Y, Z, st, prec, split, w2 ? W2_SUBTRACT : W2_MAKE | W2_SUBTRACT))) return rc;
+  if (on[T222PH] && (rc = ph_inverse(Z, prec, st, fold))) return rc;
   return IMSRG_OK;
 }
 
@@ -1527,6 +1549,7 @@ struct GroupedProducts {
   std::vector<const imsrg_op*> X, Y;
   std::vector<imsrg_op*> Z;
   int prec = IMSRG_PREC_SPLIT;
+  bool fold = false;  // comm122ss's update rides in the inverse Pandya kernel
   SplitPlan* ladder = nullptr;  // split form
   SplitPlan* zbar = nullptr;
   // FP64 form: tensor-core plans over every pair's jobs; where they do not fit,
@@ -1677,14 +1700,18 @@ int group_mid(GroupedProducts* g, cudaStream_t st)
   const Space& s = *sp->s;
   const long long* zo = g->d_zoff;
   CUDA_TRY(launch_comm221_z(s, Z->d, Z->herm, Z->d, st, zo, nz));
+  int rc = IMSRG_OK;
+  g->fold = !(g->prec == IMSRG_PREC_SPLIT && sp->comm122_fused) && inverse_folds(sp, g->prec, rc);
+  if (rc) return rc;
+  const int part = g->fold ? W2_MAKE : W2_MAKE | W2_SUBTRACT;
   if (g->prec == IMSRG_PREC_FP64)
-    CUDA_TRY(launch_comm122(s, X->d, Y->d, Z->d, sp->d_w2, Z->herm, sp->d_sym122, sp->n_sym122, st, zo, nz));
+    CUDA_TRY(launch_comm122(s, X->d, Y->d, Z->d, sp->d_w2, Z->herm, sp->d_sym122, sp->n_sym122, st, zo, nz, part));
   else if (sp->comm122_fused)
     CUDA_TRY(launch_comm122_fused_df(s, X->d, Y->d, Z->d, sp->d_xf, sp->d_yff, Z->herm, sp->d_sym122u, sp->n_sym122u,
                                      st, zo, nz));
   else
     CUDA_TRY(launch_comm122_df(s, X->d, Y->d, Z->d, sp->d_xf, sp->d_yff, (float2*)sp->d_w2, Z->herm, sp->d_sym122,
-                               sp->n_sym122, st, zo, nz));
+                               sp->n_sym122, st, zo, nz, part));
   return IMSRG_OK;
 }
 
@@ -1695,7 +1722,8 @@ int group_post(GroupedProducts* g, cudaStream_t st)
   imsrg_space* sp = g->X[0]->sp;
   const Space& s = *sp->s;
   if (g->prec == IMSRG_PREC_FP64 || sp->inv_split != 0 || sp->n_invq > 0) {
-    int rc = inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, g->prec, st, g->d_zoff, nz);
+    int rc = inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, g->prec, st, g->d_zoff, nz, g->fold ? (const void*)sp->d_w2 : nullptr,
+                            g->fold ? (g->prec == IMSRG_PREC_SPLIT ? 1 : 2) : 0);
     if (rc) return rc;
   } else {
     for (int p = 0; p < nz; ++p) {

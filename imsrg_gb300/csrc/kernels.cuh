@@ -40,10 +40,12 @@ cudaError_t launch_comm221_z(const Space& s, double* Z, int hZ, const double* Mz
                              const long long* zo = nullptr, int nz = 1);
 // comm221ss on its own
 cudaError_t launch_comm221_1b(const Space& s, const double* X, const double* Y, double* Z, int hX, int hZ, cudaStream_t st);
-// (grouped)
+// part: the W2 intermediate (it reads only X and Y), Z -= W2 + hZ W2^T, or both
+// (the inverse Pandya kernel can apply the second itself); (grouped)
+enum { W2_MAKE = 1, W2_SUBTRACT = 2 };
 cudaError_t launch_comm122(const Space& s, const double* X, const double* Y, double* Z, double* W2, int hZ,
                            const int* sym_tiles, int nsym_tiles, cudaStream_t st, const long long* zo = nullptr,
-                           int nz = 1, bool sym = true);
+                           int nz = 1, int part = W2_MAKE | W2_SUBTRACT);
 // loads launch_comm122's kernels on the current device (they are otherwise
 // loaded at their first launch under lazy module loading)
 cudaError_t load_comm122_kernels();
@@ -53,10 +55,9 @@ cudaError_t launch_to_ff(const Space& s, const double* A, float2* Af, cudaStream
                          int nz = 1, int rsrc = ZR_X, int rdst = ZR_XF);
 // split-form comm122ss from the (hi, lo) copies Xf, Yf of X and Y
 // (grouped)
-// sym = false: W2 only (the Z update is folded into the inverse Pandya kernel)
 cudaError_t launch_comm122_df(const Space& s, const double* X, const double* Y, double* Z, const float2* Xf,
                               const float2* Yf, float2* W2, int hZ, const int* sym_tiles, int nsym_tiles,
-                              cudaStream_t st, const long long* zo = nullptr, int nz = 1, bool sym = true);
+                              cudaStream_t st, const long long* zo = nullptr, int nz = 1, int part = W2_MAKE | W2_SUBTRACT);
 // the same without the W2 round trip: tile pairs (ch, a, b), a <= b, each
 // forming both W2 tiles in shared memory and updating Z(a, b) and Z(b, a)
 // (grouped)
@@ -106,7 +107,7 @@ struct InvdDev {
 void build_invd(const Space& s, InvdPlan& out, int stage_max, int res_max, bool stage_weights);
 // (grouped)
 // W2 / w2mode: comm122ss's W2 folded into the same update (Z -= W2 + hZ W2^T;
-// 1: (hi, lo) float pairs, 2: FP64), only when d.covers_all and not grouped
+// 1: (hi, lo) float pairs, 2: FP64), only when d.covers_all
 cudaError_t launch_pandya_inv_desc(const Space& s, const InvdDev& d, bool df, const double* Zb, double* Z, int hZ,
                                    cudaStream_t st, const long long* zo = nullptr, int nz = 1,
                                    const void* W2 = nullptr, int w2mode = 0);

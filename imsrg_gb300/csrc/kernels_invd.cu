@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(kThreads) k_pandya_inv_desc(const int4* __rest
   if (zo) {
     Zb = (const double*)((const char*)Zb + zo[blockIdx.z * kZRoles + ZR_ZB]);
     Z = (double*)((char*)Z + zo[blockIdx.z * kZRoles + ZR_Z]);
+    W2 = (const char*)W2 + (w2mode ? zo[blockIdx.z * kZRoles + ZR_W2] : 0);
   }
   extern __shared__ __align__(16) unsigned char smem[];
   const int4 bk = blocks[blockIdx.x];
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(kThreads) k_pandya_inv_desc(const int4* __rest
 cudaError_t launch_pandya_inv_desc(const Space& s, const InvdDev& d, bool df, const double* Zb, double* Z, int hZ,
                                    cudaStream_t st, const long long* zo, int nz, const void* W2, int w2mode)
 {
-  if (w2mode && (zo || !d.covers_all)) return cudaErrorInvalidValue;
+  if (w2mode && !d.covers_all) return cudaErrorInvalidValue;
   if (d.nblocks == 0) return cudaSuccess;
   const size_t smem = (size_t)d.stage_max * 8;
   using Kern = void (*)(const int4*, const int2*, const int2*, const int*, const unsigned short*, const int4*,

@@ -25,7 +25,7 @@
 //    every output and chunk.  The digit error is about sqrt(K) 2^-63 (unit:
 //    the rows' exponents) and that of an FP64 sum about 2^-54 sum |a||b|, so
 //    an element with 0 < sum |a||b| < 2^-9 sqrt(K) is not written but listed,
-//    and k_dgemm_exact evaluates it with FP64 FMAs.  A tile with many such
+//    and the CTA evaluates it with FP64 FMAs after its tiles.  A tile with many such
 //    elements is listed whole, and so are tiles with a row that holds an
 //    infinity, a NaN or magnitudes outside 2^-423 .. 2^477, and tiles that a
 //    timed-out wait left undone.  (Random operators list a few elements of
@@ -67,6 +67,7 @@ constexpr int NP = S + 1;    // planes: digits, then magnitudes
 constexpr int NHI = 5;       // weights summed in the leading integer word
 constexpr int CH = 20;       // K blocks per chunk: 6 x 65^2 x 32 CH < 2^24
 constexpr int NSTAGE = 2;    // 2 x 100 KB of 227 KB
+constexpr int SHORT_KB = 4;  // K blocks a job in plans that are sliced in one pass
 constexpr int NINFO = 3;     // tiles whose job, exponents and phases wait in shared memory
 constexpr int EPIW = 8;      // epilogue warps: two per TMEM lane quarter, 16 columns each
 constexpr int COLS_W = TN / 2;
@@ -112,7 +113,7 @@ struct DgemmPlan {
   DTile* d_tiles = nullptr;
   int* d_cta = nullptr;
   __nv_bfloat16* arr[2] = {nullptr, nullptr};  // planes of A and of B
-  int* d_exp = nullptr;   // [2 exp_rows] raw row exponents of A, of B; then the counts of listed tiles and elements
+  int* d_exp = nullptr;   // [2 exp_rows] raw row exponents of A, of B
   int* d_list = nullptr;  // tiles to evaluate exactly
   DElem* d_elem = nullptr;
   int4 *d_rblk = nullptr, *d_dblk = nullptr;
@@ -234,48 +235,42 @@ __device__ __forceinline__ unsigned magnitude_of(double v, int e)
   return ((unsigned)(127 + min(x, 0)) << 7) | (unsigned)((b >> 45) & 0x7F);
 }
 
-// The ten planes of A and of B: a block per listed (job, 32-row group, KB-column group), through shared
-// memory to 16-byte stores (a plane's 32 x KB values are 2 KB in a row).
-// Bound by HBM: 16 bytes read and 40 written per element pair; every operand
-// load of a thread is issued before its first conversion.
-__global__ void __launch_bounds__(256) k_dgemm_digits(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
-                                                      const double* __restrict__ Abase, const double* __restrict__ B0,
-                                                      const double* __restrict__ B1, const int* __restrict__ kidx,
-                                                      const double* __restrict__ kw, double gbscale,
-                                                      const int* __restrict__ rexpA, const int* __restrict__ rexpB,
-                                                      long long plane_rows, __nv_bfloat16* __restrict__ pA,
-                                                      __nv_bfloat16* __restrict__ pB)
+// The ten planes of A and of B for 32 rows from r0 and KB columns from t0 of
+// a job, by a block of 256 threads: through shared memory to 16-byte stores
+// (a plane's 32 x KB values are 2 KB in a row).  Bound by HBM: 16 bytes read
+// and 40 written per element pair; every operand load of a thread is issued
+// before its first conversion.  s_e: the rows' exponents in A and B.
+constexpr int RW = (KB + 2) / 2;  // 17 words a row: a warp's 32 rows in 32 banks
+struct SliceShared {
+  unsigned dg[NP][32][RW];
+  int e[2][32], col[KB], kind[KB];
+  double sc[KB];
+};
+
+__device__ __forceinline__ void slice_block(SliceShared& sh, const DJob& jb, const double* __restrict__ A,
+                                            const double* __restrict__ B, int r0, int kb, const int* __restrict__ kidx,
+                                            const double* __restrict__ kw, double gbscale, long long plane_rows,
+                                            __nv_bfloat16* __restrict__ pA, __nv_bfloat16* __restrict__ pB)
 {
-  constexpr int RW = (KB + 2) / 2;  // 17 words a row: a warp's 32 rows in 32 banks
-  __shared__ unsigned dg[NP][32][RW];
-  __shared__ int s_e[2][32], s_col[KB], s_kind[KB];
-  __shared__ double s_sc[KB];
-  const int4 bk = blocks[blockIdx.x];
-  const DJob jb = jobs[bk.x];
-  const int r0 = bk.y * 32, t0 = bk.z * KB;
-  if (threadIdx.x < 32) {
-    s_e[0][threadIdx.x] = row_e(rexpA[jb.exp_base + r0 + threadIdx.x]);
-    s_e[1][threadIdx.x] = row_e(rexpB[jb.exp_base + r0 + threadIdx.x]);
-  } else if (threadIdx.x < 32 + KB) {
+  const int t0 = kb * KB;
+  if (threadIdx.x >= 32 && threadIdx.x < 32 + KB) {
     const int tt = threadIdx.x - 32, t = t0 + tt;
-    s_col[tt] = t < jb.K ? (jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t) : 0;
-    s_sc[tt] = t < jb.K ? jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0) : 1.0;
-    s_kind[tt] = scale_kind(s_sc[tt]);
+    sh.col[tt] = t < jb.K ? (jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t) : 0;
+    sh.sc[tt] = t < jb.K ? jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0) : 1.0;
+    sh.kind[tt] = scale_kind(sh.sc[tt]);
   }
   __syncthreads();
-  const double* A = Abase + jb.a_off;
-  const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
   constexpr int NIT = 32 * (KB / 2) / 256;
   double v[2][NIT][2];
 #pragma unroll
   for (int u = 0; u < NIT; ++u) {
-    const int e = threadIdx.x + u * 256, r = e & 31, i = r0 + r;
+    const int e = threadIdx.x + u * 256, i = r0 + (e & 31);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int tt = 2 * (e >> 5) + h;
       const bool ok = t0 + tt < jb.K;
-      v[0][u][h] = ok && i < jb.m ? A[(long long)s_col[tt] * jb.lda + i] : 0.0;
-      v[1][u][h] = ok && i < jb.n ? B[(long long)s_col[tt] * jb.ldb + i] : 0.0;
+      v[0][u][h] = ok && i < jb.m ? A[(long long)sh.col[tt] * jb.lda + i] : 0.0;
+      v[1][u][h] = ok && i < jb.n ? B[(long long)sh.col[tt] * jb.ldb + i] : 0.0;
     }
   }
   long long bias = 0;  // half a digit in every lower digit: the fields of q + bias minus half are balanced
@@ -290,35 +285,94 @@ __global__ void __launch_bounds__(256) k_dgemm_digits(const DJob* __restrict__ j
       unsigned mag[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const double x = op ? scaled(v[1][u][h], s_kind[2 * tp + h], s_sc[2 * tp + h]) : v[0][u][h];
-        q[h] = fixed_of(x, s_e[op][r]) + bias;
-        mag[h] = magnitude_of(x, s_e[op][r]);
+        const double x = op ? scaled(v[1][u][h], sh.kind[2 * tp + h], sh.sc[2 * tp + h]) : v[0][u][h];
+        q[h] = fixed_of(x, sh.e[op][r]) + bias;
+        mag[h] = magnitude_of(x, sh.e[op][r]);
       }
 #pragma unroll
       for (int s = 0; s < S; ++s) {
-        const int sh = BETA * (S - 1 - s);
+        const int shf = BETA * (S - 1 - s);
         // small integer -> BF16: 1.5 * 2^23 + x minus 1.5 * 2^23, upper half; "- half" rides in the constant
         const int mg = s == 0 ? 0x4B400000 : 0x4B400000 - (1 << (BETA - 1));
         float f[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int x = s == 0 ? (int)(q[h] >> sh) : (int)((unsigned)(q[h] >> sh) & ((1u << BETA) - 1));
+          const int x = s == 0 ? (int)(q[h] >> shf) : (int)((unsigned)(q[h] >> shf) & ((1u << BETA) - 1));
           f[h] = __int_as_float(mg + x) - 12582912.0f;
         }
-        dg[s][r][tp] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
+        sh.dg[s][r][tp] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
       }
-      dg[S][r][tp] = mag[0] | (mag[1] << 16);
+      sh.dg[S][r][tp] = mag[0] | (mag[1] << 16);
     }
     __syncthreads();
     __nv_bfloat16* out = op ? pB : pA;
-    const long long row0 = jb.row_base + (long long)bk.z * jb.m_pad + r0;
+    const long long row0 = jb.row_base + (long long)kb * jb.m_pad + r0;
     for (int e = threadIdx.x; e < NP * 32 * (KB / 8); e += 256) {
       const int x = e % (KB / 8), r = (e / (KB / 8)) & 31, s = e / (32 * (KB / 8));
-      const unsigned* d = &dg[s][r][x * 4];
+      const unsigned* d = &sh.dg[s][r][x * 4];
       *(uint4*)(out + ((long long)s * plane_rows + row0 + r) * KB + x * 8) = make_uint4(d[0], d[1], d[2], d[3]);
     }
     __syncthreads();
   }
+}
+
+// long reductions: a block per listed (job, 32-row group, KB-column group),
+// the row exponents from k_dgemm_rowexp
+__global__ void __launch_bounds__(256) k_dgemm_digits(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
+                                                      const double* __restrict__ Abase, const double* __restrict__ B0,
+                                                      const double* __restrict__ B1, const int* __restrict__ kidx,
+                                                      const double* __restrict__ kw, double gbscale,
+                                                      const int* __restrict__ rexpA, const int* __restrict__ rexpB,
+                                                      long long plane_rows, __nv_bfloat16* __restrict__ pA,
+                                                      __nv_bfloat16* __restrict__ pB)
+{
+  __shared__ SliceShared sh;
+  const int4 bk = blocks[blockIdx.x];
+  const DJob jb = jobs[bk.x];
+  const int r0 = bk.y * 32;
+  if (threadIdx.x < 32) {
+    sh.e[0][threadIdx.x] = row_e(rexpA[jb.exp_base + r0 + threadIdx.x]);
+    sh.e[1][threadIdx.x] = row_e(rexpB[jb.exp_base + r0 + threadIdx.x]);
+  }
+  slice_block(sh, jb, Abase + jb.a_off, (jb.bsel ? B1 : B0) + jb.b_off, r0, bk.z, kidx, kw, gbscale, plane_rows, pA, pB);
+}
+
+// short reductions (at most SHORT_KB K blocks a job): exponents and planes of
+// a 32-row group in one block, one launch where the long form takes a clear
+// and two
+__global__ void __launch_bounds__(256) k_dgemm_slice(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
+                                                     const double* __restrict__ Abase, const double* __restrict__ B0,
+                                                     const double* __restrict__ B1, const int* __restrict__ kidx,
+                                                     const double* __restrict__ kw, double gbscale, int* __restrict__ rexpA,
+                                                     int* __restrict__ rexpB, long long plane_rows,
+                                                     __nv_bfloat16* __restrict__ pA, __nv_bfloat16* __restrict__ pB)
+{
+  __shared__ SliceShared sh;
+  __shared__ int s_max[2][8][33];
+  const int4 bk = blocks[blockIdx.x];
+  const DJob jb = jobs[bk.x];
+  const int r0 = bk.y * 32, r = threadIdx.x & 31, ty = threadIdx.x >> 5, i = r0 + r;
+  const double* A = Abase + jb.a_off;
+  const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
+  int ea = 0, eb = 0;
+#pragma unroll 4
+  for (int t = ty; t < jb.K; t += 8) {
+    const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
+    const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
+    if (i < jb.m) ea = max(ea, dexp1(A[col * jb.lda + i]));
+    if (i < jb.n) eb = max(eb, dexp1(scaled(B[col * jb.ldb + i], scale_kind(sc), sc)));
+  }
+  s_max[0][ty][r] = ea;
+  s_max[1][ty][r] = eb;
+  __syncthreads();
+  if (ty < 2) {
+    int e = 0;
+    for (int y = 0; y < 8; ++y) e = max(e, s_max[ty][y][r]);
+    sh.e[ty][r] = row_e(e);
+    (ty ? rexpB : rexpA)[jb.exp_base + i] = e;
+  }
+  for (int kb = 0; kb < jb.nkb; ++kb)  // (slice_block's first barrier covers sh.e)
+    slice_block(sh, jb, A, B, r0, kb, kidx, kw, gbscale, plane_rows, pA, pB);
 }
 
 struct DArgs {
@@ -328,9 +382,15 @@ struct DArgs {
   const int *rexpA, *rexpB;
   const int* phase;
   double* out;
-  int* nlist;  // to evaluate exactly: counts of tiles and elements, then the lists
+  // to evaluate exactly: each CTA lists its own tiles from its first tile's
+  // place, and its elements from MAX_LISTED COLS_W times that
   int* list;
   DElem* elem;
+  // for that: the operands as they are
+  const double *A, *B0, *B1;
+  const int* kidx;
+  const double* kw;
+  double gbscale;
   int gsign, accum, nomirror;
 };
 
@@ -410,6 +470,106 @@ __device__ __forceinline__ double value_of(long long hi, long long lo, int X)
   return zero ? 0.0 : __hiloint2double((int)(mh | (sg & 0x80000000u)), (int)ml);
 }
 
+// out (+)= v at (i, j) and, for a symmetrised job, its mirror
+__device__ __forceinline__ void put_exact(const DJob& jb, double* O, const int* ph, double sgn, int i, int j, double p1,
+                                          double p2, bool accumulate, int nomirror)
+{
+  double* d = O + (long long)j * jb.ldo + i;
+  if (jb.nosym) {
+    *d = accumulate ? *d + p1 : p1;
+    return;
+  }
+  const double f = sgn * (ph ? (double)(ph[i] * ph[j]) : 1.0);
+  const double v = p1 + f * p2, w = p2 + f * p1;
+  *d = accumulate ? *d + v : v;
+  if (i != j && !nomirror) {
+    double* t = O + (long long)i * jb.ldo + j;
+    *t = accumulate ? *t + w : w;
+  }
+}
+
+// The CTA's listed tiles and elements with FP64 FMAs, by its 256 epilogue
+// threads: tiles with a 4 x 4 block of both products a thread, in the
+// summation order of the FP64 kernel (kernels_gemm.cu); elements by a warp
+// each, lanes over K.  Bound by the FP64 pipe by far, so operands come
+// straight from global memory.  (As a kernel of its own it took 4 us a
+// product with nothing to do.)
+__device__ __noinline__ void exact_work(const DArgs& g, int tbeg, int ntile, int nelem)
+{
+  const int tid = threadIdx.x - 64, tx = tid & 7, ty = tid >> 3, lane = tid & 31;
+  const DElem* elem = g.elem + (long long)tbeg * MAX_LISTED * COLS_W;
+  for (int e = 0; e < ntile; ++e) {
+    const DTile tl = g.tiles[g.list[tbeg + e]];
+    const DJob jb = g.jobs[tl.job];
+    const double* A = g.A + jb.a_off;
+    const double* B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
+    const int i0 = tl.I * TM + ty * 4, j0 = tl.J * TN + tx * 4;
+    // rows past the end repeat the last one (and are not written)
+    int ia[4], ib[4], ja[4], jn[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      ia[a] = min(i0 + a, jb.m - 1);
+      ib[a] = min(i0 + a, jb.n - 1);
+      ja[a] = min(j0 + a, jb.m - 1);
+      jn[a] = min(j0 + a, jb.n - 1);
+    }
+    double acc1[4][4] = {}, acc2[4][4] = {};
+    for (int t = 0; t < jb.K; ++t) {
+      const long long col = jb.kidx_off >= 0 ? g.kidx[jb.kidx_off + t] : t;
+      const double sc = jb.bscale * g.gbscale * (jb.w_off >= 0 ? g.kw[jb.w_off + t] : 1.0);
+      double x[4], y[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        x[a] = A[col * jb.lda + ia[a]];
+        y[a] = sc * B[col * jb.ldb + jn[a]];
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc1[a][b] = fma(x[a], y[b], acc1[a][b]);
+      if (jb.nosym) continue;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        x[a] = A[col * jb.lda + ja[a]];
+        y[a] = sc * B[col * jb.ldb + ib[a]];
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc2[a][b] = fma(x[b], y[a], acc2[a][b]);
+    }
+    const int* ph = jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (i0 + a < jb.m && j0 + b < jb.n && (jb.nosym || i0 + a <= j0 + b))
+          put_exact(jb, g.out + jb.out_off, ph, jb.sign != 0 ? jb.sign : g.gsign, i0 + a, j0 + b, acc1[a][b], acc2[a][b],
+                    g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+  }
+  for (int e = tid >> 5; e < nelem; e += 8) {
+    const DTile tl = g.tiles[elem[e].tile];
+    const DJob jb = g.jobs[tl.job];
+    const double* A = g.A + jb.a_off;
+    const double* B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
+    const int i = tl.I * TM + (elem[e].ij & 0xFFFF), j = tl.J * TN + (elem[e].ij >> 16);
+    double p1 = 0.0, p2 = 0.0;
+    for (int t = lane; t < jb.K; t += 32) {
+      const long long col = jb.kidx_off >= 0 ? g.kidx[jb.kidx_off + t] : t;
+      const double sc = jb.bscale * g.gbscale * (jb.w_off >= 0 ? g.kw[jb.w_off + t] : 1.0);
+      p1 = fma(A[col * jb.lda + i], sc * B[col * jb.ldb + j], p1);
+      if (!jb.nosym) p2 = fma(A[col * jb.lda + j], sc * B[col * jb.ldb + i], p2);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+      p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+    }
+    if (lane == 0)
+      put_exact(jb, g.out + jb.out_off, jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr,
+                jb.sign != 0 ? jb.sign : g.gsign, i, j, p1, p2, g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+  }
+}
+
 // Persistent kernel, one CTA per SM, each with its own run of tiles:
 //   warp 0: TMA producer; warp 1: tensor memory and MMA issue (one thread);
 //   warps 2-9: epilogue; warp 10: tile information.
@@ -430,7 +590,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   unsigned long long* bars = (unsigned long long*)(smem + NSTAGE * STAGE);
   unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 3 + 2 * NINFO);
   __shared__ TileInfo s_info[NINFO];
-  __shared__ int s_err_, s_epi_err_;
+  __shared__ int s_err_, s_epi_err_, s_nlist[2];  // listed tiles, elements
   volatile int& s_err = s_err_;
   volatile int& s_epi_err = s_epi_err_;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -444,6 +604,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   if (threadIdx.x == 0) {
     s_err = 0;
     s_epi_err = 0;
+    s_nlist[0] = s_nlist[1] = 0;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -677,12 +838,12 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
                    : "r"(bad), "r"(EPI_T)
                    : "memory");
       if (nbad > MAX_LISTED) {
-        if (threadIdx.x == 64) g.list[atomicAdd(g.nlist, 1)] = tbeg + t;
+        if (threadIdx.x == 64) g.list[tbeg + atomicAdd(&s_nlist[0], 1)] = tbeg + t;
         mbar_arrive(info_empty(t % NINFO));
         continue;
       }
       for (unsigned b = bad; b; b &= b - 1)
-        g.elem[atomicAdd(g.nlist + 1, 1)] = {tbeg + t, row | ((cbeg + __ffs(b) - 1) << 16)};
+        g.elem[(long long)tbeg * MAX_LISTED * COLS_W + atomicAdd(&s_nlist[1], 1)] = {tbeg + t, row | ((cbeg + __ffs(b) - 1) << 16)};
       if (!nosym) {
         const int sp = f.prow[row];
 #pragma unroll
@@ -725,111 +886,18 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         }
       }
     }
-    // a wait that ran out: the tiles not written go to k_dgemm_exact
+    // a wait that ran out: the tiles not written are listed
     if (threadIdx.x == 64)
-      for (; t < ntile; ++t) g.list[atomicAdd(g.nlist, 1)] = tbeg + t;
+      for (; t < ntile; ++t) g.list[tbeg + atomicAdd(&s_nlist[0], 1)] = tbeg + t;
+    // the lists are this CTA's own: written by these threads, read by them
+    __threadfence_block();
+    asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
+    if (s_nlist[0] | s_nlist[1]) exact_work(g, tbeg, s_nlist[0], s_nlist[1]);
   }
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-  }
-}
-
-// out (+)= v at (i, j) and, for a symmetrised job, its mirror
-__device__ __forceinline__ void put_exact(const DJob& jb, double* O, const int* ph, double sgn, int i, int j, double p1,
-                                          double p2, bool accumulate, int nomirror)
-{
-  double* d = O + (long long)j * jb.ldo + i;
-  if (jb.nosym) {
-    *d = accumulate ? *d + p1 : p1;
-    return;
-  }
-  const double f = sgn * (ph ? (double)(ph[i] * ph[j]) : 1.0);
-  const double v = p1 + f * p2, w = p2 + f * p1;
-  *d = accumulate ? *d + v : v;
-  if (i != j && !nomirror) {
-    double* t = O + (long long)i * jb.ldo + j;
-    *t = accumulate ? *t + w : w;
-  }
-}
-
-// The listed tiles and elements with FP64 FMAs: tiles by 256 threads, each a
-// 4 x 4 block of both products, in the summation order of the FP64 kernel
-// (kernels_gemm.cu); elements by a warp each, lanes over K.  Bound by the
-// FP64 pipe; empty lists cost one short launch.
-__global__ void __launch_bounds__(256) k_dgemm_exact(const DJob* __restrict__ jobs, const DTile* __restrict__ tiles,
-                                                     const int* __restrict__ nlist, const int* __restrict__ list,
-                                                     const DElem* __restrict__ elem, const double* __restrict__ Abase,
-                                                     const double* __restrict__ B0, const double* __restrict__ B1,
-                                                     double* __restrict__ Obase, const int* __restrict__ kidx,
-                                                     const double* __restrict__ kw, const int* __restrict__ phase, int gsign,
-                                                     double gbscale, int accum, int nomirror)
-{
-  constexpr int TK = 8;
-  __shared__ double sAI[TK][TM], sBI[TK][TM], sAJ[TK][TN], sBJ[TK][TN];
-  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, lane = threadIdx.x & 31;
-  const int ntile = nlist[0], nelem = nlist[1];
-  for (int e = blockIdx.x; e < ntile; e += gridDim.x) {
-    const DTile tl = tiles[list[e]];
-    const DJob jb = jobs[tl.job];
-    const double* A = Abase + jb.a_off;
-    const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
-    const int i0 = tl.I * TM, j0 = tl.J * TN;
-    double acc1[4][4] = {}, acc2[4][4] = {};
-    for (int k0 = 0; k0 < jb.K; k0 += TK) {
-      const int nk = min(TK, jb.K - k0);
-      __syncthreads();
-      for (int x = threadIdx.x; x < nk * (TM + TN); x += 256) {
-        const int kk = x / (TM + TN), y = x % (TM + TN), t = k0 + kk;
-        const int r = y < TM ? i0 + y : j0 + y - TM;
-        const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
-        const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
-        const double a = r < jb.m ? A[col * jb.lda + r] : 0.0, b = r < jb.n ? sc * B[col * jb.ldb + r] : 0.0;
-        (y < TM ? sAI[kk][y] : sAJ[kk][y - TM]) = a;
-        (y < TM ? sBI[kk][y] : sBJ[kk][y - TM]) = b;
-      }
-      __syncthreads();
-      for (int kk = 0; kk < nk; ++kk)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            acc1[a][b] = fma(sAI[kk][ty * 4 + a], sBJ[kk][tx * 4 + b], acc1[a][b]);
-            if (!jb.nosym) acc2[a][b] = fma(sAJ[kk][tx * 4 + b], sBI[kk][ty * 4 + a], acc2[a][b]);
-          }
-    }
-    const int* ph = jb.phase_off >= 0 ? phase + jb.phase_off : nullptr;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int i = i0 + ty * 4 + a, j = j0 + tx * 4 + b;
-        if (i < jb.m && j < jb.n && (jb.nosym || i <= j))
-          put_exact(jb, Obase + jb.out_off, ph, jb.sign != 0 ? jb.sign : gsign, i, j, acc1[a][b], acc2[a][b],
-                    accum > 0 || (accum < 0 && jb.accumulate), nomirror);
-      }
-  }
-  for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < nelem; e += gridDim.x * 8) {
-    const DTile tl = tiles[elem[e].tile];
-    const DJob jb = jobs[tl.job];
-    const double* A = Abase + jb.a_off;
-    const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
-    const int i = tl.I * TM + (elem[e].ij & 0xFFFF), j = tl.J * TN + (elem[e].ij >> 16);
-    double p1 = 0.0, p2 = 0.0;
-    for (int t = lane; t < jb.K; t += 32) {
-      const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
-      const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
-      p1 = fma(A[col * jb.lda + i], sc * B[col * jb.ldb + j], p1);
-      if (!jb.nosym) p2 = fma(A[col * jb.lda + j], sc * B[col * jb.ldb + i], p2);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
-      p2 += __shfl_xor_sync(0xffffffffu, p2, o);
-    }
-    if (lane == 0)
-      put_exact(jb, Obase + jb.out_off, jb.phase_off >= 0 ? phase + jb.phase_off : nullptr, jb.sign != 0 ? jb.sign : gsign, i,
-                j, p1, p2, accum > 0 || (accum < 0 && jb.accumulate), nomirror);
   }
 }
 
@@ -929,14 +997,17 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     first[b + 1] = (int)sorted.size();
   }
   std::vector<int4> rb, db;
+  int nkb_max = 0;
+  for (const DJob& d : jobs) nkb_max = std::max(nkb_max, d.nkb);
+  const bool shorts = nkb_max <= SHORT_KB;  // one slicing pass (n_dblk stays 0)
   for (int j = 0; j < p->njobs; ++j) {
     const DJob& d = jobs[j];
     if (d.m == 0 || d.n == 0 || d.K == 0) continue;
     for (int y = 0; y < d.m_pad / 32; ++y)
-      for (int x = 0; x < (d.K + 255) / 256; ++x) rb.push_back(make_int4(j, y, x, 0));
+      for (int x = 0; x < (shorts ? 1 : (d.K + 255) / 256); ++x) rb.push_back(make_int4(j, y, x, 0));
   }
   // the digit pass starts on the operands that the exponent pass read last
-  for (int j = p->njobs - 1; j >= 0; --j) {
+  for (int j = p->njobs - 1; j >= 0 && !shorts; --j) {
     const DJob& d = jobs[j];
     if (d.m == 0 || d.n == 0 || d.K == 0) continue;
     for (int x = 0; x < d.nkb; ++x)
@@ -962,7 +1033,7 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
       return q;
     };
     for (int a = 0; a < 2; ++a) p->arr[a] = (__nv_bfloat16*)dm((size_t)NP * p->rows * KB * 2);
-    p->d_exp = (int*)dm(sizeof(int) * (2 * p->exp_rows + 2));
+    p->d_exp = (int*)dm(sizeof(int) * 2 * p->exp_rows);
     p->d_list = (int*)dm(sizeof(int) * p->ntiles);
     p->d_elem = (DElem*)dm(sizeof(DElem) * MAX_LISTED * COLS_W * (size_t)p->ntiles);
     p->d_jobs = (DJob*)up(jobs.data(), sizeof(DJob) * jobs.size());
@@ -1005,23 +1076,28 @@ cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, 
                          cudaStream_t st)
 {
   if (p->ntiles == 0) return cudaSuccess;
-  int *rexpA = p->d_exp, *rexpB = p->d_exp + p->exp_rows, *nlist = p->d_exp + 2 * p->exp_rows;
+  int *rexpA = p->d_exp, *rexpB = p->d_exp + p->exp_rows;
   cudaError_t e;
   {
     ProfScope ps(p->family == 0 ? "dgemm_slice_ladder" : "dgemm_slice_zbar", st);
-    if ((e = cudaMemsetAsync(p->d_exp, 0, sizeof(int) * (2 * p->exp_rows + 2), st)) != cudaSuccess) return e;
-    k_dgemm_rowexp<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB);
-    k_dgemm_digits<<<p->n_dblk, 256, 0, st>>>(p->d_jobs, p->d_dblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
-                                              p->arr[0], p->arr[1]);
-    count_launch(2);
+    if (p->n_dblk == 0) {
+      k_dgemm_slice<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
+                                               p->arr[0], p->arr[1]);
+      count_launch();
+    } else {
+      if ((e = cudaMemsetAsync(p->d_exp, 0, sizeof(int) * 2 * p->exp_rows, st)) != cudaSuccess) return e;
+      k_dgemm_rowexp<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB);
+      k_dgemm_digits<<<p->n_dblk, 256, 0, st>>>(p->d_jobs, p->d_dblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
+                                                p->arr[0], p->arr[1]);
+      count_launch(2);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   ProfScope ps(p->family == 0 ? "dgemm_ladder" : "dgemm_zbar", st);
-  DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA, rexpB, phase, O, nlist, p->d_list, p->d_elem, gsign, accum, mirror ? 0 : 1};
+  DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA,   rexpB, phase, O,  p->d_list, p->d_elem,
+          A,         B0,         B1,       kidx,    kw,    gbscale, gsign, accum, mirror ? 0 : 1};
   k_dgemm<<<p->grid, 96 + 32 * EPIW, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], a);
-  k_dgemm_exact<<<std::min(p->ntiles, 2 * p->grid), 256, 0, st>>>(p->d_jobs, p->d_tiles, nlist, p->d_list, p->d_elem, A, B0, B1, O, kidx,
-                                                                 kw, phase, gsign, gbscale, accum, a.nomirror);
-  count_launch(2);
+  count_launch();
   return cudaGetLastError();
 }
 

@@ -84,6 +84,14 @@ bool capturing(cudaStream_t st)
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
+int second_stream(imsrg_space* sp)
+{
+  if (sp->side) return IMSRG_OK;
+  CUDA_TRY(cudaStreamCreateWithFlags(&sp->side, cudaStreamNonBlocking));
+  CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_fork, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_join, cudaEventDisableTiming));
+  return IMSRG_OK;
+}
 }  // namespace imsrg
 
 // struct imsrg_space / imsrg_op: capi_internal.hpp
@@ -775,11 +783,7 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
     std::copy(g_term_on, g_term_on + NTERMS, on);
   }
   imsrg_space* sp = X->sp;
-  if (!sp->side) {
-    CUDA_TRY(cudaStreamCreateWithFlags(&sp->side, cudaStreamNonBlocking));
-    CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_fork, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_join, cudaEventDisableTiming));
-  }
+  if ((rc = second_stream(sp))) return rc;
   cudaStream_t sd = sp->side;
   ProfScope ps("CommutatorScalarScalar", st);
   const bool ladder_first = on[T222PPHH];

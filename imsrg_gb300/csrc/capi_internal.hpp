@@ -26,6 +26,8 @@ namespace imsrg {
 int set_error(int code, const char* msg);
 // whether st is being captured into a graph (nothing may be allocated then)
 bool capturing(cudaStream_t st);
+// makes the space's second stream and its events
+int second_stream(imsrg_space* sp);
 // CommutatorScalarScalar into Z (overwritten), Operator::Norm (synchronises
 // st), and the kernels' error word (synchronises st; IMSRG_ERR_KERNEL if set)
 int commutator_dev(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st);

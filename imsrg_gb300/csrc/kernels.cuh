@@ -144,9 +144,10 @@ struct TensorLayout;
 cudaError_t launch_tensor_111(const Space& s, const double* X, const double* Y, double* Z, cudaStream_t st);
 cudaError_t launch_tensor_121(const Space& s, const TensorLayout& t, const int* dev_holes, const double* X,
                               const double* Y, int hY, double* Z, int hZ, cudaStream_t st);
-// YT: scratch of layout t (Y with its blocks transposed, written here)
+// YT (layout t): Y with its blocks transposed
+cudaError_t launch_tensor_transpose(const Space& s, const TensorLayout& t, const double* Y, double* YT, cudaStream_t st);
 cudaError_t launch_tensor_122(const Space& s, const TensorLayout& t, const double* X, const double* Y, int hX,
-                              double* YT, double* Z, cudaStream_t st);
+                              const double* YT, double* Z, cudaStream_t st);
 // XW, WX: scratch of the space's arena length; D (= Mpp - Mhh), Mhh: scratch
 // arenas of layout t
 cudaError_t launch_tensor_222_221(const Space& s, const TensorLayout& t, const double* X, const double* Y,
@@ -158,12 +159,11 @@ cudaError_t launch_tensor_ph(const Space& s, const TensorLayout& t, const double
 // Operator::Norm of a tensor of layout t: partial[0 .. nrm2_off.size()] are
 // the two-body chunks' weighted sums of squares, then the one-body one
 cudaError_t launch_tensor_norm(const TensorLayout& t, const double* A, double* partial, cudaStream_t st);
-// split form: the operands the split products read (Y with its blocks
-// transposed, the tensor Pandya panels transposed and half-swapped, X bar
-// half-swapped); the ladder's remainder (Mhh, Z2 += D, the one-body part) once
+// the operands the products read besides X and Y transposed (the tensor
+// Pandya panels transposed and half-swapped, X bar half-swapped); the ladder's remainder (Mhh, Z2 += D, the one-body part) once
 // D = Mpp - Mhh is in place; the inverse tensor Pandya transform of Zbar
 cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, const double* Y, int hY,
-                                         const double* Xbar, double* YT, double* YbT, double* YbTF, double* XbF,
+                                         const double* Xbar, double* YbT, double* YbTF, double* XbF,
                                          cudaStream_t st);
 cudaError_t launch_tensor_222_221_split(const Space& s, const TensorLayout& t, const double* X, const double* Y,
                                         double* D, double* Mhh, double* Z, int hZ, cudaStream_t st);

@@ -996,15 +996,19 @@ cudaError_t launch_tensor_121(const Space& s, const TensorLayout& t, const int* 
   return cudaGetLastError();
 }
 
+cudaError_t launch_tensor_transpose(const Space& s, const TensorLayout& t, const double* Y, double* YT, cudaStream_t st)
+{
+  if (t.bra.empty() || t.max_tiles32 == 0) return cudaSuccess;
+  k_ttranspose<<<dim3((unsigned)t.max_tiles32, (unsigned)t.bra.size()), dim3(32, 8), 0, st>>>(s.dev, t.dev, Y, YT);
+  count_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_tensor_122(const Space& s, const TensorLayout& t, const double* X, const double* Y, int hX,
-                              double* YT, double* Z, cudaStream_t st)
+                              const double* YT, double* Z, cudaStream_t st)
 {
   if (t.bra.empty() || t.max_blk_elems == 0) return cudaSuccess;
   cudaError_t e;
-  // Y^T for the bra side
-  k_ttranspose<<<dim3((unsigned)t.max_tiles32, (unsigned)t.bra.size()), dim3(32, 8), 0, st>>>(s.dev, t.dev, Y, YT);
-  count_launch();
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int LY = std::max(1, 2 * t.max_ob), LX = std::max(1, 2 * t.max_tob);
   const size_t smem = (size_t)32 * (LY + LX) * (sizeof(double) + sizeof(int)) + 64 * sizeof(int);
   if (smem > 40 * 1024) {
@@ -1067,16 +1071,10 @@ cudaError_t launch_tensor_ph(const Space& s, const TensorLayout& t, const double
 
 // ---------------------------------------------------------- split form
 cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, const double* Y, int hY,
-                                         const double* Xbar, double* YT, double* YbT, double* YbTF, double* XbF,
+                                         const double* Xbar, double* YbT, double* YbTF, double* XbF,
                                          cudaStream_t st)
 {
   cudaError_t e;
-  if (!t.bra.empty() && t.max_tiles32 > 0) {
-    k_ttranspose<<<dim3((unsigned)t.max_tiles32, (unsigned)t.bra.size()), dim3(32, 8), 0, st>>>(s.dev, t.dev, Y,
-                                                                                              YT);
-    count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
   if (!t.yb_bra.empty()) {
     dim3 gy(grid_for(std::max(1, t.yb_maxelems)), (unsigned)t.yb_bra.size());
     k_tpandya<<<gy, 256, 0, st>>>(s.dev, s.work, t.dev, Y, hY, YbT, YbTF);

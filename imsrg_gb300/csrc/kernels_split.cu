@@ -256,28 +256,22 @@ __global__ void __launch_bounds__(256) k_split_rowexp(const SplitJob* __restrict
   }
 }
 
-// signed 64-bit integer times 2^X as a double, integer instructions only
-// (round to nearest even); 0 on underflow of the exponent range.
+// signed 64-bit integer times 2^X as a double, integer instructions only and
+// no branch (round to nearest even; 0 below the exponent range, infinity above)
 __device__ __forceinline__ double i64_ldexp(long long v, int X)
 {
-  if (v == 0) return 0.0;
-  unsigned long long sgn = v < 0 ? (1ull << 63) : 0ull;
-  unsigned long long u = v < 0 ? (unsigned long long)(-v) : (unsigned long long)v;
-  int lz = __clzll((long long)u);
-  unsigned long long m = u << lz;            // leading one at bit 63
-  unsigned long long mant = m >> 11;         // 53 bits
-  unsigned long long rest = m & 0x7FFull;
-  if (rest > 0x400ull || (rest == 0x400ull && (mant & 1ull))) {
-    ++mant;
-    if (mant >> 53) {
-      mant >>= 1;
-      --lz;
-    }
-  }
-  int e = (63 - lz) + 1023 + X;
-  if (e <= 0) return 0.0;
-  if (e >= 2047) return __longlong_as_double((long long)(sgn | (0x7FFull << 52)));
-  return __longlong_as_double((long long)(sgn | ((unsigned long long)e << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+  const long long sg = v >> 63;
+  unsigned long long u = (unsigned long long)((v ^ sg) - sg);
+  const int lz = __clzll((long long)u);
+  u <<= lz & 63;  // leading one at bit 63
+  const unsigned odd = (unsigned)(u >> 11) & 1u;
+  const unsigned long long mant = (u >> 11) + (((unsigned)u & 0x7FFu) + odd > 0x400u ? 1u : 0u);
+  const int e = 63 - lz + 1023 + X;
+  // the leading one carries into the exponent field (and so does a carry out of rounding)
+  unsigned long long b = mant + ((unsigned long long)(unsigned)(e - 1) << 52);
+  b = e >= 2047 ? 0x7FFull << 52 : b;
+  b = e <= 0 || lz == 64 ? 0ull : b;
+  return __longlong_as_double((long long)(b | ((unsigned long long)sg & 0x8000000000000000ull)));
 }
 
 // exponent of row i (A side) from the raw exponents: a_i = max(eA, eB - c)
@@ -497,6 +491,31 @@ struct GemmArgs {
 __host__ __device__ __forceinline__ int split_chunks(int nkt, int chunk) { return chunk ? (nkt + chunk - 1) / chunk : 1; }
 __host__ __device__ __forceinline__ int split_chunk_begin(int nkt, int n, int c) { return nkt * c / n; }
 
+// sum of n group sums (r[0] the leading one) with weights 2^(beta (n-1-g))
+template <int BETA, int N>
+__device__ __forceinline__ long long merge_groups(const unsigned (&r)[N][EPI_COLS], int cc, int beta)
+{
+  if constexpr (BETA == 0) {
+    long long v = 0;
+#pragma unroll
+    for (int g = 0; g < N; ++g) v = v * (1ll << beta) + __float2int_rn(__uint_as_float(r[g][cc]));
+    return v;
+  } else {
+    // words of at most 31 / BETA groups: their weights fit a 32-bit factor
+    constexpr int W = 30 / BETA + 1;
+    long long v = 0;
+#pragma unroll
+    for (int g0 = 0; g0 < N; g0 += W) {
+      const int n = N - g0 < W ? N - g0 : W;
+      long long w = 0;
+#pragma unroll
+      for (int g = 0; g < n; ++g) w += (long long)__float2int_rn(__uint_as_float(r[g0 + g][cc])) * (1 << (BETA * (n - 1 - g)));
+      v = g0 == 0 ? w : (long long)((unsigned long long)v << (BETA * n)) + w;
+    }
+    return v;
+  }
+}
+
 template <int S, int TN>
 struct AccPair {
   static constexpr int NB = 512 / TN;
@@ -517,8 +536,12 @@ struct AccPair {
 // epilogue's per-column partial sums take it to 168 and the commutator's two
 // streams stop overlapping.
 // CHUNKED: reductions longer than g.chunk K blocks are cut (a plan of its
-// own kernel: the loop over chunks costs the short products 4%).
-template <int S, int TN, int EPIW, bool CHUNKED>
+// own kernel: the loop over chunks costs the short products 4%).  BETA: the
+// digit width where it is a usual one, else 0 (g.beta): the merge of a column's
+// group sums is then one multiply-add a group.  With shifts by g.beta and a
+// branching conversion to FP64 it took 4.5k-6.3k cycles a tile: 114 against
+// 103 us a commutator at emax 4; at emax 10 it hides behind the TMA stream.
+template <int S, int TN, int EPIW, bool CHUNKED, int BETA>
 __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMap mAlphaA,
                                                                  const __grid_constant__ CUtensorMap mBetaA,
                                                                  const __grid_constant__ CUtensorMap mGammaA,
@@ -735,7 +758,8 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
                                 : row_exp(g.rexpA[exp_base + i], g.rexpB[exp_base + i], c);
       const int phi_i = (ph && rowok) ? ph[i] : 1;
       double* O = g.out + out_off;
-      const int Xi = ai + c - 2 * g.P + g.beta * (S - 1);
+      const int beta = BETA ? BETA : g.beta;
+      const int Xi = ai + c - 2 * g.P + beta * (S - 1);
       const bool accumulate = g.accum > 0 || (g.accum < 0 && jacc);
       // exact merge of the weight groups (group t counts 2^(beta (S-1-t))),
       // per column, over the chunks of the reduction.  Of each chunk the
@@ -769,10 +793,9 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
             tmem_wait_ld();
 #pragma unroll
             for (int cc = 0; cc < EPI_COLS; ++cc) {
-              long long E = 0;
-#pragma unroll
-              for (int gi = 0; gi < OV; ++gi) E = E * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
-              P[c0 + cc] += E * (1ll << (g.beta * (S - OV - e0)));
+              const long long E = merge_groups<BETA>(r, cc, beta);
+              // (two instances of a constant shift, or one by g.beta's multiple)
+              P[c0 + cc] += (tc & 1) ? E << (beta * (S - OV)) : E;
             }
           }
           tc_fence_before();
@@ -787,10 +810,8 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           tmem_wait_ld();
 #pragma unroll
           for (int cc = 0; cc < EPI_COLS; ++cc) {
-            long long L = 0;
-#pragma unroll
-            for (int gi = 0; gi < S - OV; ++gi) L = L * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
-            P[c0 + cc] += L * (1ll << (g.beta * (OV - l0)));
+            const long long L = merge_groups<BETA>(r, cc, beta);
+            P[c0 + cc] += (tc & 1) ? L : L << (beta * OV);
           }
         }
         tc_fence_before();
@@ -800,7 +821,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
         s_err = 1;
         break;
       }
-      const long long mulL = 1ll << (g.beta * (OV - l0));
+      const int shL = (tc & 1) ? 0 : beta * OV;
 #pragma unroll
       for (int c0 = 0; c0 < COLS_W; c0 += EPI_COLS) {
         unsigned r[S - OV][EPI_COLS];
@@ -817,10 +838,8 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           const int j = tl.J * TN + jc;
           wd[cc] = rowok && j < jn && !(tl.diag && i > j);
           wm[cc] = wd[cc] && i != j && !nosym && !g.nomirror;
-          long long L = 0;
-#pragma unroll
-          for (int gi = 0; gi < S - OV; ++gi) L = L * (1ll << g.beta) + __float2int_rn(__uint_as_float(r[gi][cc]));
-          const long long I64 = P[c0 + cc] + L * mulL;
+          const long long L = merge_groups<BETA>(r, cc, beta);
+          const long long I64 = OV > 0 || CHUNKED ? P[c0 + cc] + (L << shL) : L;
           v[cc] = i64_ldexp(I64, Xi + s_colexp[tp][jc]);
           mv[cc] = __longlong_as_double(__double_as_longlong(v[cc]) ^
                                         ((sign * phi_i * s_colph[tp][jc]) < 0 ? (long long)0x8000000000000000ull
@@ -1276,8 +1295,9 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
     ga.gsign = gsign;
     ga.accum = p->accum_override;
     ga.nomirror = p->mirror ? 0 : 1;
-    auto kern = p->chunk ? (p->tn == 64 ? k_split_gemm<S, 64, 8, true> : k_split_gemm<S, 32, 8, true>)
-                         : (p->tn == 64 ? k_split_gemm<S, 64, 8, false> : k_split_gemm<S, 32, 8, false>);
+    auto kern = p->chunk       ? (p->tn == 64 ? k_split_gemm<WIDE_S, 64, 8, true, WIDE_BETA> : k_split_gemm<WIDE_S, 32, 8, true, WIDE_BETA>)
+                : p->beta == 7 ? (p->tn == 64 ? k_split_gemm<S, 64, 8, false, 7> : k_split_gemm<S, 32, 8, false, 7>)
+                               : (p->tn == 64 ? k_split_gemm<S, 64, 8, false, 0> : k_split_gemm<S, 32, 8, false, 0>);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
     // the whole shared memory, so that the second stream's kernels find some beside the product's CTA
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);

@@ -8,7 +8,7 @@
 //  * Digits.  Each row i gets one exponent a_i for its A row and b_i = a_i + c
 //    for its B row (c is one per job), chosen so both rows fit below the
 //    exponent.  Every element is rounded to an integer q = v * 2^(P - e)
-//    (|q| <= 2^P, P = beta*S, or 37 for five 8-bit digits) and split
+//    (|q| <= 2^P, P = beta*S, or 38 for five 8-bit digits) and split
 //    into S balanced base-2^beta digits, all exact in BF16.  Only integer
 //    instructions are used (FP64 runs at 1/57 of the FP32 rate on this part).
 //  * Symmetrisation folded into K.  With the shared-exponent choice both
@@ -950,17 +950,22 @@ static void choose_digits(int Kmax, int& beta, int& S)
   if (S > MAX_S) S = MAX_S;
 }
 
-// Where that takes six digits for 36 bits (any K above 58), five of 8 bits
-// (5 in the leading one) give 37: 15 products and five planes instead of 21
-// and six.  Their leading three weight groups are exact over WIDE_CHUNK K
-// blocks ((2 x 33 x 128 + 128^2) x 672 < 2^24), so the reduction is cut into
-// chunks of that, whose sums are added as integers; what the other groups
-// round is below 2^-38 of the rows' maxima.  A chunk costs the MMAs the time
-// in which the epilogue takes the blocks that consecutive chunks share: 39
-// bits need chunks of 10 blocks.  emax=10 ladder product (beside the second
-// stream's kernels): 1135 us with six digits, 1062 with chunks of 10 blocks,
-// 945 so, 898 uncut.
-constexpr int WIDE_BETA = 8, WIDE_S = 5, WIDE_P = 37, WIDE_CHUNK = 21;
+// Where K is too long for seven-bit digits (above 339: six or fewer bits a
+// digit, 35 or 36 in all), five of 8 bits (6 in the leading one) give 38: 15
+// products and five planes instead of 21 (emax=12: 28) and six (seven).  The
+// products left out weigh 2^-38 of the rows' maxima (rms), the rounding of the
+// last digit less; with 36 bits of 6, the two together did: ladder term
+// against FP64, relative Frobenius, random operators, emax 8 / 10 / 12:
+// 2.6e-11 / 2.3e-11 / 4.8e-11 then, 1.9e-11 / 1.7e-11 / 1.8e-11 so (37 bits of
+// 8: 8.0e-11 / 6.2e-11 / 8.2e-11).  The leading three weight groups are exact
+// over WIDE_CHUNK K blocks ((2 x 65 x 128 + 128^2) x 480 < 2^24), so the
+// reduction is cut into chunks of that, whose sums are added as integers; the
+// other two round, if at all, at their own weights.  A chunk costs the MMAs
+// the time in which the epilogue takes the blocks that consecutive chunks
+// share: emax=10 commutator 3213 us with 37 bits and 21 blocks, 3243 so, 3297
+// with 39 bits and 10 blocks (error 4.7e-12); ladder product beside the second
+// stream's kernels 1135 us with six digits, 945 with 37 bits.
+constexpr int WIDE_BETA = 8, WIDE_S = 5, WIDE_P = 38, WIDE_CHUNK = 15;
 
 SplitOpts split_plan_opts(const SplitPlan* p)
 {

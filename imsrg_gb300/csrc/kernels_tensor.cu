@@ -648,12 +648,10 @@ __global__ void k_t221(DevSpace S, DevTensor T, const double* __restrict__ D, co
 // tensor Pandya transform of Y for the ordered cross-coupled pair
 // (bra, ket) = blockIdx.y (DoTensorPandyaTransformation_SingleChannel,
 // src/TensorCommutators.cc:637-752): 2 nph_bra x n_ket, rows the bra's hh
-// then ph kets (a, b) in both orders
-// Split form (YbF != nullptr): the panel is written transposed, Yb[off +
-// row n_ket + ik], and its half-swapped copy for the Z bar tails, YbF[off +
-// swap(row) n_ket + ik] = hY (-1)^(bra ph ket) (-1)^(ket ik) value.
+// then ph kets (a, b) in both orders, a thread per element (for the FP64-pipe
+// Z bar; the products' panels are k_tpandya_b's)
 __global__ void k_tpandya(DevSpace S, DevWork W, DevTensor T, const double* __restrict__ Y, int hY,
-                          double* __restrict__ Yb, double* __restrict__ YbF)
+                          double* __restrict__ Yb)
 {
   const int p = blockIdx.y;
   const int cb = T.yb_bra[p], ck = T.yb_ket[p];
@@ -666,14 +664,8 @@ __global__ void k_tpandya(DevSpace S, DevWork W, DevTensor T, const double* __re
   const int Lam = T.lam;
   const int second = row >= nph;
   const int kb = W.cc_ph[W.cc_ph_off[cb] + row - second * nph];
-  const long long et = (long long)row * nk + ik, ets = (long long)(second ? row - nph : row + nph) * nk + ik;
   if (Jbra + Jket < Lam || abs(Jbra - Jket) > Lam || ((ch_par(cb) + ch_par(ck) + T.parity) & 1)) {
-    if (YbF) {
-      out[et] = 0.0;
-      YbF[T.yb_off[p] + ets] = 0.0;
-    } else {
-      out[e] = 0.0;
-    }
+    out[e] = 0.0;
     return;
   }
   const int p0 = S.cc_p[S.cc_kofs[cb] + kb], q0 = S.cc_q[S.cc_kofs[cb] + kb];
@@ -693,14 +685,7 @@ __global__ void k_tpandya(DevSpace S, DevWork W, DevTensor T, const double* __re
       sm = fma(flip(nh, 1 + ((jb + jd) >> 1) + Jket + J2), tbme, sm);
     }
   }
-  if (YbF) {
-    out[et] = sm;
-    const int* ph_b = W.phase_tab + W.cc_phase_off[cb];
-    const int* ph_k = W.phase_tab + W.cc_phase_off[ck];
-    YbF[T.yb_off[p] + ets] = flip(sm, (hY < 0) + (ph_b[kb] < 0) + (ph_k[ik] < 0));
-  } else {
-    out[e] = sm;
-  }
+  out[e] = sm;
 }
 
 // Zbar(lo, hi) = Mleft Mright for the pair blockIdx.y (src/TensorCommutators.cc:
@@ -824,6 +809,69 @@ constexpr int kTqThreads = 256;
 // at least 1 / 256 from an integer, more than the product rounds by (checked over the range)
 __device__ __forceinline__ int small_div(int x, float r) { return __float2int_rz(__fmul_rn((float)x + 0.5f, r)); }
 
+// values v 2^(1023 - e) of each quadruple's largest exponent e, as float pairs in place
+__device__ __forceinline__ void scale_to_ff(double* in, int n, const int* s_e, int QP, float rq)
+{
+  for (int e = threadIdx.x; e < n; e += kTqThreads) {
+    const long long b = __double_as_longlong(in[e]);
+    const int ex = (int)((b >> 52) & 0x7FF), es = ex - s_e[e - small_div(e, rq) * QP] + 1023;
+    const double x = ex == 0x7FF ? in[e] : ex == 0 || es <= 0 ? 0.0 : __longlong_as_double((b & ~(0x7FFll << 52)) | ((long long)es << 52));
+    ((float2*)in)[e] = d2ff(x);
+  }
+}
+
+// z 2^(e - 1023)
+__device__ __forceinline__ double scale_back(double z, int e)
+{
+  e -= 1023;
+  z *= __longlong_as_double((long long)(1023 + e / 2) << 52);
+  return z * __longlong_as_double((long long)(1023 + e - e / 2) << 52);
+}
+
+// sum_{A, B} 9j[(A, B)][t] in[(A, B)][q0 .. q0 + 3]: A = lo + a for a < n, B within lam of A and in
+// [loB, hiB]; value v0 + a w + (B - A + lam), the 9j matrix from base with rows of nslot
+template <bool DF>
+__device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, int nslot, int t, const double* in, int v0, int QP,
+                                          int q0, int n, int lo, int loB, int hiB, double (&sum)[4])
+{
+  const int Lam = T.lam, w = 2 * Lam + 1;
+  float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
+  double sd[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int a = 0; a < n; ++a) {
+    const int A = lo + a;
+    const int b0 = max(loB, abs(A - Lam)) - A + Lam, b1 = min(hiB, A + Lam) - A + Lam;
+    for (int b = b0; b <= b1; ++b) {
+      const int v = a * w + b;
+      if (DF) {
+        const float2 c = __ldg(T.nj_hatf + base + (long long)v * nslot + t);
+        const float4* y = (const float4*)((const float2*)in + (v0 + v) * QP + q0);
+        const float4 y0 = y[0], y1 = y[1];
+        df_fma(c, make_float2(y0.x, y0.y), sh[0], sl[0]);
+        df_fma(c, make_float2(y0.z, y0.w), sh[1], sl[1]);
+        df_fma(c, make_float2(y1.x, y1.y), sh[2], sl[2]);
+        df_fma(c, make_float2(y1.z, y1.w), sh[3], sl[3]);
+      } else {
+        const double c = __ldg(T.nj_hat + base + (long long)v * nslot + t);
+        const double2* y = (const double2*)(in + (v0 + v) * QP + q0);
+        const double2 y0 = y[0], y1 = y[1];
+        sd[0] = fma(c, y0.x, sd[0]);
+        sd[1] = fma(c, y0.y, sd[1]);
+        sd[2] = fma(c, y1.x, sd[2]);
+        sd[3] = fma(c, y1.y, sd[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (DF) {
+      const float hi = __fadd_rn(sh[h], sl[h]);
+      sum[h] = ff2d(hi, __fsub_rn(sl[h], __fsub_rn(hi, sh[h])));
+    } else {
+      sum[h] = sd[h];
+    }
+  }
+}
+
 template <bool DF>
 __global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
                                                        double* __restrict__ Z, const int2* __restrict__ tq,
@@ -870,13 +918,7 @@ __global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, 
   }
   __syncthreads();
   if (DF) {
-    // v 2^(1023 - e) of the quadruple's largest exponent e, as float pairs in place
-    for (int e = tid; e < nval * QP; e += kTqThreads) {
-      const long long b = __double_as_longlong(in[e]);
-      const int ex = (int)((b >> 52) & 0x7FF), es = ex - s_e[e - small_div(e, rq) * QP] + 1023;
-      const double x = ex == 0x7FF ? in[e] : ex == 0 || es <= 0 ? 0.0 : __longlong_as_double((b & ~(0x7FFll << 52)) | ((long long)es << 52));
-      ((float2*)in)[e] = d2ff(x);
-    }
+    scale_to_ff(in, nval * QP, s_e, QP, rq);
     __syncthreads();
   }
   const int J1min = abs(ji - jj) >> 1, nslot = (((ji + jj) >> 1) - J1min + 1) * w;
@@ -891,44 +933,8 @@ __global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, 
     double sum[2][4];
     if (J2 < (abs(jk - jl) >> 1) || J2 > ((jk + jl) >> 1) || J1 >= S.NJ || J2 >= S.NJ) continue;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-      double sd[4] = {0.0, 0.0, 0.0, 0.0};
-      const int v0 = u ? n3[0] * w : 0;
-      for (int a = 0; a < n3[u]; ++a) {
-        const int J3 = lo3[u] + a;
-        const int b0 = max(lo4[u], abs(J3 - Lam)) - J3 + Lam, b1 = min(hi4[u], J3 + Lam) - J3 + Lam;
-        for (int b = b0; b <= b1; ++b) {
-          const int v = a * w + b;
-          if (DF) {
-            const float2 c = __ldg(T.nj_hatf + base[u] + (long long)v * nslot + t);
-            const float4* y = (const float4*)((const float2*)in + (v0 + v) * QP + q0);
-            const float4 y0 = y[0], y1 = y[1];
-            df_fma(c, make_float2(y0.x, y0.y), sh[0], sl[0]);
-            df_fma(c, make_float2(y0.z, y0.w), sh[1], sl[1]);
-            df_fma(c, make_float2(y1.x, y1.y), sh[2], sl[2]);
-            df_fma(c, make_float2(y1.z, y1.w), sh[3], sl[3]);
-          } else {
-            const double c = __ldg(T.nj_hat + base[u] + (long long)v * nslot + t);
-            const double2* y = (const double2*)(in + (v0 + v) * QP + q0);
-            const double2 y0 = y[0], y1 = y[1];
-            sd[0] = fma(c, y0.x, sd[0]);
-            sd[1] = fma(c, y0.y, sd[1]);
-            sd[2] = fma(c, y1.x, sd[2]);
-            sd[3] = fma(c, y1.y, sd[3]);
-          }
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        if (DF) {
-          const float hi = __fadd_rn(sh[h], sl[h]);
-          sum[u][h] = ff2d(hi, __fsub_rn(sl[h], __fsub_rn(hi, sh[h])));
-        } else {
-          sum[u][h] = sd[h];
-        }
-      }
-    }
+    for (int u = 0; u < 2; ++u)
+      quad_sums<DF>(T, base[u], nslot, t, in, u ? n3[0] * w : 0, QP, q0, n3[u], lo3[u], lo4[u], hi4[u], sum[u]);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int q = q0 + h;
@@ -942,15 +948,106 @@ __global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, 
       if (blk < 0) continue;
       // both sums carry (-1)^J2
       double z = flip(sum[0][h] + flip(sum[1][h], 1 + ((ji + jj) >> 1) - J1), J2);
-      if (DF) {
-        const int e = s_e[q] - 1023;
-        z *= __longlong_as_double((long long)(1023 + e / 2) << 52);
-        z *= __longlong_as_double((long long)(1023 + e - e / 2) << 52);
-      }
+      if (DF) z = scale_back(z, s_e[q]);
       z = unnorm(z, i == j, k == l);
       const int nb = S.ch_n[chb];
       Z[T.off[blk] + (long long)ik * nb + ib] += z;
       if (chb == chk && ik != ib) Z[T.off[blk] + (long long)ib * nb + ik] += flip(z, hZ < 0);
+    }
+  }
+}
+
+// The tensor Pandya transform for the products: the same panels as k_tpandya,
+// transposed, Yb[off + row n_ket + ik], and half-swapped for the Z bar tails,
+// YbF[off + swap(row) n_ket + ik] = hY (-1)^(bra ph ket) (-1)^(ket ik) value.
+// Like k_tinv_b, by batches of orbit quadruples (a, b ordered with a hole; c <= d)
+// of one class of j: Y's elements (a d, c b) at all (J1, J2) go to shared memory
+// once and serve every (Jbra, Jket), four quadruples to a 9j load.  Elements
+// no quadruple has are zero (cleared before).  Bound by the gather's lookups
+// and the 9j table's L2 stream.  A thread per element, looking up each element
+// of Y for each of its sums, took 1.23 ms of the commutator at emax 8, rank
+// (2, 0, +); the whole of that 9609 -> 8387 us with this kernel (emax 6, rank
+// (1, 1, +), FP64: 1358 -> 1267).  Float pairs, as k_tinv_b has them in the
+// split form, gain nothing here (8377 us) and are not used.
+__global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W, DevTensor T, const double* __restrict__ Y,
+                                                          int hY, double* __restrict__ Yb, double* __restrict__ YbF,
+                                                          const int2* __restrict__ tp, const int2* __restrict__ batches,
+                                                          const int* __restrict__ ph_loc)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* in = (double*)smem;  // [value][quadruple]
+  __shared__ int4 s_q[kTqBatch];  // a | b << 16, c | d << 16, ket (a, d), ket (c, b)
+  __shared__ int s_f[kTqBatch];
+  const int tid = threadIdx.x;
+  const int2 bt = batches[blockIdx.x];
+  const int nq = bt.y, QP = (nq + 3) & ~3;
+  if (tid < QP) {
+    const int2 v = tp[bt.x + min(tid, nq - 1)];
+    const int a = v.x & 0xFFFF, b = v.x >> 16, c = v.y & 0xFFFF, d = v.y >> 16;
+    s_q[tid] = make_int4(v.x, v.y, ket_index(S.norb, min(a, d), max(a, d)), ket_index(S.norb, min(c, b), max(c, b)));
+    s_f[tid] = chan_index(0, (S.l[a] + S.l[d]) & 1, (S.tz2[a] + S.tz2[d]) / 2) |
+               chan_index(0, (S.l[c] + S.l[b]) & 1, (S.tz2[c] + S.tz2[b]) / 2) << 4 | (a > d) << 8 | (c > b) << 9;
+  }
+  __syncthreads();
+  const int ja = S.j2[s_q[0].x & 0xFFFF], jb = S.j2[s_q[0].x >> 16], jc = S.j2[s_q[0].y & 0xFFFF], jd = S.j2[s_q[0].y >> 16];
+  const int Lam = T.lam, w = 2 * Lam + 1;
+  const int lo1 = abs(ja - jd) >> 1, n1 = ((ja + jd) >> 1) - lo1 + 1, lo2 = abs(jc - jb) >> 1, hi2 = (jc + jb) >> 1;
+  const int nval = n1 * w;
+  const float rq = 1.0f / QP, rw = 1.0f / w;
+  for (int e = tid; e < nval * QP; e += kTqThreads) {
+    const int v = small_div(e, rq), q = e - v * QP, i1 = small_div(v, rw);
+    const int J1 = lo1 + i1, J2 = J1 - Lam + v - i1 * w;
+    double x = 0.0;
+    if (q < nq && J2 >= lo2 && J2 <= hi2 && J1 < S.NJ && J2 < S.NJ) {
+      const int f = s_f[q], chb = 6 * J1 + (f & 15), chk = 6 * J2 + ((f >> 4) & 15);
+      const bool up = chb <= chk;
+      const int bi = __ldg(S.ketJ_loc + J1 * S.nkets + s_q[q].z), ki = __ldg(S.ketJ_loc + J2 * S.nkets + s_q[q].w);
+      const int blk = __ldg(T.lookup + (up ? chb * S.nch + chk : chk * S.nch + chb));
+      if (bi >= 0 && ki >= 0 && blk >= 0) {
+        const long long o = __ldg(T.off + blk) + (up ? (long long)ki * __ldg(S.ch_n + chb) + bi : (long long)bi * __ldg(S.ch_n + chk) + ki);
+        int odd = ((jb + jd) >> 1) + 1 + J2;
+        if (!up) odd += (hY < 0) + J1 - J2;
+        if ((f >> 8) & 1) odd += ((ja + jd) >> 1) + 1 + J1;
+        if ((f >> 9) & 1) odd += ((jc + jb) >> 1) + 1 + J2;
+        x = flip(__ldg(Y + o), odd);
+      }
+    }
+    in[e] = x;
+  }
+  __syncthreads();
+  const int Jbmin = abs(ja - jb) >> 1, nslot = (((ja + jb) >> 1) - Jbmin + 1) * w;
+  const int d1 = T.d1;
+  const long long base = T.nj_base[((((ja - 1) >> 1) * d1 + ((jb - 1) >> 1)) * d1 + ((jc - 1) >> 1)) * d1 + ((jd - 1) >> 1)];
+  for (int x = tid; x < nslot * (QP >> 2); x += kTqThreads) {
+    const int g4 = x / nslot, t = x - g4 * nslot, i3 = t / w, q0 = 4 * g4;
+    const int Jbra = Jbmin + i3, Jket = Jbra - Lam + t - i3 * w;
+    if (Jket < (abs(jc - jd) >> 1) || Jket > ((jc + jd) >> 1) || Jbra + Jket < Lam || Jbra >= S.NJ || Jket >= S.NJ) continue;
+    double sum[4];
+    quad_sums<false>(T, base, nslot, t, in, 0, QP, q0, n1, lo1, lo2, hi2, sum);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int q = q0 + h;
+      if (q >= nq) break;
+      const int a = s_q[q].x & 0xFFFF, b = s_q[q].x >> 16, c = s_q[q].y & 0xFFFF, d = s_q[q].y >> 16;
+      const int cb = chan_index(Jbra, (S.l[a] + S.l[b]) & 1, abs(S.tz2[a] - S.tz2[b]) / 2);
+      const int ck = chan_index(Jket, (S.l[c] + S.l[d]) & 1, abs(S.tz2[c] - S.tz2[d]) / 2);
+      const long long off = T.yb_lookup[cb * S.nch + ck];
+      if (off < 0) continue;
+      const int nph = W.cc_nph[cb], nk = S.cc_n[ck];
+      const int r = ph_loc[Jbra * S.nkets + ket_index(S.norb, min(a, b), max(a, b))];
+      const int ik = S.ccJ_loc[Jket * S.nkets + ket_index(S.norb, c, d)];
+      double z = flip(sum[h], Jket);
+      if (a == d) z *= kSqrt2t;
+      if (c == b) z *= kSqrt2t;
+      const double zf = flip(z, (hY < 0) + ((ja + jb) >> 1) + ((jc + jd) >> 1));
+      // (a pair a == b is its own swap: both rows)
+      const long long o1 = off + (long long)(a > b ? r + nph : r) * nk + ik, o2 = off + (long long)(a > b ? r : r + nph) * nk + ik;
+      Yb[o1] = z;
+      YbF[o2] = zf;
+      if (a == b) {
+        Yb[o2] = z;
+        YbF[o1] = zf;
+      }
     }
   }
 }
@@ -1058,7 +1155,7 @@ cudaError_t launch_tensor_ph(const Space& s, const TensorLayout& t, const double
 {
   if (t.yb_bra.empty()) return cudaSuccess;
   dim3 gy(grid_for(std::max(1, t.yb_maxelems)), (unsigned)t.yb_bra.size());
-  k_tpandya<<<gy, 256, 0, st>>>(s.dev, s.work, t.dev, Y, hY, Ybar, nullptr);
+  k_tpandya<<<gy, 256, 0, st>>>(s.dev, s.work, t.dev, Y, hY, Ybar);
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -1075,9 +1172,14 @@ cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, 
                                          cudaStream_t st)
 {
   cudaError_t e;
-  if (!t.yb_bra.empty()) {
-    dim3 gy(grid_for(std::max(1, t.yb_maxelems)), (unsigned)t.yb_bra.size());
-    k_tpandya<<<gy, 256, 0, st>>>(s.dev, s.work, t.dev, Y, hY, YbT, YbTF);
+  if (t.yb_total > 0) {
+    if ((e = cudaMemsetAsync(YbT, 0, t.yb_total * sizeof(double), st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(YbTF, 0, t.yb_total * sizeof(double), st)) != cudaSuccess)
+      return e;
+  }
+  if (!t.tpb.empty()) {
+    k_tpandya_b<<<(unsigned)t.tpb.size(), kTqThreads, t.tpb_smem, st>>>(s.dev, s.work, t.dev, Y, hY, YbT, YbTF, t.d_tp, t.d_tpb,
+                                                                t.d_ph_loc);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }

@@ -14,6 +14,8 @@
 namespace imsrg {
 namespace {
 
+constexpr double OCC_CUT = 1e-6;  // ModelSpace::OCC_CUT (src/ModelSpace.cc:14)
+
 int64_t round32(int64_t x) { return (x + 31) / 32 * 32; }
 
 bool triad2(int a, int b, int c)  // doubled arguments
@@ -79,6 +81,43 @@ TensorLayout::~TensorLayout()
   for (void* p : dev_allocs) cudaFree(p);
 }
 
+// an orbit quadruple with the key of its class of j
+struct Quad {
+  int key;
+  int2 v;
+};
+
+// Quadruples (x | y << 16, z | w << 16) in class order, and batches of one
+// class: as many as give each of 256 threads about one (pair of J, four
+// quadruples), within the shared memory of the gathered values.  values: (A, B)
+// with A in |x - w| .. x + w (second: and |y - w| .. y + w), 2 lam + 1 B each;
+// per_j slots for every J of |x - y| .. x + y
+static void sort_quadruples(const Space& s, const std::vector<Quad>& all, int lam, int per_j, bool second,
+                            std::vector<int2>& quads, std::vector<int2>& batches, int& smem)
+{
+  const int nkey = s.d1 * s.d1 * s.d1 * s.d1;
+  std::vector<long long> cnt(nkey + 1, 0);
+  for (const Quad& q : all) ++cnt[q.key + 1];
+  for (int x = 0; x < nkey; ++x) cnt[x + 1] += cnt[x];
+  quads.assign(all.size(), make_int2(0, 0));
+  std::vector<long long> at(cnt.begin(), cnt.end() - 1);
+  for (const Quad& q : all) quads[(size_t)at[q.key]++] = q.v;
+  batches.clear();
+  smem = 0;
+  for (int x = 0; x < nkey; ++x) {
+    if (cnt[x] == cnt[x + 1]) continue;
+    const int2 v = quads[(size_t)cnt[x]];
+    const int ja = s.j2[v.x & 0xFFFF], jb = s.j2[v.x >> 16], jd = s.j2[v.y >> 16];
+    const int nslot = (std::min(ja, jb) + 1) * per_j;
+    const int nval = (std::min(ja, jd) + 1 + (second ? std::min(jb, jd) + 1 : 0)) * (2 * lam + 1);
+    int q = std::min({kTqBatch, (1024 + nslot - 1) / nslot, kTqValues / nval});
+    q = std::max(4, q / 4 * 4);
+    for (long long b = cnt[x]; b < cnt[x + 1]; b += q)
+      batches.push_back(make_int2((int)b, (int)std::min<long long>(q, cnt[x + 1] - b)));
+    smem = std::max(smem, q * nval * 8);
+  }
+}
+
 // The orbit quadruples of the inverse tensor Pandya transform (k_tinv_b): a
 // bra ket (i <= j) and a ket ket (k <= l) with the rank's parity and |dTz|,
 // kept when some (J1, J2) gives a stored element it owns: block (chb, chk)
@@ -92,11 +131,7 @@ static void build_quadruples(const Space& s, TensorLayout& t)
       kp.push_back(p);
       kq.push_back(q);
     }
-  struct Item {
-    int key;
-    int2 v;
-  };
-  std::vector<std::vector<Item>> part(nk);
+  std::vector<std::vector<Quad>> part(nk);
 #pragma omp parallel for schedule(dynamic, 16)
   for (int kb = 0; kb < nk; ++kb) {
     const int i = kp[kb], j = kq[kb];
@@ -128,39 +163,39 @@ static void build_quadruples(const Space& s, TensorLayout& t)
       part[kb].push_back({key, make_int2(i | (j << 16), k | (l << 16))});
     }
   }
-  // counting sort by class
-  const int nkey = d1 * d1 * d1 * d1;
-  std::vector<long long> cnt(nkey + 1, 0);
-  for (const auto& v : part)
-    for (const Item& it : v) ++cnt[it.key + 1];
-  for (int x = 0; x < nkey; ++x) cnt[x + 1] += cnt[x];
-  t.tq.assign((size_t)cnt[nkey], make_int2(0, 0));
-  for (const auto& v : part)
-    for (const Item& it : v) t.tq[(size_t)cnt[it.key]++] = it.v;
-  // batches: as many quadruples as give each of 256 threads about one slot of
-  // four quadruples, within the shared memory of the gathered values
-  t.tqb.clear();
-  t.tqb_smem = 0;
-  const int w = 2 * lam + 1;
-  for (size_t a = 0; a < t.tq.size();) {
-    auto cls = [&](size_t x) {
-      return make_int4(s.j2[t.tq[x].x & 0xFFFF], s.j2[t.tq[x].x >> 16], s.j2[t.tq[x].y & 0xFFFF], s.j2[t.tq[x].y >> 16]);
-    };
-    const int4 j = cls(a);
-    size_t b = a;
-    while (b < t.tq.size()) {
-      const int4 k = cls(b);
-      if (k.x != j.x || k.y != j.y || k.z != j.z || k.w != j.w) break;
-      ++b;
+  std::vector<Quad> all;
+  for (auto& v : part) all.insert(all.end(), v.begin(), v.end());
+  // two sums: (J3, J4) values of (i, l) and of (j, l); slots J2 >= J1
+  sort_quadruples(s, all, lam, lam + 1, true, t.tq, t.tqb, t.tqb_smem);
+}
+
+// The orbit quadruples of the tensor Pandya transform (k_tpandya_b)
+static void build_pandya_quadruples(const Space& s, TensorLayout& t)
+{
+  const int N = s.norb, d1 = s.d1;
+  std::vector<std::vector<Quad>> part(N);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int a = 0; a < N; ++a)
+    for (int b = 0; b < N; ++b) {
+      if (s.occ[a] <= OCC_CUT && s.occ[b] <= OCC_CUT) continue;
+      for (int c = 0; c < N; ++c)
+        for (int d = c; d < N; ++d) {
+          if ((s.l[a] + s.l[b] + s.l[c] + s.l[d] + t.parity) & 1) continue;
+          if (std::abs(s.tz2[a] + s.tz2[d] - s.tz2[c] - s.tz2[b]) != 2 * t.trank) continue;
+          const int key = ((((s.j2[a] - 1) / 2) * d1 + (s.j2[b] - 1) / 2) * d1 + (s.j2[c] - 1) / 2) * d1 + (s.j2[d] - 1) / 2;
+          part[a].push_back({key, make_int2(a | (b << 16), c | (d << 16))});
+        }
     }
-    const int nslot = (std::min(j.x, j.y) + 1) * (lam + 1);
-    const int nval = (std::min(j.x, j.w) + 1 + std::min(j.y, j.w) + 1) * w;
-    int q = std::min({kTqBatch, (1024 + nslot - 1) / nslot, kTqValues / nval});
-    q = std::max(4, q / 4 * 4);
-    for (size_t x = a; x < b; x += q) t.tqb.push_back(make_int2((int)x, (int)std::min<size_t>(q, b - x)));
-    t.tqb_smem = std::max(t.tqb_smem, q * nval * 8);
-    a = b;
-  }
+  std::vector<Quad> all;
+  for (auto& v : part) all.insert(all.end(), v.begin(), v.end());
+  sort_quadruples(s, all, t.lam, 2 * t.lam + 1, false, t.tp, t.tpb, t.tpb_smem);
+  t.ph_loc.assign((size_t)s.NJ * s.nkets, 0);
+  for (int c = 0; c < s.nch; ++c)
+    for (int k = 0; k < s.cc_nph[c]; ++k) {
+      const Chan& C = s.cc[c];
+      const int loc = s.cc_ph[s.cc_ph_off[c] + k];
+      t.ph_loc[(size_t)C.J * s.nkets + ket_index(s.norb, C.p[loc], C.q[loc])] = k;
+    }
 }
 
 TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity)
@@ -359,6 +394,7 @@ TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity)
     t->lad_maxelems = std::max(t->lad_maxelems, (long long)jb.m * jb.K);
   }
   build_quadruples(s, *t);
+  build_pandya_quadruples(s, *t);
   t->hat2.assign((size_t)t->NJ * t->NJ, 0.0);
   for (int J1 = 0; J1 < t->NJ; ++J1)
     for (int J2 = 0; J2 < t->NJ; ++J2) t->hat2[(size_t)J1 * t->NJ + J2] = std::sqrt((double)((2 * J1 + 1) * (2 * J2 + 1)));
@@ -441,6 +477,9 @@ void tensor_upload(TensorLayout& t)
   d.tob_list = dev_copy(t, t.tob_list);
   t.d_tq = dev_copy(t, t.tq);
   t.d_tqb = dev_copy(t, t.tqb);
+  t.d_tp = dev_copy(t, t.tp);
+  t.d_tpb = dev_copy(t, t.tpb);
+  t.d_ph_loc = dev_copy(t, t.ph_loc);
   // the split form's float pairs of the 9j table; without room for them it reads the FP64 table
   d.nj_hatf = nullptr;
   void* f = nullptr;

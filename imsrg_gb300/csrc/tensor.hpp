@@ -140,6 +140,14 @@ struct TensorLayout {
   std::vector<int2> tqb;
   int tqb_smem = 0;           // shared memory of the largest batch
   int2 *d_tq = nullptr, *d_tqb = nullptr;
+  // the same for the tensor Pandya transform: (a | b << 16, c | d << 16), a, b
+  // ordered with a hole, c <= d; ph_loc[J nkets + ket]: the ket's place among
+  // the hh and ph kets of its cross-coupled channel
+  std::vector<int2> tp, tpb;
+  std::vector<int> ph_loc;
+  int tpb_smem = 0;
+  int2 *d_tp = nullptr, *d_tpb = nullptr;
+  int* d_ph_loc = nullptr;
   long long max_xbf = 0;      // largest X bar panel (2 nph x n_cc)
   DevTensor dev;
   bool dev_ready = false;

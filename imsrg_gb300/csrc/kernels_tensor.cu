@@ -829,8 +829,9 @@ __device__ __forceinline__ double scale_back(double z, int e)
 }
 
 // sum_{A, B} 9j[(A, B)][t] in[(A, B)][q0 .. q0 + 3]: A = lo + a for a < n, B within lam of A and in
-// [loB, hiB]; value v0 + a w + (B - A + lam), the 9j matrix from base with rows of nslot
-template <bool DF>
+// [loB, hiB]; value v0 + a w + (B - A + lam), the 9j matrix from base with rows of nslot.
+// SKIP0: a zero of the table takes no part, whatever the value (0 x inf)
+template <bool DF, bool SKIP0>
 __device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, int nslot, int t, const double* in, int v0, int QP,
                                           int q0, int n, int lo, int loB, int hiB, double (&sum)[4])
 {
@@ -858,6 +859,20 @@ __device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, in
         sd[1] = fma(c, y0.y, sd[1]);
         sd[2] = fma(c, y1.x, sd[2]);
         sd[3] = fma(c, y1.y, sd[3]);
+      }
+    }
+  }
+  if (SKIP0 && !isfinite((sd[0] + sd[1]) + (sd[2] + sd[3]))) {
+    for (int h = 0; h < 4; ++h) {
+      sd[h] = 0.0;
+      for (int a = 0; a < n; ++a) {
+        const int A = lo + a;
+        const int b0 = max(loB, abs(A - Lam)) - A + Lam, b1 = min(hiB, A + Lam) - A + Lam;
+        for (int b = b0; b <= b1; ++b) {
+          const int v = a * w + b;
+          const double c = __ldg(T.nj_hat + base + (long long)v * nslot + t);
+          if (!is_zero(c)) sd[h] = fma(c, in[(v0 + v) * QP + q0 + h], sd[h]);
+        }
       }
     }
   }
@@ -934,7 +949,7 @@ __global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, 
     if (J2 < (abs(jk - jl) >> 1) || J2 > ((jk + jl) >> 1) || J1 >= S.NJ || J2 >= S.NJ) continue;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
-      quad_sums<DF>(T, base[u], nslot, t, in, u ? n3[0] * w : 0, QP, q0, n3[u], lo3[u], lo4[u], hi4[u], sum[u]);
+      quad_sums<DF, false>(T, base[u], nslot, t, in, u ? n3[0] * w : 0, QP, q0, n3[u], lo3[u], lo4[u], hi4[u], sum[u]);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int q = q0 + h;
@@ -1023,7 +1038,7 @@ __global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W,
     const int Jbra = Jbmin + i3, Jket = Jbra - Lam + t - i3 * w;
     if (Jket < (abs(jc - jd) >> 1) || Jket > ((jc + jd) >> 1) || Jbra + Jket < Lam || Jbra >= S.NJ || Jket >= S.NJ) continue;
     double sum[4];
-    quad_sums<false>(T, base, nslot, t, in, 0, QP, q0, n1, lo1, lo2, hi2, sum);
+    quad_sums<false, true>(T, base, nslot, t, in, 0, QP, q0, n1, lo1, lo2, hi2, sum);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int q = q0 + h;

@@ -237,16 +237,18 @@ void setup_device_lists(imsrg_space* sp)
   sp->d_cls_list = sp->track(dcopy(s.cls_list));
   sp->d_cls_off = sp->track(dcopy(s.cls_off));
   sp->d_cls_sort = sp->track(dcopy(s.cls_sort));
-  // norm chunks: every 2b block in pieces of <= 65536 elements, weight (2J+1)^2
+  // norm chunks: every 2b block in pieces, weight (2J+1)^2; 8192 elements each
+  // (k_norm), longer ones where that would make more than about 4096 pieces
+  const long long piece = std::min<long long>(65536, std::max<long long>(8192, (s.arena / 4096 + 1023) / 1024 * 1024));
   std::vector<long long> no;
   std::vector<int> nl;
   std::vector<double> nw;
   for (int c = 0; c < s.nch; ++c) {
     long long nn = (long long)s.ch[c].n() * s.ch[c].n();
     double w = (double)(2 * s.ch[c].J + 1) * (2 * s.ch[c].J + 1);
-    for (long long o = 0; o < nn; o += 65536) {
+    for (long long o = 0; o < nn; o += piece) {
       no.push_back(s.ch[c].off + o);
-      nl.push_back((int)std::min<long long>(65536, nn - o));
+      nl.push_back((int)std::min<long long>(piece, nn - o));
       nw.push_back(w);
     }
   }
@@ -254,8 +256,10 @@ void setup_device_lists(imsrg_space* sp)
   sp->d_norm_off = sp->track(dcopy(no));
   sp->d_norm_len = sp->track(dcopy(nl));
   sp->d_norm_w = sp->track(dcopy(nw));
-  sp->d_norm_partial = sp->track(dmalloc<double>(sp->n_norm + 1));
-  sp->h_norm_partial.resize(sp->n_norm + 1);
+  sp->n_norm_partial = norm_partials(s, sp->n_norm);
+  sp->d_norm_partial = sp->track(dmalloc<double>(sp->n_norm_partial + 1));
+  if (cudaHostAlloc((void**)&sp->h_norm_partial, (sp->n_norm_partial + 1) * sizeof(double), cudaHostAllocPortable) != cudaSuccess)
+    throw std::runtime_error("cudaHostAlloc (norm)");
   sp->d_status = sp->track(dmalloc<int>(16));
   cudaMemset(sp->d_status, 0, 16 * sizeof(int));
 }
@@ -840,17 +844,22 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   return IMSRG_OK;
 }
 
+double norm_of_partials(const imsrg_space* sp)
+{
+  double n2 = 0.0;
+  for (int i = 0; i < sp->n_norm_partial; ++i) n2 += sp->h_norm_partial[i];
+  return std::sqrt(n2);
+}
+
 int norm_impl(const imsrg_op* op, double* out, cudaStream_t st)
 {
   imsrg_space* sp = op->sp;
   CUDA_TRY(launch_norm(*sp->s, op->d, sp->d_norm_off, sp->d_norm_len, sp->d_norm_w, sp->n_norm, sp->d_norm_partial,
                        st));
-  CUDA_TRY(cudaMemcpyAsync(sp->h_norm_partial.data(), sp->d_norm_partial, (sp->n_norm + 1) * sizeof(double),
+  CUDA_TRY(cudaMemcpyAsync(sp->h_norm_partial, sp->d_norm_partial, sp->n_norm_partial * sizeof(double),
                            cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
-  double n2 = 0.0;
-  for (int i = 0; i < sp->n_norm; ++i) n2 += sp->h_norm_partial[i];
-  *out = std::sqrt(sp->h_norm_partial[sp->n_norm] + n2);
+  *out = norm_of_partials(sp);
   return IMSRG_OK;
 }
 
@@ -1478,26 +1487,22 @@ int imsrg_bch_transform(const imsrg_op* OpIn, const imsrg_op* Omega, imsrg_op* O
     std::swap(nested.d, next.d);
     std::swap(nested.herm, next.herm);
     fden /= i;
-    // OpOut += fden nested and the norm of nested in one pass, then one
-    // host sync for the norm and (split form) the kernels' status word
+    // OpOut += fden nested and the norm of nested in one pass, with the
+    // kernels' status word after the norm's pieces: one copy and one host
+    // sync an iteration
     CUDA_TRY(launch_axpy_norm(*sp->s, OpOut->d, nested.d, fden, sp->d_norm_off, sp->d_norm_len, sp->d_norm_w,
-                              sp->n_norm, sp->d_norm_partial, st));
+                              sp->n_norm, sp->d_norm_partial, sp->d_status, st));
     if (n_nested) *n_nested = i;
     epsilon *= i + 1;
-    CUDA_TRY(cudaMemcpyAsync(sp->h_norm_partial.data(), sp->d_norm_partial, (sp->n_norm + 1) * sizeof(double),
+    CUDA_TRY(cudaMemcpyAsync(sp->h_norm_partial, sp->d_norm_partial, (sp->n_norm_partial + 1) * sizeof(double),
                              cudaMemcpyDeviceToHost, st));
-    int hstat = 0;
-    if (precision == IMSRG_PREC_SPLIT)
-      CUDA_TRY(cudaMemcpyAsync(&hstat, sp->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
-    if (hstat != 0) {
+    const int hstat = (int)sp->h_norm_partial[sp->n_norm_partial];
+    if (precision == IMSRG_PREC_SPLIT && hstat != 0) {
       cudaMemsetAsync(sp->d_status, 0, sizeof(int), st);
       return fail(IMSRG_ERR_KERNEL, "a kernel reported error status " + std::to_string(hstat));
     }
-    double n2 = 0.0;
-    for (int c = 0; c < sp->n_norm; ++c) n2 += sp->h_norm_partial[c];
-    const double nn = std::sqrt(sp->h_norm_partial[sp->n_norm] + n2);
-    if (nn < epsilon) break;
+    if (norm_of_partials(sp) < epsilon) break;
   }
   return IMSRG_OK;
 }

@@ -99,7 +99,9 @@ struct imsrg_space {
   double* d_norm_w = nullptr;
   int n_norm = 0;
   double* d_norm_partial = nullptr;
-  std::vector<double> h_norm_partial;
+  // (their host copy: page-locked, and then the kernels' status word)
+  double* h_norm_partial = nullptr;
+  int n_norm_partial = 0;
   // scratch
   double *d_xb = nullptr, *d_yt = nullptr, *d_yf = nullptr, *d_zb = nullptr, *d_w2 = nullptr;
   float2 *d_xf = nullptr, *d_yff = nullptr;  // (hi, lo) copies of X and Y for the double-float comm122ss
@@ -157,6 +159,7 @@ struct imsrg_space {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (side) cudaStreamDestroy(side);
+    if (h_norm_partial) cudaFreeHost(h_norm_partial);
     for (void* p : allocs) cudaFree(p);
     for (void* p : invd_allocs) cudaFree(p);
     delete s;

@@ -130,11 +130,12 @@ cudaError_t launch_generator(const Space& s, const double* H, double* Eta, doubl
                              cudaStream_t st);
 cudaError_t launch_axpy(double* y, const double* x, double a, long long n, cudaStream_t st);
 cudaError_t launch_scale(double* y, double a, long long n, cudaStream_t st);
-// y += a x and the norm pieces of x (as launch_norm: partial[0..nchunks) the
-// two-body chunks, partial[nchunks] the one-body part); x must have zero padding
+// y += a x and the norm pieces of x, then *status (x must have zero padding)
 cudaError_t launch_axpy_norm(const Space& s, double* y, const double* x, double a, const long long* chunk_off,
                              const int* chunk_len, const double* chunk_w, int nchunks, double* partial,
-                             cudaStream_t st);
+                             const int* status, cudaStream_t st);
+// norm pieces both launches write to partial: the chunks', then the one-body part's
+int norm_partials(const Space& s, int nchunks);
 cudaError_t launch_norm(const Space& s, const double* A, const long long* chunk_off, const int* chunk_len,
                         const double* chunk_w, int nchunks, double* partial, cudaStream_t st);
 

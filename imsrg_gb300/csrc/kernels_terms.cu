@@ -1201,39 +1201,26 @@ __global__ void k_scale(double* __restrict__ y, double a, long long n)
   for (; i < n; i += stride) y[i] *= a;
 }
 
-// Operator::Norm pieces: chunk c of the norm list sums weight * v^2 over its
-// range; partial[c] is written (no atomics, deterministic).
-__global__ void k_norm_chunks(const double* __restrict__ A, const long long* __restrict__ chunk_off,
-                              const int* __restrict__ chunk_len, const double* __restrict__ chunk_w,
-                              double* __restrict__ partial, int nchunks)
-{
-  __shared__ double red[32];
-  int c = blockIdx.x;
-  if (c >= nchunks) return;
-  const double* p = A + chunk_off[c];
-  int len = chunk_len[c];
-  double s = 0.0;
-  for (int t = threadIdx.x; t < len; t += blockDim.x) s = fma(p[t], p[t], s);
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    v = warp_sum(v);
-    if (threadIdx.x == 0) partial[c] = v * chunk_w[c];
-  }
-}
+// Operator::Norm's pieces (partial: no atomics, deterministic), and with AXPY
+// y += a x in the same pass (the BCH loop adds each nested commutator x and
+// tests its norm; *status goes after the pieces).  Block c < nchunks sums
+// weight x^2 over chunk c of the two-body blocks, the blocks after them kNorm1
+// elements each of the one-body part, (2 j_p + 1) O_pq^2 over p, q of one
+// channel.  x is a commutator result, whose padding between blocks is zero, so
+// those words of y are left as they are.  Bound by its reads; chunks of 8192
+// elements put several blocks on every SM from emax 7 on (65536 made 90 blocks
+// at emax 8, and one block took all of the one-body part: 84 us, and 126 + 24
+// in two launches without the update; BCH transform at emax 8 7773 -> 7081 us,
+// 6985 with the status word in the one copy of the pieces).
+constexpr int kNorm1 = 512;
 
-// y += a x together with the pieces of x's norm (the BCH loop adds each
-// nested commutator and tests its norm): block c < nchunks does norm chunk c
-// of the two-body blocks, block nchunks the zero- and one-body parts.  x is a
-// commutator result, whose padding between blocks is zero, so those words of
-// y are left as they are.
-__global__ void k_axpy_norm(DevSpace S, double* __restrict__ y, const double* __restrict__ x, double a,
-                            const long long* __restrict__ chunk_off, const int* __restrict__ chunk_len,
-                            const double* __restrict__ chunk_w, double* __restrict__ partial, int nchunks)
+template <bool AXPY>
+__global__ void __launch_bounds__(256) k_norm(DevSpace S, double* __restrict__ y, const double* __restrict__ x, double a,
+                                              const long long* __restrict__ chunk_off, const int* __restrict__ chunk_len,
+                                              const double* __restrict__ chunk_w, double* __restrict__ partial, int nchunks,
+                                              const int* __restrict__ status)
 {
-  __shared__ double red[32];
+  __shared__ double red[8];
   const int c = blockIdx.x;
   double s = 0.0;
   if (c < nchunks) {
@@ -1241,31 +1228,34 @@ __global__ void k_axpy_norm(DevSpace S, double* __restrict__ y, const double* __
     const int len = chunk_len[c];
     int t = threadIdx.x;
     // four elements' loads in flight per thread
-    for (; t + 3 * (int)blockDim.x < len; t += 4 * blockDim.x) {
+    for (; t + 3 * 256 < len; t += 4 * 256) {
       double v[4], w[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        v[u] = x[off + t + u * blockDim.x];
-        w[u] = y[off + t + u * blockDim.x];
+        v[u] = x[off + t + u * 256];
+        if (AXPY) w[u] = y[off + t + u * 256];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        y[off + t + u * blockDim.x] = fma(a, v[u], w[u]);
+        if (AXPY) y[off + t + u * 256] = fma(a, v[u], w[u]);
         s = fma(v[u], v[u], s);
       }
     }
-    for (; t < len; t += blockDim.x) {
+    for (; t < len; t += 256) {
       const double v = x[off + t];
-      y[off + t] = fma(a, v, y[off + t]);
+      if (AXPY) y[off + t] = fma(a, v, y[off + t]);
       s = fma(v, v, s);
     }
   } else {
-    const int N = S.norb;
-    if (threadIdx.x == 0) y[0] = fma(a, x[0], y[0]);
-    for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
+    const int N = S.norb, b = c - nchunks;
+    if (AXPY && b == 0 && threadIdx.x == 0) {
+      y[0] = fma(a, x[0], y[0]);
+      partial[gridDim.x] = (double)*status;
+    }
+    for (int t = b * kNorm1 + threadIdx.x; t < min(N * N, (b + 1) * kNorm1); t += 256) {
       const int p = t % N, q = t / N;
       const double v = x[32 + t];
-      y[32 + t] = fma(a, v, y[32 + t]);
+      if (AXPY) y[32 + t] = fma(a, v, y[32 + t]);
       if (S.l[p] == S.l[q] && S.j2[p] == S.j2[q] && S.tz2[p] == S.tz2[q]) s += v * v * (S.j2[p] + 1);
     }
   }
@@ -1273,32 +1263,8 @@ __global__ void k_axpy_norm(DevSpace S, double* __restrict__ y, const double* __
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    v = warp_sum(v);
+    const double v = warp_sum(threadIdx.x < 8 ? red[threadIdx.x] : 0.0);
     if (threadIdx.x == 0) partial[c] = c < nchunks ? v * chunk_w[c] : v;
-  }
-}
-
-// one-body norm: sum over p, q in one channel of (2 j_p + 1) O_pq^2
-__global__ void k_norm_onebody(DevSpace S, const double* __restrict__ A, double* __restrict__ out)
-{
-  __shared__ double red[32];
-  int N = S.norb;
-  double s = 0.0;
-  for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
-    int p = t % N, q = t / N;
-    if (S.l[p] == S.l[q] && S.j2[p] == S.j2[q] && S.tz2[p] == S.tz2[q]) {
-      double v = A[32 + t];
-      s += v * v * (S.j2[p] + 1);
-    }
-  }
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    v = warp_sum(v);
-    if (threadIdx.x == 0) *out = v;
   }
 }
 
@@ -1590,12 +1556,14 @@ cudaError_t launch_scale(double* y, double a, long long n, cudaStream_t st)
   return cudaGetLastError();
 }
 
+int norm_partials(const Space& s, int nchunks) { return nchunks + (s.norb * s.norb + kNorm1 - 1) / kNorm1; }
+
 cudaError_t launch_axpy_norm(const Space& s, double* y, const double* x, double a, const long long* chunk_off,
                              const int* chunk_len, const double* chunk_w, int nchunks, double* partial,
-                             cudaStream_t st)
+                             const int* status, cudaStream_t st)
 {
-  // the one-body block first: it is the longest
-  k_axpy_norm<<<nchunks + 1, 256, 0, st>>>(s.dev, y, x, a, chunk_off, chunk_len, chunk_w, partial, nchunks);
+  k_norm<true><<<norm_partials(s, nchunks), 256, 0, st>>>(s.dev, y, x, a, chunk_off, chunk_len, chunk_w, partial, nchunks,
+                                                         status);
   count_launch();
   return cudaGetLastError();
 }
@@ -1603,11 +1571,8 @@ cudaError_t launch_axpy_norm(const Space& s, double* y, const double* x, double 
 cudaError_t launch_norm(const Space& s, const double* A, const long long* chunk_off, const int* chunk_len,
                         const double* chunk_w, int nchunks, double* partial, cudaStream_t st)
 {
-  k_norm_onebody<<<1, 256, 0, st>>>(s.dev, A, partial + nchunks);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || nchunks == 0) return e;
-  k_norm_chunks<<<nchunks, 256, 0, st>>>(A, chunk_off, chunk_len, chunk_w, partial, nchunks);
+  k_norm<false><<<norm_partials(s, nchunks), 256, 0, st>>>(s.dev, nullptr, A, 0.0, chunk_off, chunk_len, chunk_w, partial,
+                                                          nchunks, nullptr);
   count_launch();
   return cudaGetLastError();
 }

@@ -324,6 +324,7 @@ int tune_apply(imsrg_space* sp, int t, int v)
 {
   if (!tune_valid(t, v)) return fail(IMSRG_ERR_ARG, std::string("bad value for ") + kTuneNames[t]);
   int* slot = tune_slot(sp, t);
+  if (t == 6 || t == 7) sp->inv_set[t == 6] = true;
   if (*slot == v) return IMSRG_OK;
   *slot = v;
   if (t == 0 || t == 3) (t == 0 ? sp->opt_ladder : sp->opt_zbar).nacc = v == 64 ? 1 : (v == 32 ? 2 : 0);
@@ -482,6 +483,7 @@ void drop_invd(imsrg_space* sp)
   sp->invd_allocs.clear();
   sp->invd = InvdDev{};
   sp->invd_ready = false;
+  sp->invd_tried = false;
 }
 
 // the inverse Pandya descriptors of the space (built on first use)
@@ -518,13 +520,24 @@ int ensure_invd(imsrg_space* sp)
   return IMSRG_OK;
 }
 
-// AddInversePandyaTransformation of zb into Z with the kernel the space's
-// tuning selects for the form (grouped: nz pairs at the offsets zo)
-int inverse_pandya(imsrg_space* sp, const double* zb, double* Z, int hZ, int prec, cudaStream_t st,
+// The form's inverse Pandya kernel inside a commutator: 1, 2 the descriptor
+// kernel (double-float, FP64), 0 quadruple blocks (split) or channel tiles.
+// Where neither a call nor the tuning file has chosen, the descriptors: they
+// fold comm122ss's update in and let the Z bar product skip its mirror.  Whole
+// commutators, quadruple blocks or tiles against descriptors: split 123 / 109
+// us at emax 3, 457 / 360 at 7, 1902 / 1512 at 9, 8368 / 6995 at 11; FP64 214 /
+// 180 at 5, 730 / 637 at 7 (Ca40), 3277 / 2831 at 9, 17.3 / 15.0 ms at 11.
+// Built once a space (20 ms at emax 7, 0.15 s at 9, 0.66 s at 11); beyond emax
+// 11, where that takes seconds and gigabytes on the host, only when asked for.
+// They are not built under capture, nor twice where they did not fit.
+int inv_variant(imsrg_space* sp, int prec, cudaStream_t st);
+
+// AddInversePandyaTransformation of zb into Z with that kernel (grouped: nz
+// pairs at the offsets zo)
+int inverse_pandya(imsrg_space* sp, const double* zb, double* Z, int hZ, int prec, int variant, cudaStream_t st,
                    const long long* zo = nullptr, int nz = 1, const void* w2 = nullptr, int w2mode = 0)
 {
   Space& s = *sp->s;
-  const int variant = prec == IMSRG_PREC_SPLIT ? sp->inv_split : (sp->inv_fp64 ? 2 : 0);
   if (variant == 1 || variant == 2) {
     int rc = ensure_invd(sp);
     if (rc) return rc;
@@ -543,10 +556,26 @@ int inverse_pandya(imsrg_space* sp, const double* zb, double* Z, int hZ, int pre
   return IMSRG_OK;
 }
 
-// whether the form's inverse Pandya kernel can apply comm122ss's update too
-bool inverse_folds(imsrg_space* sp, int prec, int& rc)
+int inv_variant(imsrg_space* sp, int prec, cudaStream_t st)
 {
-  const int variant = prec == IMSRG_PREC_SPLIT ? sp->inv_split : (sp->inv_fp64 ? 2 : 0);
+  const bool split = prec == IMSRG_PREC_SPLIT;
+  if (sp->inv_set[split] || sp->s->arena >= (1ll << 27)) return split ? sp->inv_split : (sp->inv_fp64 ? 2 : 0);
+  if (!sp->invd_ready && !sp->invd_tried && !capturing(st)) {
+    // (about 20 bytes an arena word; the call's other scratch and plans, made
+    // after this, take up to 140)
+    size_t room = 0, all = 0;
+    const bool fits = cudaMemGetInfo(&room, &all) == cudaSuccess && room >= 160 * (size_t)sp->s->arena;
+    const int rc = fits ? ensure_invd(sp) : IMSRG_ERR_NOMEM;
+    sp->invd_tried = true;
+    if (rc) cudaGetLastError();  // no room: the other kernel runs
+  }
+  return !sp->invd_ready ? 0 : split ? 1 : 2;
+}
+
+// whether the form's inverse Pandya kernel can apply comm122ss's update too
+bool inverse_folds(imsrg_space* sp, int prec, int& rc, cudaStream_t st)
+{
+  const int variant = inv_variant(sp, prec, st);
   if (variant != 1 && variant != 2) return false;
   rc = ensure_invd(sp);
   return rc == IMSRG_OK && sp->invd.covers_all;
@@ -738,7 +767,7 @@ int zbar_product(imsrg_space* sp, int hZ, int prec, cudaStream_t st)
     int rc = ensure_split(sp);
     if (rc) return rc;
     // the descriptor inverse kernels read only Zbar's upper triangle
-    split_plan_set_mirror(sp->split_zbar, sp->inv_split == 0 ? 1 : 0);
+    split_plan_set_mirror(sp->split_zbar, inv_variant(sp, prec, st) == 0 ? 1 : 0);
     CUDA_TRY(launch_symgemm_split(sp->split_zbar, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx,
                                   s.work.kweight, s.work.phase_tab, sp->d_status, hZ, 1.0, st));
     return IMSRG_OK;
@@ -747,7 +776,7 @@ int zbar_product(imsrg_space* sp, int hZ, int prec, cudaStream_t st)
   if (DgemmPlan* p = fp64_plan(&sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
     // the descriptor inverse kernel reads only Zbar's upper triangle
     CUDA_TRY(launch_dgemm(p, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, hZ,
-                          1.0, 0, sp->inv_fp64 == 0, st));
+                          1.0, 0, inv_variant(sp, prec, st) == 0, st));
   else
     CUDA_TRY(launch_symgemm_fp64(sp->d_zbar_jobs, sp->d_zbar_pairs, sp->n_zbar_pairs, sp->d_xb, sp->d_yt, sp->d_yf,
                                  sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, hZ, 1.0, 0, st));
@@ -760,8 +789,8 @@ int ph_inverse(imsrg_op* Z, int prec, cudaStream_t st, bool fold_w2)
 {
   imsrg_space* sp = Z->sp;
   ProfScope pinv("InversePandyaTransformation", st);
-  return inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, prec, st, nullptr, 1, fold_w2 ? (const void*)sp->d_w2 : nullptr,
-                        fold_w2 ? (prec == IMSRG_PREC_SPLIT ? 1 : 2) : 0);
+  return inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, prec, inv_variant(sp, prec, st), st, nullptr, 1,
+                        fold_w2 ? (const void*)sp->d_w2 : nullptr, fold_w2 ? (prec == IMSRG_PREC_SPLIT ? 1 : 2) : 0);
 }
 
 int do_ph(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaStream_t st)
@@ -805,7 +834,7 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   bool fold = false;
   if (w2 && on[T222PH]) {
     int rf = IMSRG_OK;
-    fold = inverse_folds(sp, prec, rf);
+    fold = inverse_folds(sp, prec, rf, st);
     if (rf) return rf;
   }
   // The terms add into Z in an order of our own (the sum is the same up to
@@ -1352,7 +1381,8 @@ int imsrg_add_inverse_pandya(const double* zbar, imsrg_op* Z, int precision, voi
   if (precision != IMSRG_PREC_FP64 && precision != IMSRG_PREC_SPLIT) return fail(IMSRG_ERR_ARG, "bad precision");
   cudaStream_t st = S_(stream);
   ProfScope ps("InversePandyaTransformation", st);
-  return inverse_pandya(Z->sp, zbar, Z->d, Z->herm, precision, st);
+  return inverse_pandya(Z->sp, zbar, Z->d, Z->herm, precision,
+                        precision == IMSRG_PREC_SPLIT ? Z->sp->inv_split : (Z->sp->inv_fp64 ? 2 : 0), st);
 }
 
 int imsrg_space_set_tuning(imsrg_space* sp, const char* name, int value)
@@ -1622,7 +1652,7 @@ GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, 
       zj.push_back(j);
     }
   }
-  if (prec == IMSRG_PREC_FP64 && s0->inv_fp64 == 0) {
+  if (prec == IMSRG_PREC_FP64 && inv_variant(s0, prec, nullptr) == 0) {
     if (why) *why = "the FP64 form's grouped inverse Pandya needs the descriptor kernel (inverse.fp64 = 1)";
     return nullptr;
   }
@@ -1710,7 +1740,7 @@ int group_mid(GroupedProducts* g, cudaStream_t st)
   const long long* zo = g->d_zoff;
   CUDA_TRY(launch_comm221_z(s, Z->d, Z->herm, Z->d, st, zo, nz));
   int rc = IMSRG_OK;
-  g->fold = !(g->prec == IMSRG_PREC_SPLIT && sp->comm122_fused) && inverse_folds(sp, g->prec, rc);
+  g->fold = !(g->prec == IMSRG_PREC_SPLIT && sp->comm122_fused) && inverse_folds(sp, g->prec, rc, st);
   if (rc) return rc;
   const int part = g->fold ? W2_MAKE : W2_MAKE | W2_SUBTRACT;
   if (g->prec == IMSRG_PREC_FP64)
@@ -1730,8 +1760,9 @@ int group_post(GroupedProducts* g, cudaStream_t st)
   imsrg_op* Z = g->Z[0];
   imsrg_space* sp = g->X[0]->sp;
   const Space& s = *sp->s;
-  if (g->prec == IMSRG_PREC_FP64 || sp->inv_split != 0 || sp->n_invq > 0) {
-    int rc = inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, g->prec, st, g->d_zoff, nz, g->fold ? (const void*)sp->d_w2 : nullptr,
+  const int variant = inv_variant(sp, g->prec, st);
+  if (variant != 0 || (g->prec == IMSRG_PREC_SPLIT && sp->n_invq > 0)) {
+    int rc = inverse_pandya(sp, sp->d_zb, Z->d, Z->herm, g->prec, variant, st, g->d_zoff, nz, g->fold ? (const void*)sp->d_w2 : nullptr,
                             g->fold ? (g->prec == IMSRG_PREC_SPLIT ? 1 : 2) : 0);
     if (rc) return rc;
   } else {
@@ -1773,7 +1804,7 @@ int grouped_zbar(GroupedProducts* g, cudaStream_t st)
   const Space& s = *s0->s;
   if (g->fp64_zbar) {
     CUDA_TRY(launch_dgemm(g->fp64_zbar, s0->d_xb, s0->d_yt, s0->d_yf, s0->d_zb, s.work.kidx, s.work.kweight,
-                          s.work.phase_tab, g->Z[0]->herm, 1.0, 0, s0->inv_fp64 == 0, st));
+                          s.work.phase_tab, g->Z[0]->herm, 1.0, 0, inv_variant(s0, g->prec, st) == 0, st));
     return IMSRG_OK;
   }
   if (g->prec == IMSRG_PREC_FP64) {
@@ -1781,7 +1812,7 @@ int grouped_zbar(GroupedProducts* g, cudaStream_t st)
                                  s.work.kweight, s.work.phase_tab, g->Z[0]->herm, 1.0, 0, st));
     return IMSRG_OK;
   }
-  split_plan_set_mirror(g->zbar, s0->inv_split == 0 ? 1 : 0);  // as group_post reads Zbar
+  split_plan_set_mirror(g->zbar, inv_variant(s0, g->prec, st) == 0 ? 1 : 0);  // as group_post reads Zbar
   CUDA_TRY(launch_symgemm_split(g->zbar, s0->d_xb, s0->d_yt, s0->d_yf, s0->d_zb, s.work.kidx, s.work.kweight,
                                 s.work.phase_tab, s0->d_status, g->Z[0]->herm, 1.0, st));
   return IMSRG_OK;

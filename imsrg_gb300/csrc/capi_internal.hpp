@@ -127,6 +127,8 @@ struct imsrg_space {
   int inv_split = 0;  // split form's inverse Pandya: 0 quadruple blocks (double-float), 1 descriptors
                       // (double-float), 2 descriptors (FP64)
   int inv_fp64 = 0;   // FP64 form's inverse Pandya: 0 channel tiles, 1 descriptors (FP64)
+  bool inv_set[2] = {false, false};  // inv_fp64, inv_split set, by a call or the tuning file (inv_variant)
+  bool invd_tried = false;
   int invq_budget = imsrg::kInvqBudget;
   int invd_stage = 2048, invd_res = 2048;
   int invd_weights = 0;  // descriptor kernel: 1 stages the 6j weight rows per block

@@ -86,10 +86,10 @@ bool capturing(cudaStream_t st)
 }
 int second_stream(imsrg_space* sp)
 {
-  if (sp->side) return IMSRG_OK;
-  CUDA_TRY(cudaStreamCreateWithFlags(&sp->side, cudaStreamNonBlocking));
-  CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_fork, cudaEventDisableTiming));
-  CUDA_TRY(cudaEventCreateWithFlags(&sp->ev_join, cudaEventDisableTiming));
+  for (cudaStream_t* s : {&sp->side, &sp->side2})
+    if (!*s) CUDA_TRY(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&sp->ev_fork, &sp->ev_join, &sp->ev_join2})
+    if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return IMSRG_OK;
 }
 }  // namespace imsrg
@@ -826,7 +826,7 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
     CUDA_TRY(cudaMemsetAsync(Z->d, 0, sp->s->arena * sizeof(double), st));
   const bool split = prec == IMSRG_PREC_SPLIT;
   // comm122ss's W2 reads only X and Y (not so the fused split form, which
-  // updates Z): it is formed on the second stream.  Its Z -= W2 + hZ W2^T
+  // updates Z): it is formed beside the second stream.  Its Z -= W2 + hZ W2^T
   // rides in the inverse Pandya kernel, which reads and writes every
   // upper-triangle element of Z and its mirror anyway, when that kernel is
   // the descriptor one and lists every element
@@ -843,24 +843,39 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   // instead of recomputing the pp dot products (ConstructScalarMpp_Mhh is
   // shared the same way by the reference's comm222_pp_hh_221ss).
   //
-  // While the ladder product runs on st, a second stream does what does not
-  // depend on it: comm122ss's W2, the zero- and one-body terms (they write
-  // only Z0 and Z1, the ladder only Z2) and comm222_phss up to Z bar, whose
-  // product takes the SMs that the ladder leaves (small spaces) or has left.
-  // The streams join before comm221ss's last part, which reads Z2 and writes
-  // Z1.  (W2 and Z bar after the ladder instead: 100 against 78 us at emax 2
-  // FP64, 310 against 279 at emax 6, 3.31 against 3.22 ms at emax 10 split.)
+  // While the ladder product runs on st, a second stream takes comm222_phss up
+  // to Z bar, whose product gets the SMs that the ladder leaves (small spaces)
+  // or has left, and a third the zero- and one-body terms (they write only Z0
+  // and Z1, the ladder only Z2) and the split form's float pairs; comm122ss's
+  // W2 follows the ladder on st.  Up to emax 7 a call is one chain of short
+  // kernels, the longest of these three: with the one-body terms and W2 in the
+  // second stream's chain 60.6 us at emax 2 FP64, 115 at 4 split, 275 at 6, 625
+  // at 7 (Ca40), 51 / 103 / 247 / 589 so; 6.59 -> 6.54 ms at emax 10 FP64, 3.26
+  // -> 3.24 split, where the chip is full either way.  (No second stream: 100 us
+  // at emax 2, 310 at 6.)  The split form's larger spaces keep all of it on the
+  // second stream, W2 before Z bar's product: it then runs beside the ladder,
+  // 7134 -> 6975 us at emax 11, 15.27 -> 14.79 ms at 12 (at 8 and 9 it costs
+  // 27 and 12 us, at 10 nothing).  All join before comm221ss's last part, which
+  // reads Z2 and writes Z1.
+  const bool beside = split && sp->s->arena >= (1ll << 26);
+  cudaStream_t sd2 = beside ? sd : sp->side2;
   CUDA_TRY(cudaEventRecord(sp->ev_fork, st));
   CUDA_TRY(cudaStreamWaitEvent(sd, sp->ev_fork, 0));
-  if (on[T122] && split && (rc = prep_122_df(X, Y, sd))) return rc;
+  if (!beside) CUDA_TRY(cudaStreamWaitEvent(sd2, sp->ev_fork, 0));
   if (on[T222PH] && (rc = prep_ph(X, Y, prec, sd))) return rc;
   const int todo = (on[T111] ? OB_111 : 0) | (on[T110] ? OB_110 : 0) | (on[T121] ? OB_121 : 0) | (on[T220] ? OB_220 : 0) |
                    (on[T221] && ladder_first ? OB_221 : 0);
-  if ((rc = do_onebody(X, Y, Z, todo, "zero- and one-body terms", sd))) return rc;
-  if (w2 && (rc = do_122(X, Y, Z, sd, prec, split, W2_MAKE))) return rc;
+  if ((rc = do_onebody(X, Y, Z, todo, "zero- and one-body terms", sd2))) return rc;
+  if (on[T122] && split && (rc = prep_122_df(X, Y, sd2))) return rc;
+  if (beside && w2 && (rc = do_122(X, Y, Z, sd, prec, split, W2_MAKE))) return rc;
+  if (!beside) CUDA_TRY(cudaEventRecord(sp->ev_join2, sd2));
   if (on[T222PH] && (rc = zbar_product(sp, Z->herm, prec, sd))) return rc;
   CUDA_TRY(cudaEventRecord(sp->ev_join, sd));
   if (ladder_first && (rc = do_ladder(X, Y, Z, prec, st, true))) return rc;
+  if (!beside) {
+    CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join2, 0));
+    if (w2 && (rc = do_122(X, Y, Z, st, prec, split, W2_MAKE))) return rc;
+  }
   CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join, 0));
   if (on[T221] && ladder_first) {
     ProfScope p221("comm221ss", st);

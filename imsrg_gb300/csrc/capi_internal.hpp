@@ -26,7 +26,7 @@ namespace imsrg {
 int set_error(int code, const char* msg);
 // whether st is being captured into a graph (nothing may be allocated then)
 bool capturing(cudaStream_t st);
-// makes the space's second stream and its events
+// makes the space's second and third stream and their events
 int second_stream(imsrg_space* sp);
 // CommutatorScalarScalar into Z (overwritten), Operator::Norm (synchronises
 // st), and the kernels' error word (synchronises st; IMSRG_ERR_KERNEL if set)
@@ -141,8 +141,9 @@ struct imsrg_space {
   std::vector<void*> invd_allocs;
   // second stream of CommutatorScalarScalar (work independent of the ladder
   // product) and the events that fork it from and join it to the caller's
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // (side2: a third, for what neither waits for)
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
 
   template <class T>
   T* track(T* p)
@@ -160,7 +161,9 @@ struct imsrg_space {
     if (fp64_ev) cudaEventDestroy(fp64_ev);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
+    if (ev_join2) cudaEventDestroy(ev_join2);
     if (side) cudaStreamDestroy(side);
+    if (side2) cudaStreamDestroy(side2);
     if (h_norm_partial) cudaFreeHost(h_norm_partial);
     for (void* p : allocs) cudaFree(p);
     for (void* p : invd_allocs) cudaFree(p);

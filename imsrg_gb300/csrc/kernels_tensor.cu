@@ -801,8 +801,8 @@ __device__ __forceinline__ double zbar_val(const DevSpace& S, const DevTensor& T
 // DF: the sums in double-float on the FP32 pipe, each quadruple's values
 // scaled by their largest exponent; else in FP64, bound by its pipe.
 // A warp per quadruple and FP64 sums took 6.43 ms at emax 8, rank (2, 0, +),
-// and 1.00 ms at emax 6, rank (1, 1, +); this takes 2.70 ms (DF) and 0.31 ms
-// (FP64).
+// and 1.00 ms at emax 6, rank (1, 1, +); this takes 2.61 ms (DF: half its issue
+// slots, the rest waiting for Z bar and the 9j rows) and 0.31 ms (FP64).
 constexpr int kTqThreads = 256;
 
 // floor(x / n) for 0 <= x < 2^16, 1 <= n <= 128 and r = 1.0f / n: (x + 1/2) / n is
@@ -887,8 +887,10 @@ __device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, in
   }
 }
 
+// (five blocks an SM in FP64: rank (1, 1, +) commutator at emax 6 1264 -> 1211
+// us; in DF the 48 registers that leaves spill: 8.42 -> 8.84 ms at emax 8)
 template <bool DF>
-__global__ void __launch_bounds__(kTqThreads) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
+__global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
                                                        double* __restrict__ Z, const int2* __restrict__ tq,
                                                        const int2* __restrict__ batches)
 {

@@ -157,8 +157,9 @@ struct TensorLayout {
 
 // the space's layout of rank (lam, trank, parity), built on first use
 // (host tables only; tensor_upload copies them to the device)
-// quadruples a batch holds at most, and the gathered values (8 bytes each)
-constexpr int kTqBatch = 128, kTqValues = 5120;
+// quadruples a batch holds at most, and the gathered values (8 bytes each:
+// 30 KB a block leave the L1 half of an SM's memory at five blocks)
+constexpr int kTqBatch = 128, kTqValues = 3840;
 TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity);
 void tensor_upload(TensorLayout& t);
 // the same view with host pointers (host-side 9j and 6j evaluation)

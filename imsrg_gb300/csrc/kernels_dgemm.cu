@@ -37,7 +37,8 @@
 // (the emax=10 ladder: 2.6 ms, tensor pipe 58%, 13.4 TB/s from L2); for the
 // short ones (Zbar, K <= 132) the epilogue.  With the FP64-pipe kernel the
 // commutator takes 142 us at emax 2, 1.26 ms at emax 6, 87.2 ms at emax 10;
-// with this one 116 us, 0.38 ms and 7.7 ms: it is used at every size, and
+// with this one, and nothing else changed, it took 116 us, 0.38 ms and 7.7 ms
+// (51 us, 0.25 ms and 6.5 ms by now): it is used at every size, and
 // the FP64-pipe kernel only where the planes do not fit (40 bytes an element
 // pair of the operands) or inside a capture that comes before them.
 #include <cuda.h>
@@ -46,6 +47,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <stdexcept>
 #include <vector>
 
@@ -109,6 +111,7 @@ struct DgemmPlan {
   int family = 0;
   int njobs = 0, ntiles = 0, grid = 0;
   long long rows = 0, exp_rows = 0;
+  void* mem = nullptr;  // everything below
   DJob* d_jobs = nullptr;
   DTile* d_tiles = nullptr;
   int* d_cta = nullptr;
@@ -1024,31 +1027,42 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
   p->n_rblk = (int)rb.size();
   p->n_dblk = (int)db.size();
   try {
-    auto dm = [](size_t bytes) {
-      void* q = nullptr;
-      if (cudaMalloc(&q, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-        cudaGetLastError();
-        throw std::runtime_error("cudaMalloc");
-      }
-      return q;
+    // one allocation and one copy a plan (a batch of new operators makes two
+    // plans a group): the tables, then the exponents, lists and planes
+    size_t size = 0;
+    auto take = [&](size_t bytes) {
+      const size_t at = size;
+      size += (std::max<size_t>(bytes, 16) + 1023) / 1024 * 1024;
+      return at;
     };
-    auto up = [&](const void* src, size_t bytes) {
-      void* q = dm(bytes);
-      if (cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(q);
-        throw std::runtime_error("cudaMemcpy");
-      }
-      return q;
-    };
-    for (int a = 0; a < 2; ++a) p->arr[a] = (__nv_bfloat16*)dm((size_t)NP * p->rows * KB * 2);
-    p->d_exp = (int*)dm(sizeof(int) * 2 * p->exp_rows);
-    p->d_list = (int*)dm(sizeof(int) * p->ntiles);
-    p->d_elem = (DElem*)dm(sizeof(DElem) * MAX_LISTED * COLS_W * (size_t)p->ntiles);
-    p->d_jobs = (DJob*)up(jobs.data(), sizeof(DJob) * jobs.size());
-    p->d_tiles = (DTile*)up(sorted.data(), sizeof(DTile) * sorted.size());
-    p->d_cta = (int*)up(first.data(), sizeof(int) * first.size());
-    p->d_rblk = (int4*)up(rb.data(), sizeof(int4) * rb.size());
-    p->d_dblk = (int4*)up(db.data(), sizeof(int4) * db.size());
+    const size_t o_jobs = take(sizeof(DJob) * jobs.size()), o_tiles = take(sizeof(DTile) * sorted.size());
+    const size_t o_cta = take(sizeof(int) * first.size());
+    const size_t o_rblk = take(sizeof(int4) * rb.size()), o_dblk = take(sizeof(int4) * db.size());
+    std::vector<char> tables(size, 0);
+    std::memcpy(tables.data() + o_jobs, jobs.data(), sizeof(DJob) * jobs.size());
+    std::memcpy(tables.data() + o_tiles, sorted.data(), sizeof(DTile) * sorted.size());
+    std::memcpy(tables.data() + o_cta, first.data(), sizeof(int) * first.size());
+    if (!rb.empty()) std::memcpy(tables.data() + o_rblk, rb.data(), sizeof(int4) * rb.size());
+    if (!db.empty()) std::memcpy(tables.data() + o_dblk, db.data(), sizeof(int4) * db.size());
+    const size_t o_exp = take(sizeof(int) * 2 * p->exp_rows), o_list = take(sizeof(int) * p->ntiles);
+    const size_t o_elem = take(sizeof(DElem) * MAX_LISTED * COLS_W * (size_t)p->ntiles);
+    const size_t o_arr[2] = {take((size_t)NP * p->rows * KB * 2), take((size_t)NP * p->rows * KB * 2)};
+    if (cudaMalloc(&p->mem, size) != cudaSuccess) {
+      p->mem = nullptr;
+      cudaGetLastError();
+      throw std::runtime_error("cudaMalloc");
+    }
+    if (cudaMemcpy(p->mem, tables.data(), tables.size(), cudaMemcpyHostToDevice) != cudaSuccess) throw std::runtime_error("cudaMemcpy");
+    char* base = (char*)p->mem;
+    p->d_jobs = (DJob*)(base + o_jobs);
+    p->d_tiles = (DTile*)(base + o_tiles);
+    p->d_cta = (int*)(base + o_cta);
+    p->d_rblk = (int4*)(base + o_rblk);
+    p->d_dblk = (int4*)(base + o_dblk);
+    p->d_exp = (int*)(base + o_exp);
+    p->d_list = (int*)(base + o_list);
+    p->d_elem = (DElem*)(base + o_elem);
+    for (int a = 0; a < 2; ++a) p->arr[a] = (__nv_bfloat16*)(base + o_arr[a]);
     for (int a = 0; a < 2; ++a) {
       plane_map(&p->maps[a], p->arr[a], p->rows, TM);
       plane_map(&p->maps[2 + a], p->arr[a], p->rows, TN);
@@ -1073,9 +1087,7 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
 void dgemm_plan_destroy(DgemmPlan* p)
 {
   if (!p) return;
-  for (void* q : {(void*)p->arr[0], (void*)p->arr[1], (void*)p->d_exp, (void*)p->d_list, (void*)p->d_elem, (void*)p->d_jobs, (void*)p->d_tiles,
-                  (void*)p->d_cta, (void*)p->d_rblk, (void*)p->d_dblk})
-    if (q) cudaFree(q);
+  if (p->mem) cudaFree(p->mem);
   delete p;
 }
 

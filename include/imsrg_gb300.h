@@ -45,7 +45,10 @@ extern "C" {
 #define IMSRG_ERR_IO 7          /* a file could not be opened, read or written */
 
 /* precision of the dense contractions (ladder and Pandya channel GEMMs) */
-#define IMSRG_PREC_FP64 0  /* plain FP64 (CUDA-core DFMA) */
+#define IMSRG_PREC_FP64 0  /* FP64: 62-bit fixed point in nine BF16 digits on the tensor cores (tcgen05), each
+                              element checked against the classical bound of an FP64 sum and formed with
+                              FP64 FMAs where the digits cannot vouch for it; CUDA-core DFMA where the
+                              digit planes do not fit, or under capture before they exist */
 #define IMSRG_PREC_SPLIT 1 /* Ozaki-style sliced BF16 tensor-core products (tcgen05), FP64 recombination */
 
 /* generator functions (src/Generator.cc:12-15) and energy-denominator
@@ -251,7 +254,8 @@ int imsrg_comm222_phss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int pr
  * selects the form of the ladder and Pandya-space (Z bar) products, as for the
  * scalar commutator: IMSRG_PREC_FP64, or IMSRG_PREC_SPLIT (tensor cores; the call
  * then synchronises the stream and checks the kernels' status word, as the
- * scalar entry points do); every other sum is FP64. */
+ * scalar entry points do; its inverse Pandya sums are double-float); every
+ * other sum is FP64. */
 int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int precision, void* stream);
 /* its terms, each accumulating into Z (src/TensorCommutators.cc) */
 /* comm111st, src/TensorCommutators.cc:25-30 */
@@ -320,7 +324,7 @@ int imsrg_get_term(const char* name, int* on);
  * commutator (both dense products included) runs as one grouped launch for
  * all pairs whose spaces have the same orbits and whose operators the same
  * hermiticities, in either precision (the FP64 form needs the descriptor
- * inverse Pandya kernel, "inverse.fp64" = 1, as tuned).
+ * inverse Pandya kernel, which it takes unless "inverse.fp64" was set to 0).
  * Creating a batch evaluates every pair once (allocating all scratch) and
  * captures the graph; the operators, their spaces and the term switches are
  * fixed from then on, and every operator must outlive the batch.  No Z may
@@ -352,8 +356,11 @@ int imsrg_batch_info(const imsrg_batch* batch, int* n_pairs, int* n_branches, in
  *   "inverse.split"                     split form: 0 orbit-quadruple blocks,
  *                                       1 descriptors with double-float sums,
  *                                       2 descriptors with FP64 sums
+ *                                       (never set: commutators of up to 2^27
+ *                                       arena words take 1, where it fits)
  *   "inverse.fp64"                      FP64 form: 0 channel tiles, 1
- *                                       descriptors (FP64 sums)
+ *                                       descriptors (FP64 sums) (never set:
+ *                                       commutators take 1, likewise)
  *   "inverse.quad_budget"               shared-memory bytes per quadruple block
  *   "inverse.desc_stage", "inverse.desc_results"
  *                                       staged values / results per descriptor block
@@ -362,10 +369,12 @@ int imsrg_batch_info(const imsrg_batch* batch, int* n_pairs, int* n_branches, in
  *   "inverse.desc_ilp"                  results each thread of the descriptor
  *                                       kernel keeps in flight: 1, 2 or 4
  *   "ladder.digits", "zbar.digits"      digits per operand of the split
- *                                       products, 5..7 (0: as many as 36 bits
- *                                       need at the digit width that keeps the
- *                                       leading FP32 sums exact); the width
- *                                       times the count is the precision
+ *                                       products, 5..7, of the width that keeps
+ *                                       the leading FP32 sums exact; the width
+ *                                       times the count is the precision (0:
+ *                                       six of 7 bits for reductions up to
+ *                                       339, beyond that five of 8 bits, 38 in
+ *                                       all, summed in exact chunks)
  *   "comm122.fused"                     split-form comm122ss: 1 forms W2 tile
  *                                       pairs in shared memory and updates Z
  *                                       directly (no W2 array)

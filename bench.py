@@ -480,7 +480,8 @@ def roofline(phases, work, emax):
                 "frac": ach / bf16_peak, "traffic": None,
                 "issued_bf16_tflops": issued * ach, "issued_frac": issued * ach / bf16_peak,
                 "note": "achieved counts FP64-equivalent algorithmic flops (the digit products issue %dx "
-                        "as many BF16 flops); peak = bf16 dense burst, %s" % (issued, peak_src)}
+                        "as many BF16 flops); timed inside the commutator, beside the other stream's "
+                        "product; peak = bf16 dense burst, %s" % (issued, peak_src)}
     else:
         ach = amount / avg_s / 1e9
         roof = {"kernel": best, "bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s",

@@ -88,7 +88,7 @@ int second_stream(imsrg_space* sp)
 {
   for (cudaStream_t* s : {&sp->side, &sp->side2})
     if (!*s) CUDA_TRY(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
-  for (cudaEvent_t* e : {&sp->ev_fork, &sp->ev_join, &sp->ev_join2})
+  for (cudaEvent_t* e : {&sp->ev_fork, &sp->ev_join, &sp->ev_join2, &sp->ev_onebody})
     if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return IMSRG_OK;
 }
@@ -846,18 +846,23 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   // While the ladder product runs on st, a second stream takes comm222_phss up
   // to Z bar, whose product gets the SMs that the ladder leaves (small spaces)
   // or has left, and a third the zero- and one-body terms (they write only Z0
-  // and Z1, the ladder only Z2) and the split form's float pairs; comm122ss's
-  // W2 follows the ladder on st.  Up to emax 7 a call is one chain of short
-  // kernels, the longest of these three: with the one-body terms and W2 in the
-  // second stream's chain 60.6 us at emax 2 FP64, 115 at 4 split, 275 at 6, 625
-  // at 7 (Ca40), 51 / 103 / 247 / 589 so; 6.59 -> 6.54 ms at emax 10 FP64, 3.26
-  // -> 3.24 split, where the chip is full either way.  (No second stream: 100 us
-  // at emax 2, 310 at 6.)  The split form's larger spaces keep all of it on the
-  // second stream, W2 before Z bar's product: it then runs beside the ladder,
-  // 7134 -> 6975 us at emax 11, 15.27 -> 14.79 ms at 12 (at 8 and 9 it costs
-  // 27 and 12 us, at 10 nothing).  All join before comm221ss's last part, which
-  // reads Z2 and writes Z1.
+  // and Z1, the ladder only Z2) and the split form's float pairs; comm221ss's
+  // last part, which reads Z2 as the ladder leaves it and adds to Z1, follows
+  // the ladder on st.  Up to emax 7 a call is chains of short kernels: with the
+  // one-body terms and W2 in the second stream's chain 60.6 us at emax 2 FP64,
+  // 115 at 4 split, 275 at 6, 625 at 7 (Ca40), 51 / 103 / 247 / 589 on three
+  // streams; 6.59 -> 6.54 ms at emax 10 FP64, 3.26 -> 3.24 split, where the chip
+  // is full either way.  (No second stream: 100 us at emax 2, 310 at 6.)
+  //
+  // comm122ss's W2 goes where it is hidden best.  After the one-body terms on
+  // the third stream in small spaces (against after the ladder: FP64 138 -> 129
+  // us at emax 5, 252 -> 247 at 6, but 589 -> 596 at 7, Ca40; split 103 -> 99 at
+  // 4, 196 -> 184 at 6, 717 -> 711 at 8, 1511 -> 1503 at 9); after the ladder on
+  // st in larger ones; and in the split form from 2^26 words before Z bar's
+  // product on the second stream, which then takes all of it, so that W2 runs
+  // beside the ladder (7134 -> 6975 us at emax 11, 15.27 -> 14.79 ms at 12).
   const bool beside = split && sp->s->arena >= (1ll << 26);
+  const bool small = sp->s->arena < (1ll << (split ? 24 : 21));
   cudaStream_t sd2 = beside ? sd : sp->side2;
   CUDA_TRY(cudaEventRecord(sp->ev_fork, st));
   CUDA_TRY(cudaStreamWaitEvent(sd, sp->ev_fork, 0));
@@ -866,23 +871,24 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   const int todo = (on[T111] ? OB_111 : 0) | (on[T110] ? OB_110 : 0) | (on[T121] ? OB_121 : 0) | (on[T220] ? OB_220 : 0) |
                    (on[T221] && ladder_first ? OB_221 : 0);
   if ((rc = do_onebody(X, Y, Z, todo, "zero- and one-body terms", sd2))) return rc;
+  CUDA_TRY(cudaEventRecord(sp->ev_onebody, sd2));
   if (on[T122] && split && (rc = prep_122_df(X, Y, sd2))) return rc;
-  if (beside && w2 && (rc = do_122(X, Y, Z, sd, prec, split, W2_MAKE))) return rc;
+  if ((beside || small) && w2 && (rc = do_122(X, Y, Z, sd2, prec, split, W2_MAKE))) return rc;
   if (!beside) CUDA_TRY(cudaEventRecord(sp->ev_join2, sd2));
   if (on[T222PH] && (rc = zbar_product(sp, Z->herm, prec, sd))) return rc;
   CUDA_TRY(cudaEventRecord(sp->ev_join, sd));
   if (ladder_first && (rc = do_ladder(X, Y, Z, prec, st, true))) return rc;
-  if (!beside) {
-    CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join2, 0));
-    if (w2 && (rc = do_122(X, Y, Z, st, prec, split, W2_MAKE))) return rc;
-  }
-  CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join, 0));
+  // (reads Z2 as the ladder leaves it, adds to Z1)
+  CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_onebody, 0));
   if (on[T221] && ladder_first) {
     ProfScope p221("comm221ss", st);
     CUDA_TRY(launch_comm221_z(*sp->s, Z->d, Z->herm, Z->d, st));
   } else if (on[T221] && (rc = do_221_1b(X, Y, Z, st))) {
     return rc;
   }
+  if (!beside) CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join2, 0));
+  if (!beside && !small && w2 && (rc = do_122(X, Y, Z, st, prec, split, W2_MAKE))) return rc;
+  CUDA_TRY(cudaStreamWaitEvent(st, sp->ev_join, 0));
   if (on[T122] && !fold && (rc = do_122(X, Y, Z, st, prec, split, w2 ? W2_SUBTRACT : W2_MAKE | W2_SUBTRACT))) return rc;
   if (on[T222PH] && (rc = ph_inverse(Z, prec, st, fold))) return rc;
   return IMSRG_OK;

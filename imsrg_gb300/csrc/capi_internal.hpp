@@ -143,7 +143,7 @@ struct imsrg_space {
   // product) and the events that fork it from and join it to the caller's
   // (side2: a third, for what neither waits for)
   cudaStream_t side = nullptr, side2 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_onebody = nullptr;
 
   template <class T>
   T* track(T* p)
@@ -162,6 +162,7 @@ struct imsrg_space {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_join2) cudaEventDestroy(ev_join2);
+    if (ev_onebody) cudaEventDestroy(ev_onebody);
     if (side) cudaStreamDestroy(side);
     if (side2) cudaStreamDestroy(side2);
     if (h_norm_partial) cudaFreeHost(h_norm_partial);

@@ -38,7 +38,7 @@
 // short ones (Zbar, K <= 132) the epilogue.  With the FP64-pipe kernel the
 // commutator takes 142 us at emax 2, 1.26 ms at emax 6, 87.2 ms at emax 10;
 // with this one, and nothing else changed, it took 116 us, 0.38 ms and 7.7 ms
-// (51 us, 0.25 ms and 6.5 ms by now): it is used at every size, and
+// (48 us, 0.24 ms and 6.5 ms by now): it is used at every size, and
 // the FP64-pipe kernel only where the planes do not fit (40 bytes an element
 // pair of the operands) or inside a capture that comes before them.
 #include <cuda.h>

@@ -1195,6 +1195,8 @@ cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, 
       return e;
   }
   if (!t.tpb.empty()) {
+    if (t.tpb_smem > 40 * 1024 && (e = cudaFuncSetAttribute(k_tpandya_b, cudaFuncAttributeMaxDynamicSharedMemorySize, t.tpb_smem)) != cudaSuccess)
+      return e;
     k_tpandya_b<<<(unsigned)t.tpb.size(), kTqThreads, t.tpb_smem, st>>>(s.dev, s.work, t.dev, Y, hY, YbT, YbTF, t.d_tp, t.d_tpb,
                                                                 t.d_ph_loc);
     count_launch();

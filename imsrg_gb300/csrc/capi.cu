@@ -1597,10 +1597,9 @@ void tensor_terms_on(bool on[5])
   on[4] = g_term_on[TS222PH];
 }
 
-// Products of several pairs whose spaces have the same structure (equal
-// orbit lists, hence equal channel tables and product job lists) and whose
-// operators have the same hermiticities, as one split-form launch per
-// product family.  The jobs of pair p address its own operands: every job
+// Products of several pairs whose spaces are groupable (equal orbits and
+// occupations, hence equal channel tables and product job lists) and whose
+// operators have the same hermiticities, as one launch per product family.  The jobs of pair p address its own operands: every job
 // offset is moved by the distance, in doubles, from pair 0's operand to pair
 // p's (all operands are 8-byte aligned device allocations), so the kernels
 // run unchanged on pair 0's base pointers, and the digit splitting (chosen
@@ -1640,6 +1639,16 @@ static long long dist(const void* a, const void* b)
   return ((long long)(intptr_t)a - (long long)(intptr_t)b) / (long long)sizeof(double);
 }
 
+bool groupable(imsrg_space* a, imsrg_space* b)
+{
+  if (a == b) return true;
+  const Space &s = *a->s, &t = *b->s;
+  if (s.emax != t.emax || s.n != t.n || s.l != t.l || s.j2 != t.j2 || s.tz2 != t.tz2 || s.occ != t.occ) return false;
+  for (int k = 0; k < kNTune; ++k)
+    if (*tune_slot(a, k) != *tune_slot(b, k)) return false;
+  return a->inv_set[0] == b->inv_set[0] && a->inv_set[1] == b->inv_set[1];
+}
+
 GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, const std::vector<const imsrg_op*>& Y,
                                          const std::vector<imsrg_op*>& Z, int prec, std::string* why)
 {
@@ -1647,9 +1656,7 @@ GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, 
   imsrg_space* s0 = X[0]->sp;
   for (size_t p = 0; p < X.size(); ++p) {
     imsrg_space* sp = X[p]->sp;
-    if (sp->s->norb != s0->s->norb || sp->s->arena != s0->s->arena || sp->s->emax != s0->s->emax ||
-        sp->ladder_jobs.size() != s0->ladder_jobs.size() || sp->zbar_jobs.size() != s0->zbar_jobs.size() ||
-        X[p]->herm != X[0]->herm || Y[p]->herm != Y[0]->herm || !sp->d_zb || !sp->d_xb) {
+    if (!groupable(sp, s0) || X[p]->herm != X[0]->herm || Y[p]->herm != Y[0]->herm || !sp->d_zb || !sp->d_xb) {
       if (why) *why = "pairs differ in structure or hermiticity";
       return nullptr;
     }

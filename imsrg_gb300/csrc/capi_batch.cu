@@ -5,11 +5,11 @@
 //
 // Two graph shapes:
 //  - grouped (either form, every term on, one model space per pair): pairs of
-//    the same structure form a group, and each group is one chain of
-//    launches in which every kernel of the commutator runs once for all the
-//    group's pairs (the grid's z runs over pairs; the two dense products are
-//    one persistent grid over the tiles of every pair), so the pairs share
-//    the GPU inside each launch instead of taking it in turn;
+//    the same orbits, occupations and tuning form a group, and each group is
+//    one chain of launches in which every kernel of the commutator runs once
+//    for all the group's pairs (the grid's z runs over pairs; the two dense
+//    products are one persistent grid over the tiles of every pair), so the
+//    pairs share the GPU inside each launch instead of taking it in turn;
 //  - branches (otherwise): pairs grouped by model space (a space's scratch
 //    serialises the pairs that share it), one branch per space running whole
 //    commutators.
@@ -87,18 +87,24 @@ int record_grouped(imsrg_batch* b)
   return IMSRG_OK;
 }
 
-// the grouped shape's product groups: pairs of equal structure and hermiticity
+// the grouped shape's product groups: pairs of groupable spaces and equal
+// hermiticities, each with the first group it fits
 int setup_grouped(imsrg_batch* b)
 {
-  std::map<std::vector<long long>, std::vector<int>> keyed;
+  std::vector<std::vector<int>> groups;
   for (size_t i = 0; i < b->X.size(); ++i) {
-    const Space& s = *b->X[i]->sp->s;
-    keyed[{s.emax, s.norb, s.nch, s.arena, b->X[i]->herm, b->Y[i]->herm}].push_back((int)i);
+    size_t g = 0;
+    for (; g < groups.size(); ++g) {
+      const int h = groups[g][0];
+      if (b->X[h]->herm == b->X[i]->herm && b->Y[h]->herm == b->Y[i]->herm && groupable(b->X[h]->sp, b->X[i]->sp)) break;
+    }
+    if (g == groups.size()) groups.emplace_back();
+    groups[g].push_back((int)i);
   }
-  for (auto& kv : keyed) {
+  for (auto& group : groups) {
     std::vector<const imsrg_op*> X, Y;
     std::vector<imsrg_op*> Z;
-    for (int i : kv.second) {
+    for (int i : group) {
       X.push_back(b->X[i]);
       Y.push_back(b->Y[i]);
       Z.push_back(b->Z[i]);

@@ -49,6 +49,11 @@ bool batch_phases_usable();
 // the scalar-tensor term switches: comm111st, comm121st, comm122st,
 // comm222_pp_hh_221st (comm222_pp_hhst and comm221st), comm222_phst
 void tensor_terms_on(bool on[5]);
+// whether a grouped launch may take pairs of both spaces: it runs every pair on
+// the first one's tables (gather lists, weights, phases, descriptors, scratch
+// layout), which follow from orbits and occupations (two references of one
+// emax have arenas, orbits and even job counts alike), and with its tuning
+bool groupable(imsrg_space* a, imsrg_space* b);
 // the ladder and Zbar products of same-structure pairs as one launch each
 // (split plans, or FP64 job lists over every pair)
 struct GroupedProducts;

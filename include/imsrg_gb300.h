@@ -322,8 +322,8 @@ int imsrg_get_term(const char* name, int* on);
  * pairs of different spaces run concurrently, one graph branch per space.
  * With every term on and one model space per pair, every kernel of the
  * commutator (both dense products included) runs as one grouped launch for
- * all pairs whose spaces have the same orbits and whose operators the same
- * hermiticities, in either precision (the FP64 form needs the descriptor
+ * all pairs whose spaces have the same orbits, occupations and tuning and whose
+ * operators the same hermiticities, in either precision (the FP64 form needs the descriptor
  * inverse Pandya kernel, which it takes unless "inverse.fp64" was set to 0).
  * Creating a batch evaluates every pair once (allocating all scratch) and
  * captures the graph; the operators, their spaces and the term switches are

@@ -92,3 +92,52 @@ def test_batch_rejects_repeated_z():
     dX, dY, dZ = ig.DeviceOperator(ms, 1), ig.DeviceOperator(ms, -1), ig.DeviceOperator(ms, 1)
     with pytest.raises(ig.IMSRGError):
         ig.CommutatorBatch([(dX, dY, dZ), (dY, dX, dZ)], "fp64")
+
+
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+@pytest.mark.parametrize("nuclei", [("C12", "O16"), ("O16", "C12"), ("O16", "C12", "O16", "C12")])
+def test_batch_groups_by_reference(nuclei, prec):
+    """References of one emax have the same orbits, arena and job counts, but
+    other occupations, so other gather lists, weights and scratch layouts: each
+    reference is a group of its own."""
+    pairs, refs = [], []
+    for i, nucleus in enumerate(nuclei):
+        ms = ig.ModelSpace(3, nucleus, nucleus)
+        ops = ig.DeviceOperator(ms, 1), ig.DeviceOperator(ms, -1), ig.DeviceOperator(ms, 1)
+        ops[0].fill_random(50 + 2 * i)
+        ops[1].fill_random(51 + 2 * i)
+        ig.Commutator.device_commutator(*ops, prec)
+        refs.append(ops[2].download())
+        ops[2].zero()
+        pairs.append(ops)
+    b = ig.CommutatorBatch(pairs, prec)
+    assert b.info()[2] == 2
+    for _, _, dZ in pairs:
+        dZ.zero()
+    b.launch()
+    b.sync()
+    for (_, _, dZ), ref in zip(pairs, refs):
+        assert max(rel_errors_any(dZ, ref)) < 1e-14
+
+
+def test_batch_groups_by_tuning():
+    """A grouped launch runs on its first pair's tuning and scratch: spaces tuned
+    apart are not grouped (the split form's fused comm122ss has no W2 scratch)."""
+    pairs, refs = [], []
+    for i in range(2):
+        ms = ig.ModelSpace(3, "O16", "O16")
+        ops = ig.DeviceOperator(ms, 1), ig.DeviceOperator(ms, -1), ig.DeviceOperator(ms, 1)
+        ms.set_tuning("comm122.fused", i)  # (the first operator reads the tuning file)
+        ops[0].fill_random(60 + 2 * i)
+        ops[1].fill_random(61 + 2 * i)
+        ig.Commutator.device_commutator(*ops, "split")
+        refs.append(ops[2].download())
+        pairs.append(ops)
+    b = ig.CommutatorBatch(pairs, "split")
+    assert b.info()[2] == 2
+    for _, _, dZ in pairs:
+        dZ.zero()
+    b.launch()
+    b.sync()
+    for (_, _, dZ), ref in zip(pairs, refs):
+        assert max(rel_errors_any(dZ, ref)) < 1e-14

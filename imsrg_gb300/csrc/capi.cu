@@ -1143,6 +1143,75 @@ int imsrg_space_tensor_layout(imsrg_space* sp, int lam, int trank, int parity, i
   return IMSRG_OK;
 }
 
+// a plain product of three tiles and two chunks, Out = A B^T with every sum an
+// integer below 2^53, in both kernels with each wait bounded at limit: the
+// split kernel gives up (its own status word, dropped here), the FP64 kernel
+// evaluates what it has not written; then with the production bound
+static int products_wait_selftest(imsrg_space* sp, unsigned limit, cudaStream_t st)
+{
+  const int m = 260, n = 70, K = 700;
+  std::vector<double> h((size_t)(m + n) * K + (size_t)m * n, 0.0);
+  for (int k = 0; k < K; ++k) {
+    for (int i = 0; i < m; ++i) h[(size_t)k * m + i] = (i + k) % 7 - 3;
+    for (int j = 0; j < n; ++j) h[(size_t)m * K + (size_t)k * n + j] = (j * k) % 5 - 2;
+  }
+  GemmJobDev j{};
+  j.b_off = (long long)m * K;
+  j.out_off = (long long)(m + n) * K;
+  j.m = j.lda = j.ldo = m;
+  j.n = j.ldb = n;
+  j.K = K;
+  j.kidx_off = j.w_off = j.phase_off = -1;
+  j.nosym = 1;
+  j.bscale = 1.0;
+  double* d = nullptr;
+  int* d_status = nullptr;
+  SplitPlan* split = nullptr;
+  DgemmPlan* fp64 = nullptr;
+  std::string bad;
+  try {
+    d = dcopy(h);
+    d_status = dmalloc<int>(1);
+    split = split_plan_create(*sp->s, {j}, 0);
+    fp64 = dgemm_plan_create({j}, 0);
+    const std::vector<double> blank((size_t)m * n, 0.5);
+    std::vector<double> out(blank.size());
+    for (unsigned bound : {0u, limit, wait_limit()})
+      for (bool fp : {false, true}) {
+        auto check = [&](cudaError_t e) {
+          if (e != cudaSuccess) throw std::runtime_error(cudaGetErrorString(e));
+        };
+        int status = 0;
+        check(cudaMemcpyAsync(d + j.out_off, blank.data(), blank.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        check(cudaMemsetAsync(d_status, 0, sizeof(int), st));
+        split_plan_set_wait(split, bound);
+        dgemm_plan_set_wait(fp64, bound);
+        check(fp ? launch_dgemm(fp64, d, d, d, d, nullptr, nullptr, nullptr, 1, 1.0, 0, true, st)
+                 : launch_symgemm_split(split, d, d, d, d, nullptr, nullptr, nullptr, d_status, 1, 1.0, st));
+        check(cudaMemcpyAsync(out.data(), d + j.out_off, out.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        check(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
+        check(cudaStreamSynchronize(st));
+        if (!fp && bound == 0 && status == 0) bad = "a split product reported no expired wait";
+        if (status != 0 && bound == wait_limit()) bad = "a product's wait ran out at the production bound";
+        if (status != 0) continue;
+        for (int c = 0; c < n && bad.empty(); ++c)
+          for (int r = 0; r < m; ++r) {
+            long long v = 0;
+            for (int k = 0; k < K; ++k) v += (long long)((r + k) % 7 - 3) * ((c * k) % 5 - 2);
+            if (out[(size_t)c * m + r] != (double)v) bad = fp ? "FP64 product with expired waits" : "split product";
+          }
+      }
+  } catch (std::exception& e) {
+    bad = e.what();
+  }
+  cudaStreamSynchronize(st);
+  if (split) split_plan_destroy(split);
+  dgemm_plan_destroy(fp64);
+  cudaFree(d);
+  cudaFree(d_status);
+  return bad.empty() ? IMSRG_OK : fail(IMSRG_ERR_CUDA, "wait self-test: " + bad);
+}
+
 int imsrg_space_wait_selftest(imsrg_space* sp, unsigned limit, long long* cycles, unsigned* production_limit,
                               void* stream)
 {
@@ -1156,11 +1225,12 @@ int imsrg_space_wait_selftest(imsrg_space* sp, unsigned limit, long long* cycles
   cudaError_t e = cudaMemsetAsync(d_cyc, 0, sizeof(long long), st);
   if (e == cudaSuccess) e = launch_wait_selftest(sp->d_status, limit, d_cyc, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_cyc, sizeof(long long), cudaMemcpyDeviceToHost, st);
-  int rc = e == cudaSuccess ? check_status(sp, st) : fail(IMSRG_ERR_CUDA, cudaGetErrorString(e));
+  int rc = e == cudaSuccess ? IMSRG_OK : fail(IMSRG_ERR_CUDA, cudaGetErrorString(e));
   cudaStreamSynchronize(st);
   cudaFree(d_cyc);
   if (cycles) *cycles = h;
-  return rc;
+  if (rc || (rc = products_wait_selftest(sp, limit, st))) return rc;
+  return check_status(sp, st);
 }
 
 int imsrg_space_ninej(imsrg_space* sp, int lam, int ja, int jd, int J1, int jb, int jc, int J2, int Jbra, int Jket,

@@ -188,6 +188,9 @@ cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int np
 struct DgemmPlan;
 DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs, int family);
 void dgemm_plan_destroy(DgemmPlan* p);
+// the bound of the kernel's barrier waits (for tests of their expiry: what the
+// CTA has not written by then it evaluates with FP64 FMAs)
+void dgemm_plan_set_wait(DgemmPlan* p, unsigned limit);
 // accum: -1 each job's own flag, 0 overwrite, 1 accumulate; mirror false:
 // symmetrised jobs write only their upper triangle
 cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, const double* B1, double* O, const int* kidx,
@@ -215,6 +218,8 @@ void split_plan_set_accumulate(SplitPlan* p, int mode);
 // 0: symmetrised jobs store only their upper triangle (for a reader of the
 // upper triangle alone, e.g. the descriptor inverse Pandya kernel); 1: both
 void split_plan_set_mirror(SplitPlan* p, int mirror);
+// the bound of the kernel's barrier waits (for tests of their expiry)
+void split_plan_set_wait(SplitPlan* p, unsigned limit);
 // one bounded mbarrier wait of `limit` iterations that runs out (no arrival):
 // status = 105, *cycles = the SM clock cycles it waited (device pointer)
 cudaError_t launch_wait_selftest(int* status, unsigned limit, long long* cycles, cudaStream_t st);

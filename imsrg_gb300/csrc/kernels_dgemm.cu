@@ -123,6 +123,7 @@ struct DgemmPlan {
   int n_rblk = 0, n_dblk = 0;
   CUtensorMap maps[4];  // A rows of A, of B (128-row boxes); B rows of A, of B (32-row boxes)
   size_t smem = 0;
+  unsigned wait = WAIT_LIMIT;
 };
 
 // ----------------------------------------------------------------- device
@@ -395,6 +396,7 @@ struct DArgs {
   const double* kw;
   double gbscale;
   int gsign, accum, nomirror;
+  unsigned wait;  // bound of every barrier wait
 };
 
 // what the roles of a CTA need to know of a tile, gathered one or two tiles
@@ -590,11 +592,11 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   constexpr int EPI_T = 32 * EPIW;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  // barriers: full[NSTAGE], empty[NSTAGE], acc_full[2], early, info_full[NINFO], info_empty[NINFO]; then the tensor-memory slot
+  // barriers: full[NSTAGE], empty[NSTAGE], acc_full[2], early, info_full[NINFO], info_empty[NINFO], drain; then the tensor-memory slot
   unsigned long long* bars = (unsigned long long*)(smem + NSTAGE * STAGE);
-  unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 3 + 2 * NINFO);
+  unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 4 + 2 * NINFO);
   __shared__ TileInfo s_info[NINFO];
-  __shared__ int s_err_, s_epi_err_, s_nlist[2];  // listed tiles, elements
+  __shared__ int s_err_, s_epi_err_, s_issued, s_nlist[2];  // listed tiles, elements
   volatile int& s_err = s_err_;
   volatile int& s_epi_err = s_epi_err_;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -605,6 +607,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   const unsigned acc_early = bar0 + 8u * (2 * NSTAGE + 2);
   auto info_full = [&](int k) { return bar0 + 8u * (2 * NSTAGE + 3 + k); };
   auto info_empty = [&](int k) { return bar0 + 8u * (2 * NSTAGE + 3 + NINFO + k); };
+  const unsigned drain = bar0 + 8u * (2 * NSTAGE + 3 + 2 * NINFO);
   if (threadIdx.x == 0) {
     s_err = 0;
     s_epi_err = 0;
@@ -616,6 +619,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     mbar_init(acc_full(0), 1);
     mbar_init(acc_full(1), 1);
     mbar_init(acc_early, EPI_T);
+    mbar_init(drain, 1);
     for (int k = 0; k < NINFO; ++k) {
       mbar_init(info_full(k), 1);
       mbar_init(info_empty(k), EPI_T + 2);
@@ -637,7 +641,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     // ------------------------------------------------ tile information
     for (int t = 0; t < ntile && !s_err; ++t) {
       const int k = t % NINFO;
-      const bool ok = mbar_wait(info_empty(k), (unsigned)((t / NINFO) & 1) ^ 1u);
+      const bool ok = mbar_wait(info_empty(k), (unsigned)((t / NINFO) & 1) ^ 1u, g.wait);
       if (!__all_sync(0xffffffffu, ok)) {
         s_err = 1;
         break;
@@ -690,7 +694,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     if (lane == 0) {
       int it = 0;
       for (int t = 0; t < ntile && !s_err; ++t) {
-        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) {
+        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1), g.wait)) {
           s_err = 1;
           break;
         }
@@ -700,7 +704,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         mbar_arrive(info_empty(t % NINFO));
         for (int k = 0; k < nhalf * nkb; ++k, ++it) {
           const int st = it % NSTAGE;
-          if (!mbar_wait(empty_bar(st), (unsigned)((it / NSTAGE) & 1) ^ 1u)) {
+          if (!mbar_wait(empty_bar(st), (unsigned)((it / NSTAGE) & 1) ^ 1u, g.wait)) {
             s_err = 1;
             break;
           }
@@ -712,6 +716,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
           tma_load_3d(sA + NP * A_SLICE, second ? &mBA : &mBB, 0, rB + row, full_bar(st));
         }
       }
+      s_issued = it;
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
@@ -719,7 +724,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
       constexpr int MAXT = 256 / TN;
       int it = 0, cc = 0;
       for (int t = 0; t < ntile && !s_err; ++t) {
-        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) {
+        if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1), g.wait)) {
           s_err = 1;
           break;
         }
@@ -730,7 +735,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
           const int c = hc >= nchunk ? hc - nchunk : hc;
           const int len = chunk_begin(nkb, nchunk, c + 1) - chunk_begin(nkb, nchunk, c);
           // the shared blocks of the chunk before have been taken (and so all of the one before that)
-          if (!mbar_wait(acc_early, (unsigned)((cc & 1) ^ 1))) {
+          if (!mbar_wait(acc_early, (unsigned)((cc & 1) ^ 1), g.wait)) {
             s_err = 1;
             break;
           }
@@ -738,7 +743,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
           const unsigned d = tmem + ((cc & 1) ? (NB - NP) * TN : 0);
           for (int kb = 0; kb < len; ++kb, ++it) {
             const int st = it % NSTAGE;
-            if (!mbar_wait(full_bar(st), (unsigned)((it / NSTAGE) & 1))) {
+            if (!mbar_wait(full_bar(st), (unsigned)((it / NSTAGE) & 1), g.wait)) {
               s_err = 1;
               break;
             }
@@ -778,9 +783,12 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     int cc = 0, t = 0;
     for (; t < ntile; ++t) {
       const TileInfo& f = s_info[t % NINFO];
-      if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1))) s_epi_err = 1;
+      if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1), g.wait)) s_epi_err = 1;
       asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
-      if (s_epi_err) break;
+      if (s_epi_err) {
+        s_err = 1;
+        break;
+      }
       const int nosym = f.nosym, nkb = f.nkb, nchunk = f.nchunk, K = f.K;
       const int i = f.I * TM + row, j0 = f.J * TN + cbeg;
       // whether this warp writes any of its 32 x 16 elements: not where they
@@ -798,7 +806,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         for (int c = 0; c < nchunk; ++c, ++cc) {
           const int kb0 = chunk_begin(nkb, nchunk, c), kb1 = chunk_begin(nkb, nchunk, c + 1);
           const float tau = 0.001953125f * __fsqrt_rn((float)(min(K, kb1 * KB) - kb0 * KB));
-          if (!mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1))) s_epi_err = 1;
+          if (!mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1), g.wait)) s_epi_err = 1;
           // the epilogue warps decide together, so none waits at a barrier alone
           asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
           if (s_epi_err) break;
@@ -906,6 +914,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     if (s_nlist[0] | s_nlist[1]) exact_work(g, tbeg, s_nlist[0], s_nlist[1]);
   }
   __syncthreads();
+  if (s_err) drain_products(s_issued, NSTAGE, full_bar, drain);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -1069,7 +1078,7 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     }
     int maxsm = 0;
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    p->smem = 1024 + NSTAGE * STAGE + (2 * NSTAGE + 3 + 2 * NINFO) * 8 + 16;
+    p->smem = 1024 + NSTAGE * STAGE + (2 * NSTAGE + 4 + 2 * NINFO) * 8 + 16;
     if (p->smem + sizeof(TileInfo) * NINFO + 64 > (size_t)maxsm) throw std::runtime_error("not enough shared memory for the FP64 product's pipeline");
     // (the whole shared memory, so that a second stream's kernels find some beside the CTA)
     if (cudaFuncSetAttribute(k_dgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem) != cudaSuccess ||
@@ -1090,6 +1099,8 @@ void dgemm_plan_destroy(DgemmPlan* p)
   if (p->mem) cudaFree(p->mem);
   delete p;
 }
+
+void dgemm_plan_set_wait(DgemmPlan* p, unsigned limit) { p->wait = limit; }
 
 cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, const double* B1, double* O, const int* kidx,
                          const double* kw, const int* phase, int gsign, double gbscale, int accum, bool mirror,
@@ -1115,7 +1126,7 @@ cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, 
   }
   ProfScope ps(p->family == 0 ? "dgemm_ladder" : "dgemm_zbar", st);
   DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA,   rexpB, phase, O,  p->d_list, p->d_elem,
-          A,         B0,         B1,       kidx,    kw,    gbscale, gsign, accum, mirror ? 0 : 1};
+          A,         B0,         B1,       kidx,    kw,    gbscale, gsign, accum, mirror ? 0 : 1, p->wait};
   k_dgemm<<<p->grid, 96 + 32 * EPIW, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], a);
   count_launch();
   return cudaGetLastError();

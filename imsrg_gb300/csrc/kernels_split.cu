@@ -107,6 +107,7 @@ struct SplitPlan {
   size_t smem = 0;
   int nstages = 0;
   int accum_override = -1;
+  unsigned wait = WAIT_LIMIT;  // bound of the kernel's barrier waits
   int mirror = 1;  // 0: symmetrised jobs write only their upper triangle
   int tn = 64, nacc = 1, epiw = 4;  // tile columns, tuning label of the tile (64 x 1 or 32 x 2), epilogue warps
   int stages_opt = 0, sched = 0;    // requested pipeline stages (0: most that fit), tile schedule
@@ -476,6 +477,7 @@ struct GemmArgs {
   int* status;
   int S, beta, P, chunk, nstages, gsign;
   int accum;  // -1: each job's flag; 0: overwrite; 1: accumulate
+  unsigned wait;  // bound of every barrier wait
   int nomirror;  // 1: symmetrised jobs skip the mirror (lower-triangle) stores
 };
 
@@ -564,8 +566,8 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
   const unsigned STAGE = S * (A_SLICE + B_SLICE);
   unsigned long long* bars = (unsigned long long*)(smem + NST * STAGE);
   // bars: full[NST], empty[NST], acc_full[2], done[2], early[1]; then the tmem slot
-  unsigned* tmem_slot = (unsigned*)(bars + 2 * NST + 5);
-  __shared__ int s_err_;
+  unsigned* tmem_slot = (unsigned*)(bars + 2 * NST + 6);
+  __shared__ int s_err_, s_issued;
   __shared__ int s_colexp[2][TN];  // indexed by tile parity: warps run at most one tile apart
   __shared__ int s_colph[2][TN];
   __shared__ int s_epi_err_;
@@ -580,6 +582,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
   auto acc_full = [&](int b) { return bar0 + 8u * (2 * NST + b); };
   auto acc_done = [&](int b) { return bar0 + 8u * (2 * NST + 2 + b); };  // epilogue finished the tile
   const unsigned acc_early = bar0 + 8u * (2 * NST + 4);                  // shared blocks read
+  const unsigned drain = bar0 + 8u * (2 * NST + 5);
 
   if (threadIdx.x == 0) {
     s_err = 0;
@@ -593,6 +596,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
     mbar_init(acc_done(0), EPI_T);
     mbar_init(acc_done(1), EPI_T);
     mbar_init(acc_early, EPI_T);
+    mbar_init(drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -626,7 +630,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
         for (int kb = 0; kb < nkt; ++kb, ++it) {
           int st = it % NST;
           unsigned ph = (unsigned)((it / NST) & 1);
-          if (!mbar_wait(empty_bar(st), ph ^ 1u)) {
+          if (!mbar_wait(empty_bar(st), ph ^ 1u, g.wait)) {
             set_status(g.status, 101);
             s_err = 1;
             break;
@@ -644,6 +648,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           tma_load_3d(sB, mb, k, rowB, full_bar(st));
         }
       }
+      s_issued = it;
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
@@ -662,8 +667,8 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           // and the shared blocks of the previous one have been read (the
           // epilogue works through them in order, so the second implies the
           // first)
-          const bool waited = OV > 0 ? mbar_wait(acc_early, (unsigned)((tc & 1) ^ 1))
-                                     : mbar_wait(acc_done(tc & 1), (unsigned)(((tc >> 1) & 1) ^ 1));
+          const bool waited = OV > 0 ? mbar_wait(acc_early, (unsigned)((tc & 1) ^ 1), g.wait)
+                                     : mbar_wait(acc_done(tc & 1), (unsigned)(((tc >> 1) & 1) ^ 1), g.wait);
           if (!waited) {
             set_status(g.status, 102);
             s_err = 1;
@@ -676,7 +681,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             int st = it % NST;
             unsigned ph = (unsigned)((it / NST) & 1);
-            if (!mbar_wait(full_bar(st), ph)) {
+            if (!mbar_wait(full_bar(st), ph, g.wait)) {
               set_status(g.status, 103);
               s_err = 1;
               ok = false;
@@ -772,7 +777,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
       unsigned lane_base = 0;
       int l0 = 0;
       for (int ch = 0; ch < nch; ++ch, ++tc) {
-        if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1))) {
+        if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1), g.wait)) {
           set_status(g.status, 104);
           s_epi_err = 1;
         }
@@ -877,8 +882,9 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
     }
   }
   // every role has left its loop: all MMAs this CTA issued have been drained
-  // by the epilogue (or the CTA gave up after a bounded wait)
+  // by the epilogue, unless the CTA gave up after a bounded wait
   __syncthreads();
+  if (s_err) drain_products(s_issued, NST, full_bar, drain);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -1223,7 +1229,7 @@ SplitPlan* split_plan_create(const Space& s, const std::vector<GemmJobDev>& jobs
     split_plan_destroy(p);
     throw std::runtime_error("not enough shared memory for the split GEMM pipeline (or fewer than 2 stages asked)");
   }
-  p->smem = 1024 + p->nstages * stage + (2 * p->nstages + 5) * 8 + 16;
+  p->smem = 1024 + p->nstages * stage + (2 * p->nstages + 6) * 8 + 16;
   return p;
 }
 
@@ -1299,6 +1305,7 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
     ga.nstages = p->nstages;
     ga.gsign = gsign;
     ga.accum = p->accum_override;
+    ga.wait = p->wait;
     ga.nomirror = p->mirror ? 0 : 1;
     auto kern = p->chunk       ? (p->tn == 64 ? k_split_gemm<WIDE_S, 64, 8, true, WIDE_BETA> : k_split_gemm<WIDE_S, 32, 8, true, WIDE_BETA>)
                 : p->beta == 7 ? (p->tn == 64 ? k_split_gemm<S, 64, 8, false, 7> : k_split_gemm<S, 32, 8, false, 7>)
@@ -1316,6 +1323,7 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
 
 void split_plan_set_accumulate(SplitPlan* p, int mode) { p->accum_override = mode; }
 void split_plan_set_mirror(SplitPlan* p, int mirror) { p->mirror = mirror ? 1 : 0; }
+void split_plan_set_wait(SplitPlan* p, unsigned limit) { p->wait = limit; }
 
 cudaError_t launch_symgemm_split(SplitPlan* p, const double* A, const double* B0, const double* B1, double* O,
                                  const int* kidx, const double* kw, const int* phase, int* dev_status, int gsign,

@@ -46,7 +46,7 @@ __device__ __forceinline__ bool mbar_try(unsigned a, unsigned parity)
 }
 
 // bounded wait: false on timeout
-__device__ __forceinline__ bool mbar_wait(unsigned a, unsigned parity, unsigned limit = WAIT_LIMIT)
+__device__ __forceinline__ bool mbar_wait(unsigned a, unsigned parity, unsigned limit)
 {
   for (unsigned it = 0; it < limit; ++it) {
     if (mbar_try(a, parity)) return true;
@@ -137,6 +137,24 @@ inline PFN_encodeTiled get_encode()
     fn = (PFN_encodeTiled)p;
   }
   return fn;
+}
+
+// After a wait that ran out, before the CTA frees its tensor memory and exits:
+// waits (again with a limit) for the TMA loads still on their way into its
+// shared memory and for the MMAs it issued.  Called by every thread once all
+// roles have left their loops; issued: loads issued so far, stage k % nstage each;
+// drain: a barrier (count 1) that nothing else uses; the MMAs are those of thread 32.
+template <class Bar>
+__device__ __forceinline__ void drain_products(int issued, int nstage, const Bar& full_bar, unsigned drain)
+{
+  if (threadIdx.x == 0) {
+    for (int k = issued > nstage ? issued - nstage : 0; k < issued; ++k)
+      mbar_wait(full_bar(k % nstage), (unsigned)((k / nstage) & 1), WAIT_LIMIT);
+  } else if (threadIdx.x == 32) {
+    tc_commit(drain);
+    mbar_wait(drain, 0, WAIT_LIMIT);
+  }
+  __syncthreads();
 }
 
 }  // namespace imsrg

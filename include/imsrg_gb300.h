@@ -159,12 +159,16 @@ int imsrg_space_tensor_layout(imsrg_space* s, int lam, int trank, int parity, in
 int imsrg_space_ninej(imsrg_space* s, int lam, int ja, int jd, int J1, int jb, int jc, int J2, int Jbra, int Jket,
                       double* out);
 
-/* Self-test of the failure path of the split products' bounded waits: one
- * kernel waits on an mbarrier that nothing arrives on, through the products'
- * own wait loop bounded at `limit` iterations (1 .. the production bound,
- * returned in *production_limit), sets the space's status word and returns;
- * the call reports it as IMSRG_ERR_KERNEL and clears the word, and *cycles
- * holds the SM clock cycles the wait took.  The context stays usable.  No
+/* Self-test of the failure path of the products' bounded waits: one kernel
+ * waits on an mbarrier that nothing arrives on, through the products' own wait
+ * loop bounded at `limit` iterations (1 .. the production bound, returned in
+ * *production_limit), sets the space's status word and returns; *cycles holds
+ * the SM clock cycles the wait took.  Then both product kernels run a small
+ * product with their waits bounded at 0, `limit` and the production bound: each
+ * returns, the FP64 form with the exact result (what it has not written when a
+ * wait runs out it evaluates with FP64 FMAs), the split form with it or a
+ * status of its own.  The call reports the status word as IMSRG_ERR_KERNEL and
+ * clears it (a wrong product: IMSRG_ERR_CUDA).  The context stays usable.  No
  * counterpart in the reference. */
 int imsrg_space_wait_selftest(imsrg_space* s, unsigned limit, long long* cycles, unsigned* production_limit,
                               void* stream);

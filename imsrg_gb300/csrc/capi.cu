@@ -420,20 +420,31 @@ int ensure_device(imsrg_space* sp)
   return IMSRG_OK;
 }
 
+// zeroes (first word, length) ranges of d before it returns, on a stream of its
+// own: the call that needs them may be under capture, where a node would run
+// at every replay but not now, and where one on the legacy stream is refused if
+// the captured stream is a blocking one
+void zero_now(double* d, const std::vector<std::pair<int64_t, int64_t>>& ranges)
+{
+  cudaStream_t st = nullptr;
+  bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+  for (auto& r : ranges) ok = ok && cudaMemsetAsync(d + r.first, 0, r.second * sizeof(double), st) == cudaSuccess;
+  ok = ok && cudaStreamSynchronize(st) == cudaSuccess;
+  if (st) cudaStreamDestroy(st);
+  if (!ok) throw std::runtime_error("cudaMemset");
+}
+
 // lazily allocated scratch of a space
 int ensure_scratch(imsrg_space* sp, bool pandya, bool w2)
 {
   try {
     Space& s = *sp->s;
     if (pandya && !sp->d_zb) {
-      sp->d_xb = sp->track(dmalloc<double>(s.xb_total));
-      sp->d_yt = sp->track(dmalloc<double>(s.xb_total));
-      sp->d_yf = sp->track(dmalloc<double>(s.xb_total));
-      sp->d_zb = sp->track(dmalloc<double>(s.zb_total));
-      // the blocks of channels without ph kets: zero for good (no product writes them)
-      for (auto& zr : sp->zbar_zero)
-        if (cudaMemset(sp->d_zb + zr.first, 0, zr.second * sizeof(double)) != cudaSuccess) throw std::runtime_error("cudaMemset");
-      if (cudaStreamSynchronize(nullptr) != cudaSuccess) throw std::runtime_error("cudaStreamSynchronize");
+      for (double** p : {&sp->d_xb, &sp->d_yt, &sp->d_yf})
+        if (!*p) *p = sp->track(dmalloc<double>(s.xb_total));
+      double* zb = sp->track(dmalloc<double>(s.zb_total));
+      zero_now(zb, sp->zbar_zero);
+      sp->d_zb = zb;
     }
     if (w2 && !sp->d_w2) sp->d_w2 = sp->track(dmalloc<double>(s.arena));
   } catch (std::exception& e) {

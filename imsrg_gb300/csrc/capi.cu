@@ -84,6 +84,47 @@ bool capturing(cudaStream_t st)
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
+bool release_plans(imsrg_space* sp)
+{
+  cudaGetLastError();  // the failed allocation's
+  if (sp->plans_captured) return false;
+  bool any = false;
+  auto drop = [&](DgemmPlan*& p) {
+    any = any || p;
+    dgemm_plan_destroy(p);
+    p = nullptr;
+  };
+  {
+    std::lock_guard<std::mutex> g(sp->fp64_mu);
+    for (DgemmPlan** p : {&sp->fp64_ladder, &sp->fp64_zbar, &sp->fp64_term}) {
+      if (*p) sp->fp64_tried[p == &sp->fp64_ladder ? 0 : p == &sp->fp64_zbar ? 1 : 2] = false;
+      drop(*p);
+    }
+  }
+  for (auto& kv : sp->s->tensors) {
+    TensorLayout* t = kv.second;
+    if (t->dg_zb2) t->dg_tried = false;
+    for (DgemmPlan** p : {&t->dg_lad1, &t->dg_lad2, &t->dg_zb1, &t->dg_zb2}) drop(*p);
+  }
+  return any;
+}
+void* space_malloc(imsrg_space* sp, size_t bytes)
+{
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, std::max<size_t>(1, bytes));
+  if (e != cudaSuccess) {
+    if (!release_plans(sp) || cudaMalloc(&p, std::max<size_t>(1, bytes)) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  return p;
+}
+bool plan_room(const imsrg_space* sp, size_t bytes)
+{
+  size_t room = 0, all = 0;
+  return cudaMemGetInfo(&room, &all) == cudaSuccess && room >= bytes + 8 * sizeof(double) * (size_t)sp->s->arena;
+}
 int second_stream(imsrg_space* sp)
 {
   for (cudaStream_t* s : {&sp->side, &sp->side2})
@@ -434,6 +475,14 @@ void zero_now(double* d, const std::vector<std::pair<int64_t, int64_t>>& ranges)
   if (!ok) throw std::runtime_error("cudaMemset");
 }
 
+template <class T>
+T* space_alloc(imsrg_space* sp, size_t count)
+{
+  T* p = (T*)space_malloc(sp, count * sizeof(T));
+  if (!p) throw std::runtime_error("cudaMalloc");
+  return sp->track(p);
+}
+
 // lazily allocated scratch of a space
 int ensure_scratch(imsrg_space* sp, bool pandya, bool w2)
 {
@@ -441,12 +490,12 @@ int ensure_scratch(imsrg_space* sp, bool pandya, bool w2)
     Space& s = *sp->s;
     if (pandya && !sp->d_zb) {
       for (double** p : {&sp->d_xb, &sp->d_yt, &sp->d_yf})
-        if (!*p) *p = sp->track(dmalloc<double>(s.xb_total));
-      double* zb = sp->track(dmalloc<double>(s.zb_total));
+        if (!*p) *p = space_alloc<double>(sp, s.xb_total);
+      double* zb = space_alloc<double>(sp, s.zb_total);
       zero_now(zb, sp->zbar_zero);
       sp->d_zb = zb;
     }
-    if (w2 && !sp->d_w2) sp->d_w2 = sp->track(dmalloc<double>(s.arena));
+    if (w2 && !sp->d_w2) sp->d_w2 = space_alloc<double>(sp, s.arena);
   } catch (std::exception& e) {
     return fail(IMSRG_ERR_NOMEM, std::string("scratch allocation failed: ") + e.what());
   }
@@ -618,18 +667,23 @@ int do_onebody(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int todo, cons
   return IMSRG_OK;
 }
 
+int ensure_pairs(imsrg_space* sp)
+{
+  try {
+    if (!sp->d_xf) sp->d_xf = space_alloc<float2>(sp, sp->s->arena);
+    if (!sp->d_yff) sp->d_yff = space_alloc<float2>(sp, sp->s->arena);
+  } catch (std::exception&) {
+    return fail(IMSRG_ERR_NOMEM, "comm122ss double-float scratch");
+  }
+  return IMSRG_OK;
+}
+
 // Split form, first half: the (hi, lo) float-pair copies of X and Y
 int prep_122_df(const imsrg_op* X, const imsrg_op* Y, cudaStream_t st)
 {
   imsrg_space* sp = X->sp;
-  int rc = ensure_scratch(sp, false, true);
-  if (rc) return rc;
-  try {
-    if (!sp->d_xf) sp->d_xf = sp->track(dmalloc<float2>(sp->s->arena));
-    if (!sp->d_yff) sp->d_yff = sp->track(dmalloc<float2>(sp->s->arena));
-  } catch (std::exception&) {
-    return fail(IMSRG_ERR_NOMEM, "comm122ss double-float scratch");
-  }
+  int rc;
+  if ((rc = ensure_scratch(sp, false, true)) || (rc = ensure_pairs(sp))) return rc;
   ProfScope ps("comm122ss prep", st);
   CUDA_TRY(launch_to_ff(*sp->s, X->d, sp->d_xf, st));
   CUDA_TRY(launch_to_ff(*sp->s, Y->d, sp->d_yff, st));
@@ -688,6 +742,7 @@ int ensure_split(imsrg_space* sp)
     if (!sp->split_ladder) sp->split_ladder = split_plan_create(*sp->s, sp->ladder_jobs, 0, sp->opt_ladder);
     if (!sp->split_zbar) sp->split_zbar = split_plan_create(*sp->s, sp->zbar_jobs, 1, sp->opt_zbar);
   } catch (std::exception& e) {
+    if (release_plans(sp)) return ensure_split(sp);
     return fail(IMSRG_ERR_NOMEM, std::string("split-precision plan: ") + e.what());
   }
   return IMSRG_OK;
@@ -695,9 +750,14 @@ int ensure_split(imsrg_space* sp)
 
 // the plan in *slot, made on first use outside a capture; null where it
 // cannot be (no room for its planes, or first used inside a capture)
-DgemmPlan* fp64_plan(DgemmPlan** slot, bool* tried, const std::vector<GemmJobDev>& jobs, int family, cudaStream_t st)
+DgemmPlan* fp64_plan(imsrg_space* sp, DgemmPlan** slot, bool* tried, const std::vector<GemmJobDev>& jobs, int family,
+                     cudaStream_t st)
 {
-  if (!*slot && !*tried && !capturing(st)) {
+  if (capturing(st)) {
+    if (*slot) sp->plans_captured = true;
+    return *slot;
+  }
+  if (!*slot && !*tried && plan_room(sp, dgemm_plan_bytes(jobs))) {
     *tried = true;
     try {
       *slot = dgemm_plan_create(jobs, family);
@@ -714,7 +774,7 @@ int ladder_term_fp64(imsrg_space* sp, const imsrg_op* X, const imsrg_op* Y, imsr
 {
   Space& s = *sp->s;
   std::lock_guard<std::mutex> g(sp->fp64_mu);
-  DgemmPlan* p = capturing(st) ? nullptr : fp64_plan(&sp->fp64_term, &sp->fp64_tried[2], sp->ladder_jobs, 0, st);
+  DgemmPlan* p = capturing(st) ? nullptr : fp64_plan(sp, &sp->fp64_term, &sp->fp64_tried[2], sp->ladder_jobs, 0, st);
   if (p) {
     if (!sp->fp64_ev) CUDA_TRY(cudaEventCreateWithFlags(&sp->fp64_ev, cudaEventDisableTiming));
     CUDA_TRY(cudaStreamWaitEvent(st, sp->fp64_ev, 0));
@@ -745,7 +805,7 @@ int do_ladder(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec, cudaS
   }
   if (prec != IMSRG_PREC_FP64) return fail(IMSRG_ERR_ARG, "unknown precision");
   if (!overwrite) return ladder_term_fp64(sp, X, Y, Z, st);
-  if (DgemmPlan* p = fp64_plan(&sp->fp64_ladder, &sp->fp64_tried[0], sp->ladder_jobs, 0, st)) {
+  if (DgemmPlan* p = fp64_plan(sp, &sp->fp64_ladder, &sp->fp64_tried[0], sp->ladder_jobs, 0, st)) {
     CUDA_TRY(launch_dgemm(p, X->d, Y->d, Y->d, Z->d, s.work.kidx, s.work.kweight, s.work.phase_tab, Z->herm,
                           (double)Y->herm, 0, true, st));
     return IMSRG_OK;
@@ -784,7 +844,7 @@ int zbar_product(imsrg_space* sp, int hZ, int prec, cudaStream_t st)
     return IMSRG_OK;
   }
   if (prec != IMSRG_PREC_FP64) return fail(IMSRG_ERR_ARG, "unknown precision");
-  if (DgemmPlan* p = fp64_plan(&sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
+  if (DgemmPlan* p = fp64_plan(sp, &sp->fp64_zbar, &sp->fp64_tried[1], sp->zbar_jobs, 1, st))
     // the descriptor inverse kernel reads only Zbar's upper triangle
     CUDA_TRY(launch_dgemm(p, sp->d_xb, sp->d_yt, sp->d_yf, sp->d_zb, s.work.kidx, s.work.kweight, s.work.phase_tab, hZ,
                           1.0, 0, inv_variant(sp, prec, st) == 0, st));
@@ -829,6 +889,10 @@ int commutator_impl(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int prec,
   imsrg_space* sp = X->sp;
   if ((rc = second_stream(sp))) return rc;
   cudaStream_t sd = sp->side;
+  // all scratch before anything that only takes room to be faster (inverse
+  // Pandya descriptors, digit planes)
+  if ((rc = ensure_scratch(sp, on[T222PH], on[T122]))) return rc;
+  if (on[T122] && prec == IMSRG_PREC_SPLIT && (rc = ensure_pairs(sp))) return rc;
   ProfScope ps("CommutatorScalarScalar", st);
   const bool ladder_first = on[T222PPHH];
   if (ladder_first)
@@ -1073,9 +1137,8 @@ int imsrg_op_create(imsrg_space* sp, int hermiticity, imsrg_op** out)
   op->sp = sp;
   op->herm = hermiticity;
   op->len = sp->s->arena;
-  if (cudaMalloc(&op->d, sp->s->arena * sizeof(double)) != cudaSuccess) {
+  if (!(op->d = (double*)space_malloc(sp, sp->s->arena * sizeof(double)))) {
     delete op;
-    cudaGetLastError();
     return fail(IMSRG_ERR_NOMEM, "operator arena allocation failed");
   }
   if (cudaMemset(op->d, 0, sp->s->arena * sizeof(double)) != cudaSuccess) {
@@ -1097,21 +1160,23 @@ int imsrg_op_create_tensor(imsrg_space* sp, int lam, int trank, int parity, int 
   int rc = ensure_device(sp);
   if (rc) return rc;
   TensorLayout* tl = nullptr;
-  try {
-    std::lock_guard<std::mutex> g(sp->mu);
-    tl = tensor_layout(*sp->s, lam, trank, parity);
-    tensor_upload(*tl);
-  } catch (std::exception& e) {
-    return fail(IMSRG_ERR_NOMEM, std::string("tensor tables: ") + e.what());
+  for (;;) {
+    try {
+      std::lock_guard<std::mutex> g(sp->mu);
+      tl = tensor_layout(*sp->s, lam, trank, parity);
+      tensor_upload(*tl);
+      break;
+    } catch (std::exception& e) {
+      if (!release_plans(sp)) return fail(IMSRG_ERR_NOMEM, std::string("tensor tables: ") + e.what());
+    }
   }
   imsrg_op* op = new imsrg_op();
   op->sp = sp;
   op->herm = hermiticity;
   op->tl = tl;
   op->len = tl->total;
-  if (cudaMalloc(&op->d, op->len * sizeof(double)) != cudaSuccess) {
+  if (!(op->d = (double*)space_malloc(sp, op->len * sizeof(double)))) {
     delete op;
-    cudaGetLastError();
     return fail(IMSRG_ERR_NOMEM, "operator arena allocation failed");
   }
   if (cudaMemset(op->d, 0, op->len * sizeof(double)) != cudaSuccess) {
@@ -1601,8 +1666,8 @@ int imsrg_bch_transform(const imsrg_op* OpIn, const imsrg_op* Omega, imsrg_op* O
   if ((rc = imsrg_op_copy(OpOut, OpIn, stream))) return rc;
   if (!(nx > threshold)) return IMSRG_OK;
   try {
-    if (!sp->d_nested) sp->d_nested = sp->track(dmalloc<double>(sp->s->arena));
-    if (!sp->d_next) sp->d_next = sp->track(dmalloc<double>(sp->s->arena));
+    if (!sp->d_nested) sp->d_nested = space_alloc<double>(sp, sp->s->arena);
+    if (!sp->d_next) sp->d_next = space_alloc<double>(sp, sp->s->arena);
   } catch (std::exception&) {
     return fail(IMSRG_ERR_NOMEM, "BCH work operators");
   }
@@ -1792,14 +1857,15 @@ GroupedProducts* grouped_products_create(const std::vector<const imsrg_op*>& X, 
       g->zbar = split_plan_create(*s0->s, zj, 1, s0->opt_zbar);
     } else {
       // (offsets from pair 0's arrays)
-      try {
-        g->fp64_ladder = dgemm_plan_create(lj, 0);
-      } catch (std::exception&) {
-      }
-      try {
-        g->fp64_zbar = dgemm_plan_create(zj, 1);
-      } catch (std::exception&) {
-      }
+      auto plan = [&](const std::vector<GemmJobDev>& jobs, int family) -> DgemmPlan* {
+        try {
+          return plan_room(s0, dgemm_plan_bytes(jobs)) ? dgemm_plan_create(jobs, family) : nullptr;
+        } catch (std::exception&) {
+          return nullptr;
+        }
+      };
+      g->fp64_ladder = plan(lj, 0);
+      g->fp64_zbar = plan(zj, 1);
       std::vector<int> lp = tile_pairs(lj, symgemm_fp64_tile()), zp = tile_pairs(zj, symgemm_fp64_tile());
       g->d_lj = dcopy(lj);
       g->d_zj = dcopy(zj);

@@ -46,11 +46,8 @@ cudaStream_t S_(void* st) { return (cudaStream_t)st; }
 int ensure_arena(imsrg_space* sp, double*& p)
 {
   if (p) return IMSRG_OK;
-  void* q = nullptr;
-  if (cudaMalloc(&q, sp->s->arena * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    return err(IMSRG_ERR_NOMEM, "work operator allocation failed");
-  }
+  void* q = space_malloc(sp, sp->s->arena * sizeof(double));
+  if (!q) return err(IMSRG_ERR_NOMEM, "work operator allocation failed");
   p = sp->track((double*)q);
   return IMSRG_OK;
 }
@@ -68,11 +65,8 @@ int generator_impl(const imsrg_op* H, imsrg_op* Eta, const GenParams& p, cudaStr
 {
   imsrg_space* sp = H->sp;
   if (!sp->d_mono) {
-    void* q = nullptr;
-    if (cudaMalloc(&q, (size_t)sp->s->norb * sp->s->norb * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return err(IMSRG_ERR_NOMEM, "generator scratch allocation failed");
-    }
+    void* q = space_malloc(sp, (size_t)sp->s->norb * sp->s->norb * sizeof(double));
+    if (!q) return err(IMSRG_ERR_NOMEM, "generator scratch allocation failed");
     sp->d_mono = sp->track((double*)q);
   }
   ProfScope ps("UpdateEta", st);

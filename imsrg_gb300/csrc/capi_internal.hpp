@@ -26,6 +26,16 @@ namespace imsrg {
 int set_error(int code, const char* msg);
 // whether st is being captured into a graph (nothing may be allocated then)
 bool capturing(cudaStream_t st);
+// cudaMalloc for a space's operators and scratch, null if it does not fit.  Where
+// memory is short the space's FP64 product plans give up their digit planes
+// first: they only make products faster, and are made again once there is room.
+// (Not if a capture has used one: its graph holds on to the planes.)
+void* space_malloc(imsrg_space* sp, size_t bytes);
+// that giving up, after an allocation that failed; whether there was anything
+bool release_plans(imsrg_space* sp);
+// whether an FP64 product plan of that size leaves room for what a program may
+// still allocate: eight operators (those of a flow step with the BCH work ones)
+bool plan_room(const imsrg_space* sp, size_t bytes);
 // makes the space's second and third stream and their events
 int second_stream(imsrg_space* sp);
 // CommutatorScalarScalar into Z (overwritten), Operator::Norm (synchronises
@@ -121,6 +131,7 @@ struct imsrg_space {
   // and fp64_ev orders their uses
   imsrg::DgemmPlan *fp64_ladder = nullptr, *fp64_zbar = nullptr, *fp64_term = nullptr;
   bool fp64_tried[3] = {false, false, false};
+  bool plans_captured = false;  // a captured graph uses one of them, or a tensor layout's
   std::mutex fp64_mu;
   cudaEvent_t fp64_ev = nullptr;
   // BCH work operators (d_prod: BCH_Product result when Z aliases X or Y)

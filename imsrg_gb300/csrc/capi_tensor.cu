@@ -42,14 +42,11 @@ int check_st(const imsrg_op* X, const imsrg_op* Y, const imsrg_op* Z)
   return IMSRG_OK;
 }
 
-int alloc(TensorLayout* tl, double*& p, long long n)
+int alloc(imsrg_space* sp, TensorLayout* tl, double*& p, long long n)
 {
   if (p) return IMSRG_OK;
-  void* q = nullptr;
-  if (cudaMalloc(&q, (size_t)std::max(1LL, n) * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    return terr(IMSRG_ERR_NOMEM, "scalar-tensor scratch allocation failed");
-  }
+  void* q = space_malloc(sp, (size_t)std::max(1LL, n) * sizeof(double));
+  if (!q) return terr(IMSRG_ERR_NOMEM, "scalar-tensor scratch allocation failed");
   tl->dev_allocs.push_back(q);
   p = (double*)q;
   return IMSRG_OK;
@@ -60,10 +57,10 @@ int scratch(imsrg_space* sp, TensorLayout* tl)
 {
   std::lock_guard<std::mutex> g(sp->mu);
   int rc;
-  if ((rc = alloc(tl, tl->d_mpp, tl->total)) || (rc = alloc(tl, tl->d_mhh, tl->total)) ||
-      (rc = alloc(tl, tl->d_xbar, sp->s->xb_total)) || (rc = alloc(tl, tl->d_ybar, tl->yb_total)) ||
-      (rc = alloc(tl, tl->d_zbar, tl->zb_total)) || (rc = alloc(tl, tl->d_xw, sp->s->arena)) ||
-      (rc = alloc(tl, tl->d_wx, sp->s->arena)) || (rc = alloc(tl, tl->d_yt, tl->total)))
+  if ((rc = alloc(sp, tl, tl->d_mpp, tl->total)) || (rc = alloc(sp, tl, tl->d_mhh, tl->total)) ||
+      (rc = alloc(sp, tl, tl->d_xbar, sp->s->xb_total)) || (rc = alloc(sp, tl, tl->d_ybar, tl->yb_total)) ||
+      (rc = alloc(sp, tl, tl->d_zbar, tl->zb_total)) || (rc = alloc(sp, tl, tl->d_xw, sp->s->arena)) ||
+      (rc = alloc(sp, tl, tl->d_wx, sp->s->arena)) || (rc = alloc(sp, tl, tl->d_yt, tl->total)))
     return rc;
   return IMSRG_OK;
 }
@@ -165,8 +162,8 @@ int product_scratch(imsrg_space* sp, TensorLayout* tl)
   int rc = scratch(sp, tl);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(sp->mu);
-  if ((rc = alloc(tl, tl->d_ybt, tl->yb_total)) || (rc = alloc(tl, tl->d_ybtf, tl->yb_total)) ||
-      (rc = alloc(tl, tl->d_xbf, sp->s->xb_total)))
+  if ((rc = alloc(sp, tl, tl->d_ybt, tl->yb_total)) || (rc = alloc(sp, tl, tl->d_ybtf, tl->yb_total)) ||
+      (rc = alloc(sp, tl, tl->d_xbf, sp->s->xb_total)))
     return rc;
   return IMSRG_OK;
 }
@@ -177,15 +174,17 @@ int split_ready(imsrg_space* sp, TensorLayout* tl)
   if (rc) return rc;
   std::lock_guard<std::mutex> g(sp->mu);
   const Space& s = *sp->s;
-  try {
-    if (!tl->sp_lad1) tl->sp_lad1 = split_plan_create(s, ladder_jobs(s, *tl, 1), 0);
-    if (!tl->sp_lad2) tl->sp_lad2 = split_plan_create(s, ladder_jobs(s, *tl, 2), 0);
-    if (!tl->sp_zb1) tl->sp_zb1 = split_plan_create(s, zbar_jobs(s, *tl, 1), 1);
-    if (!tl->sp_zb2) tl->sp_zb2 = split_plan_create(s, zbar_jobs(s, *tl, 2), 1);
-  } catch (std::exception& e) {
-    return terr(IMSRG_ERR_NOMEM, std::string("split-precision plan: ") + e.what());
+  for (;;) {
+    try {
+      if (!tl->sp_lad1) tl->sp_lad1 = split_plan_create(s, ladder_jobs(s, *tl, 1), 0);
+      if (!tl->sp_lad2) tl->sp_lad2 = split_plan_create(s, ladder_jobs(s, *tl, 2), 0);
+      if (!tl->sp_zb1) tl->sp_zb1 = split_plan_create(s, zbar_jobs(s, *tl, 1), 1);
+      if (!tl->sp_zb2) tl->sp_zb2 = split_plan_create(s, zbar_jobs(s, *tl, 2), 1);
+      return IMSRG_OK;
+    } catch (std::exception& e) {
+      if (!release_plans(sp)) return terr(IMSRG_ERR_NOMEM, std::string("split-precision plan: ") + e.what());
+    }
   }
-  return IMSRG_OK;
 }
 
 // the FP64 form's product plans, made on first use outside a capture; false
@@ -194,15 +193,26 @@ int split_ready(imsrg_space* sp, TensorLayout* tl)
 // 1.58 ms with the FP64-pipe kernels
 bool fp64_ready(imsrg_space* sp, TensorLayout* tl, cudaStream_t st)
 {
-  if (!tl->dg_tried && !capturing(st)) {
-    if (product_scratch(sp, tl) != IMSRG_OK) return false;
-    std::lock_guard<std::mutex> g(sp->mu);
+  if (capturing(st)) {
+    if (tl->dg_zb2) sp->plans_captured = true;
+    return tl->dg_zb2 != nullptr;
+  }
+  if (!tl->dg_zb2 && !tl->dg_tried) {
     const Space& s = *sp->s;
+    // all scratch of either route before the planes, which only make it faster
+    if (scratch(sp, tl) != IMSRG_OK) return false;
+    std::vector<GemmJobDev> jobs[4];
+    size_t bytes = sizeof(double) * (2 * (size_t)tl->yb_total + (size_t)s.xb_total);
+    for (int k = 0; k < 4; ++k) {
+      jobs[k] = k < 2 ? ladder_jobs(s, *tl, k + 1) : zbar_jobs(s, *tl, k - 1);
+      bytes += dgemm_plan_bytes(jobs[k]);
+    }
+    if (!plan_room(sp, bytes) || product_scratch(sp, tl) != IMSRG_OK) return false;
+    std::lock_guard<std::mutex> g(sp->mu);
     DgemmPlan* p[4] = {};
     tl->dg_tried = true;
     try {
-      for (int k = 0; k < 4; ++k)
-        p[k] = k < 2 ? dgemm_plan_create(ladder_jobs(s, *tl, k + 1), 0) : dgemm_plan_create(zbar_jobs(s, *tl, k - 1), 1);
+      for (int k = 0; k < 4; ++k) p[k] = dgemm_plan_create(jobs[k], k < 2 ? 0 : 1);
     } catch (std::exception&) {
       for (DgemmPlan* q : p) dgemm_plan_destroy(q);
       return false;
@@ -286,7 +296,7 @@ int bch_scratch(imsrg_space* sp, TensorLayout* tl)
 {
   std::lock_guard<std::mutex> g(sp->mu);
   int rc;
-  if ((rc = alloc(tl, tl->d_bch_nested, tl->total)) || (rc = alloc(tl, tl->d_bch_next, tl->total))) return rc;
+  if ((rc = alloc(sp, tl, tl->d_bch_nested, tl->total)) || (rc = alloc(sp, tl, tl->d_bch_next, tl->total))) return rc;
   return IMSRG_OK;
 }
 

@@ -187,6 +187,8 @@ cudaError_t launch_symgemm_fp64(const GemmJobDev* jobs, const int* pairs, int np
 // order.  family: 0 ladder, 1 Zbar (phase timers)
 struct DgemmPlan;
 DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs, int family);
+// device memory a plan of these jobs takes
+size_t dgemm_plan_bytes(const std::vector<GemmJobDev>& jobs);
 void dgemm_plan_destroy(DgemmPlan* p);
 // the bound of the kernel's barrier waits (for tests of their expiry: what the
 // CTA has not written by then it evaluates with FP64 FMAs)

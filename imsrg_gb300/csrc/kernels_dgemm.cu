@@ -937,6 +937,19 @@ void plane_map(CUtensorMap* m, void* base, long long rows, int box_rows)
 }  // namespace
 
 // ------------------------------------------------------------------ host
+size_t dgemm_plan_bytes(const std::vector<GemmJobDev>& jobs)
+{
+  // (planes, and the exponents and lists of the tiles; the job tables are small)
+  size_t bytes = 1 << 20;
+  for (const GemmJobDev& j : jobs) {
+    const size_t n = j.nosym ? j.n : j.m, m_pad = (std::max<size_t>(j.m, n) + TM - 1) / TM * TM;
+    const size_t nkb = std::max(1, (j.K + KB - 1) / KB);
+    bytes += m_pad * (nkb * KB * 2 * NP * 2 + 2 * sizeof(int));
+    bytes += (m_pad / TM) * ((n + TN - 1) / TN) * (sizeof(DTile) + sizeof(int) + sizeof(DElem) * MAX_LISTED * COLS_W);
+  }
+  return bytes;
+}
+
 DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
 {
   DgemmPlan* p = new DgemmPlan();

@@ -277,11 +277,11 @@ int t222_finish(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, cudaStream_t 
   return IMSRG_OK;
 }
 
-int tph_finish(imsrg_op* Z, int prec, cudaStream_t st)
+int tph_finish(imsrg_op* Z, cudaStream_t st)
 {
   TensorLayout* tl = Z->tl;
   ProfScope ps("comm222_phst", st);
-  T_CUDA(launch_tensor_inverse_pandya(*Z->sp->s, *tl, tl->d_zbar, Z->d, Z->herm, prec == IMSRG_PREC_SPLIT, st));
+  T_CUDA(launch_tensor_inverse_pandya(*Z->sp->s, *tl, tl->d_zbar, Z->d, Z->herm, st));
   return IMSRG_OK;
 }
 
@@ -400,7 +400,7 @@ int imsrg_comm222_phst(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int pr
   const bool split = precision == IMSRG_PREC_SPLIT;
   if (!split && !fp64_ready(X->sp, Y->tl, st)) return tph(X, Y, Z, st);
   if ((split && (rc = split_ready(X->sp, Y->tl))) || (rc = product_operands(X, Y, st)) ||
-      (rc = tph_zbar(X, Y, precision, st)) || (rc = tph_finish(Z, precision, st)))
+      (rc = tph_zbar(X, Y, precision, st)) || (rc = tph_finish(Z, st)))
     return rc;
   return split ? end_status(X->sp, st) : IMSRG_OK;
 }
@@ -445,7 +445,7 @@ int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_o
       (on[4] && (rc = tph_zbar(X, Y, precision, st))))
     return rc;
   T_CUDA(cudaStreamWaitEvent(st, sp->ev_join, 0));
-  if ((on[3] && (rc = t222_finish(X, Y, Z, st))) || (on[4] && (rc = tph_finish(Z, precision, st)))) return rc;
+  if ((on[3] && (rc = t222_finish(X, Y, Z, st))) || (on[4] && (rc = tph_finish(Z, st)))) return rc;
   return split ? end_status(sp, st) : IMSRG_OK;
 }
 

@@ -168,11 +168,8 @@ cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, 
                                          cudaStream_t st);
 cudaError_t launch_tensor_222_221_split(const Space& s, const TensorLayout& t, const double* X, const double* Y,
                                         double* D, double* Mhh, double* Z, int hZ, cudaStream_t st);
-// df: double-float sums (split form), where the float-pair 9j table exists
 cudaError_t launch_tensor_inverse_pandya(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ,
-                                         bool df, cudaStream_t st);
-// (hi, lo) float pairs of a table
-cudaError_t launch_ff_table(const double* src, float2* dst, long long n, cudaStream_t st);
+                                         cudaStream_t st);
 
 // kernels_gemm.cu
 int symgemm_fp64_tile();

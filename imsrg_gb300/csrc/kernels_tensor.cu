@@ -9,7 +9,6 @@
 
 #include <algorithm>
 
-#include "dfloat.cuh"
 #include "kernels.cuh"
 #include "prof.hpp"
 #include "tensor.hpp"
@@ -798,68 +797,37 @@ __device__ __forceinline__ double zbar_val(const DevSpace& S, const DevTensor& T
 //   3. each result whose element the quadruple owns (a stored block, the
 //      upper triangle of a diagonal one; exactly one quadruple owns each)
 //      updates Z.
-// DF: the sums in double-float on the FP32 pipe, each quadruple's values
-// scaled by their largest exponent; else in FP64, bound by its pipe.
-// A warp per quadruple and FP64 sums took 6.43 ms at emax 8, rank (2, 0, +),
-// and 1.00 ms at emax 6, rank (1, 1, +); this takes 2.61 ms (DF: half its issue
-// slots, the rest waiting for Z bar and the 9j rows) and 0.31 ms (FP64).
+// The sums are FP64 in both forms, bound by its pipe.  A warp per quadruple took
+// 1.00 ms at emax 6, rank (1, 1, +), this 0.31; at emax 8, rank (2, 0, +), the
+// split commutator takes 8.70 ms (8.39 with double-float sums on the FP32 pipe,
+// which carry five bits less than the FP64 ones).
 constexpr int kTqThreads = 256;
 
 // floor(x / n) for 0 <= x < 2^16, 1 <= n <= 128 and r = 1.0f / n: (x + 1/2) / n is
 // at least 1 / 256 from an integer, more than the product rounds by (checked over the range)
 __device__ __forceinline__ int small_div(int x, float r) { return __float2int_rz(__fmul_rn((float)x + 0.5f, r)); }
 
-// values v 2^(1023 - e) of each quadruple's largest exponent e, as float pairs in place
-__device__ __forceinline__ void scale_to_ff(double* in, int n, const int* s_e, int QP, float rq)
-{
-  for (int e = threadIdx.x; e < n; e += kTqThreads) {
-    const long long b = __double_as_longlong(in[e]);
-    const int ex = (int)((b >> 52) & 0x7FF), es = ex - s_e[e - small_div(e, rq) * QP] + 1023;
-    const double x = ex == 0x7FF ? in[e] : ex == 0 || es <= 0 ? 0.0 : __longlong_as_double((b & ~(0x7FFll << 52)) | ((long long)es << 52));
-    ((float2*)in)[e] = d2ff(x);
-  }
-}
-
-// z 2^(e - 1023)
-__device__ __forceinline__ double scale_back(double z, int e)
-{
-  e -= 1023;
-  z *= __longlong_as_double((long long)(1023 + e / 2) << 52);
-  return z * __longlong_as_double((long long)(1023 + e - e / 2) << 52);
-}
-
 // sum_{A, B} 9j[(A, B)][t] in[(A, B)][q0 .. q0 + 3]: A = lo + a for a < n, B within lam of A and in
 // [loB, hiB]; value v0 + a w + (B - A + lam), the 9j matrix from base with rows of nslot.
 // SKIP0: a zero of the table takes no part, whatever the value (0 x inf)
-template <bool DF, bool SKIP0>
+template <bool SKIP0>
 __device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, int nslot, int t, const double* in, int v0, int QP,
                                           int q0, int n, int lo, int loB, int hiB, double (&sum)[4])
 {
   const int Lam = T.lam, w = 2 * Lam + 1;
-  float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
   double sd[4] = {0.0, 0.0, 0.0, 0.0};
   for (int a = 0; a < n; ++a) {
     const int A = lo + a;
     const int b0 = max(loB, abs(A - Lam)) - A + Lam, b1 = min(hiB, A + Lam) - A + Lam;
     for (int b = b0; b <= b1; ++b) {
       const int v = a * w + b;
-      if (DF) {
-        const float2 c = __ldg(T.nj_hatf + base + (long long)v * nslot + t);
-        const float4* y = (const float4*)((const float2*)in + (v0 + v) * QP + q0);
-        const float4 y0 = y[0], y1 = y[1];
-        df_fma(c, make_float2(y0.x, y0.y), sh[0], sl[0]);
-        df_fma(c, make_float2(y0.z, y0.w), sh[1], sl[1]);
-        df_fma(c, make_float2(y1.x, y1.y), sh[2], sl[2]);
-        df_fma(c, make_float2(y1.z, y1.w), sh[3], sl[3]);
-      } else {
-        const double c = __ldg(T.nj_hat + base + (long long)v * nslot + t);
-        const double2* y = (const double2*)(in + (v0 + v) * QP + q0);
-        const double2 y0 = y[0], y1 = y[1];
-        sd[0] = fma(c, y0.x, sd[0]);
-        sd[1] = fma(c, y0.y, sd[1]);
-        sd[2] = fma(c, y1.x, sd[2]);
-        sd[3] = fma(c, y1.y, sd[3]);
-      }
+      const double c = __ldg(T.nj_hat + base + (long long)v * nslot + t);
+      const double2* y = (const double2*)(in + (v0 + v) * QP + q0);
+      const double2 y0 = y[0], y1 = y[1];
+      sd[0] = fma(c, y0.x, sd[0]);
+      sd[1] = fma(c, y0.y, sd[1]);
+      sd[2] = fma(c, y1.x, sd[2]);
+      sd[3] = fma(c, y1.y, sd[3]);
     }
   }
   if (SKIP0 && !isfinite((sd[0] + sd[1]) + (sd[2] + sd[3]))) {
@@ -877,20 +845,11 @@ __device__ __forceinline__ void quad_sums(const DevTensor& T, long long base, in
     }
   }
 #pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    if (DF) {
-      const float hi = __fadd_rn(sh[h], sl[h]);
-      sum[h] = ff2d(hi, __fsub_rn(sl[h], __fsub_rn(hi, sh[h])));
-    } else {
-      sum[h] = sd[h];
-    }
-  }
+  for (int h = 0; h < 4; ++h) sum[h] = sd[h];
 }
 
-// (five blocks an SM in FP64: rank (1, 1, +) commutator at emax 6 1264 -> 1211
-// us; in DF the 48 registers that leaves spill: 8.42 -> 8.84 ms at emax 8)
-template <bool DF>
-__global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
+// (five blocks an SM: rank (1, 1, +) commutator at emax 6 1264 -> 1211 us)
+__global__ void __launch_bounds__(kTqThreads, 5) k_tinv_b(DevSpace S, DevTensor T, const double* __restrict__ Zb, int hZ,
                                                        double* __restrict__ Z, const int2* __restrict__ tq,
                                                        const int2* __restrict__ batches)
 {
@@ -898,7 +857,6 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
   double* in = (double*)smem;  // [value of sum 1, then of sum 2][quadruple]
   __shared__ int2 s_q[kTqBatch];
   __shared__ ZbarKets s_z[2][kTqBatch];
-  __shared__ int s_e[kTqBatch];
   const int tid = threadIdx.x;
   const int2 bt = batches[blockIdx.x];
   const int nq = bt.y, QP = (nq + 3) & ~3;
@@ -908,7 +866,6 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
     s_q[tid] = v;
     s_z[0][tid] = zbar_kets(S, i, j, k, l);
     s_z[1][tid] = zbar_kets(S, j, i, k, l);
-    s_e[tid] = 0;
   }
   __syncthreads();
   const int ji = S.j2[s_q[0].x & 0xFFFF], jj = S.j2[s_q[0].x >> 16], jk = S.j2[s_q[0].y & 0xFFFF], jl = S.j2[s_q[0].y >> 16];
@@ -928,16 +885,8 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
     if (q < nq && J4 >= lo4[sum] && J4 <= hi4[sum])
       x = zbar_val(S, T, Zb, hZ, s_z[sum][q], J3, J4, (((sum ? ji : jj) + jl) >> 1) + J4);
     in[e] = x;
-    if (DF) {
-      const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
-      if (ex) atomicMax(&s_e[q], ex);
-    }
   }
   __syncthreads();
-  if (DF) {
-    scale_to_ff(in, nval * QP, s_e, QP, rq);
-    __syncthreads();
-  }
   const int J1min = abs(ji - jj) >> 1, nslot = (((ji + jj) >> 1) - J1min + 1) * w;
   const int d1 = T.d1, ci = (ji - 1) >> 1, cj = (jj - 1) >> 1, ck = (jk - 1) >> 1, cl = (jl - 1) >> 1;
   const long long base[2] = {T.nj_base[((ci * d1 + cj) * d1 + ck) * d1 + cl], T.nj_base[((cj * d1 + ci) * d1 + ck) * d1 + cl]};
@@ -951,7 +900,7 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
     if (J2 < (abs(jk - jl) >> 1) || J2 > ((jk + jl) >> 1) || J1 >= S.NJ || J2 >= S.NJ) continue;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
-      quad_sums<DF, false>(T, base[u], nslot, t, in, u ? n3[0] * w : 0, QP, q0, n3[u], lo3[u], lo4[u], hi4[u], sum[u]);
+      quad_sums<false>(T, base[u], nslot, t, in, u ? n3[0] * w : 0, QP, q0, n3[u], lo3[u], lo4[u], hi4[u], sum[u]);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int q = q0 + h;
@@ -965,7 +914,6 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
       if (blk < 0) continue;
       // both sums carry (-1)^J2
       double z = flip(sum[0][h] + flip(sum[1][h], 1 + ((ji + jj) >> 1) - J1), J2);
-      if (DF) z = scale_back(z, s_e[q]);
       z = unnorm(z, i == j, k == l);
       const int nb = S.ch_n[chb];
       Z[T.off[blk] + (long long)ik * nb + ib] += z;
@@ -984,8 +932,8 @@ __global__ void __launch_bounds__(kTqThreads, DF ? 4 : 5) k_tinv_b(DevSpace S, D
 // and the 9j table's L2 stream.  A thread per element, looking up each element
 // of Y for each of its sums, took 1.23 ms of the commutator at emax 8, rank
 // (2, 0, +); the whole of that 9609 -> 8387 us with this kernel (emax 6, rank
-// (1, 1, +), FP64: 1358 -> 1267).  Float pairs, as k_tinv_b has them in the
-// split form, gain nothing here (8377 us) and are not used.
+// (1, 1, +), FP64: 1358 -> 1267).  Float
+// pairs gain nothing here (8377 us).
 __global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W, DevTensor T, const double* __restrict__ Y,
                                                           int hY, double* __restrict__ Yb, double* __restrict__ YbF,
                                                           const int2* __restrict__ tp, const int2* __restrict__ batches,
@@ -1040,7 +988,7 @@ __global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W,
     const int Jbra = Jbmin + i3, Jket = Jbra - Lam + t - i3 * w;
     if (Jket < (abs(jc - jd) >> 1) || Jket > ((jc + jd) >> 1) || Jbra + Jket < Lam || Jbra >= S.NJ || Jket >= S.NJ) continue;
     double sum[4];
-    quad_sums<false, true>(T, base, nslot, t, in, 0, QP, q0, n1, lo1, lo2, hi2, sum);
+    quad_sums<true>(T, base, nslot, t, in, 0, QP, q0, n1, lo1, lo2, hi2, sum);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int q = q0 + h;
@@ -1071,24 +1019,17 @@ __global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W,
 
 unsigned grid_for(long long n) { return (unsigned)std::max(1LL, (n + 255) / 256); }
 
-cudaError_t launch_tinv(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ, bool df,
+cudaError_t launch_tinv(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ,
                         cudaStream_t st)
 {
   if (t.tqb.empty()) return cudaSuccess;
-  auto kern = df && t.dev.nj_hatf ? k_tinv_b<true> : k_tinv_b<false>;
   if (t.tqb_smem > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, t.tqb_smem);
+    cudaError_t e = cudaFuncSetAttribute(k_tinv_b, cudaFuncAttributeMaxDynamicSharedMemorySize, t.tqb_smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<(unsigned)t.tqb.size(), kTqThreads, t.tqb_smem, st>>>(s.dev, t.dev, Zbar, hZ, Z, t.d_tq, t.d_tqb);
+  k_tinv_b<<<(unsigned)t.tqb.size(), kTqThreads, t.tqb_smem, st>>>(s.dev, t.dev, Zbar, hZ, Z, t.d_tq, t.d_tqb);
   count_launch();
   return cudaGetLastError();
-}
-
-__global__ void k_ff_table(const double* __restrict__ src, float2* __restrict__ dst, long long n)
-{
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = d2ff(src[i]);
 }
 
 }  // namespace
@@ -1180,7 +1121,7 @@ cudaError_t launch_tensor_ph(const Space& s, const TensorLayout& t, const double
   k_tzbar<<<gz, 256, 0, st>>>(s.dev, s.work, t.dev, Xbar, Ybar, hX, hY, Zbar, s.work.phase_tab);
   count_launch();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  return launch_tinv(s, t, Zbar, Z, hZ, false, st);
+  return launch_tinv(s, t, Zbar, Z, hZ, st);
 }
 
 // ---------------------------------------------------------- split form
@@ -1228,17 +1169,9 @@ cudaError_t launch_tensor_222_221_split(const Space& s, const TensorLayout& t, c
 }
 
 cudaError_t launch_tensor_inverse_pandya(const Space& s, const TensorLayout& t, const double* Zbar, double* Z, int hZ,
-                                         bool df, cudaStream_t st)
+                                         cudaStream_t st)
 {
-  return launch_tinv(s, t, Zbar, Z, hZ, df, st);
-}
-
-cudaError_t launch_ff_table(const double* src, float2* dst, long long n, cudaStream_t st)
-{
-  if (n <= 0) return cudaSuccess;
-  k_ff_table<<<(unsigned)std::min<long long>((n + 255) / 256, 65536), 256, 0, st>>>(src, dst, n);
-  count_launch();
-  return cudaGetLastError();
+  return launch_tinv(s, t, Zbar, Z, hZ, st);
 }
 
 // Operator::Norm of a tensor operator: blocks 0 .. n2-1 sum their chunk's

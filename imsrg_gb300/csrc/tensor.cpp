@@ -480,18 +480,6 @@ void tensor_upload(TensorLayout& t)
   t.d_tp = dev_copy(t, t.tp);
   t.d_tpb = dev_copy(t, t.tpb);
   t.d_ph_loc = dev_copy(t, t.ph_loc);
-  // the split form's float pairs of the 9j table; without room for them it reads the FP64 table
-  d.nj_hatf = nullptr;
-  void* f = nullptr;
-  if (!t.nj_hat.empty() && cudaMalloc(&f, t.nj_hat.size() * sizeof(float2)) == cudaSuccess) {
-    t.dev_allocs.push_back(f);
-    if (launch_ff_table(d.nj_hat, (float2*)f, (long long)t.nj_hat.size(), nullptr) != cudaSuccess ||
-        cudaStreamSynchronize(nullptr) != cudaSuccess)
-      throw std::runtime_error("9j float-pair table");
-    d.nj_hatf = (const float2*)f;
-  } else {
-    cudaGetLastError();
-  }
   d.lad_koff = dev_copy(t, t.lad_koff);
   d.lad_woff = dev_copy(t, t.lad_woff);
   d.lad_n = dev_copy(t, t.lad_n);

@@ -57,7 +57,6 @@ struct DevTensor {
   const long long* nj_base = nullptr;
   const double* nj_val = nullptr;
   const double* nj_hat = nullptr;
-  const float2* nj_hatf = nullptr;  // nj_hat as (hi, lo) float pairs (split form; null: none)
   int d1 = 0;
   const double* hat2 = nullptr;  // [J1 * NJ + J2] = sqrt((2J1+1)(2J2+1))
   // per orbit i: the orbits j with <i||T||j> allowed (tob_list[tob_off[i] ..

@@ -258,8 +258,7 @@ int imsrg_comm222_phss(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int pr
  * selects the form of the ladder and Pandya-space (Z bar) products, as for the
  * scalar commutator: IMSRG_PREC_FP64, or IMSRG_PREC_SPLIT (tensor cores; the call
  * then synchronises the stream and checks the kernels' status word, as the
- * scalar entry points do; its inverse Pandya sums are double-float); every
- * other sum is FP64. */
+ * scalar entry points do); every other sum is FP64. */
 int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int precision, void* stream);
 /* its terms, each accumulating into Z (src/TensorCommutators.cc) */
 /* comm111st, src/TensorCommutators.cc:25-30 */

@@ -596,9 +596,8 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   unsigned long long* bars = (unsigned long long*)(smem + NSTAGE * STAGE);
   unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 4 + 2 * NINFO);
   __shared__ TileInfo s_info[NINFO];
-  __shared__ int s_err_, s_epi_err_, s_issued, s_nlist[2];  // listed tiles, elements
+  __shared__ int s_err_, s_issued, s_nlist[2];  // listed tiles, elements
   volatile int& s_err = s_err_;
-  volatile int& s_epi_err = s_epi_err_;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned sbase = smem_u32(smem), bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
@@ -610,7 +609,6 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   const unsigned drain = bar0 + 8u * (2 * NSTAGE + 3 + 2 * NINFO);
   if (threadIdx.x == 0) {
     s_err = 0;
-    s_epi_err = 0;
     s_nlist[0] = s_nlist[1] = 0;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full_bar(s), 1);
@@ -639,9 +637,10 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
 
   if (warp == 2 + EPIW) {
     // ------------------------------------------------ tile information
-    for (int t = 0; t < ntile && !s_err; ++t) {
+    for (int t = 0; t < ntile; ++t) {
       const int k = t % NINFO;
-      const bool ok = mbar_wait(info_empty(k), (unsigned)((t / NINFO) & 1) ^ 1u, g.wait);
+      // (the lanes decide together too)
+      const bool ok = !s_err && mbar_wait(info_empty(k), (unsigned)((t / NINFO) & 1) ^ 1u, g.wait);
       if (!__all_sync(0xffffffffu, ok)) {
         s_err = 1;
         break;
@@ -783,9 +782,9 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     int cc = 0, t = 0;
     for (; t < ntile; ++t) {
       const TileInfo& f = s_info[t % NINFO];
-      if (!mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1), g.wait)) s_epi_err = 1;
-      asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
-      if (s_epi_err) {
+      // the epilogue warps decide together, so none waits at a barrier alone
+      bool expired = barrier_any(1, EPI_T, !mbar_wait(info_full(t % NINFO), (unsigned)((t / NINFO) & 1), g.wait));
+      if (expired) {
         s_err = 1;
         break;
       }
@@ -806,10 +805,8 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         for (int c = 0; c < nchunk; ++c, ++cc) {
           const int kb0 = chunk_begin(nkb, nchunk, c), kb1 = chunk_begin(nkb, nchunk, c + 1);
           const float tau = 0.001953125f * __fsqrt_rn((float)(min(K, kb1 * KB) - kb0 * KB));
-          if (!mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1), g.wait)) s_epi_err = 1;
-          // the epilogue warps decide together, so none waits at a barrier alone
-          asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
-          if (s_epi_err) break;
+          expired = barrier_any(1, EPI_T, !mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1), g.wait));
+          if (expired) break;
           tc_fence_after();
           const unsigned lane_base = tmem + ((unsigned)(q * 32) << 16) + cbeg;
           if (cc & 1) {
@@ -825,7 +822,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
             take_run<0, NP - OV>(lane_base, hi, lo, tau, bad, live);
           }
         }
-        if (s_epi_err) break;
+        if (expired) break;
         if (!live) continue;
         const int raw_i = f.rrow[half][row];
         if (row_bad(raw_i)) bad = (1u << COLS_W) - 1;
@@ -840,7 +837,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
             v1[c] = v;
         }
       }
-      if (s_epi_err) {
+      if (expired) {
         s_err = 1;
         break;
       }

@@ -570,9 +570,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
   __shared__ int s_err_, s_issued;
   __shared__ int s_colexp[2][TN];  // indexed by tile parity: warps run at most one tile apart
   __shared__ int s_colph[2][TN];
-  __shared__ int s_epi_err_;
   volatile int& s_err = s_err_;
-  volatile int& s_epi_err = s_epi_err_;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned sbase = smem_u32(smem);
@@ -586,7 +584,6 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
 
   if (threadIdx.x == 0) {
     s_err = 0;
-    s_epi_err = 0;
     for (int s = 0; s < NST; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -775,16 +772,15 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
 #pragma unroll
       for (int cc = 0; cc < COLS_W; ++cc) P[cc] = 0;
       unsigned lane_base = 0;
+      bool expired = false;
       int l0 = 0;
       for (int ch = 0; ch < nch; ++ch, ++tc) {
-        if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1), g.wait)) {
-          set_status(g.status, 104);
-          s_epi_err = 1;
-        }
+        const bool late = !mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1), g.wait);
+        if (late) set_status(g.status, 104);
         // the epilogue warps decide together (named barrier 1), so a timeout
         // never leaves one of them waiting at a barrier alone
-        asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
-        if (s_epi_err) break;
+        expired = barrier_any(1, EPI_T, late);
+        if (expired) break;
         tc_fence_after();
         lane_base = tmem + ((unsigned)(q * 32) << 16) + Acc::base(tc);
         const int e0 = Acc::early_lo(tc);
@@ -822,7 +818,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
         tc_fence_before();
         mbar_arrive(acc_done(tc & 1));
       }
-      if (s_epi_err) {
+      if (expired) {
         s_err = 1;
         break;
       }

@@ -932,8 +932,8 @@ __global__ void __launch_bounds__(kTqThreads, 5) k_tinv_b(DevSpace S, DevTensor 
 // and the 9j table's L2 stream.  A thread per element, looking up each element
 // of Y for each of its sums, took 1.23 ms of the commutator at emax 8, rank
 // (2, 0, +); the whole of that 9609 -> 8387 us with this kernel (emax 6, rank
-// (1, 1, +), FP64: 1358 -> 1267).  Float
-// pairs gain nothing here (8377 us).
+// (1, 1, +), FP64: 1358 -> 1267).  Float pairs gain
+// nothing here (8377 us).
 __global__ void __launch_bounds__(kTqThreads) k_tpandya_b(DevSpace S, DevWork W, DevTensor T, const double* __restrict__ Y,
                                                           int hY, double* __restrict__ Yb, double* __restrict__ YbF,
                                                           const int2* __restrict__ tp, const int2* __restrict__ batches,

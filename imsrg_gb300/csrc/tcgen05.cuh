@@ -139,6 +139,19 @@ inline PFN_encodeTiled get_encode()
   return fn;
 }
 
+// Named barrier `id` over `n` threads that tells all of them whether any arrived
+// with bad set.  (A shared flag read after a plain barrier can be set by a
+// thread that is past it already: some would leave, others wait for them.)
+__device__ __forceinline__ bool barrier_any(int id, int n, bool bad)
+{
+  unsigned any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n}"
+               : "=r"(any)
+               : "r"(bad ? 1u : 0u), "r"(id), "r"(n)
+               : "memory");
+  return any != 0;
+}
+
 // After a wait that ran out, before the CTA frees its tensor memory and exits:
 // waits (again with a limit) for the TMA loads still on their way into its
 // shared memory and for the MMAs it issued.  Called by every thread once all

@@ -22,15 +22,29 @@
 //    to 2^-53 of each element, so the two differ where a sum is small against
 //    its rows' maxima.  A tenth plane holds |a| and |b| as BF16 magnitudes
 //    (exponents clamped at 2^-60), and one more MMA a step gives sum |a||b| of
-//    every output and chunk.  The digit error is about sqrt(K) 2^-63 (unit:
-//    the rows' exponents) and that of an FP64 sum about 2^-54 sum |a||b|, so
-//    an element with 0 < sum |a||b| < 2^-9 sqrt(K) is not written but listed,
-//    and the CTA evaluates it with FP64 FMAs after its tiles.  A tile with many such
-//    elements is listed whole, and so are tiles with a row that holds an
-//    infinity, a NaN or magnitudes outside 2^-423 .. 2^477, and tiles that a
-//    timed-out wait left undone.  (Random operators list a few elements of
-//    the channels with K < 8; listing whole tiles for those cost 30 us a
-//    product at emax=10.)
+//    every output and chunk.  A product with a zero factor has zero digits and
+//    no error, so the digit error of a sum with n nonzero products is about
+//    sqrt(n) 2^-63 (unit: the rows' exponents), that of an FP64 sum about
+//    2^-54 sum |a||b|.  An element whose sum |a||b| is not zero, but below
+//    2^-9 sqrt(n) in every chunk (n: the smaller of the two rows' counts of
+//    nonzero elements), is not written but listed, and evaluated with FP64
+//    FMAs; so is one of a row that holds an infinity, a NaN or magnitudes
+//    outside 2^-423 .. 2^477, and what a timed-out wait left undone.  (An
+//    estimate of the two errors, not a bound for the worst signs; but then too
+//    a sum above that line stays within the classical bound of an FP64 sum,
+//    (n + 5) 2^-53 sum |a||b| against n 2^-60.)
+//  * Listed elements (exact_work): blocks of 8 x 8 with a mask, shared out over
+//    all CTAs at the end, since one 128 x 32 tile of K = 1000 keeps an SM's FP64
+//    pipe busy for 2 ms.  So the time depends on the operands.  FP64 commutator,
+//    emax 6 / 8 / 10, in ms (on the FP64 pipe alone: 1.25 / 11.1 / 87.2):
+//      random operators, none to a few elements listed    0.24 / 1.21 / 6.5
+//      one a generator, 0.1 to 1% of the FP64 work        0.34 / 1.52 / 7.0
+//      both falling off as e^(-1.0 |de|)                  0.70 / 4.4  / 36
+//      a dominating diagonal                              0.71 / 4.8  / 51
+//      both falling off as 2^(-4 |de|), 70 to 90% of it   1.22 / 9.3  / 80
+//    (With the chunk's length as n and whole tiles of 128 x 32 listed, evaluated
+//    by the CTA that found them: generator 0.95 / 4.7 / 20.8, falling off
+//    1.25 / 11.6 / 97 and 1.62 / 14.6 / 112, diagonal 1.54 / 12.8 / 99.)
 //
 // What bounds it: for the long products the MMAs, 46 of 128 x 32 x 16 a K16
 // step (merged to 11 instructions), next to the TMA stream of the ten planes
@@ -73,6 +87,8 @@ constexpr int SHORT_KB = 4;  // K blocks a job in plans that are sliced in one p
 constexpr int NINFO = 3;     // tiles whose job, exponents and phases wait in shared memory
 constexpr int EPIW = 8;      // epilogue warps: two per TMEM lane quarter, 16 columns each
 constexpr int COLS_W = TN / 2;
+constexpr int BLK = 8;                // rows and columns of a listed block
+constexpr int TILE_BLKS = (TM / BLK) * (TN / BLK);
 constexpr int NB = 512 / TN;         // tensor-memory blocks
 constexpr int OV = 2 * NP - NB;      // blocks that consecutive chunks share (see k_dgemm)
 constexpr unsigned A_SLICE = TM * KB * 2, B_SLICE = TN * KB * 2;
@@ -96,11 +112,10 @@ struct DTile {
   int job, I, J;
 };
 
-// at most MAX_LISTED threads of a tile list their elements (each up to
-// COLS_W); with more the tile is listed
-constexpr int MAX_LISTED = 8;
-struct DElem {
-  int tile, ij;  // row and column within the tile: row | column << 16
+// listed elements of a tile's block: bit 8 r + c of mask is row + r, column + c
+struct DBlock {
+  unsigned long long mask;
+  int tile, at;  // at: row | column << 16 of the block within the tile
 };
 
 __host__ __device__ __forceinline__ int chunk_begin(int nkb, int nchunk, int c) { return (int)((long long)nkb * c / nchunk); }
@@ -116,9 +131,10 @@ struct DgemmPlan {
   DTile* d_tiles = nullptr;
   int* d_cta = nullptr;
   __nv_bfloat16* arr[2] = {nullptr, nullptr};  // planes of A and of B
-  int* d_exp = nullptr;   // [2 exp_rows] raw row exponents of A, of B
-  int* d_list = nullptr;  // tiles to evaluate exactly
-  DElem* d_elem = nullptr;
+  // [2 exp_rows] raw row exponents of A, of B, [2 exp_rows] the rows' counts of
+  // nonzero elements, [2 grid] listed blocks of each CTA: published, taken
+  int* d_exp = nullptr;
+  DBlock* d_list = nullptr;
   int4 *d_rblk = nullptr, *d_dblk = nullptr;
   int n_rblk = 0, n_dblk = 0;
   CUtensorMap maps[4];  // A rows of A, of B (128-row boxes); B rows of A, of B (32-row boxes)
@@ -143,7 +159,11 @@ __device__ __forceinline__ int dexp1(double v)
 // instruction an element otherwise: 250 us instead of 55 for the emax=10
 // ladder's exponents.)
 enum { SC_PLUS = 0, SC_MINUS = 1, SC_OTHER = 2 };
-__device__ __forceinline__ int scale_kind(double sc) { return sc == 1.0 ? SC_PLUS : sc == -1.0 ? SC_MINUS : SC_OTHER; }
+__device__ __forceinline__ int scale_kind(double sc)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(sc);  // (not on the FP64 pipe)
+  return (b & 0x7FFFFFFFFFFFFFFFull) == 0x3FF0000000000000ull ? (b >> 63 ? SC_MINUS : SC_PLUS) : SC_OTHER;
+}
 __device__ __forceinline__ double scaled(double v, int kind, double sc)
 {
   if (kind == SC_OTHER) return v * sc;
@@ -160,9 +180,10 @@ __global__ void __launch_bounds__(256) k_dgemm_rowexp(const DJob* __restrict__ j
                                                       const double* __restrict__ Abase, const double* __restrict__ B0,
                                                       const double* __restrict__ B1, const int* __restrict__ kidx,
                                                       const double* __restrict__ kw, double gbscale,
-                                                      int* __restrict__ rexpA, int* __restrict__ rexpB)
+                                                      int* __restrict__ rexpA, int* __restrict__ rexpB,
+                                                      int* __restrict__ cntA, int* __restrict__ cntB)
 {
-  __shared__ int sa[8][33], sb[8][33];
+  __shared__ int sa[8][33], sb[8][33];  // largest exponent | count of nonzeros << 11
   __shared__ int s_col[256], s_kind[256];
   __shared__ double s_sc[256];
   const int4 bk = blocks[blockIdx.x];
@@ -182,7 +203,12 @@ __global__ void __launch_bounds__(256) k_dgemm_rowexp(const DJob* __restrict__ j
   const double* A = Abase + jb.a_off;
   const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
   const bool oka = i < jb.m, okb = i < jb.n;
-  int ea = 0, eb = 0;
+  int ea = 0, eb = 0, na = 0, nb = 0;
+  auto see = [](double v, int& e, int& n) {
+    const int x = dexp1(v);
+    e = max(e, x);
+    n += x != 0;
+  };
   int t = t0 + ty;
   for (; t + 24 < tend; t += 32) {
     double a[4], b[4];
@@ -194,25 +220,29 @@ __global__ void __launch_bounds__(256) k_dgemm_rowexp(const DJob* __restrict__ j
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      ea = max(ea, dexp1(a[u]));
-      eb = max(eb, dexp1(scaled(b[u], s_kind[t + 8 * u - t0], s_sc[t + 8 * u - t0])));
+      see(a[u], ea, na);
+      see(scaled(b[u], s_kind[t + 8 * u - t0], s_sc[t + 8 * u - t0]), eb, nb);
     }
   }
   for (; t < tend; t += 8) {
     const long long col = s_col[t - t0];
-    if (oka) ea = max(ea, dexp1(A[col * jb.lda + i]));
-    if (okb) eb = max(eb, dexp1(scaled(B[col * jb.ldb + i], s_kind[t - t0], s_sc[t - t0])));
+    if (oka) see(A[col * jb.lda + i], ea, na);
+    if (okb) see(scaled(B[col * jb.ldb + i], s_kind[t - t0], s_sc[t - t0]), eb, nb);
   }
-  sa[ty][r] = ea;
-  sb[ty][r] = eb;
+  sa[ty][r] = ea | na << 11;
+  sb[ty][r] = eb | nb << 11;
   __syncthreads();
   if (ty == 0) {
     for (int y = 1; y < 8; ++y) {
-      ea = max(ea, sa[y][r]);
-      eb = max(eb, sb[y][r]);
+      ea = max(ea, sa[y][r] & 0x7FF);
+      eb = max(eb, sb[y][r] & 0x7FF);
+      na += sa[y][r] >> 11;
+      nb += sb[y][r] >> 11;
     }
     if (ea) atomicMax(rexpA + jb.exp_base + i, ea);
     if (eb) atomicMax(rexpB + jb.exp_base + i, eb);
+    if (na) atomicAdd(cntA + jb.exp_base + i, na);
+    if (nb) atomicAdd(cntB + jb.exp_base + i, nb);
   }
 }
 
@@ -341,14 +371,15 @@ __global__ void __launch_bounds__(256) k_dgemm_digits(const DJob* __restrict__ j
   slice_block(sh, jb, Abase + jb.a_off, (jb.bsel ? B1 : B0) + jb.b_off, r0, bk.z, kidx, kw, gbscale, plane_rows, pA, pB);
 }
 
-// short reductions (at most SHORT_KB K blocks a job): exponents and planes of
-// a 32-row group in one block, one launch where the long form takes a clear
-// and two
+// short reductions (at most SHORT_KB K blocks a job): exponents, counts and
+// planes of a 32-row group in one block, one launch where the long form takes a
+// clear and two (the lists' counters are cleared here too)
 __global__ void __launch_bounds__(256) k_dgemm_slice(const DJob* __restrict__ jobs, const int4* __restrict__ blocks,
                                                      const double* __restrict__ Abase, const double* __restrict__ B0,
                                                      const double* __restrict__ B1, const int* __restrict__ kidx,
                                                      const double* __restrict__ kw, double gbscale, int* __restrict__ rexpA,
-                                                     int* __restrict__ rexpB, long long plane_rows,
+                                                     int* __restrict__ rexpB, int* __restrict__ cntA, int* __restrict__ cntB,
+                                                     int* __restrict__ nlist, int nclear, long long plane_rows,
                                                      __nv_bfloat16* __restrict__ pA, __nv_bfloat16* __restrict__ pB)
 {
   __shared__ SliceShared sh;
@@ -358,22 +389,31 @@ __global__ void __launch_bounds__(256) k_dgemm_slice(const DJob* __restrict__ jo
   const int r0 = bk.y * 32, r = threadIdx.x & 31, ty = threadIdx.x >> 5, i = r0 + r;
   const double* A = Abase + jb.a_off;
   const double* B = (jb.bsel ? B1 : B0) + jb.b_off;
-  int ea = 0, eb = 0;
+  for (int c = blockIdx.x * 256 + threadIdx.x; c < nclear; c += gridDim.x * 256) nlist[c] = 0;
+  int ea = 0, eb = 0, na = 0, nb = 0;
 #pragma unroll 4
   for (int t = ty; t < jb.K; t += 8) {
     const long long col = jb.kidx_off >= 0 ? kidx[jb.kidx_off + t] : t;
     const double sc = jb.bscale * gbscale * (jb.w_off >= 0 ? kw[jb.w_off + t] : 1.0);
-    if (i < jb.m) ea = max(ea, dexp1(A[col * jb.lda + i]));
-    if (i < jb.n) eb = max(eb, dexp1(scaled(B[col * jb.ldb + i], scale_kind(sc), sc)));
+    const int xa = i < jb.m ? dexp1(A[col * jb.lda + i]) : 0;
+    const int xb = i < jb.n ? dexp1(scaled(B[col * jb.ldb + i], scale_kind(sc), sc)) : 0;
+    ea = max(ea, xa);
+    eb = max(eb, xb);
+    na += xa != 0;
+    nb += xb != 0;
   }
-  s_max[0][ty][r] = ea;
-  s_max[1][ty][r] = eb;
+  s_max[0][ty][r] = ea | na << 11;
+  s_max[1][ty][r] = eb | nb << 11;
   __syncthreads();
   if (ty < 2) {
-    int e = 0;
-    for (int y = 0; y < 8; ++y) e = max(e, s_max[ty][y][r]);
+    int e = 0, n = 0;
+    for (int y = 0; y < 8; ++y) {
+      e = max(e, s_max[ty][y][r] & 0x7FF);
+      n += s_max[ty][y][r] >> 11;
+    }
     sh.e[ty][r] = row_e(e);
     (ty ? rexpB : rexpA)[jb.exp_base + i] = e;
+    (ty ? cntB : cntA)[jb.exp_base + i] = n;
   }
   for (int kb = 0; kb < jb.nkb; ++kb)  // (slice_block's first barrier covers sh.e)
     slice_block(sh, jb, A, B, r0, kb, kidx, kw, gbscale, plane_rows, pA, pB);
@@ -383,13 +423,13 @@ struct DArgs {
   const DJob* jobs;
   const DTile* tiles;
   const int* cta_first;
-  const int *rexpA, *rexpB;
+  const int *rexpA, *rexpB, *cntA, *cntB;
   const int* phase;
   double* out;
-  // to evaluate exactly: each CTA lists its own tiles from its first tile's
-  // place, and its elements from MAX_LISTED COLS_W times that
-  int* list;
-  DElem* elem;
+  // to evaluate exactly: each CTA lists from TILE_BLKS times its first tile's
+  // place; published[cta] entries of it are complete, taken[cta] taken
+  DBlock* list;
+  int *published, *taken;
   // for that: the operands as they are
   const double *A, *B0, *B1;
   const int* kidx;
@@ -407,36 +447,59 @@ struct TileInfo {
   double* O;
   int m, n, K, ldo, nosym, nkb, nchunk, m_pad, row_base, accumulate, I, J;
   int rrow[2][TM], rcol[2][TN];  // raw exponents of the tile's rows and columns, in each half
+  float nrow[2][TM], ncol[2][TN];  // their counts of nonzero elements, times 2^-18
   int prow[TM], pcol[TN];        // phases (rows carry the job's sign too)
 };
 
-// adds 16 columns of block g (a weight, or the magnitudes) to the thread's sums
+// what the magnitudes of a half's chunks say of a thread's 16 columns: sum
+// |a||b| is not zero, and at least 2^-9 sqrt(count) in one of them
+struct Guard {
+  unsigned nonzero, enough;
+};
+
+// adds 16 columns of block g (a weight) to the thread's sums, or (g = S) tests
+// the magnitudes, eight columns at a time (registers); n and nc: the row's and
+// the columns' counts times 2^-18
 template <int G>
-__device__ __forceinline__ void take(unsigned taddr, long long (&hi)[COLS_W], long long (&lo)[COLS_W], float tau, unsigned& bad)
+__device__ __forceinline__ void take(unsigned taddr, long long (&hi)[COLS_W], long long (&lo)[COLS_W], Guard& gd, float n,
+                                     const float* nc)
 {
-  unsigned r[2][8];
-  tmem_ld8(taddr, r[0]);
-  tmem_ld8(taddr + 8, r[1]);
-  tmem_wait_ld();
+  if constexpr (G == S) {
 #pragma unroll
-  for (int c = 0; c < COLS_W; ++c) {
-    const float x = __uint_as_float(r[c >> 3][c & 7]);
-    if (G == S)
-      bad |= (x != 0.f && x < tau ? 1u : 0u) << c;
-    else if (G < NHI)
-      hi[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (NHI - 1 - (G < NHI ? G : 0))));
-    else
-      lo[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (S - 1 - (G < S ? G : 0))));
+    for (int h = 0; h < COLS_W; h += 8) {
+      unsigned r[8];
+      tmem_ld8(taddr + h, r);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float x = __uint_as_float(r[c]);
+        gd.nonzero |= (x != 0.f ? 1u : 0u) << (h + c);
+        gd.enough |= (x * x >= fminf(n, nc[h + c]) ? 1u : 0u) << (h + c);
+      }
+    }
+  } else {
+    unsigned r[2][8];
+    tmem_ld8(taddr, r[0]);
+    tmem_ld8(taddr + 8, r[1]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < COLS_W; ++c) {
+      const float x = __uint_as_float(r[c >> 3][c & 7]);
+      if (G < NHI)
+        hi[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (NHI - 1 - (G < NHI ? G : 0))));
+      else
+        lo[c] += (long long)__float2int_rn(x) * (1ll << (BETA * (S - 1 - (G < S ? G : 0))));
+    }
   }
 }
 
 template <int G, int N>
-__device__ __forceinline__ void take_run(unsigned base, long long (&hi)[COLS_W], long long (&lo)[COLS_W], float tau, unsigned& bad,
-                                         bool live)
+__device__ __forceinline__ void take_run(unsigned base, long long (&hi)[COLS_W], long long (&lo)[COLS_W], Guard& gd, float n,
+                                         const float* nc, bool live)
 {
   if constexpr (N > 0) {
-    if (live) take<G>(base + G * TN, hi, lo, tau, bad);
-    take_run<G + 1, N - 1>(base, hi, lo, tau, bad, live);
+    if (live) take<G>(base + G * TN, hi, lo, gd, n, nc);
+    take_run<G + 1, N - 1>(base, hi, lo, gd, n, nc, live);
   }
 }
 
@@ -494,85 +557,254 @@ __device__ __forceinline__ void put_exact(const DJob& jb, double* O, const int* 
   }
 }
 
-// The CTA's listed tiles and elements with FP64 FMAs, by its 256 epilogue
-// threads: tiles with a 4 x 4 block of both products a thread, in the
-// summation order of the FP64 kernel (kernels_gemm.cu); elements by a warp
-// each, lanes over K.  Bound by the FP64 pipe by far, so operands come
-// straight from global memory.  (As a kernel of its own it took 4 us a
-// product with nothing to do.)
-__device__ __noinline__ void exact_work(const DArgs& g, int tbeg, int ntile, int nelem)
+// a thread's columns that the tile's matrix has, on or above the diagonal of a
+// symmetrised job (those below are another element's mirror)
+__device__ __forceinline__ unsigned own_columns(int i, int j0, int m, int n, int nosym)
 {
-  const int tid = threadIdx.x - 64, tx = tid & 7, ty = tid >> 3, lane = tid & 31;
-  const DElem* elem = g.elem + (long long)tbeg * MAX_LISTED * COLS_W;
-  for (int e = 0; e < ntile; ++e) {
-    const DTile tl = g.tiles[g.list[tbeg + e]];
-    const DJob jb = g.jobs[tl.job];
-    const double* A = g.A + jb.a_off;
-    const double* B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
-    const int i0 = tl.I * TM + ty * 4, j0 = tl.J * TN + tx * 4;
-    // rows past the end repeat the last one (and are not written)
-    int ia[4], ib[4], ja[4], jn[4];
+  unsigned b = i >= m || j0 >= n ? 0u : n - j0 < COLS_W ? (1u << (n - j0)) - 1 : (1u << COLS_W) - 1;
+  if (!nosym && i > j0) b &= i - j0 < COLS_W ? ~0u << (i - j0) : 0u;
+  return b;
+}
+
+// lists the bad columns of a warp's 32 rows x 16 columns, by blocks
+__device__ __forceinline__ void list_blocks(DBlock* list, int* n, int tile, int row, int col, unsigned bad)
+{
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      ia[a] = min(i0 + a, jb.m - 1);
-      ib[a] = min(i0 + a, jb.n - 1);
-      ja[a] = min(j0 + a, jb.m - 1);
-      jn[a] = min(j0 + a, jb.n - 1);
+  for (int c = 0; c < COLS_W / BLK; ++c) {
+    const unsigned b = (bad >> (BLK * c)) & 0xFFu;
+    unsigned lo = (lane & 4) ? 0u : b << (8 * (lane & 3)), hi = (lane & 4) ? b << (8 * (lane & 3)) : 0u;
+#pragma unroll
+    for (int o = 1; o < BLK; o <<= 1) {
+      lo |= __shfl_xor_sync(0xffffffffu, lo, o);
+      hi |= __shfl_xor_sync(0xffffffffu, hi, o);
     }
-    double acc1[4][4] = {}, acc2[4][4] = {};
-    for (int t = 0; t < jb.K; ++t) {
-      const long long col = jb.kidx_off >= 0 ? g.kidx[jb.kidx_off + t] : t;
-      const double sc = jb.bscale * g.gbscale * (jb.w_off >= 0 ? g.kw[jb.w_off + t] : 1.0);
-      double x[4], y[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        x[a] = A[col * jb.lda + ia[a]];
-        y[a] = sc * B[col * jb.ldb + jn[a]];
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc1[a][b] = fma(x[a], y[b], acc1[a][b]);
-      if (jb.nosym) continue;
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        x[a] = A[col * jb.lda + ja[a]];
-        y[a] = sc * B[col * jb.ldb + ib[a]];
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc2[a][b] = fma(x[b], y[a], acc2[a][b]);
-    }
-    const int* ph = jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (i0 + a < jb.m && j0 + b < jb.n && (jb.nosym || i0 + a <= j0 + b))
-          put_exact(jb, g.out + jb.out_off, ph, jb.sign != 0 ? jb.sign : g.gsign, i0 + a, j0 + b, acc1[a][b], acc2[a][b],
-                    g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+    if ((lane & 7) == 0 && (lo | hi))
+      list[atomicAdd(n, 1)] = {(unsigned long long)hi << 32 | lo, tile, row | (col + BLK * c) << 16};
   }
-  for (int e = tid >> 5; e < nelem; e += 8) {
-    const DTile tl = g.tiles[elem[e].tile];
-    const DJob jb = g.jobs[tl.job];
-    const double* A = g.A + jb.a_off;
-    const double* B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
-    const int i = tl.I * TM + (elem[e].ij & 0xFFFF), j = tl.J * TN + (elem[e].ij >> 16);
-    double p1 = 0.0, p2 = 0.0;
-    for (int t = lane; t < jb.K; t += 32) {
-      const long long col = jb.kidx_off >= 0 ? g.kidx[jb.kidx_off + t] : t;
-      const double sc = jb.bscale * g.gbscale * (jb.w_off >= 0 ? g.kw[jb.w_off + t] : 1.0);
-      p1 = fma(A[col * jb.lda + i], sc * B[col * jb.ldb + j], p1);
-      if (!jb.nosym) p2 = fma(A[col * jb.lda + j], sc * B[col * jb.ldb + i], p2);
+}
+
+// the entries before n, written before this thread's last barrier, for other CTAs
+__device__ __forceinline__ void publish(int* at, int n)
+{
+  __threadfence();
+  *(volatile int*)at = n;
+}
+
+// the rank-th set bit of a block's mask
+__device__ __forceinline__ int nth_bit(unsigned long long mask, int rank)
+{
+  int bit = 0;
+#pragma unroll
+  for (int w = 32; w > 0; w >>= 1) {
+    const int c = __popcll((mask >> bit) & ((1ull << w) - 1));
+    if (rank >= c) {
+      rank -= c;
+      bit += w;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
-      p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+  }
+  return bit;
+}
+
+__device__ __forceinline__ void put_listed(const DArgs& g, const DJob& jb, int i, int j, double p1, double p2)
+{
+  put_exact(jb, g.out + jb.out_off, jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr, jb.sign != 0 ? jb.sign : g.gsign, i, j,
+            p1, p2, g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+}
+
+// At most FEW elements of a block, by a warp: 32 / n lanes an element take K by
+// turns and meet in a fixed tree; operands straight from L1 and L2, eight
+// columns a lane in flight.
+constexpr int FEW = 16;
+__device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const DBlock& e, int i0, int j0, int n)
+{
+  const int lane = threadIdx.x & 31, nosym = jb.nosym;
+  const double *A = g.A + jb.a_off, *B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
+  const int* kidx = jb.kidx_off >= 0 ? g.kidx + jb.kidx_off : nullptr;
+  const double* kw = jb.w_off >= 0 ? g.kw + jb.w_off : nullptr;
+  const double sc0 = jb.bscale * g.gbscale;
+  const int kind0 = scale_kind(sc0);
+  int sh = 0;  // 2^sh slots for n elements (a slot too many repeats the last one)
+  while ((1 << sh) < n) ++sh;
+  const int slot = lane & ((1 << sh) - 1), part = lane >> sh, parts = 32 >> sh;
+  const int bit = nth_bit(e.mask, min(slot, n - 1)), i = i0 + (bit >> 3), j = j0 + (bit & 7);
+  double p1 = 0.0, p2 = 0.0;
+  constexpr int U = 8;
+  for (int t0 = 0; t0 < jb.K; t0 += 32) {
+    const int t = min(t0 + lane, jb.K - 1), nt = min(32, jb.K - t0);
+    const int col = kidx ? kidx[t] : t;
+    const double sc = kw ? scaled(kw[t], kind0, sc0) : sc0;
+    const int kind = scale_kind(sc);
+    const bool fractions = __any_sync(0xffffffffu, kind == SC_OTHER);
+    for (int u0 = 0; u0 < nt; u0 += U * parts) {
+      double x[U], y[U], x2[U], y2[U];
+#pragma unroll
+      for (int v = 0; v < U; ++v) {
+        const int k = u0 + v * parts + part;
+        const long long c = __shfl_sync(0xffffffffu, col, min(k, nt - 1));
+        const double *a = A + c * jb.lda, *b = B + c * jb.ldb;
+        x[v] = k < nt ? a[i] : 0.0;
+        y[v] = k < nt ? b[j] : 0.0;
+        x2[v] = k < nt && !nosym ? a[j] : 0.0;
+        y2[v] = k < nt && !nosym ? b[i] : 0.0;
+      }
+#pragma unroll
+      for (int v = 0; v < U; ++v) {
+        if (u0 + v * parts >= nt) break;
+        const int k = min(u0 + v * parts + part, nt - 1), kd = __shfl_sync(0xffffffffu, kind, k);
+        if (fractions) {
+          const double s = __shfl_sync(0xffffffffu, sc, k);
+          y[v] = scaled(y[v], kd, s);
+          y2[v] = scaled(y2[v], kd, s);
+        } else {  // (a sign flip: no multiply on the FP64 pipe)
+          y[v] = scaled(y[v], kd & 1, 1.0);
+          y2[v] = scaled(y2[v], kd & 1, 1.0);
+        }
+        p1 = fma(x[v], y[v], p1);
+        if (!nosym) p2 = fma(x2[v], y2[v], p2);
+      }
     }
-    if (lane == 0)
-      put_exact(jb, g.out + jb.out_off, jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr,
-                jb.sign != 0 ? jb.sign : g.gsign, i, j, p1, p2, g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+  }
+  for (int o = 1 << sh; o < 32; o <<= 1) {
+    p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+    p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+  }
+  if (part == 0 && slot < n) put_listed(g, jb, i, j, p1, p2);
+}
+
+// More elements, E a lane.  A column of the operands at the block's eight rows
+// i and eight rows j is one asynchronous copy of 8 bytes a lane into the warp's
+// part of the pipeline's shared memory, two steps of XK columns ahead; B is
+// scaled there, once.  Bound by the FP64 pipe (81% busy at emax 10, operands
+// falling off as 2^(-4 |de|)), one FMA a warp every 16 cycles of an SM.  (Read
+// straight from L1 and L2 like the few: 92 against 90 ms there, 7.1 against 6.6
+// at emax 8 as e^(-1.5 |de|); the few this way: 1.70 against 1.46 ms with a generator.)
+constexpr int XK = 32, XLD = 32;  // columns a step, and the words of one
+constexpr int XSTAGES = 3;
+constexpr int XWARP = XSTAGES * XK * XLD;  // doubles a warp
+static_assert(EPIW * XWARP * 8 <= NSTAGE * (int)STAGE, "exact_work's buffers exceed the pipeline's");
+
+template <int E>
+__device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const DBlock& e, int i0, int j0, int n, double* buf)
+{
+  const int lane = threadIdx.x & 31, nosym = jb.nosym;
+  // what this lane copies: A(i0 + 0..7), B(i0 + ..), A(j0 + ..), B(j0 + ..); rows
+  // past the end repeat the last one (and are not used), a plain job needs no more than the outer two
+  const int strip = lane >> 3, row = min((strip < 2 ? i0 : j0) + (lane & 7), (strip & 1 ? jb.n : jb.m) - 1);
+  const double* src = (strip & 1 ? (jb.bsel ? g.B1 : g.B0) + jb.b_off : g.A + jb.a_off) + row;
+  const int ld = strip & 1 ? jb.ldb : jb.lda;
+  const bool copies = !nosym || strip == 0 || strip == 3;
+  const unsigned dst = smem_u32(buf) + lane * 8;
+  const int* kidx = jb.kidx_off >= 0 ? g.kidx + jb.kidx_off : nullptr;
+  const double* kw = jb.w_off >= 0 ? g.kw + jb.w_off : nullptr;
+  const double sc0 = jb.bscale * g.gbscale;
+  const int kind0 = scale_kind(sc0);
+  int er[E], ec[E];  // row and column within the block (a lane too many repeats the last element)
+  double p1[E], p2[E];
+#pragma unroll
+  for (int h = 0; h < E; ++h) {
+    const int bit = nth_bit(e.mask, min(lane + 32 * h, n - 1));
+    er[h] = bit >> 3;
+    ec[h] = bit & 7;
+    p1[h] = p2[h] = 0.0;
+  }
+  const int steps = (jb.K + XK - 1) / XK;
+  auto column = [&](int step) { return kidx ? kidx[min(step * XK + lane, jb.K - 1)] : step * XK + lane; };
+  int col = column(0);
+  auto copy = [&](int step) {  // always one group, an empty one past the end
+    if (step < steps) {
+      const unsigned d = dst + (step % XSTAGES) * (XK * XLD * 8);
+      const int nk = min(XK, jb.K - step * XK);
+      for (int k = 0; k < nk; ++k) {
+        const double* a = src + (long long)__shfl_sync(0xffffffffu, col, k) * ld;
+        if (copies)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + k * (XLD * 8)), "l"(__cvta_generic_to_global(a))
+                       : "memory");
+      }
+      col = column(step + 1);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  copy(0);
+  copy(1);
+  for (int step = 0; step < steps; ++step) {
+    copy(step + 2);
+    double* x = buf + (step % XSTAGES) * (XK * XLD);
+    const int t0 = step * XK, nk = min(XK, jb.K - t0);
+    const double w = kw ? kw[t0 + min(lane, nk - 1)] : 1.0;
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncwarp();
+    const double sc = scaled(w, kind0, sc0);
+    const int kind = scale_kind(sc);
+    if (__any_sync(0xffffffffu, kind != SC_PLUS)) {
+      for (int k = 0; k < nk; ++k) {
+        const int kd = __shfl_sync(0xffffffffu, kind, k);
+        const double s = __shfl_sync(0xffffffffu, sc, k);
+        if (kd != SC_PLUS && (strip & 1)) x[k * XLD + lane] = scaled(x[k * XLD + lane], kd, s);
+      }
+      __syncwarp();
+    }
+#pragma unroll 4
+    for (int k = 0; k < nk; ++k) {
+      const double* q = x + k * XLD;
+#pragma unroll
+      for (int h = 0; h < E; ++h) {
+        p1[h] = fma(q[er[h]], q[24 + ec[h]], p1[h]);
+        if (!nosym) p2[h] = fma(q[16 + ec[h]], q[8 + er[h]], p2[h]);
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int h = 0; h < E; ++h)
+    if (lane + 32 * h < n) put_listed(g, jb, i0 + er[h], j0 + ec[h], p1[h], p2[h]);
+}
+
+// The listed blocks, a warp at a time: this CTA's own n (all complete), then
+// those that other CTAs have published by now.  Nothing waits: every CTA ends
+// with its own list taken, by itself or by others.
+__device__ __noinline__ void exact_work(const DArgs& g, int n, double* buf)
+{
+  const int lane = threadIdx.x & 31, grid = gridDim.x;
+  auto cta = [&](int d) { return (int)blockIdx.x + d < grid ? blockIdx.x + d : blockIdx.x + d - grid; };
+  auto listed = [&](int d) { return d == 0 ? n : d < grid ? *(volatile int*)(g.published + cta(d)) : 0; };
+  int any = 0;
+  for (int d = lane; d < grid; d += 32) any |= listed(d);
+  if (!__any_sync(0xffffffffu, any)) return;
+  for (int d0 = 0; d0 < grid; d0 += 32) {
+    const int have = listed(d0 + lane);
+    __threadfence();  // the entries after their count
+    for (unsigned m = __ballot_sync(0xffffffffu, have > 0); m; m &= m - 1) {
+      const int c = cta(d0 + __ffs(m) - 1), cn = __shfl_sync(0xffffffffu, have, __ffs(m) - 1);
+      const DBlock* list = g.list + (long long)g.cta_first[c] * TILE_BLKS;
+      for (;;) {
+        int k = 0;
+        if (lane == 0) {
+          k = *(volatile int*)(g.taken + c);
+          while (k < cn) {
+            const int old = atomicCAS(g.taken + c, k, k + 1);
+            if (old == k) break;
+            k = old;
+          }
+        }
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= cn) break;
+        DBlock e;
+        e.mask = __ldcg(&list[k].mask);
+        e.tile = __ldcg(&list[k].tile);
+        e.at = __ldcg(&list[k].at);
+        const DTile tl = g.tiles[e.tile];
+        const DJob jb = g.jobs[tl.job];
+        const int total = __popcll(e.mask);
+        const int i0 = tl.I * TM + (e.at & 0xFFFF), j0 = tl.J * TN + (e.at >> 16);
+        if (total <= FEW)
+          exact_few(g, jb, e, i0, j0, total);
+        else if (total <= 32)
+          exact_many<1>(g, jb, e, i0, j0, total, buf);
+        else
+          exact_many<2>(g, jb, e, i0, j0, total, buf);
+      }
+    }
   }
 }
 
@@ -596,7 +828,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   unsigned long long* bars = (unsigned long long*)(smem + NSTAGE * STAGE);
   unsigned* tmem_slot = (unsigned*)(bars + 2 * NSTAGE + 4 + 2 * NINFO);
   __shared__ TileInfo s_info[NINFO];
-  __shared__ int s_err_, s_issued, s_nlist[2];  // listed tiles, elements
+  __shared__ int s_err_, s_issued, s_nlist, s_published;  // listed blocks, how many of them are published
   volatile int& s_err = s_err_;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned sbase = smem_u32(smem), bar0 = smem_u32(bars);
@@ -609,7 +841,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
   const unsigned drain = bar0 + 8u * (2 * NSTAGE + 3 + 2 * NINFO);
   if (threadIdx.x == 0) {
     s_err = 0;
-    s_nlist[0] = s_nlist[1] = 0;
+    s_nlist = s_published = 0;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -652,23 +884,31 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
       const int sign = jb.sign != 0 ? jb.sign : g.gsign;
       const int* ra = g.rexpA + jb.exp_base;
       const int* rb = g.rexpB + jb.exp_base;
-      int x[2][TM / 32 + 1], p[TM / 32 + 1];
+      const int *na = g.cntA + jb.exp_base, *nb = g.cntB + jb.exp_base;
+      int x[2][TM / 32 + 1], y[2][TM / 32 + 1], p[TM / 32 + 1];
 #pragma unroll
       for (int u = 0; u <= TM / 32; ++u) {
         const int r = u < TM / 32 ? tl.I * TM + u * 32 + lane : tl.J * TN + lane;  // the last: the tile's columns
         const int lim = u < TM / 32 ? jb.m : jb.n;
         x[0][u] = r < lim ? (u < TM / 32 ? ra[r] : rb[r]) : 0;
         x[1][u] = r < lim && !jb.nosym ? (u < TM / 32 ? rb[r] : ra[r]) : 0;
+        y[0][u] = r < lim ? (u < TM / 32 ? na[r] : nb[r]) : 0;
+        y[1][u] = r < lim && !jb.nosym ? (u < TM / 32 ? nb[r] : na[r]) : 0;
         p[u] = ph && r < lim ? ph[r] : 1;
       }
+      constexpr float N2 = 1.0f / (1 << 18);
 #pragma unroll
       for (int u = 0; u < TM / 32; ++u) {
         f.rrow[0][u * 32 + lane] = x[0][u];
         f.rrow[1][u * 32 + lane] = x[1][u];
+        f.nrow[0][u * 32 + lane] = (float)y[0][u] * N2;
+        f.nrow[1][u * 32 + lane] = (float)y[1][u] * N2;
         f.prow[u * 32 + lane] = sign * p[u];
       }
       f.rcol[0][lane] = x[0][TM / 32];
       f.rcol[1][lane] = x[1][TM / 32];
+      f.ncol[0][lane] = (float)y[0][TM / 32] * N2;
+      f.ncol[1][lane] = (float)y[1][TM / 32] * N2;
       f.pcol[lane] = p[TM / 32];
       if (lane == 0) {
         f.O = g.out + jb.out_off;
@@ -788,7 +1028,9 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         s_err = 1;
         break;
       }
-      const int nosym = f.nosym, nkb = f.nkb, nchunk = f.nchunk, K = f.K;
+      // (the listing of the tile before is complete, that of this one not begun)
+      if (threadIdx.x == 64 && s_nlist > s_published) publish(g.published + blockIdx.x, s_published = s_nlist);
+      const int nosym = f.nosym, nchunk = f.nchunk;
       const int i = f.I * TM + row, j0 = f.J * TN + cbeg;
       // whether this warp writes any of its 32 x 16 elements: not where they
       // lie outside the matrix or below the diagonal.  A small job's tile is
@@ -802,30 +1044,29 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         long long hi[COLS_W], lo[COLS_W];
 #pragma unroll
         for (int c = 0; c < COLS_W; ++c) hi[c] = lo[c] = 0;
+        Guard gd{0, 0};
         for (int c = 0; c < nchunk; ++c, ++cc) {
-          const int kb0 = chunk_begin(nkb, nchunk, c), kb1 = chunk_begin(nkb, nchunk, c + 1);
-          const float tau = 0.001953125f * __fsqrt_rn((float)(min(K, kb1 * KB) - kb0 * KB));
           expired = barrier_any(1, EPI_T, !mbar_wait(acc_full(cc & 1), (unsigned)((cc >> 1) & 1), g.wait));
           if (expired) break;
           tc_fence_after();
           const unsigned lane_base = tmem + ((unsigned)(q * 32) << 16) + cbeg;
           if (cc & 1) {
             const unsigned base = lane_base + (NB - NP) * TN;
-            take_run<0, OV>(base, hi, lo, tau, bad, live);
+            take_run<0, OV>(base, hi, lo, gd, f.nrow[half][row], f.ncol[half] + cbeg, live);
             tc_fence_before();
             mbar_arrive(acc_early);
-            take_run<OV, NP - OV>(base, hi, lo, tau, bad, live);
+            take_run<OV, NP - OV>(base, hi, lo, gd, f.nrow[half][row], f.ncol[half] + cbeg, live);
           } else {
-            take_run<NP - OV, OV>(lane_base, hi, lo, tau, bad, live);
+            take_run<NP - OV, OV>(lane_base, hi, lo, gd, f.nrow[half][row], f.ncol[half] + cbeg, live);
             tc_fence_before();
             mbar_arrive(acc_early);
-            take_run<0, NP - OV>(lane_base, hi, lo, tau, bad, live);
+            take_run<0, NP - OV>(lane_base, hi, lo, gd, f.nrow[half][row], f.ncol[half] + cbeg, live);
           }
         }
         if (expired) break;
         if (!live) continue;
         const int raw_i = f.rrow[half][row];
-        if (row_bad(raw_i)) bad = (1u << COLS_W) - 1;
+        bad |= row_bad(raw_i) ? (1u << COLS_W) - 1 : gd.nonzero & ~gd.enough;
 #pragma unroll
         for (int c = 0; c < COLS_W; ++c) {
           const int raw_j = f.rcol[half][cbeg + c];
@@ -842,24 +1083,13 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         break;
       }
       const int m = f.m, n = f.n, ldo = f.ldo;
-      const bool accumulate = f.accumulate, rowok = i < m;
+      const bool accumulate = f.accumulate;
       double* O = f.O;
-      if (!rowok || (!nosym && i > j0 + COLS_W - 1)) bad = 0;
-      if (!nosym && i > j0) bad &= ~0u << min(i - j0, 31);  // columns below the diagonal are another element's mirror
-      bad &= j0 >= n ? 0u : n - j0 < COLS_W ? (1u << (n - j0)) - 1 : ~0u;
-      // the epilogue threads decide together whether the tile is listed
-      unsigned nbad;
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.popc.u32 %0, 2, %2, p;\n}"
-                   : "=r"(nbad)
-                   : "r"(bad), "r"(EPI_T)
-                   : "memory");
-      if (nbad > MAX_LISTED) {
-        if (threadIdx.x == 64) g.list[tbeg + atomicAdd(&s_nlist[0], 1)] = tbeg + t;
-        mbar_arrive(info_empty(t % NINFO));
-        continue;
-      }
-      for (unsigned b = bad; b; b &= b - 1)
-        g.elem[(long long)tbeg * MAX_LISTED * COLS_W + atomicAdd(&s_nlist[1], 1)] = {tbeg + t, row | ((cbeg + __ffs(b) - 1) << 16)};
+      // columns this thread writes: in the matrix, on or above the diagonal, not listed
+      unsigned wd = own_columns(i, j0, m, n, nosym);
+      bad &= wd;
+      wd &= ~bad;
+      if (__any_sync(0xffffffffu, bad)) list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, tbeg + t, row & ~7, cbeg, bad);
       if (!nosym && live) {
         const int sp = f.prow[row];
 #pragma unroll
@@ -870,10 +1100,6 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         }
       }
       mbar_arrive(info_empty(t % NINFO));
-      // columns this thread writes: in the matrix, on or above the diagonal, not listed
-      unsigned wd = !rowok || j0 >= n ? 0u : n - j0 < COLS_W ? (1u << (n - j0)) - 1 : (1u << COLS_W) - 1;
-      if (!nosym && i > j0) wd &= i - j0 < COLS_W ? ~0u << (i - j0) : 0u;
-      wd &= ~bad;
       unsigned wm = nosym || g.nomirror ? 0u : wd;
       if (i >= j0 && i < j0 + COLS_W) wm &= ~(1u << (i - j0));
       double* od = O + (long long)j0 * ldo + i;
@@ -903,18 +1129,23 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
       }
     }
     // a wait that ran out: the tiles not written are listed
-    if (threadIdx.x == 64)
-      for (; t < ntile; ++t) g.list[tbeg + atomicAdd(&s_nlist[0], 1)] = tbeg + t;
-    // the lists are this CTA's own: written by these threads, read by them
-    __threadfence_block();
-    asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
-    if (s_nlist[0] | s_nlist[1]) exact_work(g, tbeg, s_nlist[0], s_nlist[1]);
+    for (; t < ntile; ++t) {
+      const DTile tl = g.tiles[tbeg + t];
+      const DJob& jb = g.jobs[tl.job];
+      list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, tbeg + t, row & ~7, cbeg, own_columns(tl.I * TM + row, tl.J * TN + cbeg, jb.m, jb.n, jb.nosym));
+    }
   }
+  // every role has left its loop, and so has every copy and MMA, unless a wait
+  // ran out; the lists are complete
   __syncthreads();
   if (s_err) drain_products(s_issued, NSTAGE, full_bar, drain);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  } else if (warp >= 2 && warp < 2 + EPIW) {
+    const int n = s_nlist;
+    if (threadIdx.x == 64 && n > s_published) publish(g.published + blockIdx.x, n);
+    exact_work(g, n, (double*)smem + (warp - 2) * XWARP);  // (the pipeline's shared memory is free)
   }
 }
 
@@ -941,8 +1172,8 @@ size_t dgemm_plan_bytes(const std::vector<GemmJobDev>& jobs)
   for (const GemmJobDev& j : jobs) {
     const size_t n = j.nosym ? j.n : j.m, m_pad = (std::max<size_t>(j.m, n) + TM - 1) / TM * TM;
     const size_t nkb = std::max(1, (j.K + KB - 1) / KB);
-    bytes += m_pad * (nkb * KB * 2 * NP * 2 + 2 * sizeof(int));
-    bytes += (m_pad / TM) * ((n + TN - 1) / TN) * (sizeof(DTile) + sizeof(int) + sizeof(DElem) * MAX_LISTED * COLS_W);
+    bytes += m_pad * (nkb * KB * 2 * NP * 2 + 4 * sizeof(int));
+    bytes += (m_pad / TM) * ((n + TN - 1) / TN) * (sizeof(DTile) + sizeof(DBlock) * TILE_BLKS);
   }
   return bytes;
 }
@@ -1063,8 +1294,8 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     std::memcpy(tables.data() + o_cta, first.data(), sizeof(int) * first.size());
     if (!rb.empty()) std::memcpy(tables.data() + o_rblk, rb.data(), sizeof(int4) * rb.size());
     if (!db.empty()) std::memcpy(tables.data() + o_dblk, db.data(), sizeof(int4) * db.size());
-    const size_t o_exp = take(sizeof(int) * 2 * p->exp_rows), o_list = take(sizeof(int) * p->ntiles);
-    const size_t o_elem = take(sizeof(DElem) * MAX_LISTED * COLS_W * (size_t)p->ntiles);
+    const size_t o_exp = take(sizeof(int) * (4 * p->exp_rows + 2 * p->grid));
+    const size_t o_list = take(sizeof(DBlock) * TILE_BLKS * (size_t)p->ntiles);
     const size_t o_arr[2] = {take((size_t)NP * p->rows * KB * 2), take((size_t)NP * p->rows * KB * 2)};
     if (cudaMalloc(&p->mem, size) != cudaSuccess) {
       p->mem = nullptr;
@@ -1079,8 +1310,7 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     p->d_rblk = (int4*)(base + o_rblk);
     p->d_dblk = (int4*)(base + o_dblk);
     p->d_exp = (int*)(base + o_exp);
-    p->d_list = (int*)(base + o_list);
-    p->d_elem = (DElem*)(base + o_elem);
+    p->d_list = (DBlock*)(base + o_list);
     for (int a = 0; a < 2; ++a) p->arr[a] = (__nv_bfloat16*)(base + o_arr[a]);
     for (int a = 0; a < 2; ++a) {
       plane_map(&p->maps[a], p->arr[a], p->rows, TM);
@@ -1117,17 +1347,18 @@ cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, 
                          cudaStream_t st)
 {
   if (p->ntiles == 0) return cudaSuccess;
-  int *rexpA = p->d_exp, *rexpB = p->d_exp + p->exp_rows;
+  int *rexpA = p->d_exp, *rexpB = p->d_exp + p->exp_rows, *cntA = p->d_exp + 2 * p->exp_rows, *cntB = cntA + p->exp_rows;
+  int* nlist = cntB + p->exp_rows;
   cudaError_t e;
   {
     ProfScope ps(p->family == 0 ? "dgemm_slice_ladder" : "dgemm_slice_zbar", st);
     if (p->n_dblk == 0) {
-      k_dgemm_slice<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
-                                               p->arr[0], p->arr[1]);
+      k_dgemm_slice<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, cntA, cntB,
+                                               nlist, 2 * p->grid, p->rows, p->arr[0], p->arr[1]);
       count_launch();
     } else {
-      if ((e = cudaMemsetAsync(p->d_exp, 0, sizeof(int) * 2 * p->exp_rows, st)) != cudaSuccess) return e;
-      k_dgemm_rowexp<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB);
+      if ((e = cudaMemsetAsync(p->d_exp, 0, sizeof(int) * (4 * p->exp_rows + 2 * p->grid), st)) != cudaSuccess) return e;
+      k_dgemm_rowexp<<<p->n_rblk, 256, 0, st>>>(p->d_jobs, p->d_rblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, cntA, cntB);
       k_dgemm_digits<<<p->n_dblk, 256, 0, st>>>(p->d_jobs, p->d_dblk, A, B0, B1, kidx, kw, gbscale, rexpA, rexpB, p->rows,
                                                 p->arr[0], p->arr[1]);
       count_launch(2);
@@ -1135,8 +1366,8 @@ cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, 
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   ProfScope ps(p->family == 0 ? "dgemm_ladder" : "dgemm_zbar", st);
-  DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA,   rexpB, phase, O,  p->d_list, p->d_elem,
-          A,         B0,         B1,       kidx,    kw,    gbscale, gsign, accum, mirror ? 0 : 1, p->wait};
+  DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA, rexpB, cntA, cntB, phase, O, p->d_list, nlist, nlist + p->grid,
+          A, B0, B1, kidx, kw, gbscale, gsign, accum, mirror ? 0 : 1, p->wait};
   k_dgemm<<<p->grid, 96 + 32 * EPIW, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], a);
   count_launch();
   return cudaGetLastError();

@@ -567,10 +567,15 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
   unsigned long long* bars = (unsigned long long*)(smem + NST * STAGE);
   // bars: full[NST], empty[NST], acc_full[2], done[2], early[1]; then the tmem slot
   unsigned* tmem_slot = (unsigned*)(bars + 2 * NST + 6);
-  __shared__ int s_err_, s_issued;
+  // s_late: a wait ran out before the epilogue's barrier of an even, odd chunk
+  // (with one flag a thread past the barrier could set it at the next one before
+  // a slow thread has read it, and some would leave while others wait for them;
+  // a barrier that reduces the outcomes costs the emax 12 flow step 1%)
+  __shared__ int s_err_, s_issued, s_late_[2];
   __shared__ int s_colexp[2][TN];  // indexed by tile parity: warps run at most one tile apart
   __shared__ int s_colph[2][TN];
   volatile int& s_err = s_err_;
+  volatile int* s_late = s_late_;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned sbase = smem_u32(smem);
@@ -583,7 +588,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
   const unsigned drain = bar0 + 8u * (2 * NST + 5);
 
   if (threadIdx.x == 0) {
-    s_err = 0;
+    s_err = s_late[0] = s_late[1] = 0;
     for (int s = 0; s < NST; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -772,15 +777,16 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
 #pragma unroll
       for (int cc = 0; cc < COLS_W; ++cc) P[cc] = 0;
       unsigned lane_base = 0;
-      bool expired = false;
       int l0 = 0;
       for (int ch = 0; ch < nch; ++ch, ++tc) {
-        const bool late = !mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1), g.wait);
-        if (late) set_status(g.status, 104);
+        if (!mbar_wait(acc_full(tc & 1), (unsigned)((tc >> 1) & 1), g.wait)) {
+          set_status(g.status, 104);
+          s_late[tc & 1] = 1;
+        }
         // the epilogue warps decide together (named barrier 1), so a timeout
         // never leaves one of them waiting at a barrier alone
-        expired = barrier_any(1, EPI_T, late);
-        if (expired) break;
+        asm volatile("bar.sync 1, %0;" ::"r"(EPI_T) : "memory");
+        if (s_late[tc & 1]) break;
         tc_fence_after();
         lane_base = tmem + ((unsigned)(q * 32) << 16) + Acc::base(tc);
         const int e0 = Acc::early_lo(tc);
@@ -818,7 +824,7 @@ __global__ void __maxnreg__(128) k_split_gemm(const __grid_constant__ CUtensorMa
         tc_fence_before();
         mbar_arrive(acc_done(tc & 1));
       }
-      if (expired) {
+      if (s_late[tc & 1]) {
         s_err = 1;
         break;
       }

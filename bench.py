@@ -459,8 +459,27 @@ def profiled_phases(L, step, nsteps):
     return phases
 
 
-def roofline(phases, work, emax):
+def issued_products(ms, product):
+    """BF16 digit products per multiply-add of the split form's "ladder" or
+    "zbar" product: S (S + 1) / 2 of S digits, the tuned count, or the rule's:
+    five where the longest reduction (the gathered kets of a channel; the ph
+    kets of a cross-coupled one, taken twice) passes 339, else six."""
+    occ = [o[4] for o in ms.orbits]
+    digits = ms.tuning()[product + ".digits"]
+    if not digits:
+        if product == "ladder":
+            # kets with a weight: (1 - n_p)(1 - n_q) - n_p n_q
+            longest = max(sum((1 - occ[p]) * (1 - occ[q]) != occ[p] * occ[q] for p, q in c["kets"]) for c in ms.channels)
+        else:
+            # hh and ph kets
+            longest = max(2 * sum(occ[p] > 1e-6 or occ[q] > 1e-6 for p, q in ms.cc_channel(c)["kets"]) for c in range(ms.nch))
+        digits = 5 if longest > 339 else 6
+    return digits * (digits + 1) // 2
+
+
+def roofline(phases, work, ms):
     """Roofline entry of the dominant profiled phase."""
+    emax = ms.emax
     hbm_peak, bf16_peak, peak_src = measured_peaks()
     best = None
     for name, (tot, cnt) in phases.items():
@@ -473,9 +492,7 @@ def roofline(phases, work, emax):
     avg_s = phases[best][0] / phases[best][1] / 1000.0
     if bound == "tensor":
         ach = amount / avg_s / 1e12
-        # digit products per multiply-add: five digits' 15 where the longest reduction passes 339
-        # (the ladder from emax 8), six digits' 21 elsewhere
-        issued = 15 if emax >= 8 and "ladder" in best else 21
+        issued = issued_products(ms, best.rsplit("_", 1)[1])
         roof = {"kernel": best, "bound": "tensor", "achieved": ach, "peak": bf16_peak, "unit": "TFLOP/s",
                 "frac": ach / bf16_peak, "traffic": None,
                 "issued_bf16_tflops": issued * ach, "issued_frac": issued * ach / bf16_peak,
@@ -572,7 +589,7 @@ def run_gb300(args):
     phases = profiled_phases(L, step, nprof)
     ms.check_status()
     work = algorithmic_work(ms)
-    roof = roofline(phases, work, args.emax)
+    roof = roofline(phases, work, ms)
     Zs = dZ.download()  # the split result of the timed region's inputs
     # ---- plain FP64 form (the metric compares split vs FP64)
     fp64 = None

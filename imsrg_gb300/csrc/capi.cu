@@ -552,24 +552,22 @@ int ensure_invd(imsrg_space* sp)
   if (sp->invd_ready) return IMSRG_OK;
   drop_invd(sp);
   try {
-    InvdPlan plan;
+    InvdPack plan;
     build_invd(*sp->s, plan, sp->invd_stage, sp->invd_res, sp->invd_weights != 0);
-    auto up = [&](const auto& v) {
-      auto* p = dcopy(v);
-      sp->invd_allocs.push_back((void*)p);
-      return p;
-    };
-    sp->invd.blocks = up(plan.blocks);
-    sp->invd.wblk = up(plan.wblk);
-    sp->invd.wrow = up(plan.wrow);
-    sp->invd.sslot = up(plan.sslot);
-    sp->invd.sidx = up(plan.sidx);
-    sp->invd.dA = up(plan.dA);
-    sp->invd.dB = up(plan.dB);
-    sp->invd.nblocks = (int)plan.blocks.size();
+    char* base = dmalloc<char>(plan.bytes);
+    sp->invd_allocs.push_back(base);
+    if (cudaMemcpy(base, plan.data.get(), plan.bytes, cudaMemcpyHostToDevice) != cudaSuccess) throw std::runtime_error("cudaMemcpy");
+    sp->invd.blocks = (const int4*)(base + plan.at[InvdPack::BLOCKS]);
+    sp->invd.wblk = (const int2*)(base + plan.at[InvdPack::WBLK]);
+    sp->invd.wrow = (const int2*)(base + plan.at[InvdPack::WROW]);
+    sp->invd.sslot = (const unsigned short*)(base + plan.at[InvdPack::SSLOT]);
+    sp->invd.sidx = (const int*)(base + plan.at[InvdPack::SIDX]);
+    sp->invd.dA = (const int4*)(base + plan.at[InvdPack::DA]);
+    sp->invd.dB = (const int2*)(base + plan.at[InvdPack::DB]);
+    sp->invd.nblocks = (int)plan.count[InvdPack::BLOCKS];
     long long upper = 0;  // upper-triangle elements (diagonal included) of every two-body block
     for (const Chan& C : sp->s->ch) upper += (long long)C.n() * (C.n() + 1) / 2;
-    sp->invd.covers_all = (long long)plan.dA.size() == upper;
+    sp->invd.covers_all = (long long)plan.count[InvdPack::DA] == upper;
     sp->invd.stage_max = plan.stage_max;
     sp->invd.staged_weights = sp->invd_weights != 0;
   } catch (std::exception& e) {
@@ -587,8 +585,12 @@ int ensure_invd(imsrg_space* sp)
 // commutators, quadruple blocks or tiles against descriptors: split 123 / 109
 // us at emax 3, 457 / 360 at 7, 1902 / 1512 at 9, 8368 / 6995 at 11; FP64 214 /
 // 180 at 5, 730 / 637 at 7 (Ca40), 3277 / 2831 at 9, 17.3 / 15.0 ms at 11.
-// Built once a space (20 ms at emax 7, 0.15 s at 9, 0.66 s at 11); beyond emax
-// 11, where that takes seconds and gigabytes on the host, only when asked for.
+// They are built once a space, by its first such call: 9 ms at emax 7, 53 at 9,
+// 0.23 s at 11, what about 90 / 130 / 170 split commutators there save (with a
+// step of a flow some ten), so a program of a few commutators in a space pays
+// for more than it gets; "inverse.split" or "inverse.fp64" = 0 is for it.
+// Beyond emax 11, where that takes seconds and gigabytes on the host, only when
+// asked for.
 // They are not built under capture, nor twice where they did not fit.
 int inv_variant(imsrg_space* sp, int prec, cudaStream_t st);
 

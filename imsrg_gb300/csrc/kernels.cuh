@@ -1,6 +1,8 @@
 // Kernel launchers of the GB300 IMSRG(2) commutator (host-callable).
 #pragma once
 
+#include <memory>
+
 #include <cuda_runtime.h>
 
 #include "space.hpp"
@@ -89,6 +91,13 @@ struct InvdPlan {
   std::vector<int2> dB;      // per result: staged offsets, counts and combination bits
   int stage_max = 0;         // most staged values + weights in one block (shared-memory words)
 };
+// the same arrays in one buffer, each from a multiple of 256 bytes
+struct InvdPack {
+  enum { BLOCKS, WBLK, WROW, SIDX, SSLOT, DA, DB, ARRAYS };
+  std::unique_ptr<char[]> data;  // (not cleared: its pages are first touched in parallel)
+  size_t bytes = 0, at[ARRAYS] = {}, count[ARRAYS] = {};
+  int stage_max = 0;
+};
 struct InvdDev {
   const int4* blocks = nullptr;
   const int2* wblk = nullptr;
@@ -104,7 +113,7 @@ struct InvdDev {
 };
 // blocks of at most stage_max staged values (and, staging weights, as many
 // weights) and res_max results
-void build_invd(const Space& s, InvdPlan& out, int stage_max, int res_max, bool stage_weights);
+void build_invd(const Space& s, InvdPack& out, int stage_max, int res_max, bool stage_weights);
 // (grouped)
 // W2 / w2mode: comm122ss's W2 folded into the same update (Z -= W2 + hZ W2^T;
 // 1: (hi, lo) float pairs, 2: FP64), only when d.covers_all

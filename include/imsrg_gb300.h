@@ -46,9 +46,11 @@ extern "C" {
 
 /* precision of the dense contractions (ladder and Pandya channel GEMMs) */
 #define IMSRG_PREC_FP64 0  /* FP64: 62-bit fixed point in nine BF16 digits on the tensor cores (tcgen05), each
-                              element checked against the classical bound of an FP64 sum and formed with
-                              FP64 FMAs where the digits cannot vouch for it; CUDA-core DFMA where the
-                              digit planes do not fit, or under capture before they exist */
+                              element's sum |a||b| checked against an estimate of the digits' error and formed
+                              with FP64 FMAs where that is above an FP64 sum's (the time depends on the
+                              operands: at emax 8 1.2 ms for random ones, 1.5 with a generator, 9.3 where
+                              both fall off steeply from the diagonal); CUDA-core DFMA where the digit
+                              planes do not fit, or under capture before they exist */
 #define IMSRG_PREC_SPLIT 1 /* Ozaki-style sliced BF16 tensor-core products (tcgen05), FP64 recombination */
 
 /* generator functions (src/Generator.cc:12-15) and energy-denominator
@@ -295,8 +297,9 @@ int imsrg_space_zbar_layout(const imsrg_space* s, int ch_cc, int* rows, int* col
 /* Commutator::AddInversePandyaTransformation (src/Commutator.cc:1501-1616):
  * Z += the inverse Pandya transform of zbar, a device buffer of the
  * imsrg_space_zbar_layout layout; Z's hermiticity selects the symmetrisation.
- * precision selects the kernel that comm222_phss uses in that form
- * (imsrg_space_set_tuning "inverse.split" / "inverse.fp64").  zbar must have
+ * precision selects the form; the kernel is the one that "inverse.split" /
+ * "inverse.fp64" hold (imsrg_space_set_tuning; never set: quadruple blocks or
+ * channel tiles, where comm222_phss takes the descriptors).  zbar must have
  * the symmetry of comm222_phss's Z bar, which every kernel relies on: head
  * Zbar(r, c) = hZ Zbar(c, r), tail Zbar(r, n + c) = phi_r phi_c Zbar(c, n + r)
  * with phi of a ket (p, q) = (-1)^((j_p + j_q) / 2); the descriptor kernels
@@ -360,7 +363,10 @@ int imsrg_batch_info(const imsrg_batch* batch, int* n_pairs, int* n_branches, in
  *                                       1 descriptors with double-float sums,
  *                                       2 descriptors with FP64 sums
  *                                       (never set: commutators of up to 2^27
- *                                       arena words take 1, where it fits)
+ *                                       arena words take 1, where it fits; the
+ *                                       space's first one then builds the
+ *                                       descriptors, 10 ms at emax 7, 0.25 s at
+ *                                       11, earned back by some hundred calls)
  *   "inverse.fp64"                      FP64 form: 0 channel tiles, 1
  *                                       descriptors (FP64 sums) (never set:
  *                                       commutators take 1, likewise)

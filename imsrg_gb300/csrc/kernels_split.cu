@@ -107,6 +107,7 @@ struct SplitPlan {
   size_t smem = 0;
   int nstages = 0;
   int accum_override = -1;
+  bool any_accumulate = false;  // of the jobs' own flags
   unsigned wait = WAIT_LIMIT;  // bound of the kernel's barrier waits
   int mirror = 1;  // 0: symmetrised jobs write only their upper triangle
   int tn = 64, nacc = 1, epiw = 4;  // tile columns, tuning label of the tile (64 x 1 or 32 x 2), epilogue warps
@@ -1074,6 +1075,7 @@ SplitPlan* split_plan_create(const Space& s, const std::vector<GemmJobDev>& jobs
     sj.exp_base = erow;
     erow += sj.m_pad;
     kstride = std::max(kstride, sj.K_pad);
+    p->any_accumulate = p->any_accumulate || sj.accumulate;
     p->jobs.push_back(sj);
   }
   for (int jix : order) {
@@ -1313,8 +1315,15 @@ static cudaError_t launch_s(SplitPlan* p, const double* A, const double* B0, con
                 : p->beta == 7 ? (p->tn == 64 ? k_split_gemm<S, 64, 8, false, 7> : k_split_gemm<S, 32, 8, false, 7>)
                                : (p->tn == 64 ? k_split_gemm<S, 64, 8, false, 0> : k_split_gemm<S, 32, 8, false, 0>);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
-    // the whole shared memory, so that the second stream's kernels find some beside the product's CTA
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    // a product that overwrites (one of a whole commutator's): the whole shared
+    // memory, so that the other streams' kernels find some beside its CTA.  One
+    // that accumulates reads its output through L1 and wants what there is of
+    // that: comm222_pp_hhss at emax 6 / 8 / 10 40 / 230 / 1220 us with the first
+    // choice, 33 / 172 / 1033 so
+    const bool accumulates = p->accum_override > 0 || (p->accum_override < 0 && p->any_accumulate);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               accumulates ? cudaSharedmemCarveoutDefault : cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     kern<<<p->grid, 64 + 32 * 8, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], p->maps[4], p->maps[5], ga);
     count_launch();

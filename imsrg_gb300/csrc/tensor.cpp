@@ -92,16 +92,34 @@ struct Quad {
 // quadruples), within the shared memory of the gathered values.  values: (A, B)
 // with A in |x - w| .. x + w (second: and |y - w| .. y + w), 2 lam + 1 B each;
 // per_j slots for every J of |x - y| .. x + y
-static void sort_quadruples(const Space& s, const std::vector<Quad>& all, int lam, int per_j, bool second,
+static void sort_quadruples(const Space& s, const std::vector<std::vector<Quad>>& part, int lam, int per_j, bool second,
                             std::vector<int2>& quads, std::vector<int2>& batches, int& smem)
 {
-  const int nkey = s.d1 * s.d1 * s.d1 * s.d1;
+  // a counting sort, in the parts' order within a class: runs of parts counted
+  // and placed in parallel (one after the other, this and the list for the
+  // tensor Pandya transform took an operator's creation at emax 8 from 84 to 97 ms)
+  const int nkey = s.d1 * s.d1 * s.d1 * s.d1, runs = std::min<int>(64, (int)part.size());
+  auto begin = [&](int r) { return part.size() * r / runs; };
+  std::vector<std::vector<long long>> at(runs, std::vector<long long>(nkey, 0));
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int r = 0; r < runs; ++r)
+    for (size_t p = begin(r); p < begin(r + 1); ++p)
+      for (const Quad& q : part[p]) ++at[r][q.key];
   std::vector<long long> cnt(nkey + 1, 0);
-  for (const Quad& q : all) ++cnt[q.key + 1];
-  for (int x = 0; x < nkey; ++x) cnt[x + 1] += cnt[x];
-  quads.assign(all.size(), make_int2(0, 0));
-  std::vector<long long> at(cnt.begin(), cnt.end() - 1);
-  for (const Quad& q : all) quads[(size_t)at[q.key]++] = q.v;
+  for (int x = 0; x < nkey; ++x) {
+    long long n = cnt[x];
+    for (int r = 0; r < runs; ++r) {
+      const long long c = at[r][x];
+      at[r][x] = n;
+      n += c;
+    }
+    cnt[x + 1] = n;
+  }
+  quads.assign((size_t)cnt[nkey], make_int2(0, 0));
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int r = 0; r < runs; ++r)
+    for (size_t p = begin(r); p < begin(r + 1); ++p)
+      for (const Quad& q : part[p]) quads[(size_t)at[r][q.key]++] = q.v;
   batches.clear();
   smem = 0;
   for (int x = 0; x < nkey; ++x) {
@@ -163,10 +181,8 @@ static void build_quadruples(const Space& s, TensorLayout& t)
       part[kb].push_back({key, make_int2(i | (j << 16), k | (l << 16))});
     }
   }
-  std::vector<Quad> all;
-  for (auto& v : part) all.insert(all.end(), v.begin(), v.end());
   // two sums: (J3, J4) values of (i, l) and of (j, l); slots J2 >= J1
-  sort_quadruples(s, all, lam, lam + 1, true, t.tq, t.tqb, t.tqb_smem);
+  sort_quadruples(s, part, lam, lam + 1, true, t.tq, t.tqb, t.tqb_smem);
 }
 
 // The orbit quadruples of the tensor Pandya transform (k_tpandya_b)
@@ -186,9 +202,7 @@ static void build_pandya_quadruples(const Space& s, TensorLayout& t)
           part[a].push_back({key, make_int2(a | (b << 16), c | (d << 16))});
         }
     }
-  std::vector<Quad> all;
-  for (auto& v : part) all.insert(all.end(), v.begin(), v.end());
-  sort_quadruples(s, all, t.lam, 2 * t.lam + 1, false, t.tp, t.tpb, t.tpb_smem);
+  sort_quadruples(s, part, t.lam, 2 * t.lam + 1, false, t.tp, t.tpb, t.tpb_smem);
   t.ph_loc.assign((size_t)s.NJ * s.nkets, 0);
   for (int c = 0; c < s.nch; ++c)
     for (int k = 0; k < s.cc_nph[c]; ++k) {

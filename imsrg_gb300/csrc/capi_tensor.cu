@@ -162,9 +162,8 @@ int product_scratch(imsrg_space* sp, TensorLayout* tl)
   int rc = scratch(sp, tl);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(sp->mu);
-  if ((rc = alloc(sp, tl, tl->d_ybt, tl->yb_total)) || (rc = alloc(sp, tl, tl->d_ybtf, tl->yb_total)) ||
-      (rc = alloc(sp, tl, tl->d_xbf, sp->s->xb_total)))
-    return rc;
+  if ((rc = alloc(sp, tl, tl->d_ybt, 2 * tl->yb_total)) || (rc = alloc(sp, tl, tl->d_xbf, sp->s->xb_total))) return rc;
+  tl->d_ybtf = tl->d_ybt + tl->yb_total;  // one clear for both
   return IMSRG_OK;
 }
 
@@ -186,6 +185,19 @@ int split_ready(imsrg_space* sp, TensorLayout* tl)
     }
   }
 }
+
+// The multiply-adds from which the FP64 form runs its products on the tensor
+// cores: of the ladder for its term, of Z bar for comm222_phst and for a whole
+// commutator.  Below, the chain of clearing, transposing, slicing and product
+// launches (35 to 45 us more) takes longer than the FP64-pipe kernels do for
+// all.  Products against those, us: comm222_pp_hh_221st, rank (0, 1, +) at emax
+// 3, 4, 5, 6, 79 / 43, 96 / 61, 139 / 131, 203 / 374 (2.4e5, 3.3e6, 2.8e7, 1.8e8
+// multiply-adds), rank (1, 1, +) at emax 5, 230 / 241 (8e7); comm222_phst 107 /
+// 64, 120 / 108, 156 / 258, 263 / 734 (1.2e6, 7.8e6, 3.9e7, 1.5e8), rank (1, 1, +)
+// at emax 4, 155 / 198 (2.1e7).  A whole commutator hides part of the chain
+// behind its other terms: rank (0, 1, +) at emax 2 and 3 173 / 147 and 191 / 200,
+// (1, 1, +) at 2 197 / 197 (Z bar 9.4e4, 1.2e6, 2.3e5).
+constexpr double kLadderTerm = 5e7, kZbarTerm = 1e7, kWholeZbar = 2.5e5;
 
 // the FP64 form's product plans, made on first use outside a capture; false
 // where they cannot be (the FP64-pipe kernels run then).  Rank (1, 1, +) at
@@ -385,7 +397,7 @@ int imsrg_comm222_pp_hh_221st(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z,
   if (rc || (rc = check_prec(precision))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const bool split = precision == IMSRG_PREC_SPLIT;
-  if (!split && !fp64_ready(X->sp, Y->tl, st)) return t222(X, Y, Z, st);
+  if (!split && (Y->tl->ladder_work < kLadderTerm || !fp64_ready(X->sp, Y->tl, st))) return t222(X, Y, Z, st);
   if ((split && (rc = split_ready(X->sp, Y->tl))) || (rc = y_transposed(Y, st)) || (rc = t222_d(X, Y, precision, st)) ||
       (rc = t222_finish(X, Y, Z, st)))
     return rc;
@@ -398,7 +410,7 @@ int imsrg_comm222_phst(const imsrg_op* X, const imsrg_op* Y, imsrg_op* Z, int pr
   if (rc || (rc = check_prec(precision))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const bool split = precision == IMSRG_PREC_SPLIT;
-  if (!split && !fp64_ready(X->sp, Y->tl, st)) return tph(X, Y, Z, st);
+  if (!split && (Y->tl->zbar_work < kZbarTerm || !fp64_ready(X->sp, Y->tl, st))) return tph(X, Y, Z, st);
   if ((split && (rc = split_ready(X->sp, Y->tl))) || (rc = product_operands(X, Y, st)) ||
       (rc = tph_zbar(X, Y, precision, st)) || (rc = tph_finish(Z, st)))
     return rc;
@@ -420,7 +432,7 @@ int imsrg_commutator_scalar_tensor(const imsrg_op* X, const imsrg_op* Y, imsrg_o
   ProfScope ps("CommutatorScalarTensor", st);
   T_CUDA(cudaMemsetAsync(Z->d, 0, Z->len * sizeof(double), st));
   const bool split = precision == IMSRG_PREC_SPLIT;
-  const bool products = (on[3] || on[4]) && (split || fp64_ready(X->sp, Y->tl, st));
+  const bool products = (on[3] || on[4]) && (split || (Y->tl->zbar_work >= kWholeZbar && fp64_ready(X->sp, Y->tl, st)));
   if ((on[2] || products) && ((rc = scratch(X->sp, Y->tl)) || (rc = y_transposed(Y, st)))) return rc;
   if (!products) {
     if ((on[0] && (rc = t111(X, Y, Z, st))) || (on[1] && (rc = t121(X, Y, Z, st))) || (on[2] && (rc = t122(X, Y, Z, st))) ||

@@ -1130,11 +1130,8 @@ cudaError_t launch_tensor_split_operands(const Space& s, const TensorLayout& t, 
                                          cudaStream_t st)
 {
   cudaError_t e;
-  if (t.yb_total > 0) {
-    if ((e = cudaMemsetAsync(YbT, 0, t.yb_total * sizeof(double), st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(YbTF, 0, t.yb_total * sizeof(double), st)) != cudaSuccess)
-      return e;
-  }
+  // (YbTF follows YbT)
+  if (t.yb_total > 0 && (e = cudaMemsetAsync(YbT, 0, 2 * t.yb_total * sizeof(double), st)) != cudaSuccess) return e;
   if (!t.tpb.empty()) {
     if (t.tpb_smem > 40 * 1024 && (e = cudaFuncSetAttribute(k_tpandya_b, cudaFuncAttributeMaxDynamicSharedMemorySize, t.tpb_smem)) != cudaSuccess)
       return e;

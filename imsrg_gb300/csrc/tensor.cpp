@@ -407,6 +407,12 @@ TensorLayout* tensor_layout(Space& s, int lam, int trank, int parity)
     t->lad_n[c] = jb.K;
     t->lad_maxelems = std::max(t->lad_maxelems, (long long)jb.m * jb.K);
   }
+  for (size_t b = 0; b < t->bra.size(); ++b)
+    t->ladder_work += (double)s.ch[t->bra[b]].n() * s.ch[t->ket[b]].n() * (t->lad_n[t->bra[b]] + t->lad_n[t->ket[b]]);
+  for (size_t p = 0; p < t->zb_bra.size(); ++p) {
+    const int lo = t->zb_bra[p], hi = t->zb_ket[p];
+    t->zbar_work += 4.0 * s.cc[lo].n() * s.cc[hi].n() * (s.cc_nph[lo] + s.cc_nph[hi]);
+  }
   build_quadruples(s, *t);
   build_pandya_quadruples(s, *t);
   t->hat2.assign((size_t)t->NJ * t->NJ, 0.0);

@@ -130,6 +130,7 @@ struct TensorLayout {
   // once: without them (their planes do not fit) the FP64-pipe kernels run
   DgemmPlan *dg_lad1 = nullptr, *dg_lad2 = nullptr, *dg_zb1 = nullptr, *dg_zb2 = nullptr;
   bool dg_tried = false;
+  double ladder_work = 0, zbar_work = 0;  // multiply-adds of the ladder's, of Z bar's products
   int max_tiles32 = 0;        // largest block in 32 x 32 tiles (transpose grid)
   // orbit quadruples of the inverse tensor Pandya transform: (i | j << 16,
   // k | l << 16) for every bra ket i <= j and ket ket k <= l that own at

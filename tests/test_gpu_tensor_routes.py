@@ -49,3 +49,37 @@ def test_products_vs_fp64_pipe(emax, nucleus, rank, herm, term, inf):
     assert np.array_equal(fine, np.isfinite(prod))
     top = np.max(abs(pipe[fine]), initial=0.0)
     assert np.max(abs(pipe[fine] - prod[fine]), initial=0.0) <= 4e-12 * top
+
+
+@pytest.mark.parametrize("emax,nucleus,rank,herm", [(5, "O16", (2, 0, 0), 1), (5, "O18", (3, 0, 1), -1), (6, "O16", (0, 1, 0), 1)])
+@pytest.mark.parametrize("term", ["comm222_phst", "comm222_pp_hh_221st"])
+@pytest.mark.parametrize("inf", [False, True])
+def test_products_vs_fp64_pipe_above_the_rule(emax, nucleus, rank, herm, term, inf):
+    """At sizes from which a call outside a capture takes the products (5e7
+    multiply-adds of the ladder, 1e7 of Z bar)."""
+    test_products_vs_fp64_pipe(emax, nucleus, rank, herm, term, inf)
+
+
+@pytest.mark.parametrize("emax,nucleus,rank,herm", [(1, "O16", (1, 1, 0), 1), (2, "O16", (0, 1, 0), 1), (2, "O16", (2, 0, 0), -1), (3, "O18", (2, 0, 0), 1)])
+def test_whole_commutator_either_side_of_the_rule(emax, nucleus, rank, herm):
+    """Captured (FP64-pipe kernels throughout) against not captured (products
+    from 2.5e5 multiply-adds of Z bar): same bound."""
+    ref = RefModelSpace(emax, *{"O16": (16, 8), "O18": (18, 8)}[nucleus])
+    ms = ig.ModelSpace(emax, nucleus, nucleus)
+    X, Y = ref.random_operator(5, True), ref.random_tensor(6, *rank)
+    with ig.DeviceOperator(ms, 1) as dX, ig.DeviceOperator(ms, herm, rank) as dY, ig.DeviceOperator(ms, 1, rank) as dZ:
+        dX.upload(X)
+        dY.upload(Y)
+        st = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st, capture_error_mode="relaxed"):
+            ig.Commutator.device_scalar_tensor(dX, dY, dZ, "fp64", st.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        pipe = dZ.download()
+        ig.Commutator.device_scalar_tensor(dX, dY, dZ, "fp64")
+        torch.cuda.synchronize()
+        prod = dZ.download()
+    assert np.max(abs(pipe), initial=0.0) > 0
+    assert np.max(abs(pipe - prod)) <= 4e-12 * np.max(abs(pipe))

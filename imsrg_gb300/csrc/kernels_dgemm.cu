@@ -37,11 +37,11 @@
 //    all CTAs at the end, since one 128 x 32 tile of K = 1000 keeps an SM's FP64
 //    pipe busy for 2 ms.  So the time depends on the operands.  FP64 commutator,
 //    emax 6 / 8 / 10, in ms (on the FP64 pipe alone: 1.25 / 11.1 / 87.2):
-//      random operators, none to a few elements listed    0.24 / 1.21 / 6.5
-//      one a generator, 0.1 to 1% of the FP64 work        0.34 / 1.52 / 7.0
-//      both falling off as e^(-1.0 |de|)                  0.70 / 4.4  / 36
-//      a dominating diagonal                              0.71 / 4.8  / 51
-//      both falling off as 2^(-4 |de|), 70 to 90% of it   1.22 / 9.3  / 80
+//      random operators, none to a few elements listed    0.24 / 1.20 / 6.5
+//      one a generator, 0.1 to 1% of the FP64 work        0.31 / 1.39 / 6.9
+//      both falling off as e^(-1.0 |de|)                  0.64 / 4.0  / 35
+//      a dominating diagonal                              0.65 / 4.5  / 50
+//      both falling off as 2^(-4 |de|), 70 to 90% of it   1.09 / 8.8  / 78
 //    (With the chunk's length as n and whole tiles of 128 x 32 listed, evaluated
 //    by the CTA that found them: generator 0.95 / 4.7 / 20.8, falling off
 //    1.25 / 11.6 / 97 and 1.62 / 14.6 / 112, diagonal 1.54 / 12.8 / 99.)
@@ -89,6 +89,7 @@ constexpr int EPIW = 8;      // epilogue warps: two per TMEM lane quarter, 16 co
 constexpr int COLS_W = TN / 2;
 constexpr int BLK = 8;                // rows and columns of a listed block
 constexpr int TILE_BLKS = (TM / BLK) * (TN / BLK);
+constexpr int SHARE = 1 << 15;        // FP64 FMAs of a tile (8 us of an SM) from which listed blocks are shared out
 constexpr int NB = 512 / TN;         // tensor-memory blocks
 constexpr int OV = 2 * NP - NB;      // blocks that consecutive chunks share (see k_dgemm)
 constexpr unsigned A_SLICE = TM * KB * 2, B_SLICE = TN * KB * 2;
@@ -112,10 +113,12 @@ struct DTile {
   int job, I, J;
 };
 
-// listed elements of a tile's block: bit 8 r + c of mask is row + r, column + c
-struct DBlock {
+// listed elements of a job's block: bit 8 r + c of mask is (i + r, j + c)
+struct __align__(16) DBlock {
   unsigned long long mask;
-  int tile, at;  // at: row | column << 16 of the block within the tile
+  int job;
+  int i, j;
+  int pad[3];
 };
 
 __host__ __device__ __forceinline__ int chunk_begin(int nkb, int nchunk, int c) { return (int)((long long)nkb * c / nchunk); }
@@ -139,6 +142,7 @@ struct DgemmPlan {
   int n_rblk = 0, n_dblk = 0;
   CUtensorMap maps[4];  // A rows of A, of B (128-row boxes); B rows of A, of B (32-row boxes)
   size_t smem = 0;
+  bool share = false;  // listed blocks among all CTAs
   unsigned wait = WAIT_LIMIT;
 };
 
@@ -435,7 +439,7 @@ struct DArgs {
   const int* kidx;
   const double* kw;
   double gbscale;
-  int gsign, accum, nomirror;
+  int gsign, accum, nomirror, share;
   unsigned wait;  // bound of every barrier wait
 };
 
@@ -445,7 +449,7 @@ struct DArgs {
 // epilogue 30k of its 45k cycles a tile of the emax=10 Zbar product
 struct TileInfo {
   double* O;
-  int m, n, K, ldo, nosym, nkb, nchunk, m_pad, row_base, accumulate, I, J;
+  int job, m, n, ldo, nosym, nkb, nchunk, m_pad, row_base, accumulate, I, J;
   int rrow[2][TM], rcol[2][TN];  // raw exponents of the tile's rows and columns, in each half
   float nrow[2][TM], ncol[2][TN];  // their counts of nonzero elements, times 2^-18
   int prow[TM], pcol[TN];        // phases (rows carry the job's sign too)
@@ -540,15 +544,15 @@ __device__ __forceinline__ double value_of(long long hi, long long lo, int X)
 }
 
 // out (+)= v at (i, j) and, for a symmetrised job, its mirror
-__device__ __forceinline__ void put_exact(const DJob& jb, double* O, const int* ph, double sgn, int i, int j, double p1,
-                                          double p2, bool accumulate, int nomirror)
+// (f: the job's sign and the phases of i and j)
+__device__ __forceinline__ void put_exact(const DJob& jb, double* O, double f, int i, int j, double p1, double p2, bool accumulate,
+                                          int nomirror)
 {
   double* d = O + (long long)j * jb.ldo + i;
   if (jb.nosym) {
     *d = accumulate ? *d + p1 : p1;
     return;
   }
-  const double f = sgn * (ph ? (double)(ph[i] * ph[j]) : 1.0);
   const double v = p1 + f * p2, w = p2 + f * p1;
   *d = accumulate ? *d + v : v;
   if (i != j && !nomirror) {
@@ -566,8 +570,9 @@ __device__ __forceinline__ unsigned own_columns(int i, int j0, int m, int n, int
   return b;
 }
 
-// lists the bad columns of a warp's 32 rows x 16 columns, by blocks
-__device__ __forceinline__ void list_blocks(DBlock* list, int* n, int tile, int row, int col, unsigned bad)
+// lists the bad columns of a warp's 32 rows x 16 columns, by blocks; i, j: the
+// first element of the lane's block
+__device__ __forceinline__ void list_blocks(DBlock* list, int* n, int job, int i, int j, unsigned bad)
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -580,7 +585,7 @@ __device__ __forceinline__ void list_blocks(DBlock* list, int* n, int tile, int 
       hi |= __shfl_xor_sync(0xffffffffu, hi, o);
     }
     if ((lane & 7) == 0 && (lo | hi))
-      list[atomicAdd(n, 1)] = {(unsigned long long)hi << 32 | lo, tile, row | (col + BLK * c) << 16};
+      list[atomicAdd(n, 1)] = {(unsigned long long)hi << 32 | lo, job, i, j + BLK * c};
   }
 }
 
@@ -606,17 +611,21 @@ __device__ __forceinline__ int nth_bit(unsigned long long mask, int rank)
   return bit;
 }
 
-__device__ __forceinline__ void put_listed(const DArgs& g, const DJob& jb, int i, int j, double p1, double p2)
+__device__ __forceinline__ int sign_of(const DArgs& g, const DJob& jb, int i, int j)
 {
-  put_exact(jb, g.out + jb.out_off, jb.phase_off >= 0 ? g.phase + jb.phase_off : nullptr, jb.sign != 0 ? jb.sign : g.gsign, i, j,
-            p1, p2, g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
+  return (jb.sign != 0 ? jb.sign : g.gsign) * (jb.phase_off >= 0 ? g.phase[jb.phase_off + i] * g.phase[jb.phase_off + j] : 1);
+}
+
+__device__ __forceinline__ void put_listed(const DArgs& g, const DJob& jb, int sign, int i, int j, double p1, double p2)
+{
+  put_exact(jb, g.out + jb.out_off, (double)sign, i, j, p1, p2, g.accum > 0 || (g.accum < 0 && jb.accumulate), g.nomirror);
 }
 
 // At most FEW elements of a block, by a warp: 32 / n lanes an element take K by
 // turns and meet in a fixed tree; operands straight from L1 and L2, eight
 // columns a lane in flight.
 constexpr int FEW = 16;
-__device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const DBlock& e, int i0, int j0, int n)
+__device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const DBlock& e, int n)
 {
   const int lane = threadIdx.x & 31, nosym = jb.nosym;
   const double *A = g.A + jb.a_off, *B = (jb.bsel ? g.B1 : g.B0) + jb.b_off;
@@ -627,7 +636,8 @@ __device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const 
   int sh = 0;  // 2^sh slots for n elements (a slot too many repeats the last one)
   while ((1 << sh) < n) ++sh;
   const int slot = lane & ((1 << sh) - 1), part = lane >> sh, parts = 32 >> sh;
-  const int bit = nth_bit(e.mask, min(slot, n - 1)), i = i0 + (bit >> 3), j = j0 + (bit & 7);
+  const int bit = nth_bit(e.mask, min(slot, n - 1)), i = e.i + (bit >> 3), j = e.j + (bit & 7);
+  const int sign = sign_of(g, jb, i, j);
   double p1 = 0.0, p2 = 0.0;
   constexpr int U = 8;
   for (int t0 = 0; t0 < jb.K; t0 += 32) {
@@ -669,7 +679,7 @@ __device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const 
     p1 += __shfl_xor_sync(0xffffffffu, p1, o);
     p2 += __shfl_xor_sync(0xffffffffu, p2, o);
   }
-  if (part == 0 && slot < n) put_listed(g, jb, i, j, p1, p2);
+  if (part == 0 && slot < n) put_listed(g, jb, sign, i, j, p1, p2);
 }
 
 // More elements, E a lane.  A column of the operands at the block's eight rows
@@ -685,12 +695,12 @@ constexpr int XWARP = XSTAGES * XK * XLD;  // doubles a warp
 static_assert(EPIW * XWARP * 8 <= NSTAGE * (int)STAGE, "exact_work's buffers exceed the pipeline's");
 
 template <int E>
-__device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const DBlock& e, int i0, int j0, int n, double* buf)
+__device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const DBlock& e, int n, double* buf)
 {
   const int lane = threadIdx.x & 31, nosym = jb.nosym;
-  // what this lane copies: A(i0 + 0..7), B(i0 + ..), A(j0 + ..), B(j0 + ..); rows
+  // what this lane copies: A(i + 0..7), B(i + ..), A(j + ..), B(j + ..); rows
   // past the end repeat the last one (and are not used), a plain job needs no more than the outer two
-  const int strip = lane >> 3, row = min((strip < 2 ? i0 : j0) + (lane & 7), (strip & 1 ? jb.n : jb.m) - 1);
+  const int strip = lane >> 3, row = min((strip < 2 ? e.i : e.j) + (lane & 7), (strip & 1 ? jb.n : jb.m) - 1);
   const double* src = (strip & 1 ? (jb.bsel ? g.B1 : g.B0) + jb.b_off : g.A + jb.a_off) + row;
   const int ld = strip & 1 ? jb.ldb : jb.lda;
   const bool copies = !nosym || strip == 0 || strip == 3;
@@ -757,52 +767,72 @@ __device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const
   }
 #pragma unroll
   for (int h = 0; h < E; ++h)
-    if (lane + 32 * h < n) put_listed(g, jb, i0 + er[h], j0 + ec[h], p1[h], p2[h]);
+    if (lane + 32 * h < n) put_listed(g, jb, sign_of(g, jb, e.i + er[h], e.j + ec[h]), e.i + er[h], e.j + ec[h], p1[h], p2[h]);
+}
+
+// the k-th block of a list that another CTA may have written
+__device__ __forceinline__ void exact_block(const DArgs& g, const DBlock* at, double* buf)
+{
+  DBlock e;
+  e.mask = __ldcg(&at->mask);
+  e.job = __ldcg(&at->job);
+  e.i = __ldcg(&at->i);
+  e.j = __ldcg(&at->j);
+  const DJob jb = g.jobs[e.job];
+  const int n = __popcll(e.mask);
+  if (n <= FEW)
+    exact_few(g, jb, e, n);
+  else if (n <= 32)
+    exact_many<1>(g, jb, e, n, buf);
+  else
+    exact_many<2>(g, jb, e, n, buf);
 }
 
 // The listed blocks, a warp at a time: this CTA's own n (all complete), then
 // those that other CTAs have published by now.  Nothing waits: every CTA ends
-// with its own list taken, by itself or by others.
+// with its own list taken, by itself or by others.  Plans whose whole tiles
+// take a few microseconds share nothing: looking at the other lists and drawing
+// tickets would be as long (replay of nine FP64 pairs at emax 2 138.7 us
+// against 128).
 __device__ __noinline__ void exact_work(const DArgs& g, int n, double* buf)
 {
   const int lane = threadIdx.x & 31, grid = gridDim.x;
+  {
+    // the first blocks by warp, then tickets, each drawn while the block before
+    // is worked on (n is final, so counting past it harms nobody)
+    const DBlock* list = g.list + (long long)g.cta_first[blockIdx.x] * TILE_BLKS;
+    for (int k = (threadIdx.x >> 5) - 2; k < n;) {
+      int next = k + EPIW;
+      if (g.share && lane == 0) next = EPIW + atomicAdd(g.taken + blockIdx.x, 1);
+      exact_block(g, list + k, buf);
+      k = __shfl_sync(0xffffffffu, next, 0);
+    }
+  }
+  if (!g.share) return;
   auto cta = [&](int d) { return (int)blockIdx.x + d < grid ? blockIdx.x + d : blockIdx.x + d - grid; };
-  auto listed = [&](int d) { return d == 0 ? n : d < grid ? *(volatile int*)(g.published + cta(d)) : 0; };
+  auto listed = [&](int d) { return d > 0 && d < grid ? *(volatile int*)(g.published + cta(d)) : 0; };
   int any = 0;
-  for (int d = lane; d < grid; d += 32) any |= listed(d);
+  for (int d = lane; d < grid; d += 32) any |= listed(d) > EPIW;
   if (!__any_sync(0xffffffffu, any)) return;
   for (int d0 = 0; d0 < grid; d0 += 32) {
     const int have = listed(d0 + lane);
     __threadfence();  // the entries after their count
-    for (unsigned m = __ballot_sync(0xffffffffu, have > 0); m; m &= m - 1) {
+    for (unsigned m = __ballot_sync(0xffffffffu, have > EPIW); m; m &= m - 1) {
       const int c = cta(d0 + __ffs(m) - 1), cn = __shfl_sync(0xffffffffu, have, __ffs(m) - 1);
       const DBlock* list = g.list + (long long)g.cta_first[c] * TILE_BLKS;
       for (;;) {
         int k = 0;
         if (lane == 0) {
           k = *(volatile int*)(g.taken + c);
-          while (k < cn) {
+          while (EPIW + k < cn) {
             const int old = atomicCAS(g.taken + c, k, k + 1);
             if (old == k) break;
             k = old;
           }
         }
-        k = __shfl_sync(0xffffffffu, k, 0);
+        k = EPIW + __shfl_sync(0xffffffffu, k, 0);
         if (k >= cn) break;
-        DBlock e;
-        e.mask = __ldcg(&list[k].mask);
-        e.tile = __ldcg(&list[k].tile);
-        e.at = __ldcg(&list[k].at);
-        const DTile tl = g.tiles[e.tile];
-        const DJob jb = g.jobs[tl.job];
-        const int total = __popcll(e.mask);
-        const int i0 = tl.I * TM + (e.at & 0xFFFF), j0 = tl.J * TN + (e.at >> 16);
-        if (total <= FEW)
-          exact_few(g, jb, e, i0, j0, total);
-        else if (total <= 32)
-          exact_many<1>(g, jb, e, i0, j0, total, buf);
-        else
-          exact_many<2>(g, jb, e, i0, j0, total, buf);
+        exact_block(g, list + k, buf);
       }
     }
   }
@@ -914,7 +944,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
         f.O = g.out + jb.out_off;
         f.m = jb.m;
         f.n = jb.n;
-        f.K = jb.K;
+        f.job = tl.job;
         f.ldo = jb.ldo;
         f.nosym = jb.nosym;
         f.nkb = jb.nkb;
@@ -1089,7 +1119,7 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
       unsigned wd = own_columns(i, j0, m, n, nosym);
       bad &= wd;
       wd &= ~bad;
-      if (__any_sync(0xffffffffu, bad)) list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, tbeg + t, row & ~7, cbeg, bad);
+      if (__any_sync(0xffffffffu, bad)) list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, f.job, i & ~7, j0, bad);
       if (!nosym && live) {
         const int sp = f.prow[row];
 #pragma unroll
@@ -1132,7 +1162,8 @@ __global__ void __launch_bounds__(96 + 32 * EPIW, 1) k_dgemm(const __grid_consta
     for (; t < ntile; ++t) {
       const DTile tl = g.tiles[tbeg + t];
       const DJob& jb = g.jobs[tl.job];
-      list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, tbeg + t, row & ~7, cbeg, own_columns(tl.I * TM + row, tl.J * TN + cbeg, jb.m, jb.n, jb.nosym));
+      const int i = tl.I * TM + row, j0 = tl.J * TN + cbeg;
+      list_blocks(g.list + (long long)tbeg * TILE_BLKS, &s_nlist, tl.job, i & ~7, j0, own_columns(i, j0, jb.m, jb.n, jb.nosym));
     }
   }
   // every role has left its loop, and so has every copy and MMA, unless a wait
@@ -1219,6 +1250,7 @@ DgemmPlan* dgemm_plan_create(const std::vector<GemmJobDev>& jobs_in, int family)
     const int jix = (int)jobs.size();
     jobs.push_back(d);
     if (d.m == 0 || d.n == 0 || d.K == 0) continue;
+    p->share = p->share || (long long)std::min(d.m, TM) * std::min(d.n, TN) * d.K * (d.nosym ? 1 : 2) > SHARE;
     // a tile costs its K blocks and, per chunk, about three of them in the epilogue, plus its stores
     const long long c = (d.nosym ? 1 : 2) * (d.nkb + 3 * d.nchunk) + 4;
     for (int I = 0; I * TM < d.m; ++I)
@@ -1367,7 +1399,7 @@ cudaError_t launch_dgemm(const DgemmPlan* p, const double* A, const double* B0, 
   }
   ProfScope ps(p->family == 0 ? "dgemm_ladder" : "dgemm_zbar", st);
   DArgs a{p->d_jobs, p->d_tiles, p->d_cta, rexpA, rexpB, cntA, cntB, phase, O, p->d_list, nlist, nlist + p->grid,
-          A, B0, B1, kidx, kw, gbscale, gsign, accum, mirror ? 0 : 1, p->wait};
+          A, B0, B1, kidx, kw, gbscale, gsign, accum, mirror ? 0 : 1, p->share ? 1 : 0, p->wait};
   k_dgemm<<<p->grid, 96 + 32 * EPIW, p->smem, st>>>(p->maps[0], p->maps[1], p->maps[2], p->maps[3], a);
   count_launch();
   return cudaGetLastError();

@@ -52,9 +52,10 @@
 // short ones (Zbar, K <= 132) the epilogue.  With the FP64-pipe kernel the
 // commutator takes 142 us at emax 2, 1.26 ms at emax 6, 87.2 ms at emax 10;
 // with this one, and nothing else changed, it took 116 us, 0.38 ms and 7.7 ms
-// (48 us, 0.24 ms and 6.5 ms by now): it is used at every size, and
-// the FP64-pipe kernel only where the planes do not fit (40 bytes an element
-// pair of the operands) or inside a capture that comes before them.
+// (47 us, 0.24 ms and 6.5 ms by now): scalar products use it at every size,
+// tensor ones from the sizes that capi_tensor.cu gives, and the FP64-pipe
+// kernels run below those, where the planes do not fit (40 bytes an element
+// pair of the operands) and inside a capture that comes before them.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -50,7 +50,8 @@ extern "C" {
                               with FP64 FMAs where that is above an FP64 sum's (the time depends on the
                               operands: at emax 8 1.2 ms for random ones, 1.4 with a generator, 8.8 where
                               both fall off steeply from the diagonal); CUDA-core DFMA where the digit
-                              planes do not fit, or under capture before they exist */
+                              planes do not fit, under capture before they exist, and for the products of
+                              small tensors */
 #define IMSRG_PREC_SPLIT 1 /* Ozaki-style sliced BF16 tensor-core products (tcgen05), FP64 recombination */
 
 /* generator functions (src/Generator.cc:12-15) and energy-denominator

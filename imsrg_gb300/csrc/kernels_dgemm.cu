@@ -39,12 +39,16 @@
 //    emax 6 / 8 / 10, in ms (on the FP64 pipe alone: 1.25 / 11.1 / 87.2):
 //      random operators, none to a few elements listed    0.24 / 1.20 / 6.5
 //      one a generator, 0.1 to 1% of the FP64 work        0.31 / 1.39 / 6.9
-//      both falling off as e^(-1.0 |de|)                  0.64 / 4.0  / 35
-//      a dominating diagonal                              0.65 / 4.5  / 50
-//      both falling off as 2^(-4 |de|), 70 to 90% of it   1.09 / 8.8  / 78
+//      both falling off as e^(-1.0 |de|)                  0.54 / 3.4  / 30
+//      a dominating diagonal                              0.61 / 4.1  / 39
+//      both falling off as 2^(-4 |de|), 70 to 90% of it   0.96 / 7.2  / 61
 //    (With the chunk's length as n and whole tiles of 128 x 32 listed, evaluated
 //    by the CTA that found them: generator 0.95 / 4.7 / 20.8, falling off
-//    1.25 / 11.6 / 97 and 1.62 / 14.6 / 112, diagonal 1.54 / 12.8 / 99.)
+//    1.25 / 11.6 / 97 and 1.62 / 14.6 / 112, diagonal 1.54 / 12.8 / 99.)  Tensor
+//    commutators likewise: rank (2, 0, +), emax 6 / 8, 1.70 / 9.9 ms random, 4.7 /
+//    43 falling off as 2^(-4 |de|), 4.9 / 51 on the FP64 pipe; smaller ones of such
+//    operands are slower than there (emax 4 0.81 against 0.57), since an 8 x 8
+//    block of a small matrix is half padding.
 //
 // What bounds it: for the long products the MMAs, 46 of 128 x 32 x 16 a K16
 // step (merged to 11 instructions), next to the TMA stream of the ten planes
@@ -623,8 +627,9 @@ __device__ __forceinline__ void put_listed(const DArgs& g, const DJob& jb, int s
 }
 
 // At most FEW elements of a block, by a warp: 32 / n lanes an element take K by
-// turns and meet in a fixed tree; operands straight from L1 and L2, eight
-// columns a lane in flight.
+// turns and meet in a fixed tree; operands straight from L1 and L2, two columns
+// a lane in flight (eight: 4.47 against 4.08 ms at emax 8 with a dominating
+// diagonal, and the code of a launch's first block is read cold).
 constexpr int FEW = 16;
 __device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const DBlock& e, int n)
 {
@@ -640,7 +645,7 @@ __device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const 
   const int bit = nth_bit(e.mask, min(slot, n - 1)), i = e.i + (bit >> 3), j = e.j + (bit & 7);
   const int sign = sign_of(g, jb, i, j);
   double p1 = 0.0, p2 = 0.0;
-  constexpr int U = 8;
+  constexpr int U = 2;
   for (int t0 = 0; t0 < jb.K; t0 += 32) {
     const int t = min(t0 + lane, jb.K - 1), nt = min(32, jb.K - t0);
     const int col = kidx ? kidx[t] : t;
@@ -683,28 +688,35 @@ __device__ __forceinline__ void exact_few(const DArgs& g, const DJob& jb, const 
   if (part == 0 && slot < n) put_listed(g, jb, sign, i, j, p1, p2);
 }
 
-// More elements, E a lane.  A column of the operands at the block's eight rows
-// i and eight rows j is one asynchronous copy of 8 bytes a lane into the warp's
-// part of the pipeline's shared memory, two steps of XK columns ahead; B is
-// scaled there, once.  Bound by the FP64 pipe (81% busy at emax 10, operands
-// falling off as 2^(-4 |de|)), one FMA a warp every 16 cycles of an SM.  (Read
-// straight from L1 and L2 like the few: 92 against 90 ms there, 7.1 against 6.6
-// at emax 8 as e^(-1.5 |de|); the few this way: 1.70 against 1.46 ms with a generator.)
-constexpr int XK = 32, XLD = 32;  // columns a step, and the words of one
+// More elements, E a lane.  Columns of the operands at the block's eight rows i
+// and eight rows j are asynchronous copies of 8 bytes a lane into the warp's
+// part of the pipeline's shared memory (one column a copy, or two of a plain
+// job's), two steps of XK columns ahead; the few columns with a weight that is
+// not 1 are scaled there, a common sign is applied at the end.  Bound by the
+// FP64 pipe, one FMA a warp every 16 cycles of an SM.  (With every column scaled
+// and one column of a plain job a copy: 78 against 61 ms for the emax 10
+// commutator of operands falling off as 2^(-4 |de|), 80 against 44 for the tensor
+// one at emax 8; the few this way: 1.70 against 1.46 ms at emax 8 with a
+// generator.)
+constexpr int XK = 32;  // columns a step
 constexpr int XSTAGES = 3;
-constexpr int XWARP = XSTAGES * XK * XLD;  // doubles a warp
+constexpr int XWARP = XSTAGES * XK * 32;  // doubles a warp
 static_assert(EPIW * XWARP * 8 <= NSTAGE * (int)STAGE, "exact_work's buffers exceed the pipeline's");
 
-template <int E>
+// ALL: all 64 elements (E = 2): a lane's two are in one column
+template <int E, bool NOSYM, bool ALL>
 __device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const DBlock& e, int n, double* buf)
 {
-  const int lane = threadIdx.x & 31, nosym = jb.nosym;
-  // what this lane copies: A(i + 0..7), B(i + ..), A(j + ..), B(j + ..); rows
-  // past the end repeat the last one (and are not used), a plain job needs no more than the outer two
-  const int strip = lane >> 3, row = min((strip < 2 ? e.i : e.j) + (lane & 7), (strip & 1 ? jb.n : jb.m) - 1);
+  constexpr int W = NOSYM ? 16 : 32;          // words of a column: A(i ..), [B(i ..), A(j ..),] B(j ..)
+  constexpr int AT_AJ = 16, AT_BI = 8, AT_BJ = NOSYM ? 8 : 24;
+  constexpr int STEP = XK * 32;               // doubles from one step's buffer to the next
+  const int lane = threadIdx.x & 31;
+  // what this lane copies (rows past the end repeat the last one, and are not
+  // used): column k + half of row, k + half even in a plain job's first half
+  const int strip = NOSYM ? ((lane >> 3) & 1) * 3 : lane >> 3, half = NOSYM ? lane >> 4 : 0;
+  const int row = min((strip < 2 ? e.i : e.j) + (lane & 7), (strip & 1 ? jb.n : jb.m) - 1);
   const double* src = (strip & 1 ? (jb.bsel ? g.B1 : g.B0) + jb.b_off : g.A + jb.a_off) + row;
   const int ld = strip & 1 ? jb.ldb : jb.lda;
-  const bool copies = !nosym || strip == 0 || strip == 3;
   const unsigned dst = smem_u32(buf) + lane * 8;
   const int* kidx = jb.kidx_off >= 0 ? g.kidx + jb.kidx_off : nullptr;
   const double* kw = jb.w_off >= 0 ? g.kw + jb.w_off : nullptr;
@@ -714,23 +726,21 @@ __device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const
   double p1[E], p2[E];
 #pragma unroll
   for (int h = 0; h < E; ++h) {
-    const int bit = nth_bit(e.mask, min(lane + 32 * h, n - 1));
+    const int bit = ALL ? lane + 32 * h : nth_bit(e.mask, min(lane + 32 * h, n - 1));
     er[h] = bit >> 3;
-    ec[h] = bit & 7;
+    ec[h] = ALL ? lane & 7 : bit & 7;
     p1[h] = p2[h] = 0.0;
   }
   const int steps = (jb.K + XK - 1) / XK;
-  auto column = [&](int step) { return kidx ? kidx[min(step * XK + lane, jb.K - 1)] : step * XK + lane; };
+  auto column = [&](int step) { return kidx ? kidx[min(step * XK + lane, jb.K - 1)] : min(step * XK + lane, jb.K - 1); };
   int col = column(0);
-  auto copy = [&](int step) {  // always one group, an empty one past the end
+  auto copy = [&](int step) {  // always one group, an empty one past the end (columns past it repeat the last)
     if (step < steps) {
-      const unsigned d = dst + (step % XSTAGES) * (XK * XLD * 8);
-      const int nk = min(XK, jb.K - step * XK);
-      for (int k = 0; k < nk; ++k) {
-        const double* a = src + (long long)__shfl_sync(0xffffffffu, col, k) * ld;
-        if (copies)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + k * (XLD * 8)), "l"(__cvta_generic_to_global(a))
-                       : "memory");
+      const unsigned d = dst + (step % XSTAGES) * (STEP * 8);
+#pragma unroll 8
+      for (int k = 0; k < XK; k += 32 / W) {
+        const double* a = src + (long long)__shfl_sync(0xffffffffu, col, k + half) * ld;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + k * (W * 8)), "l"(__cvta_generic_to_global(a)) : "memory");
       }
       col = column(step + 1);
     }
@@ -740,35 +750,49 @@ __device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const
   copy(1);
   for (int step = 0; step < steps; ++step) {
     copy(step + 2);
-    double* x = buf + (step % XSTAGES) * (XK * XLD);
+    double* x = buf + (step % XSTAGES) * STEP;
     const int t0 = step * XK, nk = min(XK, jb.K - t0);
-    const double w = kw ? kw[t0 + min(lane, nk - 1)] : 1.0;
+    const double w = kw && lane < nk ? kw[t0 + lane] : 1.0;
     asm volatile("cp.async.wait_group 2;" ::: "memory");
     __syncwarp();
-    const double sc = scaled(w, kind0, sc0);
-    const int kind = scale_kind(sc);
-    if (__any_sync(0xffffffffu, kind != SC_PLUS)) {
-      for (int k = 0; k < nk; ++k) {
-        const int kd = __shfl_sync(0xffffffffu, kind, k);
+    const double sc = kind0 == SC_OTHER ? sc0 * w : w;
+    const int kind = lane < nk ? scale_kind(sc) : SC_PLUS;
+    const unsigned scales = __ballot_sync(0xffffffffu, kind != SC_PLUS);
+    if (scales) {
+      for (unsigned m = scales; m; m &= m - 1) {
+        const int k = __ffs(m) - 1, kd = __shfl_sync(0xffffffffu, kind, k);
         const double s = __shfl_sync(0xffffffffu, sc, k);
-        if (kd != SC_PLUS && (strip & 1)) x[k * XLD + lane] = scaled(x[k * XLD + lane], kd, s);
+        if (lane < W && (lane >> 3 & 1)) x[k * W + lane] = scaled(x[k * W + lane], kd, s);
       }
       __syncwarp();
     }
 #pragma unroll 4
     for (int k = 0; k < nk; ++k) {
-      const double* q = x + k * XLD;
+      const double* q = x + k * W;
 #pragma unroll
       for (int h = 0; h < E; ++h) {
-        p1[h] = fma(q[er[h]], q[24 + ec[h]], p1[h]);
-        if (!nosym) p2[h] = fma(q[16 + ec[h]], q[8 + er[h]], p2[h]);
+        p1[h] = fma(q[er[h]], q[AT_BJ + (ALL ? ec[0] : ec[h])], p1[h]);
+        if (!NOSYM) p2[h] = fma(q[AT_AJ + (ALL ? ec[0] : ec[h])], q[AT_BI + er[h]], p2[h]);
       }
     }
     __syncwarp();
   }
 #pragma unroll
   for (int h = 0; h < E; ++h)
-    if (lane + 32 * h < n) put_listed(g, jb, sign_of(g, jb, e.i + er[h], e.j + ec[h]), e.i + er[h], e.j + ec[h], p1[h], p2[h]);
+    if (lane + 32 * h < n)
+      put_listed(g, jb, sign_of(g, jb, e.i + er[h], e.j + ec[h]), e.i + er[h], e.j + ec[h], kind0 == SC_MINUS ? -p1[h] : p1[h],
+                 kind0 == SC_MINUS ? -p2[h] : p2[h]);
+}
+
+template <bool NOSYM>
+__device__ __forceinline__ void exact_many(const DArgs& g, const DJob& jb, const DBlock& e, int n, double* buf)
+{
+  if (n <= 32)
+    exact_many<1, NOSYM, false>(g, jb, e, n, buf);
+  else if (n < 64)
+    exact_many<2, NOSYM, false>(g, jb, e, n, buf);
+  else
+    exact_many<2, NOSYM, true>(g, jb, e, n, buf);
 }
 
 // the k-th block of a list that another CTA may have written
@@ -783,10 +807,10 @@ __device__ __forceinline__ void exact_block(const DArgs& g, const DBlock* at, do
   const int n = __popcll(e.mask);
   if (n <= FEW)
     exact_few(g, jb, e, n);
-  else if (n <= 32)
-    exact_many<1>(g, jb, e, n, buf);
+  else if (jb.nosym)
+    exact_many<true>(g, jb, e, n, buf);
   else
-    exact_many<2>(g, jb, e, n, buf);
+    exact_many<false>(g, jb, e, n, buf);
 }
 
 // The listed blocks, a warp at a time: this CTA's own n (all complete), then

@@ -48,7 +48,7 @@ extern "C" {
 #define IMSRG_PREC_FP64 0  /* FP64: 62-bit fixed point in nine BF16 digits on the tensor cores (tcgen05), each
                               element's sum |a||b| checked against an estimate of the digits' error and formed
                               with FP64 FMAs where that is above an FP64 sum's (the time depends on the
-                              operands: at emax 8 1.2 ms for random ones, 1.4 with a generator, 8.8 where
+                              operands: at emax 8 1.2 ms for random ones, 1.4 with a generator, 7.2 where
                               both fall off steeply from the diagonal); CUDA-core DFMA where the digit
                               planes do not fit, under capture before they exist, and for the products of
                               small tensors */
